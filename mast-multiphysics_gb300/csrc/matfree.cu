@@ -1325,7 +1325,8 @@ __global__ void __launch_bounds__(256) mg_prolong_kernel(const MfProblem *__rest
 
 // coarse moduli: E_c = 2 mean(E of the 8 children); the factor 2 is the
 // element-size scaling of the 3D stiffness (K(2h) = 2 K(h)), so every level
-// uses the fine-grid reference stiffness K0
+// uses the fine-grid reference stiffness K0.  The last element of an odd direction
+// reaches one fine element beyond the grid: those children count as void (0).
 __global__ void mg_coarsen_kernel(const MfProblem *__restrict__ probs, int plo,
                                   float *__restrict__ E32) {
     const MfProblem C = probs[plo + blockIdx.y];
@@ -1338,7 +1339,8 @@ __global__ void mg_coarsen_kernel(const MfProblem *__restrict__ probs, int plo,
         for (int dz = 0; dz < 2; dz++)
             for (int dy = 0; dy < 2; dy++)
                 for (int dx = 0; dx < 2; dx++)
-                    s += E32[F.elem_off + ((int64_t)(2 * ez + dz) * F.ny + 2 * ey + dy) * F.pitch_e + 2 * ex + dx];
+                    if (2 * ex + dx < F.nx && 2 * ey + dy < F.ny && 2 * ez + dz < F.nz)
+                        s += E32[F.elem_off + ((int64_t)(2 * ez + dz) * F.ny + 2 * ey + dy) * F.pitch_e + 2 * ex + dx];
         E32[C.elem_off + ((int64_t)ez * C.ny + ey) * C.pitch_e + ex] = 0.25f * s;
     }
 }
@@ -1487,8 +1489,6 @@ __device__ void bottom_residual(const BottomLevel &L, const float *sK) {
 // the level's moduli and K0 like the level operators (Dirichlet dofs: identity
 // rows and zero columns), so the inverse is symmetric and the V-cycle stays a
 // fixed symmetric preconditioner.
-constexpr int kCoarseDirectMax = 144;
-
 struct BottomCheb {
     float inv_theta_s, inv_theta_c;
     float c1s[32], c2s[32], c1c[32], c2c[32];
@@ -3010,9 +3010,9 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         const int start = (int)b.h_probs.size();
         for (int f = lo; f < hi; f++) {
             const MfProblem F = b.h_probs[f];
-            if (F.nx % 2 || F.ny % 2 || F.nz % 2 || F.nx < 4 || F.ny < 4 || F.nz < 4) continue;
+            if (!mg_coarsens(F.nx, F.ny, F.nz)) continue;
             MfProblem C{};
-            C.nx = F.nx / 2; C.ny = F.ny / 2; C.nz = F.nz / 2;
+            C.nx = (F.nx + 1) / 2; C.ny = (F.ny + 1) / 2; C.nz = (F.nz + 1) / 2;
             C.level = lev;
             C.root = F.root;
             C.fine = f;
@@ -3384,7 +3384,8 @@ int mf_batch_set_bc(MfBatch &b, int i, const uint8_t *node_fix_host, const doubl
     cudaStream_t s = b.stream;
     if (node_fix_host) {
         MG_CUDA_TRY(cudaMemcpyAsync(b.node_fix + P.node_off, node_fix_host, nn, cudaMemcpyHostToDevice, s));
-        // coarse levels: a coarse node is constrained where its fine node (2I,2J,2K) is
+        // coarse levels: a coarse node is constrained where its fine node (2I,2J,2K) is; the
+        // last node of an odd direction lies beyond the grid and takes the last fine node's
         std::vector<uint8_t> fine(node_fix_host, node_fix_host + nn), coarse;
         for (int f = i; b.h_probs[f].coarse >= 0; f = b.h_probs[f].coarse) {
             const MfProblem &F = b.h_probs[f], &C = b.h_probs[F.coarse];
@@ -3393,7 +3394,8 @@ int mf_batch_set_bc(MfBatch &b, int i, const uint8_t *node_fix_host, const doubl
                 for (int J = 0; J < C.NY; J++)
                     for (int I = 0; I < C.NX; I++)
                         coarse[I + (size_t)C.NX * (J + (size_t)C.NY * K)] =
-                            fine[2 * I + (size_t)F.NX * (2 * J + (size_t)F.NY * 2 * K)];
+                            fine[std::min(2 * I, F.nx) +
+                                 (size_t)F.NX * (std::min(2 * J, F.ny) + (size_t)F.NY * std::min(2 * K, F.nz))];
             MG_CUDA_TRY(cudaMemcpyAsync(b.node_fix + C.node_off, coarse.data(), coarse.size(),
                                         cudaMemcpyHostToDevice, s));
             MG_CUDA_TRY(cudaStreamSynchronize(s));

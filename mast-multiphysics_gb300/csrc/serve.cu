@@ -90,8 +90,8 @@ int64_t chain_bytes(int nx, int ny, int nz, int cases) {
         dofs += pitch * (y + 1) * (z + 1);
         elems += (int64_t)((x + 3) / 4 * 4) * y * z;
         nodes += (int64_t)(x + 1) * (y + 1) * (z + 1);
-        if (x % 2 || y % 2 || z % 2 || x < 4 || y < 4 || z < 4) break;
-        x /= 2; y /= 2; z /= 2;
+        if (!mg_coarsens(x, y, z)) break;
+        x = (x + 1) / 2; y = (y + 1) / 2; z = (z + 1) / 2;
     }
     // 13 FP32 + 3 FP64 vectors per dof, 3 element tables per design, dc + densities
     return cases * (dofs * (13 * 4 + 3 * 8) + nodes + 8LL * nx * ny * nz) + elems * 20 +
