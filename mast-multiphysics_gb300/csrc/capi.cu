@@ -336,6 +336,8 @@ int create_impl(const mg_mesh_desc *mesh, const mg_material_desc *mat, const mg_
     });
     p->A.n = n;
     p->A.nnz = nnz;
+    p->A.max_row = 0;
+    for (int64_t i = 0; i < n; i++) p->A.max_row = std::max(p->A.max_row, rowptr[i + 1] - rowptr[i]);
     p->A.dpn = dpn;
 
     // ---- Dirichlet elimination tables ----

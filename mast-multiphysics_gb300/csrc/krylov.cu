@@ -28,6 +28,9 @@ constexpr int kBS = 256;
 // lanes per node in the SpMV: few lanes keep the FP64 work near one FMA per
 // stored value (GB300's FP64 rate is the binding limit next to HBM)
 constexpr int kSpmvLanes = 4;
+// iterations per launch of the one-kernel form: the host looks at the wall-clock limit
+// between launches (a few ms), a launch and its state copy cost about 20 us
+constexpr int kResidentIters = 256;
 
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double *partials, int stride) {
@@ -459,9 +462,13 @@ int krylov_init(mg_problem *p) {
     double **vecs[] = {&w.r, &w.z, &w.p0, &w.p1, &w.q, &w.dinv, &w.rh, &w.v, &w.y, &w.s, &w.t};
     for (double **v : vecs) MG_TRY(dev_alloc_n(v, (size_t)n));
     MG_TRY(dev_alloc_n(&w.partials, (size_t)3 * w.grid));
-    MG_TRY(dev_alloc(reinterpret_cast<void **>(&w.state), sizeof(KrylovState)));
+    // the state, then the one-kernel form's exchange scratch and its error flag
+    const size_t slots_at = (sizeof(KrylovState) + 255) / 256 * 256, err_at = slots_at + krylov_resident_bytes();
+    MG_TRY(dev_alloc(reinterpret_cast<void **>(&w.state), err_at + sizeof(int)));
+    w.slots = reinterpret_cast<char *>(w.state) + slots_at;
+    w.slot_err = reinterpret_cast<int *>(reinterpret_cast<char *>(w.state) + err_at);
     MG_CUDA_TRY(cudaMallocHost(reinterpret_cast<void **>(&w.state_host), sizeof(KrylovState)));
-    MG_CUDA_TRY(cudaMemsetAsync(w.state, 0, sizeof(KrylovState), p->stream));
+    MG_CUDA_TRY(cudaMemsetAsync(w.state, 0, err_at + sizeof(int), p->stream));
     return MG_OK;
 }
 
@@ -503,6 +510,7 @@ int transpose_csr(mg_problem *p, const CsrMatrix &A, CsrMatrix *At) {
     At->n = A.n;
     At->nnz = A.nnz;
     At->dpn = A.dpn;
+    At->max_row = A.max_row;
     int32_t *perm = nullptr;
     MG_TRY(dev_alloc_n(&perm, (size_t)A.nnz));
     MG_TRY(dev_alloc_n(&At->vals, (size_t)A.nnz));
@@ -565,6 +573,33 @@ int krylov_solve(mg_problem *p, const CsrMatrix &A, const double *d_b, double *d
                                          w.partials, nparts);
     MG_CUDA_TRY(cudaGetLastError());
     count_launches(3);
+    const double t0 = wall_time();
+    // one cooperative kernel per kResidentIters iterations where the vectors fit the SMs'
+    // shared memory (up to about 216,000 HEX8 nodes; faster there at every size measured,
+    // krylov_resident.cu)
+    for (;;) {
+        int launched = 0;
+        MG_TRY(krylov_resident_launch(p, A, d_x, krylov == MG_KRYLOV_CG, kResidentIters, &launched));
+        if (!launched) break;
+        int err = 0;
+        MG_CUDA_TRY(cudaMemcpyAsync(&err, w.slot_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        MG_TRY(read_state(p));
+        if (err) {
+            MG_CUDA_TRY(cudaMemsetAsync(w.slot_err, 0, sizeof(int), s));
+            set_error("Krylov solve: a grid exchange exceeded its bound");
+            return MG_ETIMEDOUT;
+        }
+        if (w.state_host->done) {
+            const KrylovState &h = *w.state_host;
+            if (iters) *iters = h.iter;
+            if (relres) *relres = (h.bb > 0 ? sqrt(h.rr / h.bb) : sqrt(h.rr));
+            return h.status;
+        }
+        if (o.timeout_s > 0 && wall_time() - t0 > o.timeout_s) {
+            set_error("Krylov solve exceeded %.1f s", o.timeout_s);
+            return MG_ETIMEDOUT;
+        }
+    }
     // CG: p0 = 0 and beta = 0, so the first p update forms p = z
     const int chunk = o.graph_chunk > 0 ? o.graph_chunk : 16;
     cudaGraph_t graph = nullptr;
@@ -599,7 +634,6 @@ int krylov_solve(mg_problem *p, const CsrMatrix &A, const double *d_b, double *d
         set_error("graph instantiate: %s", cudaGetErrorString(ce));
         return MG_ECUDA;
     }
-    const double t0 = wall_time();
     int rc = MG_OK;
     for (;;) {
         rc = read_state(p);

@@ -58,6 +58,8 @@ struct KrylovWork {
     double *partials = nullptr; // 3 * grid
     KrylovState *state = nullptr;
     KrylovState *state_host = nullptr; // pinned mirror
+    void *slots = nullptr;      // exchange scratch of the one-kernel form (krylov_resident.cu; in state's buffer)
+    int *slot_err = nullptr;    // set there when a bounded wait ran out
     cudaGraphExec_t graph_cg[2] = {nullptr, nullptr};
     int graph_chunk = 0;
     cudaGraphExec_t graph_bicg = nullptr;
@@ -67,6 +69,7 @@ struct KrylovWork {
 struct CsrMatrix {
     int64_t n = 0, nnz = 0;
     int dpn = 1;
+    int max_row = 1 << 30;  // longest row (columns); unknown: no bound
     int32_t *rowptr = nullptr, *cols = nullptr;
     double *vals = nullptr;
 };
@@ -172,6 +175,10 @@ void krylov_free(mg_problem *p);
 int spmv(mg_problem *p, const CsrMatrix &A, const double *d_x, double *d_y);
 int krylov_solve(mg_problem *p, const CsrMatrix &A, const double *d_b, double *d_x,
                  const mg_solve_opts &o, int krylov, int *iters, double *relres);
+// the one-kernel form (krylov_resident.cu)
+size_t krylov_resident_bytes();
+int krylov_resident_launch(mg_problem *p, const CsrMatrix &A, double *d_x, bool cg, int max_iters,
+                           int *launched);
 int dot(mg_problem *p, const double *a, const double *b, int64_t n, double *out);
 int transpose_csr(mg_problem *p, const CsrMatrix &A, CsrMatrix *At);
 void free_csr(CsrMatrix *A);
