@@ -91,9 +91,9 @@ def parse():
 def nonlinear_assembly(args, M):
     """Time the nonlinear-strain HEX8 assembly (residual and tangent of every colour,
     scattered into the CSR) on a 64x32x32 cantilever at a random 1e-3-strain state.
-    FP64 operations per element, from the per-pair formulation of the element:
-    tangent blocks 64 pairs x 8 points x 82 = 41,984; Jacobians, gradients, stresses,
-    projections and forces about 10,000: about 52,000 in all.  Bytes per element: the 576-entry tangent scattered as
+    FP64 operations per element: tangent blocks 36 pairs x (8 points x 42 + 45) = 13,700,
+    Jacobians, gradients, stresses, projections and forces about 8,100: about 21,800 in all.
+    Bytes per element: the 576-entry tangent scattered as
     read-modify-write (9,216 B), 24 residual entries (384 B), coordinates, state,
     connectivity and modulus (424 B)."""
     import torch
@@ -115,7 +115,7 @@ def nonlinear_assembly(args, M):
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / reps
     n_el = nx * ny * nz
-    flops = 52000.0 * n_el
+    flops = 21800.0 * n_el
     bytes_ = (9216 + 384 + 424) * n_el
     pk = peaks()
     print(json.dumps({

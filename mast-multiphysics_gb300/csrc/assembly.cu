@@ -215,8 +215,7 @@ __global__ void __launch_bounds__(256) hex8_kernel(
 // ---------------------------------------------------------------------------
 // Green-Lagrange HEX8 (the NONLINEAR_STRAIN branch, hex8_gl.cuh): one warp per
 // element, four warps per block, the element workspace in shared memory.
-// MODE 0: scatter the tangent (vals != null) and the internal force (R != null)
-// of coloured elements; MODE 1: element tangent (var-blocked) and force;
+// MODE 1: element tangent (var-blocked) and force;
 // MODE 2: out[e] = E_elem[e] a_e . f1_e(X) with f1 the internal force at unit
 // modulus (f_int is linear in E at fixed displacement: the density term of the
 // adjoint sensitivity, E_elem = dE/drho).
@@ -228,10 +227,8 @@ __global__ void __launch_bounds__(kGlWarps * 32) hex8_gl_kernel(
     const double *__restrict__ coords, const int32_t *__restrict__ conn,
     const int32_t *__restrict__ elem_list, int64_t first, int64_t n_items,
     const double *__restrict__ E_elem, double lam1, double mu1, const double *__restrict__ Xg,
-    const int32_t *__restrict__ rowptr, const uint16_t *__restrict__ emap,
-    double *__restrict__ vals, double *__restrict__ R, double *__restrict__ Ke_out,
-    double *__restrict__ fe_out, const double *__restrict__ va, const uint8_t *__restrict__ fixed,
-    double *__restrict__ out, int *__restrict__ status) {
+    double *__restrict__ Ke_out, double *__restrict__ fe_out, const double *__restrict__ va,
+    const uint8_t *__restrict__ fixed, double *__restrict__ out, int *__restrict__ status) {
     __shared__ gl::Work sh[kGlWarps];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     gl::Work &s = sh[w];
@@ -269,36 +266,97 @@ __global__ void __launch_bounds__(kGlWarps * 32) hex8_gl_kernel(
             if (lane < 24) {
                 const int a = lane / 3, i = lane % 3;
                 const double fl = gl::phase_force(s, lane);
-                if (MODE == 0 && R) R[(int64_t)en[a] * 3 + i] += fl;
-                if (MODE == 1 && fe_out) fe_out[(e - first) * 24 + i * 8 + a] = fl;
+                if (fe_out) fe_out[(e - first) * 24 + i * 8 + a] = fl;
             }
-            if (MODE == 1 || vals) {
 #pragma unroll 1
-                for (int h = 0; h < 2; h++) {
-                    const int p = lane + 32 * h, a = p >> 3, b = p & 7;
-                    double K[9];
-                    gl::phase_tangent(s, a, b, lam, mu, K);
-                    if (MODE == 0) {
-                        const int64_t na = en[a];
-                        const int off = emap[e * 64 + a * 8 + b];
+            for (int h = 0; h < 2; h++) {
+                const int p = lane + 32 * h, a = p >> 3, b = p & 7;
+                double K[9];
+                gl::phase_tangent(s, a, b, lam, mu, K);
+                double *dst = Ke_out + (e - first) * 576;
 #pragma unroll
-                        for (int i = 0; i < 3; i++) {
-                            double *dst = vals + rowptr[na * 3 + i] + off;
+                for (int i = 0; i < 3; i++)
 #pragma unroll
-                            for (int j = 0; j < 3; j++) dst[j] += K[i * 3 + j];
-                        }
-                    } else {
-                        double *dst = Ke_out + (e - first) * 576;
-#pragma unroll
-                        for (int i = 0; i < 3; i++)
-#pragma unroll
-                            for (int j = 0; j < 3; j++) dst[(i * 8 + a) * 24 + j * 8 + b] = K[i * 3 + j];
-                    }
-                }
+                    for (int j = 0; j < 3; j++) dst[(i * 8 + a) * 24 + j * 8 + b] = K[i * 3 + j];
             }
         }
         __syncwarp();
     }
+}
+
+// Residual and tangent of the coloured elements into the CSR (vals, nullable) and R
+// (nullable).  FP64-pipe bound (two DFMA per cycle and SM, 16 cycles a warp instruction
+// whatever its active lanes), so the items are packed: eight elements per block of nine
+// warps, their 64 Gauss points in two warps, their 288 node pairs (the upper half of the
+// symmetric tangent; the other half is written as the transpose) in exactly nine.
+// 64x32x32 (65,536 elements, 8 colours): one warp per element and all 64 pairs 5.39 ms an
+// assembly, this form 1.61 ms.
+constexpr int kGlBlockEl = 8;
+constexpr int kGlPairs = 36;
+constexpr int kGlBlock = kGlBlockEl * kGlPairs;
+constexpr int kGlBlockSmem = kGlBlockEl * (int)sizeof(gl::Work);
+
+__global__ void __launch_bounds__(kGlBlock, 3) hex8_gl_scatter_kernel(
+    const double *__restrict__ coords, const int32_t *__restrict__ conn,
+    const int32_t *__restrict__ elem_list, int64_t n_items, const double *__restrict__ E_elem,
+    double lam1, double mu1, const double *__restrict__ Xg, const int32_t *__restrict__ rowptr,
+    const uint16_t *__restrict__ emap, double *__restrict__ vals, double *__restrict__ R,
+    int *__restrict__ status) {
+    extern __shared__ __align__(16) unsigned char gl_smem[];
+    gl::Work *sh = reinterpret_cast<gl::Work *>(gl_smem);
+    __shared__ int32_t s_node[kGlBlockEl][8];
+    __shared__ double s_E[kGlBlockEl];
+    const int tid = threadIdx.x;
+    const int64_t item0 = (int64_t)blockIdx.x * kGlBlockEl;
+    const int ne = (int)min((int64_t)kGlBlockEl, n_items - item0);
+    if (tid < ne * 8) s_node[tid >> 3][tid & 7] = conn[(int64_t)elem_list[item0 + (tid >> 3)] * 8 + (tid & 7)];
+    if (tid >= 64 && tid < 64 + ne) s_E[tid - 64] = E_elem[elem_list[item0 + tid - 64]];
+    __syncthreads();
+    if (tid < ne * 24) {
+        const int k = tid / 24, i = tid - 24 * k;
+        const int64_t g = (int64_t)s_node[k][i / 3] * 3 + i % 3;
+        sh[k].X[i] = coords[g];
+        sh[k].u[i] = Xg[g];
+    }
+    __syncthreads();
+    if (tid < ne * 8 && !gl::jacobian_item(sh[tid >> 3], tid & 7)) atomicOr(status, 1);
+    __syncthreads();
+    for (int t = tid; t < ne * 64; t += kGlBlock) gl::gradient_item(sh[t >> 6], t >> 3 & 7, t & 7);
+    __syncthreads();
+    if (tid < ne * 8) gl::stress_item(sh[tid >> 3], tid & 7, s_E[tid >> 3] * lam1, s_E[tid >> 3] * mu1);
+    __syncthreads();
+    for (int t = tid; t < ne * 64; t += kGlBlock) gl::projection_item(sh[t >> 6], t >> 3 & 7, t & 7);
+    __syncthreads();
+    if (R && tid < ne * 24) {
+        const int k = tid / 24, i = tid - 24 * k;
+        R[(int64_t)s_node[k][i / 3] * 3 + i % 3] += gl::force_item(sh[k], i / 3, i % 3);
+    }
+    const int k = tid / kGlPairs;
+    if (!vals || k >= ne) return;
+    int a = 0, b = tid - k * kGlPairs;  // pair index -> a <= b
+    while (b >= 8 - a) {
+        b -= 8 - a;
+        a++;
+    }
+    b += a;
+    const int64_t e = elem_list[item0 + k];
+    double K[9];
+    gl::phase_tangent(sh[k], a, b, s_E[k] * lam1, s_E[k] * mu1, K);
+    const int64_t na = (int64_t)s_node[k][a] * 3, nb = (int64_t)s_node[k][b] * 3;
+    const int ab = emap[e * 64 + a * 8 + b], ba = emap[e * 64 + b * 8 + a];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        double *dst = vals + rowptr[na + i] + ab;
+#pragma unroll
+        for (int j = 0; j < 3; j++) dst[j] += K[i * 3 + j];
+    }
+    if (a != b)
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            double *dst = vals + rowptr[nb + i] + ba;
+#pragma unroll
+            for (int j = 0; j < 3; j++) dst[j] += K[j * 3 + i];
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -954,6 +1012,21 @@ int build_emap(mg_problem *p) {
     return read_status(p, st);
 }
 
+namespace {
+
+// one colour of the Green-Lagrange assembly
+int launch_gl_scatter(mg_problem *p, const int32_t *elems, int64_t count, double lam1, double mu1,
+                      const double *d_X, double *vals, double *d_R, int *st) {
+    MG_CUDA_TRY(cudaFuncSetAttribute(hex8_gl_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kGlBlockSmem));
+    hex8_gl_scatter_kernel<<<blocks_for(count, kGlBlockEl), kGlBlock, kGlBlockSmem, p->stream>>>(
+        p->d_coords, p->d_conn, elems, count, p->d_E, lam1, mu1, d_X, p->A.rowptr, p->d_emap, vals, d_R, st);
+    MG_CUDA_TRY(cudaGetLastError());
+    return MG_OK;
+}
+
+}  // namespace
+
 int assemble_system(mg_problem *p, const double *d_X, double *d_R, bool want_jacobian,
                     bool consistent) {
     int *st = status_slot(p);
@@ -997,11 +1070,8 @@ int assemble_system(mg_problem *p, const double *d_X, double *d_R, bool want_jac
         if (d_R) MG_CUDA_TRY(cudaMemsetAsync(d_R, 0, p->n_dofs * sizeof(double), p->stream));
         for (int c = 0; c < p->n_colors; c++) {
             int64_t cnt = p->color_ptr[c + 1] - p->color_ptr[c];
-            hex8_gl_kernel<0><<<blocks_for(cnt, kGlWarps), kGlWarps * 32, 0, p->stream>>>(
-                p->d_coords, p->d_conn, p->d_color_elems + p->color_ptr[c], 0, cnt, p->d_E, lam1,
-                mu1, d_X, p->A.rowptr, p->d_emap, want_jacobian ? p->A.vals : nullptr, d_R, nullptr,
-                nullptr, nullptr, nullptr, nullptr, st);
-            MG_CUDA_TRY(cudaGetLastError());
+            MG_TRY(launch_gl_scatter(p, p->d_color_elems + p->color_ptr[c], cnt, lam1, mu1, d_X,
+                                     want_jacobian ? p->A.vals : nullptr, d_R, st));
         }
         count_launches(p->n_colors);
         if (want_jacobian && (p->n_fix_zero || p->n_fix_diag)) {
@@ -1166,11 +1236,8 @@ int launch_assembly(mg_problem *p, const double *d_X, int reps) {
         MG_CUDA_TRY(cudaMemsetAsync(p->d_R, 0, p->n_dofs * sizeof(double), p->stream));
         for (int c = 0; c < p->n_colors; c++) {
             int64_t cnt = p->color_ptr[c + 1] - p->color_ptr[c];
-            hex8_gl_kernel<0><<<blocks_for(cnt, kGlWarps), kGlWarps * 32, 0, p->stream>>>(
-                p->d_coords, p->d_conn, p->d_color_elems + p->color_ptr[c], 0, cnt, p->d_E, lam1,
-                mu1, d_X, p->A.rowptr, p->d_emap, p->A.vals, p->d_R, nullptr, nullptr, nullptr,
-                nullptr, nullptr, st);
-            MG_CUDA_TRY(cudaGetLastError());
+            MG_TRY(launch_gl_scatter(p, p->d_color_elems + p->color_ptr[c], cnt, lam1, mu1, d_X, p->A.vals,
+                                     p->d_R, st));
         }
     }
     count_launches((long long)reps * p->n_colors);
@@ -1193,8 +1260,8 @@ int element_matrices(mg_problem *p, const double *d_X, int64_t first, int64_t co
         double lam1, mu1;
         lame_3d(p->mat.nu, lam1, mu1);
         hex8_gl_kernel<1><<<blocks_for(count, kGlWarps), kGlWarps * 32, 0, p->stream>>>(
-            p->d_coords, p->d_conn, nullptr, first, count, p->d_E, lam1, mu1, d_X, nullptr,
-            nullptr, nullptr, nullptr, d_Ke, d_fe, nullptr, nullptr, nullptr, st);
+            p->d_coords, p->d_conn, nullptr, first, count, p->d_E, lam1, mu1, d_X, d_Ke, d_fe,
+            nullptr, nullptr, nullptr, st);
     } else if (p->physics == MG_PHYSICS_MEMBRANE_QUAD4) {
         double nu = p->mat.nu;
         membrane_kernel<1><<<blocks_for(count, 128), 128, 0, p->stream>>>(
@@ -1235,7 +1302,7 @@ int elem_sensitivity(mg_problem *p, const double *d_X, const double *d_lambda, i
         lame_3d(p->mat.nu, lam1, mu1);
         hex8_gl_kernel<2><<<blocks_for(p->n_elems, kGlWarps), kGlWarps * 32, 0, p->stream>>>(
             p->d_coords, p->d_conn, nullptr, 0, p->n_elems, p->d_dE, lam1, mu1, d_X, nullptr,
-            nullptr, nullptr, nullptr, nullptr, nullptr, d_lambda, p->d_fixed, d_out_elem, st);
+            nullptr, d_lambda, p->d_fixed, d_out_elem, st);
     } else if (p->physics == MG_PHYSICS_HEAT_QUAD4 &&
                (kind == MG_PARAM_K0 || kind == MG_PARAM_ELEM_SCALE)) {
         heat_sens_kernel<<<blocks_for(p->n_elems, 128), 128, 0, p->stream>>>(
@@ -1274,8 +1341,8 @@ int assemble_param_residual(mg_problem *p, const double *d_X, int kind, int64_t 
             elem_matvec_kernel<<<1, 32, 0, p->stream>>>(Ke, d_X, p->d_conn, index, 1, 8, 3, fe);
         } else {
             hex8_gl_kernel<1><<<1, kGlWarps * 32, 0, p->stream>>>(
-                p->d_coords, p->d_conn, nullptr, index, 1, p->d_dE, lam1, mu1, d_X, nullptr,
-                nullptr, nullptr, nullptr, Ke, fe, nullptr, nullptr, nullptr, st);
+                p->d_coords, p->d_conn, nullptr, index, 1, p->d_dE, lam1, mu1, d_X, Ke, fe, nullptr,
+                nullptr, nullptr, st);
         }
         MG_CUDA_TRY(cudaGetLastError());
         std::vector<double> hfe(24);
@@ -1413,8 +1480,8 @@ int element_sensitivity(mg_problem *p, int64_t e, const double *d_sol, int kind,
             elem_matvec_kernel<<<1, 32, 0, p->stream>>>(Ke, p->d_tmp, p->d_conn, e, 1, 8, 3, d_dfe);
         } else {
             hex8_gl_kernel<1><<<1, kGlWarps * 32, 0, p->stream>>>(
-                p->d_coords, p->d_conn, nullptr, e, 1, p->d_dE, lam1, mu1, p->d_tmp, nullptr, nullptr,
-                nullptr, nullptr, Ke, d_dfe, nullptr, nullptr, nullptr, st);
+                p->d_coords, p->d_conn, nullptr, e, 1, p->d_dE, lam1, mu1, p->d_tmp, Ke, d_dfe,
+                nullptr, nullptr, nullptr, st);
         }
         MG_CUDA_TRY(cudaGetLastError());
         count_launches(2);

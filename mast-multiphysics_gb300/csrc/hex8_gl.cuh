@@ -16,10 +16,16 @@
 // with S = lam tr(E) I + 2 mu E, E = (Fd^T Fd - I)/2 (the second Piola-Kirchhoff
 // stress of C applied to the Green-Lagrange strain in Voigt form).
 //
-// One warp evaluates one element.  The work is split into phases over a
-// per-warp workspace; a phase is a function of the lane index, and lanes only
-// read what earlier phases wrote, so the kernel separates phases by
-// __syncwarp() and a host loop over the 32 lanes runs the same source.
+// With the sums T = sum_qp JxW (Fd g_a) (x) (Fd g_b) and s = sum_qp JxW g_a.S.g_b, the block
+// of nodes a, b is lam T + mu T^T + mu sum_qp JxW (g_a.g_b) Fd Fd^T + s I: 21 products per
+// Gauss point instead of 41 with the terms scaled inside the sum, and the block of b, a is
+// its transpose.
+//
+// The work is split into items ((point), (point, node), (dof), (node pair)) over the
+// element's workspace; the items of a phase only read what earlier phases wrote, so a
+// kernel may spread them over any threads with a barrier between phases.  The phase_*
+// functions do the items of one lane of a warp per element (the host tests run the same
+// source as a loop over 32 lanes).
 #pragma once
 
 #include <math.h>
@@ -33,41 +39,42 @@
 namespace mg {
 namespace gl {
 
-// element workspace of one warp (doubles; 924 = 7.4 KB)
+// element workspace (doubles; 1,064 = 8.5 KB)
 struct Work {
-    double X[24];        // node coordinates, node-major (3 a + d)
-    double u[24];        // displacements, node-major (3 a + c)
-    double w[8];         // JxW per Gauss point (unit weights)
-    double inv[8][9];    // inverse Jacobian per Gauss point
-    double g[8][8][3];   // physical gradients g[q][a]
-    double Fd[8][9];     // deformation gradient I + grad u per Gauss point
-    double S[8][9];      // second Piola-Kirchhoff stress (symmetric, full 3 x 3)
-    double B[8][9];      // Fd Fd^T (f_i . f_j)
-    double Fg[8][8][3];  // Fd g_a  (f_i . g_a)
-    double Sg[8][8][3];  // S g_a
+    double X[24];         // node coordinates, node-major (3 a + d)
+    double u[24];         // displacements, node-major (3 a + c)
+    double w[8];          // JxW per Gauss point (unit weights)
+    double inv[8][9];     // inverse Jacobian per Gauss point
+    double g[8][8][3];    // physical gradients g[q][a]
+    double Fd[8][9];      // deformation gradient I + grad u per Gauss point
+    double wS[8][6];      // JxW times the second Piola-Kirchhoff stress: xx, yy, zz, xy, yz, zx
+    double wB[8][6];      // JxW Fd Fd^T (f_i . f_j), in the same order
+    double Fg[8][8][3];   // Fd g_a  (f_i . g_a)
+    double wFg[8][8][3];  // JxW Fd g_a
+    double wSg[8][8][3];  // JxW S g_a
 };
 
-constexpr double kGauss = 0.57735026918962576451;  // 1/sqrt(3)
-
 // reference gradient of shape function a at Gauss point q = i + 2 j + 4 k
-// (libMesh HEX8 node order: x signs - + + -, y signs - - + +, z - for nodes 0-3)
+// (libMesh HEX8 node order: x signs - + + -, y signs - - + +, z - for nodes 0-3).
+// Each component is +-1/2 times the other two directions' hats, each (1 + 1/sqrt 3) / 2 at
+// the node's own side and (1 - 1/sqrt 3) / 2 at the other: one of three constants.
 GL_HD void dref(int q, int a, double d[3]) {
-    const double xi = (q & 1) ? kGauss : -kGauss, eta = (q >> 1 & 1) ? kGauss : -kGauss,
-                 zeta = (q >> 2 & 1) ? kGauss : -kGauss;
-    const double sx = ((a + 1) >> 1 & 1) ? 1.0 : -1.0, sy = (a >> 1 & 1) ? 1.0 : -1.0,
-                 sz = (a >> 2 & 1) ? 1.0 : -1.0;
-    const double fx = 0.5 * (1.0 + sx * xi), fy = 0.5 * (1.0 + sy * eta), fz = 0.5 * (1.0 + sz * zeta);
-    d[0] = 0.5 * sx * fy * fz;
-    d[1] = 0.5 * sy * fx * fz;
-    d[2] = 0.5 * sz * fx * fy;
+    constexpr double near = 0.5 * (1.0 + 0.57735026918962576451), far = 0.5 * (1.0 - 0.57735026918962576451);
+    constexpr double c0 = 0.5 * far * far, c1 = 0.5 * near * far, c2 = 0.5 * near * near;
+    const int ax = (a + 1) >> 1 & 1, ay = a >> 1 & 1, az = a >> 2 & 1;
+    const int mx = (q & 1) == ax, my = (q >> 1 & 1) == ay, mz = (q >> 2 & 1) == az;
+    const double x = my & mz ? c2 : my | mz ? c1 : c0;
+    const double y = mx & mz ? c2 : mx | mz ? c1 : c0;
+    const double z = mx & my ? c2 : mx | my ? c1 : c0;
+    d[0] = ax ? x : -x;
+    d[1] = ay ? y : -y;
+    d[2] = az ? z : -z;
 }
 
-// phase 1 (lanes 0-7, q = lane): Jacobian, JxW, inverse.  Returns false for a
-// non-positive determinant.  (W: any workspace with X, w, inv.)
+// item (q): Jacobian, JxW, inverse.  Returns false for a non-positive determinant.
+// (W: any workspace with X, w, inv.)
 template <class W>
-GL_HD bool phase_jacobian(W &s, int lane) {
-    if (lane >= 8) return true;
-    const int q = lane;
+GL_HD bool jacobian_item(W &s, int q) {
     double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // J[i][j] = d x_j / d xi_i
     for (int a = 0; a < 8; a++) {
         double d[3];
@@ -75,109 +82,129 @@ GL_HD bool phase_jacobian(W &s, int lane) {
         for (int i = 0; i < 3; i++)
             for (int j = 0; j < 3; j++) J[i * 3 + j] += d[i] * s.X[a * 3 + j];
     }
-    const double det = J[0] * (J[4] * J[8] - J[5] * J[7]) - J[1] * (J[3] * J[8] - J[5] * J[6]) +
-                       J[2] * (J[3] * J[7] - J[4] * J[6]);
-    double *iv = s.inv[q];
-    iv[0] = (J[4] * J[8] - J[5] * J[7]) / det;
-    iv[1] = (J[2] * J[7] - J[1] * J[8]) / det;
-    iv[2] = (J[1] * J[5] - J[2] * J[4]) / det;
-    iv[3] = (J[5] * J[6] - J[3] * J[8]) / det;
-    iv[4] = (J[0] * J[8] - J[2] * J[6]) / det;
-    iv[5] = (J[2] * J[3] - J[0] * J[5]) / det;
-    iv[6] = (J[3] * J[7] - J[4] * J[6]) / det;
-    iv[7] = (J[1] * J[6] - J[0] * J[7]) / det;
-    iv[8] = (J[0] * J[4] - J[1] * J[3]) / det;
+    double iv[9];
+    iv[0] = J[4] * J[8] - J[5] * J[7];
+    iv[1] = J[2] * J[7] - J[1] * J[8];
+    iv[2] = J[1] * J[5] - J[2] * J[4];
+    iv[3] = J[5] * J[6] - J[3] * J[8];
+    iv[4] = J[0] * J[8] - J[2] * J[6];
+    iv[5] = J[2] * J[3] - J[0] * J[5];
+    iv[6] = J[3] * J[7] - J[4] * J[6];
+    iv[7] = J[1] * J[6] - J[0] * J[7];
+    iv[8] = J[0] * J[4] - J[1] * J[3];
+    const double det = J[0] * iv[0] + J[1] * iv[3] + J[2] * iv[6];
+    const double r = 1.0 / det;
+    for (int k = 0; k < 9; k++) s.inv[q][k] = iv[k] * r;
     s.w[q] = det;
     return det > 0.0;
 }
 
-// phase 2 (every lane, (q, a) = (p >> 3, p & 7) for p = lane, lane + 32):
-// physical gradients g_j = sum_k (d xi_k / d x_j) d phi / d xi_k
+// item (q, a): physical gradient g_j = sum_k (d xi_k / d x_j) d phi / d xi_k
 template <class W>
-GL_HD void phase_gradients(W &s, int lane) {
-    for (int h = 0; h < 2; h++) {
-        const int p = lane + 32 * h, q = p >> 3, a = p & 7;
-        double d[3];
-        dref(q, a, d);
-        const double *iv = s.inv[q];
-        for (int j = 0; j < 3; j++) s.g[q][a][j] = iv[j * 3] * d[0] + iv[j * 3 + 1] * d[1] + iv[j * 3 + 2] * d[2];
-    }
+GL_HD void gradient_item(W &s, int q, int a) {
+    double d[3];
+    dref(q, a, d);
+    const double *iv = s.inv[q];
+    for (int j = 0; j < 3; j++) s.g[q][a][j] = iv[j * 3] * d[0] + iv[j * 3 + 1] * d[1] + iv[j * 3 + 2] * d[2];
 }
 
-// phase 3 (lanes 0-7, q = lane): Fd, Green-Lagrange strain, S, Fd Fd^T.  The
-// strain is formed from H = grad u as (H + H^T + H^T H) / 2, not as
-// (Fd^T Fd - I) / 2, whose subtraction would cancel the leading digits of small
-// strains (a 1e-8 strain would keep only 8 significant digits).
-GL_HD void phase_stress(Work &s, int lane, double lam, double mu) {
-    if (lane >= 8) return;
-    const int q = lane;
+// item (q): Fd, Green-Lagrange strain, JxW S, JxW Fd Fd^T.  The strain is formed from
+// H = grad u as (H + H^T + H^T H) / 2, not as (Fd^T Fd - I) / 2, whose subtraction would
+// cancel the leading digits of small strains (a 1e-8 strain would keep only 8 significant
+// digits).
+GL_HD void stress_item(Work &s, int q, double lam, double mu) {
     double H[9], Fd[9];
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) {
-            double v = 0.0;
-            for (int a = 0; a < 8; a++) v += s.u[a * 3 + i] * s.g[q][a][j];
-            H[i * 3 + j] = v;
-            Fd[i * 3 + j] = v + (i == j ? 1.0 : 0.0);
-        }
-    double E[9];
-    for (int j = 0; j < 3; j++)
-        for (int k = 0; k < 3; k++) {
-            double c = 0.0;
-            for (int m = 0; m < 3; m++) c += H[m * 3 + j] * H[m * 3 + k];
-            E[j * 3 + k] = 0.5 * (H[j * 3 + k] + H[k * 3 + j] + c);
-        }
-    const double tr = E[0] + E[4] + E[8];
-    for (int j = 0; j < 3; j++)
-        for (int k = 0; k < 3; k++) {
-            s.S[q][j * 3 + k] = 2.0 * mu * E[j * 3 + k] + (j == k ? lam * tr : 0.0);
-            double b = 0.0;
-            for (int m = 0; m < 3; m++) b += Fd[j * 3 + m] * Fd[k * 3 + m];
-            s.B[q][j * 3 + k] = b;
-            s.Fd[q][j * 3 + k] = Fd[j * 3 + k];
-        }
-}
-
-// phase 4 (every lane, (q, a) as in phase 2): Fd g_a and S g_a
-GL_HD void phase_projections(Work &s, int lane) {
-    for (int h = 0; h < 2; h++) {
-        const int p = lane + 32 * h, q = p >> 3, a = p & 7;
-        const double *g = s.g[q][a];
-        for (int i = 0; i < 3; i++) {
-            s.Fg[q][a][i] = s.Fd[q][i * 3] * g[0] + s.Fd[q][i * 3 + 1] * g[1] + s.Fd[q][i * 3 + 2] * g[2];
-            s.Sg[q][a][i] = s.S[q][i * 3] * g[0] + s.S[q][i * 3 + 1] * g[1] + s.S[q][i * 3 + 2] * g[2];
-        }
+    for (int i = 0; i < 9; i++) H[i] = 0.0;
+    for (int a = 0; a < 8; a++)
+        for (int i = 0; i < 3; i++)
+            for (int j = 0; j < 3; j++) H[i * 3 + j] += s.u[a * 3 + i] * s.g[q][a][j];
+    for (int i = 0; i < 9; i++) {
+        Fd[i] = H[i] + (i % 4 == 0 ? 1.0 : 0.0);
+        s.Fd[q][i] = Fd[i];
     }
+    const double w = s.w[q];
+    double E[6];  // xx, yy, zz, xy, yz, zx
+    for (int r = 0; r < 6; r++) {
+        const int j = r % 3, k = r < 3 ? j : (j + 1) % 3;
+        double c = 0.0;
+        for (int m = 0; m < 3; m++) c += H[m * 3 + j] * H[m * 3 + k];
+        E[r] = 0.5 * (H[j * 3 + k] + H[k * 3 + j] + c);
+        double b = 0.0;
+        for (int m = 0; m < 3; m++) b += Fd[j * 3 + m] * Fd[k * 3 + m];
+        s.wB[q][r] = w * b;
+    }
+    const double ltr = lam * (E[0] + E[1] + E[2]);
+    for (int r = 0; r < 6; r++) s.wS[q][r] = w * (2.0 * mu * E[r] + (r < 3 ? ltr : 0.0));
 }
 
-// phase 5a (lanes 0-23, lane = 3 a + i): internal force of dof (i, a)
-GL_HD double phase_force(const Work &s, int lane) {
-    const int a = lane / 3, i = lane % 3;
+// item (q, a): Fd g_a, JxW Fd g_a and JxW S g_a
+GL_HD void projection_item(Work &s, int q, int a) {
+    const double g[3] = {s.g[q][a][0], s.g[q][a][1], s.g[q][a][2]};
+    const double w = s.w[q];
+    const double *S = s.wS[q];
+    for (int i = 0; i < 3; i++) {
+        const double f = s.Fd[q][i * 3] * g[0] + s.Fd[q][i * 3 + 1] * g[1] + s.Fd[q][i * 3 + 2] * g[2];
+        s.Fg[q][a][i] = f;
+        s.wFg[q][a][i] = w * f;
+    }
+    s.wSg[q][a][0] = S[0] * g[0] + S[3] * g[1] + S[5] * g[2];
+    s.wSg[q][a][1] = S[3] * g[0] + S[1] * g[1] + S[4] * g[2];
+    s.wSg[q][a][2] = S[5] * g[0] + S[4] * g[1] + S[2] * g[2];
+}
+
+// item (a, i): internal force of dof (i, a)
+GL_HD double force_item(const Work &s, int a, int i) {
     double f = 0.0;
     for (int q = 0; q < 8; q++) {
         const double *Fd = s.Fd[q] + i * 3;
-        const double *Sg = s.Sg[q][a];
-        f += s.w[q] * (Fd[0] * Sg[0] + Fd[1] * Sg[1] + Fd[2] * Sg[2]);
+        const double *Sg = s.wSg[q][a];
+        f += Fd[0] * Sg[0] + Fd[1] * Sg[1] + Fd[2] * Sg[2];
     }
     return f;
 }
 
-// phase 5b (node pair (a, b)): the 3 x 3 tangent block K[i][j] = K_ia,jb
+// item (node pair (a, b)): the 3 x 3 tangent block K[i][j] = K_ia,jb
 GL_HD void phase_tangent(const Work &s, int a, int b, double lam, double mu, double K[9]) {
-    for (int k = 0; k < 9; k++) K[k] = 0.0;
+    double T[9], B[6], sg = 0.0;
+    for (int k = 0; k < 9; k++) T[k] = 0.0;
+    for (int k = 0; k < 6; k++) B[k] = 0.0;
+#ifdef __CUDA_ARCH__
+#pragma unroll 2
+#endif
     for (int q = 0; q < 8; q++) {
-        const double *ga = s.g[q][a], *gb = s.g[q][b];
-        const double *Fa = s.Fg[q][a], *Fb = s.Fg[q][b];
-        const double wq = s.w[q];
+        const double *ga = s.g[q][a], *gb = s.g[q][b], *Sb = s.wSg[q][b];
+        const double *Fa = s.wFg[q][a], *Fb = s.Fg[q][b], *wB = s.wB[q];
         const double gab = ga[0] * gb[0] + ga[1] * gb[1] + ga[2] * gb[2];
-        const double gsg = ga[0] * s.Sg[q][b][0] + ga[1] * s.Sg[q][b][1] + ga[2] * s.Sg[q][b][2];
+        sg += ga[0] * Sb[0] + ga[1] * Sb[1] + ga[2] * Sb[2];
         for (int i = 0; i < 3; i++)
-            for (int j = 0; j < 3; j++) {
-                double k = lam * Fa[i] * Fb[j] + mu * (s.B[q][i * 3 + j] * gab + Fb[i] * Fa[j]);
-                if (i == j) k += gsg;
-                K[i * 3 + j] += wq * k;
-            }
+            for (int j = 0; j < 3; j++) T[i * 3 + j] += Fa[i] * Fb[j];
+        for (int r = 0; r < 6; r++) B[r] += gab * wB[r];
+    }
+    for (int i = 0; i < 3; i++) {
+        K[i * 4] = (lam + mu) * T[i * 4] + (mu * B[i] + sg);
+        const int j = (i + 1) % 3;
+        const double m = mu * B[3 + i];
+        K[i * 3 + j] = lam * T[i * 3 + j] + (mu * T[j * 3 + i] + m);
+        K[j * 3 + i] = lam * T[j * 3 + i] + (mu * T[i * 3 + j] + m);
     }
 }
+
+// the items of lane `lane` of a warp that evaluates one element (workspaces with X, u)
+template <class W>
+GL_HD bool phase_jacobian(W &s, int lane) {
+    return lane >= 8 || jacobian_item(s, lane);
+}
+template <class W>
+GL_HD void phase_gradients(W &s, int lane) {
+    for (int p = lane; p < 64; p += 32) gradient_item(s, p >> 3, p & 7);
+}
+GL_HD void phase_stress(Work &s, int lane, double lam, double mu) {
+    if (lane < 8) stress_item(s, lane, lam, mu);
+}
+GL_HD void phase_projections(Work &s, int lane) {
+    for (int p = lane; p < 64; p += 32) projection_item(s, p >> 3, p & 7);
+}
+GL_HD double phase_force(const Work &s, int lane) { return force_item(s, lane / 3, lane % 3); }
 
 // ---------------------------------------------------------------------------
 // Stress output (StructuralElement3D::calculate_stress, solid_element_3d.cpp:
