@@ -81,26 +81,19 @@ __device__ __forceinline__ double quad4_qp(const double X[8], int q, double phi[
 constexpr int kWarpsPerBlock = 8;
 
 // ---------------------------------------------------------------------------
-// HEX8: one warp per element.  MODE 0: scatter into CSR; MODE 1: write the
-// 24x24 element matrix (var-blocked); MODE 2: per-element bilinear form
-// out[e] = scale_e * a_e^T K1_e b_e (K1 = stiffness at E = 1).
+// HEX8: one warp per element, writes the 24x24 element matrix (var-blocked).
 // ---------------------------------------------------------------------------
-template <int MODE>
-__global__ void __launch_bounds__(256) hex8_kernel(
-    const double *__restrict__ coords, const int32_t *__restrict__ conn,
-    const int32_t *__restrict__ elem_list, int64_t first, int64_t n_items,
+__global__ void __launch_bounds__(256) hex8_matrix_kernel(
+    const double *__restrict__ coords, const int32_t *__restrict__ conn, int64_t first, int64_t n_items,
     const double *__restrict__ E_elem, const double *__restrict__ E_qp, double lam1, double mu1,
-    const int32_t *__restrict__ rowptr, const uint16_t *__restrict__ emap,
-    double *__restrict__ vals, double *__restrict__ Ke_out,
-    const double *__restrict__ va, const double *__restrict__ vb,
-    const uint8_t *__restrict__ fixed, double *__restrict__ out, int *__restrict__ status) {
+    double *__restrict__ Ke_out, int *__restrict__ status) {
     __shared__ double sh_g[kWarpsPerBlock][8][8][3];
     __shared__ double sh_w[kWarpsPerBlock][8];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
     for (int64_t item = (int64_t)blockIdx.x * kWarpsPerBlock + w; item < n_items;
          item += (int64_t)gridDim.x * kWarpsPerBlock) {
-        const int64_t e = elem_list ? elem_list[item] : first + item;
+        const int64_t e = first + item;
         const int32_t *en = conn + e * 8;
         double xv = 0.0;
         if (lane < 24) xv = coords[(int64_t)en[lane / 3] * 3 + lane % 3];
@@ -146,7 +139,6 @@ __global__ void __launch_bounds__(256) hex8_kernel(
                 sh_g[w][qq][a][j] = iv[j * 3] * d[0] + iv[j * 3 + 1] * d[1] + iv[j * 3 + 2] * d[2];
         }
         __syncwarp();
-        double acc_mode2 = 0.0;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int p = lane + 32 * h, a = p >> 3, b = p & 7;
@@ -166,7 +158,7 @@ __global__ void __launch_bounds__(256) hex8_kernel(
 #pragma unroll
                     for (int j = 0; j < 3; j++) S[i * 3 + j] = fma(ga[i], gb[j], S[i * 3 + j]);
             }
-            const double Ee = (MODE == 2 || E_qp) ? 1.0 : E_elem[e];
+            const double Ee = E_qp ? 1.0 : E_elem[e];
             const double lam = Ee * lam1, mu = Ee * mu1, tr = S[0] + S[4] + S[8];
             double K[9];
 #pragma unroll
@@ -174,39 +166,11 @@ __global__ void __launch_bounds__(256) hex8_kernel(
 #pragma unroll
                 for (int j = 0; j < 3; j++)
                     K[i * 3 + j] = lam * S[i * 3 + j] + mu * S[j * 3 + i] + (i == j ? mu * tr : 0.0);
-            if (MODE == 0) {
-                const int64_t na = en[a];
-                const int off = emap[e * 64 + a * 8 + b];
+            double *dst = Ke_out + (e - first) * 576;
 #pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    double *dst = vals + rowptr[na * 3 + i] + off;
+            for (int i = 0; i < 3; i++)
 #pragma unroll
-                    for (int j = 0; j < 3; j++) dst[j] += K[i * 3 + j];
-                }
-            } else if (MODE == 1) {
-                double *dst = Ke_out + (e - first) * 576;
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int j = 0; j < 3; j++) dst[(i * 8 + a) * 24 + j * 8 + b] = K[i * 3 + j];
-            } else {
-                const int64_t na = en[a], nb = en[b];
-                double ua[3], ub[3];
-#pragma unroll
-                for (int i = 0; i < 3; i++) {
-                    ua[i] = (fixed && fixed[na * 3 + i]) ? 0.0 : va[na * 3 + i];
-                    ub[i] = (fixed && fixed[nb * 3 + i]) ? 0.0 : vb[nb * 3 + i];
-                }
-#pragma unroll
-                for (int i = 0; i < 3; i++)
-#pragma unroll
-                    for (int j = 0; j < 3; j++) acc_mode2 = fma(ua[i] * K[i * 3 + j], ub[j], acc_mode2);
-            }
-        }
-        if (MODE == 2) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc_mode2 += __shfl_xor_sync(full, acc_mode2, o);
-            if (lane == 0) out[e] = E_elem[e] * acc_mode2;
+                for (int j = 0; j < 3; j++) dst[(i * 8 + a) * 24 + j * 8 + b] = K[i * 3 + j];
         }
         __syncwarp();
     }
@@ -284,6 +248,27 @@ __global__ void __launch_bounds__(kGlWarps * 32) hex8_gl_kernel(
     }
 }
 
+// adds the block K of nodes a <= b of element e, and its transpose for b, a
+__device__ __forceinline__ void scatter_pair(const int32_t *node, int64_t e, int a, int b, const double (&K)[9],
+                                             const int32_t *__restrict__ rowptr,
+                                             const uint16_t *__restrict__ emap, double *__restrict__ vals) {
+    const int64_t na = (int64_t)node[a] * 3, nb = (int64_t)node[b] * 3;
+    const int ab = emap[e * 64 + a * 8 + b], ba = emap[e * 64 + b * 8 + a];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        double *dst = vals + rowptr[na + i] + ab;
+#pragma unroll
+        for (int j = 0; j < 3; j++) dst[j] += K[i * 3 + j];
+    }
+    if (a != b)
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            double *dst = vals + rowptr[nb + i] + ba;
+#pragma unroll
+            for (int j = 0; j < 3; j++) dst[j] += K[j * 3 + i];
+        }
+}
+
 // Residual and tangent of the coloured elements into the CSR (vals, nullable) and R
 // (nullable).  FP64-pipe bound (two DFMA per cycle and SM, 16 cycles a warp instruction
 // whatever its active lanes), so the items are packed: eight elements per block of nine
@@ -342,21 +327,116 @@ __global__ void __launch_bounds__(kGlBlock, 3) hex8_gl_scatter_kernel(
     const int64_t e = elem_list[item0 + k];
     double K[9];
     gl::phase_tangent(sh[k], a, b, s_E[k] * lam1, s_E[k] * mu1, K);
-    const int64_t na = (int64_t)s_node[k][a] * 3, nb = (int64_t)s_node[k][b] * 3;
-    const int ab = emap[e * 64 + a * 8 + b], ba = emap[e * 64 + b * 8 + a];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        double *dst = vals + rowptr[na + i] + ab;
-#pragma unroll
-        for (int j = 0; j < 3; j++) dst[j] += K[i * 3 + j];
+    scatter_pair(s_node[k], e, a, b, K, rowptr, emap, vals);
+}
+
+// Linear-strain stiffness of the coloured elements into the CSR: the packing of
+// hex8_gl_scatter_kernel (eight elements per block, the upper half of the node pairs).
+// Latency-bound below a few thousand elements a colour: 24x12x12 43 us a colour with one warp
+// per element and all pairs, 22 us this way.
+__global__ void __launch_bounds__(kGlBlock, 4) hex8_scatter_kernel(
+    const double *__restrict__ coords, const int32_t *__restrict__ conn,
+    const int32_t *__restrict__ elem_list, int64_t n_items, const double *__restrict__ E_elem,
+    const double *__restrict__ E_qp, double lam1, double mu1, const int32_t *__restrict__ rowptr,
+    const uint16_t *__restrict__ emap, double *__restrict__ vals, int *__restrict__ status) {
+    __shared__ gl::LinearWork sh[kGlBlockEl];
+    __shared__ int32_t s_node[kGlBlockEl][8];
+    const int tid = threadIdx.x;
+    const int64_t item0 = (int64_t)blockIdx.x * kGlBlockEl;
+    const int ne = (int)min((int64_t)kGlBlockEl, n_items - item0);
+    if (tid < ne * 8) s_node[tid >> 3][tid & 7] = conn[(int64_t)elem_list[item0 + (tid >> 3)] * 8 + (tid & 7)];
+    __syncthreads();
+    if (tid < ne * 24) {
+        const int k = tid / 24, i = tid - 24 * k;
+        sh[k].X[i] = coords[(int64_t)s_node[k][i / 3] * 3 + i % 3];
     }
-    if (a != b)
+    __syncthreads();
+    if (tid < ne * 8 && !gl::jacobian_item(sh[tid >> 3], tid & 7)) atomicOr(status, 1);
+    __syncthreads();
+    for (int t = tid; t < ne * 64; t += kGlBlock) {
+        gl::LinearWork &s = sh[t >> 6];
+        const int q = t >> 3 & 7, n = t & 7;
+        gl::gradient_item(s, q, n);
+        // a nodal density field gives the modulus per Gauss point, else it scales the element
+        const double w = E_qp ? s.w[q] * E_qp[(int64_t)elem_list[item0 + (t >> 6)] * 8 + q] : s.w[q];
+        for (int j = 0; j < 3; j++) s.wg[q][n][j] = w * s.g[q][n][j];
+    }
+    __syncthreads();
+    const int k = tid / kGlPairs;
+    if (k >= ne) return;
+    int a = 0, b = tid - k * kGlPairs;  // pair index -> a <= b
+    while (b >= 8 - a) {
+        b -= 8 - a;
+        a++;
+    }
+    b += a;
+    const int64_t e = elem_list[item0 + k];
+    const double Ee = E_qp ? 1.0 : E_elem[e];
+    double K[9];
+    gl::linear_pair_item(sh[k], a, b, Ee * lam1, Ee * mu1, K);
+    scatter_pair(s_node[k], e, a, b, K, rowptr, emap, vals);
+}
+
+// out[e] = scale_e a_e . K1_e b_e (K1 = stiffness at E = 1; a, b zero on fixed dofs), from the
+// strains of a and b at the Gauss points: sum_qp JxW (lam tr(ea) tr(eb) + 2 mu ea : eb).
+// One thread per Gauss point, 32 elements per block; FP64-pipe bound; at 24x12x12
+// 123 us for the form through the 24 x 24 products (one warp per element), 26 us this way.
+constexpr int kEnergyEl = 32;
+
+__global__ void __launch_bounds__(kEnergyEl * 8) hex8_energy_kernel(
+    const double *__restrict__ coords, const int32_t *__restrict__ conn, int64_t n_elems,
+    const double *__restrict__ scale, double lam1, double mu1, const double *__restrict__ va,
+    const double *__restrict__ vb, const uint8_t *__restrict__ fixed, double *__restrict__ out,
+    int *__restrict__ status) {
+    __shared__ double sX[kEnergyEl][25], sa[kEnergyEl][25], sb[kEnergyEl][25];  // padded: 8 elements per warp row
+    const int64_t e0 = (int64_t)blockIdx.x * kEnergyEl;
+    const int ne = (int)min((int64_t)kEnergyEl, n_elems - e0);
+    const bool same = va == vb;
+    for (int t = threadIdx.x; t < ne * 24; t += kEnergyEl * 8) {
+        const int k = t / 24, i = t - 24 * k;
+        const int64_t g = (int64_t)conn[(e0 + k) * 8 + i / 3] * 3 + i % 3;
+        const bool fx = fixed && fixed[g];
+        sX[k][i] = coords[g];
+        sa[k][i] = fx ? 0.0 : va[g];
+        if (!same) sb[k][i] = fx ? 0.0 : vb[g];
+    }
+    __syncthreads();
+    const int k = threadIdx.x >> 3, q = threadIdx.x & 7;
+    double v = 0.0;
+    if (k < ne) {
+        struct { const double *X; double inv[1][9], w[1]; } s{sX[k], {}, {}};
+        if (!gl::jacobian_at(s, q, 0)) atomicOr(status, 1);
+        double A[9], B[9];
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            double *dst = vals + rowptr[nb + i] + ba;
+        for (int i = 0; i < 9; i++) A[i] = B[i] = 0.0;
 #pragma unroll
-            for (int j = 0; j < 3; j++) dst[j] += K[j * 3 + i];
+        for (int n = 0; n < 8; n++) {
+            double d[3], g[3];
+            gl::dref(q, n, d);
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+                g[j] = s.inv[0][j * 3] * d[0] + s.inv[0][j * 3 + 1] * d[1] + s.inv[0][j * 3 + 2] * d[2];
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int j = 0; j < 3; j++) A[i * 3 + j] = fma(sa[k][n * 3 + i], g[j], A[i * 3 + j]);
+            if (!same)
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) B[i * 3 + j] = fma(sb[k][n * 3 + i], g[j], B[i * 3 + j]);
         }
+        if (same)
+#pragma unroll
+            for (int i = 0; i < 9; i++) B[i] = A[i];
+        // 2 ea : eb = 2 sum of the diagonal products + the products of the engineering shears
+        const double dd = A[0] * B[0] + A[4] * B[4] + A[8] * B[8];
+        const double ss = (A[1] + A[3]) * (B[1] + B[3]) + (A[5] + A[7]) * (B[5] + B[7]) + (A[2] + A[6]) * (B[2] + B[6]);
+        v = s.w[0] * (lam1 * (A[0] + A[4] + A[8]) * (B[0] + B[4] + B[8]) + mu1 * (2.0 * dd + ss));
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (k < ne && q == 0) out[e0 + k] = scale[e0 + k] * v;
 }
 
 // ---------------------------------------------------------------------------
@@ -1099,11 +1179,9 @@ int assemble_system(mg_problem *p, const double *d_X, double *d_R, bool want_jac
             lame_3d(p->mat.nu, lam1, mu1);
             for (int c = 0; c < p->n_colors; c++) {
                 int64_t cnt = p->color_ptr[c + 1] - p->color_ptr[c];
-                unsigned grid = blocks_for(cnt, kWarpsPerBlock);
-                hex8_kernel<0><<<grid, 256, 0, p->stream>>>(
-                    p->d_coords, p->d_conn, p->d_color_elems + p->color_ptr[c], 0, cnt, p->d_E,
-                    p->nodal_design ? p->d_Eq : nullptr, lam1, mu1, p->A.rowptr, p->d_emap, p->A.vals,
-                    nullptr, nullptr, nullptr, nullptr, nullptr, st);
+                hex8_scatter_kernel<<<blocks_for(cnt, kGlBlockEl), kGlBlock, 0, p->stream>>>(
+                    p->d_coords, p->d_conn, p->d_color_elems + p->color_ptr[c], cnt, p->d_E,
+                    p->nodal_design ? p->d_Eq : nullptr, lam1, mu1, p->A.rowptr, p->d_emap, p->A.vals, st);
                 MG_CUDA_TRY(cudaGetLastError());
             }
         } else {
@@ -1253,9 +1331,9 @@ int element_matrices(mg_problem *p, const double *d_X, int64_t first, int64_t co
     if (p->physics == MG_PHYSICS_ELASTICITY_HEX8) {
         double lam1, mu1;
         lame_3d(p->mat.nu, lam1, mu1);
-        hex8_kernel<1><<<blocks_for(count, kWarpsPerBlock), 256, 0, p->stream>>>(
-            p->d_coords, p->d_conn, nullptr, first, count, p->d_E, p->nodal_design ? p->d_Eq : nullptr,
-            lam1, mu1, nullptr, nullptr, nullptr, d_Ke, nullptr, nullptr, nullptr, nullptr, st);
+        hex8_matrix_kernel<<<blocks_for(count, kWarpsPerBlock), 256, 0, p->stream>>>(
+            p->d_coords, p->d_conn, first, count, p->d_E, p->nodal_design ? p->d_Eq : nullptr, lam1, mu1, d_Ke,
+            st);
     } else if (p->physics == MG_PHYSICS_ELASTICITY_HEX8_NONLINEAR) {
         double lam1, mu1;
         lame_3d(p->mat.nu, lam1, mu1);
@@ -1293,9 +1371,8 @@ int elem_sensitivity(mg_problem *p, const double *d_X, const double *d_lambda, i
     if (p->physics == MG_PHYSICS_ELASTICITY_HEX8 && kind == MG_PARAM_DENSITY) {
         double lam1, mu1;
         lame_3d(p->mat.nu, lam1, mu1);
-        hex8_kernel<2><<<blocks_for(p->n_elems, kWarpsPerBlock), 256, 0, p->stream>>>(
-            p->d_coords, p->d_conn, nullptr, 0, p->n_elems, p->d_dE, nullptr, lam1, mu1, nullptr,
-            nullptr, nullptr, nullptr, d_lambda, d_X, p->d_fixed, d_out_elem, st);
+        hex8_energy_kernel<<<blocks_for(p->n_elems, kEnergyEl), kEnergyEl * 8, 0, p->stream>>>(
+            p->d_coords, p->d_conn, p->n_elems, p->d_dE, lam1, mu1, d_lambda, d_X, p->d_fixed, d_out_elem, st);
     } else if (p->physics == MG_PHYSICS_ELASTICITY_HEX8_NONLINEAR && kind == MG_PARAM_DENSITY) {
         // out[e] = dE_e lambda_e . f1_e(X)
         double lam1, mu1;
@@ -1334,9 +1411,8 @@ int assemble_param_residual(mg_problem *p, const double *d_X, int kind, int64_t 
         double lam1, mu1;
         lame_3d(p->mat.nu, lam1, mu1);
         if (p->physics == MG_PHYSICS_ELASTICITY_HEX8) {
-            hex8_kernel<1><<<1, 256, 0, p->stream>>>(p->d_coords, p->d_conn, nullptr, index, 1,
-                                                     p->d_dE, nullptr, lam1, mu1, nullptr, nullptr,
-                                                     nullptr, Ke, nullptr, nullptr, nullptr, nullptr, st);
+            hex8_matrix_kernel<<<1, 256, 0, p->stream>>>(p->d_coords, p->d_conn, index, 1, p->d_dE, nullptr,
+                                                         lam1, mu1, Ke, st);
             MG_CUDA_TRY(cudaGetLastError());
             elem_matvec_kernel<<<1, 32, 0, p->stream>>>(Ke, d_X, p->d_conn, index, 1, 8, 3, fe);
         } else {
@@ -1473,9 +1549,8 @@ int element_sensitivity(mg_problem *p, int64_t e, const double *d_sol, int kind,
         lame_3d(p->mat.nu, lam1, mu1);
         double *Ke = p->d_tmp2;  // 576 doubles
         if (p->physics == MG_PHYSICS_ELASTICITY_HEX8) {
-            hex8_kernel<1><<<1, 256, 0, p->stream>>>(p->d_coords, p->d_conn, nullptr, e, 1, p->d_dE,
-                                                     nullptr, lam1, mu1, nullptr, nullptr, nullptr, Ke,
-                                                     nullptr, nullptr, nullptr, nullptr, st);
+            hex8_matrix_kernel<<<1, 256, 0, p->stream>>>(p->d_coords, p->d_conn, e, 1, p->d_dE, nullptr, lam1,
+                                                         mu1, Ke, st);
             MG_CUDA_TRY(cudaGetLastError());
             elem_matvec_kernel<<<1, 32, 0, p->stream>>>(Ke, p->d_tmp, p->d_conn, e, 1, 8, 3, d_dfe);
         } else {

@@ -39,6 +39,12 @@
 namespace mg {
 namespace gl {
 
+// workspace of the linear-strain element (doubles; 488 = 3.9 KB)
+struct LinearWork {
+    double X[24], w[8], inv[8][9], g[8][8][3];
+    double wg[8][8][3];  // JxW (times the point's modulus, if it has one) g_a
+};
+
 // element workspace (doubles; 1,064 = 8.5 KB)
 struct Work {
     double X[24];         // node coordinates, node-major (3 a + d)
@@ -71,10 +77,10 @@ GL_HD void dref(int q, int a, double d[3]) {
     d[2] = az ? z : -z;
 }
 
-// item (q): Jacobian, JxW, inverse.  Returns false for a non-positive determinant.
-// (W: any workspace with X, w, inv.)
+// item (q): Jacobian, JxW, inverse into s.inv[at], s.w[at].  Returns false for a
+// non-positive determinant.  (W: any workspace with X, w, inv.)
 template <class W>
-GL_HD bool jacobian_item(W &s, int q) {
+GL_HD bool jacobian_at(W &s, int q, int at) {
     double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // J[i][j] = d x_j / d xi_i
     for (int a = 0; a < 8; a++) {
         double d[3];
@@ -94,9 +100,13 @@ GL_HD bool jacobian_item(W &s, int q) {
     iv[8] = J[0] * J[4] - J[1] * J[3];
     const double det = J[0] * iv[0] + J[1] * iv[3] + J[2] * iv[6];
     const double r = 1.0 / det;
-    for (int k = 0; k < 9; k++) s.inv[q][k] = iv[k] * r;
-    s.w[q] = det;
+    for (int k = 0; k < 9; k++) s.inv[at][k] = iv[k] * r;
+    s.w[at] = det;
     return det > 0.0;
+}
+template <class W>
+GL_HD bool jacobian_item(W &s, int q) {
+    return jacobian_at(s, q, q);
 }
 
 // item (q, a): physical gradient g_j = sum_k (d xi_k / d x_j) d phi / d xi_k
@@ -186,6 +196,25 @@ GL_HD void phase_tangent(const Work &s, int a, int b, double lam, double mu, dou
         const double m = mu * B[3 + i];
         K[i * 3 + j] = lam * T[i * 3 + j] + (mu * T[j * 3 + i] + m);
         K[j * 3 + i] = lam * T[j * 3 + i] + (mu * T[i * 3 + j] + m);
+    }
+}
+
+// item (node pair (a, b)) of the linear element: lam T + mu T^T + mu tr(T) I with
+// T = sum_qp JxW g_a (x) g_b
+GL_HD void linear_pair_item(const LinearWork &s, int a, int b, double lam, double mu, double K[9]) {
+    double T[9];
+    for (int k = 0; k < 9; k++) T[k] = 0.0;
+    for (int q = 0; q < 8; q++) {
+        const double *ga = s.wg[q][a], *gb = s.g[q][b];
+        for (int i = 0; i < 3; i++)
+            for (int j = 0; j < 3; j++) T[i * 3 + j] += ga[i] * gb[j];
+    }
+    const double mtr = mu * (T[0] + T[4] + T[8]);
+    for (int i = 0; i < 3; i++) {
+        K[i * 4] = (lam + mu) * T[i * 4] + mtr;
+        const int j = (i + 1) % 3;
+        K[i * 3 + j] = lam * T[i * 3 + j] + mu * T[j * 3 + i];
+        K[j * 3 + i] = lam * T[j * 3 + i] + mu * T[i * 3 + j];
     }
 }
 
