@@ -11,8 +11,9 @@
 //
 // Two layouts:
 //   * structured grids: the element centroids form a lattice, so the weights
-//     are one stencil of integer offsets; a kernel applies it with the per-point
-//     normalisation (which only differs near the boundary) precomputed;
+//     are one stencil of integer offsets, applied with the per-point normalisation
+//     (which only differs near the boundary) precomputed: with mirrored offsets
+//     folded together where it is a ball of cells, else one point per thread;
 //   * arbitrary points: the neighbour lists are found on the host with a
 //     bucket grid of cell size r and stored as a CSR matrix and its transpose;
 //     FP64 CSR products apply F and F^T.
@@ -79,6 +80,115 @@ __global__ void stencil_apply_kernel(StencilArgs a, const double *__restrict__ i
     }
 }
 
+// The same stencil where it is a ball of up to kFoldMax cells.  The weights depend on |a|, |b|, |c| only, so values at
+// mirrored offsets are added before they are multiplied: along x into F_a = v(x - a) +
+// v(x + a), along y into G_ab = F_a(y - b) + F_a(y + b), and the plane sums P_c = sum_ab
+// w_abc G_ab go to the outputs at z - c and z + c.  For a radius of 2.5 cells that is 32 FP64
+// operations a point instead of 81, on a GPU whose FP64 pipe (two DFMA per cycle and SM)
+// binds the filter.  A block of 32 x 4 points marches through a chunk of z planes; the
+// outputs still open sit in registers, the next plane is fetched while one is folded.
+// Microseconds at 128x64x64, one point per thread -> folded: radius 1.5 25 -> 25 (transpose
+// 43 -> 29), 2.5 86 -> 60 (166 -> 72), 3.5 184 -> 107 (358 -> 125); 32x16x16 with 2.5 cells 14.5 ->
+// 8.4 (16.6 -> 10.5).  Larger radii and uneven spacings keep the form above.
+constexpr int kFoldX = 32, kFoldY = 4, kFoldMax = 3;  // kFoldMax: most cells of the radius
+
+struct FoldWeights {
+    double w[(kFoldMax + 1) * (kFoldMax + 1) * (kFoldMax + 1)];  // [c][b][a]
+};
+
+// A: cells of the radius; D: the stencil is a^2 + b^2 + c^2 <= D (known to the compiler: with
+// a test per weight the sums became chains of single instructions, twice the time)
+template <int A, int D>
+__global__ void __launch_bounds__(kFoldX * kFoldY) stencil_fold_kernel(
+    int nx, int ny, int nz, int zc, const FoldWeights W, const double *__restrict__ inv_s,
+    const uint8_t *__restrict__ dv, const double *__restrict__ in, double *__restrict__ out, int transpose) {
+    constexpr int H = kFoldY + 2 * A, NR = (H + kFoldY - 1) / kFoldY;  // rows of a plane, per warp
+    __shared__ double F[2][A + 1][H][kFoldX];                          // F_0 = v; double-buffered
+    auto weight = [&](int c, int b, int a) { return W.w[(c * (kFoldMax + 1) + b) * (kFoldMax + 1) + a]; };
+    auto inside = [](int c, int b, int a) { return a * a + b * b + c * c <= D; };
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int x0 = blockIdx.x * kFoldX, y0 = blockIdx.y * kFoldY, z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+    const int x = x0 + tx, y = y0 + ty;
+    const bool own = x < nx && y < ny;
+    const int64_t plane = (int64_t)nx * ny, col = x + (int64_t)nx * y;
+    // a warp's rows: lane = x, and the row's 2 A halo points (A left, then A right) in lanes 0 .. 2 A - 1
+    const int xh = tx < A ? x0 - A + tx : x0 + kFoldX + tx - A;
+    const bool in_x = x < nx, in_h = tx < 2 * A && xh >= 0 && xh < nx;
+    auto value = [&](int64_t e) { return !transpose ? in[e] : (!dv || dv[e]) ? in[e] * inv_s[e] : 0.0; };
+    auto fetch = [&](int p, double (&v)[NR], double (&h)[NR]) {
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            const int r = ty + k * kFoldY, j = y0 - A + r;
+            const bool row = r < H && j >= 0 && j < ny && p >= 0 && p < nz;
+            const int64_t e = (int64_t)nx * j + plane * p;
+            v[k] = row && in_x ? value(e + x) : 0.0;
+            h[k] = row && in_h ? value(e + xh) : 0.0;
+        }
+    };
+    double acc[2 * A + 1], v[NR], h[NR];  // acc[j]: the output plane p - A + j
+#pragma unroll
+    for (int j = 0; j <= 2 * A; j++) acc[j] = 0.0;
+    fetch(z0 - A, v, h);
+    for (int p = z0 - A; p < z1 + A; p++) {
+        const bool live = p >= 0 && p < nz;  // uniform
+        // what the output completed by this plane needs, fetched before the arithmetic
+        const int z = p - A;
+        const bool emit = own && z >= z0;
+        const int64_t eo = emit ? col + plane * z : 0;
+        const bool is_dv = !emit || !dv || dv[eo];
+        const double so = emit && !transpose ? inv_s[eo] : 0.0, keep = emit && dv ? in[eo] : 0.0;
+        double(*Fp)[H][kFoldX] = F[p & 1];
+        if (live) {
+#pragma unroll
+            for (int k = 0; k < NR; k++) {
+                const int r = ty + k * kFoldY;
+                if (r >= H) break;  // whole warps
+                Fp[0][r][tx] = v[k];
+#pragma unroll
+                for (int a = 1; a <= A; a++) {
+                    // v(x - a): the halo's lane A + x - a where x < a; v(x + a) likewise
+                    const double l = __shfl_sync(0xffffffffu, v[k], (tx - a) & 31),
+                                 lh = __shfl_sync(0xffffffffu, h[k], (A + tx - a) & 31),
+                                 g = __shfl_sync(0xffffffffu, v[k], (tx + a) & 31),
+                                 gh = __shfl_sync(0xffffffffu, h[k], (A + tx + a - kFoldX) & 31);
+                    Fp[a][r][tx] = (tx < a ? lh : l) + (tx + a >= kFoldX ? gh : g);
+                }
+            }
+        }
+        if (p + 1 < z1 + A) fetch(p + 1, v, h);
+        __syncthreads();
+        if (live) {
+            double G[A + 1][A + 1];  // [b][a]
+#pragma unroll
+            for (int b = 0; b <= A; b++)
+#pragma unroll
+                for (int a = 0; a <= A; a++) {
+                    if (!inside(0, b, a)) continue;  // then no plane uses it
+                    G[b][a] = Fp[a][ty + A - b][tx];
+                    if (b) G[b][a] += Fp[a][ty + A + b][tx];
+                }
+#pragma unroll
+            for (int c = 0; c <= A; c++) {
+                // planes outside the chunk take nothing from this one
+                const bool below = p - c >= z0 && p - c < z1, above = c && p + c >= z0 && p + c < z1;
+                if (!(below || above)) continue;
+                double P = 0.0;
+#pragma unroll
+                for (int b = 0; b <= A; b++)
+#pragma unroll
+                    for (int a = 0; a <= A; a++)
+                        if (inside(c, b, a)) P = fma(weight(c, b, a), G[b][a], P);
+                if (below) acc[A - c] += P;
+                if (above) acc[A + c] += P;
+            }
+        }
+        if (emit) out[eo] = transpose ? (is_dv ? acc[0] : acc[0] + keep) : (is_dv ? acc[0] * so : keep);
+#pragma unroll
+        for (int j = 0; j < 2 * A; j++) acc[j] = acc[j + 1];
+        acc[2 * A] = 0.0;
+    }
+}
+
 // y_i = (pass_i ? x_i : 0) + sum_k vals_k x_cols_k (one warp per row)
 __global__ void csr_filter_kernel(int64_t n, const int64_t *__restrict__ rowptr, const int32_t *__restrict__ cols,
                                   const double *__restrict__ vals, const uint8_t *__restrict__ pass,
@@ -108,6 +218,8 @@ struct mg_filter {
     int64_t n = 0, nnz = 0;
     bool grid = false;
     StencilArgs st{};
+    FoldWeights fold{};
+    int fold_a = 0, fold_d = 0, fold_zc = 0;  // the folded form's shape (fold_a = 0: not used), planes per block
     int *d_ox = nullptr, *d_oy = nullptr, *d_oz = nullptr;
     double *d_w = nullptr, *d_inv_s = nullptr;
     uint8_t *d_dv = nullptr, *d_not_dv = nullptr;
@@ -141,6 +253,90 @@ int finish_create(mg_filter *f, const uint8_t *dv) {
     return MG_OK;
 }
 
+// z planes per block of the folded form.  A plane of a block takes the FP64 pipe for
+// kFoldCycles per warp instruction (counted from the stencil) and about kFoldLatency cycles
+// more before its results are there (barrier, shared memory, one chain of sums), which only
+// other blocks of the SM can fill; a halo plane is partial work.  The cheapest choice by that
+// model: 128x64x64 with 2.5 cells takes 16 planes, two blocks on most SMs.
+constexpr double kFoldCycles = 18.0, kFoldLatency = 2500.0;
+
+int fold_chunk(const mg_filter *f, int sms) {
+    const int A = f->fold_a, nz = f->st.nz;
+    int pairs = 0, products = 0;
+    for (int c = 0; c <= A; c++)
+        for (int b = 0; b <= A; b++)
+            for (int a = 0; a <= A; a++)
+                if (a * a + b * b + c * c <= f->fold_d) {
+                    products++;
+                    pairs += c == 0;
+                }
+    const double work = kFoldCycles * (A * (kFoldY + 2 * A) + kFoldY * (pairs - A - 1 + products + 2 * A + 2));
+    const int64_t tiles = (int64_t)((f->st.nx + kFoldX - 1) / kFoldX) * ((f->st.ny + kFoldY - 1) / kFoldY);
+    int best = 1;
+    double least = 1e300;
+    for (int zc = 1; zc <= nz; zc++) {
+        const int64_t rounds = (tiles * ((nz + zc - 1) / zc) + sms - 1) / sms;
+        const double cost = (zc + 1.2 * A) * std::max(rounds * work, work + kFoldLatency);
+        if (cost < least) {
+            least = cost;
+            best = zc;
+        }
+    }
+    return best;
+}
+
+template <int A, int D>
+void launch_fold(const mg_filter *f, const double *in, double *out, int transpose, cudaStream_t s) {
+    const StencilArgs &a = f->st;
+    const dim3 grid((a.nx + kFoldX - 1) / kFoldX, (a.ny + kFoldY - 1) / kFoldY, (a.nz + f->fold_zc - 1) / f->fold_zc);
+    stencil_fold_kernel<A, D><<<grid, dim3(kFoldX, kFoldY), 0, s>>>(a.nx, a.ny, a.nz, f->fold_zc, f->fold, f->d_inv_s,
+                                                                    f->d_dv, in, out, transpose);
+}
+
+// the squared radii (in cells) between which a ball of cells changes, up to kFoldMax cells
+constexpr int kFoldBalls[] = {1, 2, 3, 4, 5, 6, 8, 9, 10, 11, 12, 13, 14};
+
+void dispatch_fold(const mg_filter *f, const double *in, double *out, int transpose, cudaStream_t s) {
+    switch (f->fold_d) {
+        case 1: launch_fold<1, 1>(f, in, out, transpose, s); break;
+        case 2: launch_fold<1, 2>(f, in, out, transpose, s); break;
+        case 3: launch_fold<1, 3>(f, in, out, transpose, s); break;
+        case 4: launch_fold<2, 4>(f, in, out, transpose, s); break;
+        case 5: launch_fold<2, 5>(f, in, out, transpose, s); break;
+        case 6: launch_fold<2, 6>(f, in, out, transpose, s); break;
+        case 8: launch_fold<2, 8>(f, in, out, transpose, s); break;
+        case 9: launch_fold<3, 9>(f, in, out, transpose, s); break;
+        case 10: launch_fold<3, 10>(f, in, out, transpose, s); break;
+        case 11: launch_fold<3, 11>(f, in, out, transpose, s); break;
+        case 12: launch_fold<3, 12>(f, in, out, transpose, s); break;
+        case 13: launch_fold<3, 13>(f, in, out, transpose, s); break;
+        case 14: launch_fold<3, 14>(f, in, out, transpose, s); break;
+    }
+}
+
+// The folded form's shape for a stencil of offsets (a, b, c) with weights w, or none: the
+// offsets have to be exactly those of a ball of cells (2D grids: a disc).
+void plan_fold(mg_filter *f, const std::vector<int> &ox, const std::vector<int> &oy, const std::vector<int> &oz,
+               const std::vector<double> &w, bool flat) {
+    int far = 0;
+    for (size_t o = 0; o < w.size(); o++) far = std::max(far, ox[o] * ox[o] + oy[o] * oy[o] + oz[o] * oz[o]);
+    // 2D: the smallest ball whose disc holds the stencil (the planes above and below are empty)
+    for (int d : kFoldBalls) {
+        if (d < far) continue;
+        size_t count = 0;
+        for (int c = flat ? 0 : -kFoldMax; c <= (flat ? 0 : kFoldMax); c++)
+            for (int b = -kFoldMax; b <= kFoldMax; b++)
+                for (int a = -kFoldMax; a <= kFoldMax; a++) count += a * a + b * b + c * c <= d;
+        if (count != w.size()) continue;
+        f->fold_d = d;
+        f->fold_a = d < 4 ? 1 : d < 9 ? 2 : 3;
+        for (size_t o = 0; o < w.size(); o++)
+            if (ox[o] >= 0 && oy[o] >= 0 && oz[o] >= 0)
+                f->fold.w[(oz[o] * (kFoldMax + 1) + oy[o]) * (kFoldMax + 1) + ox[o]] = w[o];
+        return;
+    }
+}
+
 int run(mg_filter *f, const double *in, double *out, int transpose, cudaStream_t s) {
     static int sms = 0;
     if (!sms) {
@@ -148,7 +344,10 @@ int run(mg_filter *f, const double *in, double *out, int transpose, cudaStream_t
         MG_CUDA_TRY(cudaGetDevice(&dev));
         MG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     }
-    if (f->grid) {
+    if (f->grid && f->fold_a) {
+        if (!f->fold_zc) f->fold_zc = fold_chunk(f, sms);
+        dispatch_fold(f, in, out, transpose, s);
+    } else if (f->grid) {
         const unsigned g = std::min(blocks_for(f->n, 256), (unsigned)(8 * sms));
         stencil_apply_kernel<<<g, 256, 0, s>>>(f->st, f->d_inv_s, f->d_dv, in, out, transpose);
     } else {
@@ -219,6 +418,7 @@ int mg_filter_create_grid(int32_t nx, int32_t ny, int32_t nz, double hx, double 
     if ((rc = upload(&f->d_w, w.data(), w.size(), f->stream)) != MG_OK) return fail(rc);
     if ((rc = dev_alloc_n(&f->d_inv_s, (size_t)f->n)) != MG_OK) return fail(rc);
     f->st = StencilArgs{nx, ny, NZ, (int)w.size(), f->d_ox, f->d_oy, f->d_oz, f->d_w};
+    if (ny <= kFoldY * 65535 && NZ <= 65535) plan_fold(f, ox, oy, oz, w, NZ == 1);
     stencil_norm_kernel<<<std::min(blocks_for(f->n, 256), 4096u), 256, 0, f->stream>>>(f->st, f->d_inv_s);
     count_launches(1);
     if (cudaGetLastError() != cudaSuccess) return fail(MG_ECUDA);
