@@ -33,17 +33,17 @@ constexpr int kMaxLevels = 8;                  // multigrid levels per design
 constexpr int kBottomMaxLevels = 6;            // levels of a bottom chain (one-CTA or cluster kernel)
 constexpr int kCoarseDirectMax = 144;          // most dofs of a coarsest grid that is solved directly
 
-// Whether a grid gets a coarser level (ceil(n / 2) elements a side).  It does until
-// its dofs fit the direct coarse solve, or a side has fewer than three elements.  An
-// odd side counts as padded by one void element: the coarse grid reaches one fine
-// element beyond it, its moduli average the void in, and the same trilinear transfers
-// apply (fine nodes beyond the grid do not exist and are skipped).  Stopping at the
-// first odd side instead left e.g. 6x3x3 (under 48x24x24) or 45x23x19 (under 90x46x38)
-// to the Chebyshev smoother alone: 72 against 38 CG iterations and 9.1 against 5.1 ms
-// (48x24x24 to 1e-10), 449 against 42 and 63.0 against 8.5 ms (90x46x38 to 1e-9).
+// Whether a grid gets a coarser level (ceil(n / 2) elements a side): until its dofs fit the
+// direct coarse solve.  An odd side counts as padded by one void element: the coarse grid
+// reaches one fine element beyond it, its moduli average the void in, and the same trilinear
+// transfers apply (fine nodes beyond the grid do not exist and are skipped); a side of one
+// element stays one.  Stopping at the first odd side, or at fewer than four elements, leaves
+// e.g. 6x3x3 (under 48x24x24), 45x23x19 (under 90x46x38) or 20x2x2 to the Chebyshev smoother
+// alone: 72 against 38 CG iterations and 9.1 against 5.1 ms (48x24x24 to 1e-10), 449 against
+// 42 and 63.0 against 8.5 ms (90x46x38 to 1e-9), 432 against 57 and 34.0 against 4.7 ms
+// (40x4x4), 4,750 against 153 and 120 against 13 ms (31x17x2).
 inline bool mg_coarsens(int nx, int ny, int nz) {
-    const int side = nx < ny ? (nx < nz ? nx : nz) : (ny < nz ? ny : nz);
-    return side >= 3 && 3LL * (nx + 1) * (ny + 1) * (nz + 1) > kCoarseDirectMax;
+    return 3LL * (nx + 1) * (ny + 1) * (nz + 1) > kCoarseDirectMax;
 }
 
 // level table of the cluster bottom kernel (one chain, one cluster)

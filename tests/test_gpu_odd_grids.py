@@ -9,10 +9,10 @@ import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(4, 3, 3), (7, 3, 3), (9, 5, 4), (23, 13, 9), (33, 15, 17), (31, 17, 2)])
+@pytest.mark.parametrize("shape", [(4, 3, 3), (7, 3, 3), (9, 5, 4), (23, 13, 9), (33, 15, 17), (31, 17, 2), (40, 4, 4), (30, 5, 1)])
 def test_odd_grid_design_matches_the_oracle(shape):
     """Smallest grid with a coarse level, odd in one to three sides at one or more levels,
-    and a side too short to coarsen.  Mixed-form tolerances (1e-8 residual, 1e-6 results)."""
+    and sides of one and two elements.  Mixed-form tolerances (1e-8 residual, 1e-6 results)."""
     nx, ny, nz = shape
     rho = np.random.default_rng(21).uniform(0.01, 1.0, nx * ny * nz)
     o = M.default_opts(precision=M.MIXED_TF32X3, rtol=1e-8, inner_rtol=1e-2, timeout_s=300.0)
