@@ -809,14 +809,25 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
 // and 2w+1 of the kFEX x kFEY element plane around the owned nodes (lane = x;
 // halo elements are recomputed by the neighbouring tiles).  The node planes
 // (input, D^-1 and the per-mode node vectors) and the moduli plane arrive by
-// TMA two planes ahead into a four-slot ring.  Per element plane: gather the
-// corner values from the two node planes, apply the factored stiffness scaled
-// by E_e, then sum the corner results into the owned nodes: along x with a warp
-// shuffle (left element + right element), along y inside the thread (rows 2w,
-// 2w+1) or through shared memory (row 2w+1 with the next warp's row 2w+2),
-// along z through registers (the top corners of plane z-1 + the bottom corners
-// of plane z).  Every node's sum has the same fixed order (deterministic and
-// independent of the tiling).
+// TMA ahead of their use into a four-slot ring.
+//
+// The transform to sum/difference modes is a product of an x, y part, which
+// belongs to a node plane, and a z part, which joins two planes.  So each node
+// plane is gathered and transformed in x, y once, kept in registers, and met by
+// the next plane in the z stage of the element plane between them; on the way
+// back the z stage leaves a part for the plane below and one for the plane
+// above, the two parts of a node plane are added in mode space, and one inverse
+// x, y transform per node plane returns to the corners: two thirds of the
+// butterflies, half the gathers, shuffles and exchanges of a form that treats
+// each element plane by itself.  The corners are then summed into the owned
+// nodes: along x with a warp shuffle (left element + right element), along y
+// inside the thread (rows 2w, 2w+1) or through shared memory (row 2w+1 with the
+// next warp's row 2w+2).  Every node's sum has the same fixed order
+// (deterministic and independent of the tiling).  Issue-bound with 16 warps per
+// SM: 128 registers, no spills (D^-1 and the third plane are read behind the
+// plane's barrier: read before it they spilled, and MODE 6 took 144 us where it
+// takes 85).  MODE 2, 58 problems of 12.9 M dofs: 95 -> 84 us a launch; y = A x at
+// 128x64x64 13.9 -> 12.2 us, at 192x96x96 31.6 -> 27.3 us.
 constexpr int kFEX = 32, kFEY = 16;                // elements per tile plane
 constexpr int kFNX = kFEX - 1, kFNY = kFEY - 1;    // owned nodes per tile plane
 constexpr int kFPX = kFEX + 1, kFPY = kFEY + 1;    // tile node plane (with halo)
@@ -827,32 +838,38 @@ constexpr int kFBoxX = 104;                        // TMA node box: 104 floats (
 constexpr int kFPlaneF = 1792;                     // floats per node plane in the ring (7168 B, 128 B aligned)
 constexpr int kFBoxE = 36;                         // TMA moduli box: 36 elements x kFEY rows
 constexpr int kFModF = kFBoxE * kFEY;              // 576 floats
-constexpr int kFXch = 6 * kFThreads;               // row exchange: 6 floats per thread
+constexpr int kFXch = 3 * kFThreads;               // row exchange: 3 floats per thread
 static_assert(kFBoxX * kFPY <= kFPlaneF && kFBoxX >= 3 + 3 * kFPX && kFBoxE >= 3 + kFEX, "boxes");
 static_assert(kFThreads == 32 * (kFEY / 2) && kFEX == 32, "warp = element row pair, lane = x");
 // tensor maps per problem for this kernel: node vectors with the 104 x 17 x 1 box
 // and the moduli with the 36 x 16 x 1 box
-enum FacMap { kFMapMx = 0, kFMapMd, kFMapMy, kFMapMb, kFMapR, kFMapDinv, kFMapMr, kFMapE, kFacMaps };
-// node planes per ring slot: the input, D^-1 and (MODE 2 rhs, MODE 4 r, MODE 5 the iterate)
+enum FacMap { kFMapMx = 0, kFMapMd, kFMapMy, kFMapMb, kFMapR, kFMapDinv, kFMapMr, kFMapZ, kFMapE, kFacMaps };
+// node planes per ring slot: the input, D^-1 and (MODE 2, 5 rhs, MODE 4 r, MODE 6 the iterate)
 __host__ __device__ constexpr int fac_planes(int mode) { return mode == 3 ? 2 : 3; }
 __host__ __device__ constexpr int fac_slot(int mode) { return fac_planes(mode) * kFPlaneF + kFModF; }
 __host__ __device__ constexpr int fac_smem(int mode) { return (kFRing * fac_slot(mode) + 2 * kFXch) * 4 + 128; }
-// MODE 3: 77,696 B; MODE 2, 4, 5: 106,368 B: two CTAs per SM
+// MODE 3: 72,832 B; MODE 2, 4, 5, 6: 101,504 B: two CTAs per SM
 
 struct FacArgs {
     int in_map, b_map;  // tensor maps (FacMap) of the input and of the third node plane
-    float *y;           // MODE 2, 3: output; MODE 4, 5: the new direction
-    float *r, *xs;      // MODE 4, 5: Chebyshev residual and iterate
+    float *y;           // MODE 2, 3: output (MODE 2: nullable); MODE 4, 5: the new direction
+    float *z;           // MODE 2: D^-1 times the output (nullable)
+    float *r, *xs;      // MODE 4, 5: Chebyshev residual; MODE 4, 5, 6: iterate
     float c1, c2, inv_theta;
-    int x0_zero;        // MODE 5: the iterate starts at 0 (its plane is not loaded)
+    int x0_zero;        // MODE 5, 6: the iterate starts at 0
 };
 
-// MODE 2: y = rhs - A x.  MODE 3: y = A x.  (Both 0 where dinv = 0.)
+// MODE 2: y = rhs - A x, z = D^-1 y.  MODE 3: y = A x.  (All 0 where dinv = 0.)
 // MODE 4: one Chebyshev step on direction x = d: r -= A d; y = d' = c1 d +
 //         c2 D^-1 r; xs += d' (mg_cheb_next_kernel's sequence, fused).
-// MODE 5: the first two Chebyshev steps on rhs x = b: d = D^-1 b / theta,
+// MODE 5: the first two Chebyshev steps on rhs b from x = z = D^-1 b: d = z / theta,
 //         xs (+)= d, r = b - A d, y = d' = c1 d + c2 D^-1 r, xs += d'
 //         (mg_cheb_first_kernel's and mg_cheb_next_kernel's sequence, fused).
+// MODE 6: the same two steps when no third follows: only xs changes, and with
+//         D^-1 r = z - D^-1 A d the rhs is not needed either.
+// The producers of a rhs write z beside it (the CG update, the restriction, MODE 2):
+// formed here from b and D^-1 at every corner it took twice the shared loads of MODE 2 (a
+// batch of 58 problems, 12.9 M dofs: 159 us a launch against 85 us for MODE 6).
 // A TMA wait that exceeds its bound sets bit 4 of *err and ends the block.
 template <int MODE>
 __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
@@ -866,7 +883,7 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
     // slot k: [input plane | D^-1 plane | third plane (NP = 3) | moduli]
     auto plane_of = [&](int slot, int part) { return fsm + slot * fac_slot(MODE) + part * kFPlaneF; };
     auto mod_of = [&](int slot) { return fsm + slot * fac_slot(MODE) + NP * kFPlaneF; };
-    float(*sX)[6][kFThreads] = reinterpret_cast<float(*)[6][kFThreads]>(fsm + kFRing * fac_slot(MODE));
+    float(*sX)[3][kFThreads] = reinterpret_cast<float(*)[3][kFThreads]>(fsm + kFRing * fac_slot(MODE));
     const int tid = threadIdx.x, tx = tid & 31, w = tid >> 5;
     const uint32_t bar0 = smem_u32(&bars[0]);
     if (tid == 0)
@@ -883,7 +900,8 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
     uint32_t phase = 0;   // bit k: parity of slot k's next completion
     uint32_t issued = 0;  // bit k: a load into slot k is outstanding (thread 0)
     bool failed = false;
-    const bool third = MODE == 2 || MODE == 4 || (MODE == 5 && !A.x0_zero);
+    const bool third = MODE == 2 || MODE == 4 || MODE == 5 || (MODE == 6 && !A.x0_zero);
+    const float2 neg1 = make_float2(-1.0f, -1.0f);
     for (int ti = t_lo + blockIdx.x; ti < t_hi && !failed; ti += gridDim.x) {
         const MfCol T = tiles[ti];
         const MfProblem P = probs[T.prob];
@@ -930,77 +948,95 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
         }
         bool ok = arrive(0);
         ok = arrive(1) && ok;
-        float pt[2][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};  // top-corner sums of the previous plane
+        // the xy modes (q = mx + 2 my) of node plane p at the element pair: element A = rows
+        // 2w, 2w+1 of the plane in .x, B = rows 2w+1, 2w+2 in .y
+        auto plane_modes = [&](int p, float2 (&m)[3][4]) {
+            const float *n0 = plane_of(p % kFRing, 0) + ox;
+            float nv[3][2][3];  // [row 2w + 0..2][bx][c]
+#pragma unroll
+            for (int r3 = 0; r3 < 3; r3++)
+#pragma unroll
+                for (int bx = 0; bx < 2; bx++) {
+                    const int o = (2 * w + r3) * kFBoxX + 3 * (tx + bx);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) nv[r3][bx][c] = n0[o + c];
+                }
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float2 sx[2], dx[2];  // [by]
+#pragma unroll
+                for (int by = 0; by < 2; by++) {
+                    const float2 lo = make_float2(nv[by][0][c], nv[by + 1][0][c]);
+                    const float2 hi = make_float2(nv[by][1][c], nv[by + 1][1][c]);
+                    sx[by] = __fadd2_rn(lo, hi);
+                    dx[by] = __ffma2_rn(lo, neg1, hi);  // hi - lo
+                }
+                m[c][0] = __fadd2_rn(sx[0], sx[1]);
+                m[c][1] = __fadd2_rn(dx[0], dx[1]);
+                m[c][2] = __ffma2_rn(sx[0], neg1, sx[1]);
+                m[c][3] = __ffma2_rn(dx[0], neg1, dx[1]);
+            }
+        };
+        float2 low[3][4], car[3][4];  // modes of node plane s; the top-face results of element plane s - 1 on it
+        plane_modes(0, low);
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) car[c][q] = make_float2(0.0f, 0.0f);
         int64_t g1 = P.dof_off + ((int64_t)(z0 - 1) * P.NY + gy1) * P.pitch + 3 * gx;
         for (int s = 0; s < S; s++) {
-            // plane s + 3 into the slot of plane s - 1, whose readers (the element phases
-            // of steps s - 2, s - 1 and the node-phase reads of step s - 1) are behind
-            // the barrier of step s - 1
-            if (tid == 0 && s + 3 <= S) {
-                issue(s + 3);
-                issued |= 1u << ((s + 3) % kFRing);
-            }
-            // element phase: corner values of the element pair, packed (A in .x, B in .y)
-            float2 v[3][8];
+            // element phase: the z stage of the transform joins node planes s and s + 1, the
+            // result is split again into the plane below (completing node plane s together
+            // with the carried results of the element plane below it) and the plane above
+            float2 node[3][4];
             {
-                const float *n0 = plane_of(s % kFRing, 0) + ox, *n1 = plane_of((s + 1) % kFRing, 0) + ox;
-                const float *m0 = plane_of(s % kFRing, 1) + ox, *m1 = plane_of((s + 1) % kFRing, 1) + ox;
-                float nv[2][3][2][3];  // [bz][row 2w + 0..2][bx][c]
+                float2 high[3][4], v[3][8];
+                plane_modes(s + 1, high);
 #pragma unroll
-                for (int bz = 0; bz < 2; bz++)
+                for (int c = 0; c < 3; c++)
 #pragma unroll
-                    for (int r3 = 0; r3 < 3; r3++)
-#pragma unroll
-                        for (int bx = 0; bx < 2; bx++) {
-                            const int o = (2 * w + r3) * kFBoxX + 3 * (tx + bx);
-#pragma unroll
-                            for (int c = 0; c < 3; c++) {
-                                float val = (bz ? n1 : n0)[o + c];
-                                if (MODE == 5) val = (bz ? m1 : m0)[o + c] * val * A.inv_theta;
-                                nv[bz][r3][bx][c] = val;
-                            }
-                        }
-#pragma unroll
-                for (int b = 0; b < 8; b++) {
-                    const int bx = b & 1, by = (b >> 1) & 1, bz = b >> 2;
-#pragma unroll
-                    for (int c = 0; c < 3; c++) v[c][b] = make_float2(nv[bz][by][bx][c], nv[bz][by + 1][bx][c]);
-                }
-            }
-            const float *Es = mod_of(s % kFRing) + oe + tx;
-            const float2 e2 = make_float2(Es[2 * w * kFBoxE], Es[(2 * w + 1) * kFBoxE]);
-            hex8_factored_apply2(K, e2, v);  // E = 0 (outside the grid) gives exact zeros
-            // along x: node x0 + tx = corner dx = 1 of this lane's element + dx = 0 of the next lane's
-            float2 xsum[3][2][2];  // [c][by][bz]
-#pragma unroll
-            for (int c = 0; c < 3; c++)
-#pragma unroll
-                for (int by = 0; by < 2; by++)
-#pragma unroll
-                    for (int bz = 0; bz < 2; bz++) {
-                        const float2 lo = v[c][2 * by + 4 * bz], hi = v[c][1 + 2 * by + 4 * bz];
-                        float2 nb;
-                        nb.x = __shfl_down_sync(0xffffffffu, lo.x, 1);
-                        nb.y = __shfl_down_sync(0xffffffffu, lo.y, 1);
-                        xsum[c][by][bz] = __fadd2_rn(hi, nb);
+                    for (int q = 0; q < 4; q++) {
+                        v[c][q] = __fadd2_rn(low[c][q], high[c][q]);
+                        v[c][q + 4] = __ffma2_rn(low[c][q], neg1, high[c][q]);
+                        low[c][q] = high[c][q];
                     }
-            // along y: row 2w of this warp (element 2w at by = 0) goes to the warp above
+                const float *Es = mod_of(s % kFRing) + oe + tx;
+                const float2 e2 = make_float2(Es[2 * w * kFBoxE], Es[(2 * w + 1) * kFBoxE]);
+                hex8_factored_khat2(K, e2, v);  // E = 0 (outside the grid) gives exact zeros
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        // mode 0 is zero
+                        const float2 down = q ? __ffma2_rn(v[c][q + 4], neg1, v[c][q]) : __fmul2_rn(v[c][4], neg1);
+                        const float2 up = q ? __fadd2_rn(v[c][q], v[c][q + 4]) : v[c][4];
+                        node[c][q] = __fadd2_rn(car[c][q], down);
+                        car[c][q] = up;
+                    }
+            }
+            // node plane s (s >= 1; the halo plane 0 is the tile below's): back to the corners
+            float2 xsum[3][2];  // [c][by]
             float(*X)[kFThreads] = sX[s & 1];
-#pragma unroll
-            for (int bz = 0; bz < 2; bz++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) X[bz * 3 + c][tid] = xsum[c][0][bz].x;
-            // node-phase inputs at the owned nodes of node plane s (its slot is refilled
-            // in the next step): the input in un, D^-1 in dv, the third plane in bv
-            float un[2][3], dv[2][3], bv[2][3];
-#pragma unroll
-            for (int rr = 0; rr < 2; rr++) {
-                const int o = ox + (2 * w + 1 + rr) * kFBoxX + 3 * (tx + 1);
+            if (s >= 1) {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    un[rr][c] = plane_of(s % kFRing, 0)[o + c];
-                    dv[rr][c] = plane_of(s % kFRing, 1)[o + c];
-                    bv[rr][c] = third ? plane_of(s % kFRing, 2)[o + c] : 0.0f;
+                    float2 f[2][2];  // [by][bx]
+                    const float2 y0 = __ffma2_rn(node[c][2], neg1, node[c][0]), y1 = __fadd2_rn(node[c][0], node[c][2]);
+                    const float2 d0 = __ffma2_rn(node[c][3], neg1, node[c][1]), d1 = __fadd2_rn(node[c][1], node[c][3]);
+                    f[0][0] = __ffma2_rn(d0, neg1, y0);
+                    f[0][1] = __fadd2_rn(y0, d0);
+                    f[1][0] = __ffma2_rn(d1, neg1, y1);
+                    f[1][1] = __fadd2_rn(y1, d1);
+                    // along x: node x0 + tx = corner dx = 1 of this lane's element + dx = 0 of the next lane's
+#pragma unroll
+                    for (int by = 0; by < 2; by++) {
+                        float2 nb;
+                        nb.x = __shfl_down_sync(0xffffffffu, f[by][0].x, 1);
+                        nb.y = __shfl_down_sync(0xffffffffu, f[by][0].y, 1);
+                        xsum[c][by] = __fadd2_rn(f[by][1], nb);
+                    }
+                    // along y: row 2w of this warp (element 2w at by = 0) goes to the warp above
+                    X[c][tid] = xsum[c][0].x;
                 }
             }
             // the next step's top plane (s + 2) has landed
@@ -1011,47 +1047,61 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
                 if (tid == 0) atomicOr(err, 4);
                 break;
             }
-            float nn[2][2][3];  // [row][bz][c]; node plane z0 - 1 + s gets its bottom-corner sums now
-#pragma unroll
-            for (int bz = 0; bz < 2; bz++)
+            // plane s + 3 into the slot of plane s - 1, whose readers (the element phases of
+            // steps s - 2, s - 1 and the node phase of step s - 1) are behind this barrier
+            if (tid == 0 && s + 3 <= S) {
+                issue(s + 3);
+                issued |= 1u << ((s + 3) % kFRing);
+            }
+            if (s >= 1) {
+                float nn[2][3];  // [row][c]: the operator at the owned nodes of node plane s
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
-                    nn[0][bz][c] = xsum[c][1][bz].x + xsum[c][0][bz].y;  // element 2w (by = 1) + 2w+1 (by = 0)
-                    nn[1][bz][c] = xsum[c][1][bz].y + (w < kFEY / 2 - 1 ? X[bz * 3 + c][tid + 32] : 0.0f);
+                    nn[0][c] = xsum[c][1].x + xsum[c][0].y;  // element 2w (by = 1) + 2w+1 (by = 0)
+                    nn[1][c] = xsum[c][1].y + (w < kFEY / 2 - 1 ? X[c][tid + 32] : 0.0f);
                 }
 #pragma unroll
-            for (int rr = 0; rr < 2; rr++) {
-                const bool own = rr ? own2 : own1;
-                if (own && s >= 1) {
+                for (int rr = 0; rr < 2; rr++) {
+                    const bool own = rr ? own2 : own1;
+                    if (!own) continue;
                     const int64_t g = g1 + (rr ? P.pitch : 0);
 #pragma unroll
                     for (int c = 0; c < 3; c++) {
-                        const float a = pt[rr][c] + nn[rr][0][c];
+                        const float a = nn[rr][c];
+                        // the input, D^-1 and the third plane at the node
+                        const int o = ox + (2 * w + 1 + rr) * kFBoxX + 3 * (tx + 1) + c;
+                        const float uu = plane_of(s % kFRing, 0)[o], dd = plane_of(s % kFRing, 1)[o];
+                        const float bb = third ? plane_of(s % kFRing, 2)[o] : 0.0f;
                         if (MODE == 2) {
-                            A.y[g + c] = dv[rr][c] == 0.0f ? 0.0f : bv[rr][c] - a;
+                            const float v = dd == 0.0f ? 0.0f : bb - a;
+                            if (A.y) A.y[g + c] = v;
+                            if (A.z) A.z[g + c] = dd * v;
                         } else if (MODE == 3) {
-                            A.y[g + c] = dv[rr][c] == 0.0f ? 0.0f : a;
+                            A.y[g + c] = dd == 0.0f ? 0.0f : a;
                         } else if (MODE == 4) {
-                            const float rv = bv[rr][c] - (dv[rr][c] == 0.0f ? 0.0f : a);
-                            const float dn2 = fmaf(A.c1, un[rr][c], A.c2 * dv[rr][c] * rv);
+                            const float rv = bb - (dd == 0.0f ? 0.0f : a);
+                            const float dn2 = fmaf(A.c1, uu, A.c2 * dd * rv);
                             A.r[g + c] = rv;
                             A.y[g + c] = dn2;
                             A.xs[g + c] += dn2;
                         } else {
-                            // d = D^-1 b / theta at the node, its iterate, residual and next direction
-                            const float dd = dv[rr][c], bb = un[rr][c];
-                            const float d0 = dd * bb * A.inv_theta;
-                            const float xv = A.x0_zero ? d0 : bv[rr][c] + d0;
-                            const float rv = bb - (dd == 0.0f ? 0.0f : a);
-                            const float dn2 = fmaf(A.c1, d0, A.c2 * dd * rv);
-                            A.r[g + c] = rv;
-                            A.y[g + c] = dn2;
-                            A.xs[g + c] = xv + dn2;
+                            // the input is z: a is A z, so A d = a / theta
+                            const float d0 = uu * A.inv_theta;
+                            float dr;  // D^-1 r
+                            if (MODE == 5) {
+                                const float rv = dd == 0.0f ? bb : fmaf(-A.inv_theta, a, bb);
+                                A.r[g + c] = rv;
+                                dr = dd * rv;
+                            } else {
+                                dr = fmaf(-A.inv_theta * dd, a, uu);
+                            }
+                            const float dn2 = fmaf(A.c1, d0, A.c2 * dr);
+                            if (MODE == 5) A.y[g + c] = dn2;
+                            const float x0 = A.x0_zero ? 0.0f : MODE == 5 ? A.xs[g + c] : bb;
+                            A.xs[g + c] = x0 + d0 + dn2;
                         }
                     }
                 }
-#pragma unroll
-                for (int c = 0; c < 3; c++) pt[rr][c] = nn[rr][1][c];
             }
             g1 += plane_stride;
         }
@@ -1066,8 +1116,8 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
 // ---------------------------------------------------------------- vector phase
 // x += alpha p; r -= alpha q (r stays 0 on Dirichlet dofs, D^-1 = 0 there);
 // z = D^-1 r; rz, rr -> beta, stop test.  float4 over 16-byte aligned chunks.
-// mg = 1: z comes from the multigrid V-cycle; only rr (stop test) is reduced
-// here and beta is formed after the V-cycle (mf_dot_rz_kernel).
+// mg = 1: z starts the multigrid V-cycle's first smoother; only rr (stop test) is
+// reduced here and beta is formed after the V-cycle (mf_dot_rz_kernel).
 __global__ void __launch_bounds__(kThreads) mf_update_kernel(
     const MfChunkDesc *__restrict__ chunks, int n_chunks, const MfProblem *__restrict__ probs,
     float *__restrict__ x, float *__restrict__ r, float *__restrict__ z,
@@ -1098,7 +1148,7 @@ __global__ void __launch_bounds__(kThreads) mf_update_kernel(
             const float4 zv = make_float4(dv.x * rv.x, dv.y * rv.y, dv.z * rv.z, dv.w * rv.w);
             *reinterpret_cast<float4 *>(x + i) = xv;
             *reinterpret_cast<float4 *>(r + i) = rv;
-            if (!mg) *reinterpret_cast<float4 *>(z + i) = zv;
+            *reinterpret_cast<float4 *>(z + i) = zv;
             rz = fmaf(rv.x, zv.x, fmaf(rv.y, zv.y, fmaf(rv.z, zv.z, fmaf(rv.w, zv.w, rz))));
             rr = fmaf(rv.x, rv.x, fmaf(rv.y, rv.y, fmaf(rv.z, rv.z, fmaf(rv.w, rv.w, rr))));
         }
@@ -1241,10 +1291,12 @@ __global__ void __launch_bounds__(kThreads) mg_cheb_next_kernel(
 }
 
 // restriction (transpose of trilinear interpolation) into the coarse problems
-// plo..phi-1: mb_c[I] = sum_d w(d) my_f[2I + d], d in {-1,0,1}^3, w = prod (1 - |d|/2)
+// plo..phi-1: mb_c[I] = sum_d w(d) my_f[2I + d], d in {-1,0,1}^3, w = prod (1 - |d|/2);
+// z_c = D^-1 mb_c
 __global__ void __launch_bounds__(256) mg_restrict_kernel(const MfProblem *__restrict__ probs, int plo,
                                                           const MfState *states, const float *__restrict__ my,
-                                                          float *__restrict__ mb, const float *__restrict__ dinv) {
+                                                          float *__restrict__ mb, float *__restrict__ z,
+                                                          const float *__restrict__ dinv) {
     pdl_enter();
     const MfProblem C = probs[plo + blockIdx.y];
     if (states[C.root].done) return;
@@ -1276,7 +1328,9 @@ __global__ void __launch_bounds__(256) mg_restrict_kernel(const MfProblem *__res
                 const float w = (dz ? 0.5f : 1.0f) * (dy ? 0.5f : 1.0f) * (dx ? 0.5f : 1.0f);
                 out = fmaf(w, v[q][c], out);
             }
-            mb[o + c] = dinv[o + c] != 0.0f ? out : 0.0f;
+            const float dv = dinv[o + c];
+            mb[o + c] = dv != 0.0f ? out : 0.0f;
+            z[o + c] = dv * out;  // the smoother's start
         }
     }
 }
@@ -2718,12 +2772,13 @@ int fac_map_of(const MfBatch &b, const float *v) {
     if (v == b.mb) return kFMapMb;
     if (v == b.r) return kFMapR;
     if (v == b.mr) return kFMapMr;
+    if (v == b.z) return kFMapZ;
     return -1;
 }
 
 template <int MODE>
 void launch_fac(MfBatch &b, int lo, int hi, int sel, const FacArgs &a) {
-    if (a.in_map < 0 || ((MODE == 2 || MODE == 4) && a.b_map < 0)) {
+    if (a.in_map < 0 || ((MODE == 2 || MODE == 4 || MODE == 5) && a.b_map < 0)) {
         b.enqueue_error = MG_EINVAL;  // reported by the caller of the enqueue
         return;
     }
@@ -2733,12 +2788,13 @@ void launch_fac(MfBatch &b, int lo, int hi, int sel, const FacArgs &a) {
                                                                       b.fac_maps, b.states, a, b.err);
 }
 
+// y = A x (MODE 3) or rhs - A x (MODE 2; z, nullable: D^-1 y, the factored operator only)
 template <int MODE>
 void launch_level_op(MfBatch &b, bool fac, int prec, int l, int in_slot, const float *x, const float *rhs,
-                     float *y, int sel) {
+                     float *y, int sel, float *z = nullptr) {
     if (fac) {
         launch_fac<MODE>(b, b.lvl_fac_lo[l], b.lvl_fac_hi[l], sel,
-                         FacArgs{fac_map_of(b, x), rhs ? fac_map_of(b, rhs) : -1, y, nullptr, nullptr, 0.0f, 0.0f,
+                         FacArgs{fac_map_of(b, x), rhs ? fac_map_of(b, rhs) : -1, y, z, nullptr, nullptr, 0.0f, 0.0f,
                                  0.0f, 0});
     } else {
         ApplyArgs a{b.lvl_col_lo[l], b.lvl_col_hi[l], in_slot, 0, rhs, y, sel};
@@ -2777,6 +2833,7 @@ int configure_kernels() {
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(3)));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(4)));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(5)));
+    MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(6)));
     MG_CUDA_TRY(cudaFuncSetAttribute(mg_bottom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kBottomSmemMax));
     MG_CUDA_TRY(cudaFuncSetAttribute(mg_coarse_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3298,7 +3355,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     std::vector<CUtensorMap> fmaps((size_t)b.n_probs * kFacMaps);
     for (int pi = 0; pi < b.n_probs; pi++) {
         const MfProblem &P = b.h_probs[pi];
-        float *vecs[kFMapE] = {b.mx, b.md, b.my, b.mb, b.r, b.dinv, b.mr};
+        float *vecs[kFMapE] = {b.mx, b.md, b.my, b.mb, b.r, b.dinv, b.mr, b.z};
         for (int k = 0; k < kFMapE; k++)
             MG_TRY(make_map(enc, &fmaps[(size_t)pi * kFacMaps + k], vecs[k] + P.dof_off, 3 * (uint64_t)P.NX, P.NY,
                             P.NZ, (uint64_t)P.pitch * 4, (uint64_t)P.pitch * P.NY * 4, kFBoxX, kFPY, 1));
@@ -3460,7 +3517,7 @@ int mf_apply(MfBatch &b, int precision, const double *x_host, double *y_host, in
     MG_CUDA_TRY(cudaMemsetAsync(b.states, 0, b.n_probs * sizeof(MfState), b.stream));
     if (precision == MG_OPERATOR_FACTORED_FP32) {
         launch_fac<3>(b, P.fac_begin, P.fac_begin + P.fac_count, -1,
-                      FacArgs{kFMapMx, -1, b.my, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0});
+                      FacArgs{kFMapMx, -1, b.my, nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0});
     } else {
         ApplyArgs a{P.col_begin, P.col_begin + P.col_count, 4, 0, nullptr, b.my};
         launch_apply_prec<3>(b, precision, a);
@@ -3531,16 +3588,23 @@ long long enqueue_smooth(MfBatch &b, bool fac, int prec, int l, const float *rin
     const int clo = b.lvl_chunk_lo[l], chi = b.lvl_chunk_hi[l];
     const int grid = std::max(1, std::min(chi - clo, b.vec_grid));
     if (fac && deg >= 2) {
-        // fused: the first two steps in one launch (direction into md, which is
-        // never rin), then one launch per step, the direction alternating md / my
+        // fused, from z = D^-1 rin (in b.z): the first two steps in one launch, then one launch
+        // per step, the direction alternating md / my (md is never rin)
         const int lo = b.lvl_fac_lo[l], hi = b.lvl_fac_hi[l];
+        if (deg == 2) {
+            launch_fac<6>(b, lo, hi, sel,
+                          FacArgs{kFMapZ, kFMapMx, nullptr, nullptr, nullptr, b.mx, cc.c1[1], cc.c2[1], cc.inv_theta,
+                                  x0_zero});
+            return 1;
+        }
         launch_fac<5>(b, lo, hi, sel,
-                      FacArgs{fac_map_of(b, rin), kFMapMx, b.md, b.mr, b.mx, cc.c1[1], cc.c2[1], cc.inv_theta, x0_zero});
+                      FacArgs{kFMapZ, fac_map_of(b, rin), b.md, nullptr, b.mr, b.mx, cc.c1[1], cc.c2[1], cc.inv_theta,
+                              x0_zero});
         float *din = b.md, *dout = b.my;
         long long n = 1;
         for (int k = 2; k < deg; k++) {
             launch_fac<4>(b, lo, hi, sel,
-                          FacArgs{fac_map_of(b, din), kFMapMr, dout, b.mr, b.mx, cc.c1[k], cc.c2[k], 0.0f, 0});
+                          FacArgs{fac_map_of(b, din), kFMapMr, dout, nullptr, b.mr, b.mx, cc.c1[k], cc.c2[k], 0.0f, 0});
             std::swap(din, dout);
             n += 1;
         }
@@ -3588,7 +3652,7 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
         for (int pi = clo; pi < chi; pi++)
             maxnodes = std::max<int64_t>(maxnodes, (int64_t)b.h_probs[pi].NX * b.h_probs[pi].NY * b.h_probs[pi].NZ);
         dim3 grid(std::max(1u, std::min(blocks_for(maxnodes, 256), 4096u)), chi - clo);
-        launch_pdl(mg_restrict_kernel, grid, 256, 0, b.stream, b.probs, clo, b.states, b.my, b.mb, b.dinv);
+        launch_pdl(mg_restrict_kernel, grid, 256, 0, b.stream, b.probs, clo, b.states, b.my, b.mb, b.z, b.dinv);
         n += 2;
         if (own_coarsest(l)) n += enqueue_smooth(b, fac, prec, l, rin, 1, cdeg, cc, 1);
     }
@@ -3622,7 +3686,10 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
                 maxnodes = std::max<int64_t>(maxnodes, (int64_t)b.h_probs[pi].NX * b.h_probs[pi].NY * b.h_probs[pi].NZ);
         dim3 grid(std::max(1u, std::min(blocks_for(maxnodes, 256), 4096u)), fhi - flo);
         launch_pdl(mg_prolong_kernel, grid, 256, 0, b.stream, b.probs, flo, b.states, b.mx, b.dinv);
-        launch_level_op<2>(b, fac, prec, l, 4, b.mx, rin, b.my, 0);  // my = rin - A mx
+        // my = rin - A mx; the fused smoother starts from z = D^-1 my (and of degree 2 needs no more)
+        const bool from_z = fac && sdeg >= 2;
+        launch_level_op<2>(b, fac, prec, l, 4, b.mx, rin, from_z && sdeg == 2 ? nullptr : b.my, 0,
+                           from_z ? b.z : nullptr);
         n += 2 + enqueue_smooth(b, fac, prec, l, b.my, 0, sdeg, cs, 0);
     }
     return n;
