@@ -2332,22 +2332,40 @@ __global__ void mf_refine_kernel(const MfChunkDesc *__restrict__ chunks, int n_c
 }
 
 // after the refinement update: a stopped inner CG sends its problem back to the
-// FP64 residual, or ends it on a breakdown / NaN (one thread per problem)
-__global__ void mf_phase_kernel(MfState *states, int n_fine) {
+// FP64 residual, or ends it on a breakdown / NaN (one block).  LOOP: the last kernel of a
+// while-loop body; the loop goes on while a problem is unfinished, no wait has timed out
+// and fewer than `limit` bodies have run since the launch (loop[0]; loop[1] counts them all).
+constexpr int kPhaseThreads = 256;
+template <bool LOOP>
+__global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states, int n_fine,
+                                                                 cudaGraphConditionalHandle handle, int *loop,
+                                                                 int limit, const int *err) {
     pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_fine) return;
-    MfState *st = states + i;
-    if (st->phase != kPhaseCG || !st->done) return;
-    if (st->status != 0 && st->status != MG_ENOCONV) {
-        st->ref_status = st->status;
-        st->ref_done = 1;
-        st->phase = kPhaseFin;
-    } else {
-        st->refine += 1;
-        st->status = 0;
-        st->u_zero = 0;  // u has been corrected
-        st->phase = kPhaseResid;
+    int active = 0;
+    for (int i = threadIdx.x; i < n_fine; i += kPhaseThreads) {
+        MfState *st = states + i;
+        if (st->phase == kPhaseCG && st->done) {
+            if (st->status != 0 && st->status != MG_ENOCONV) {
+                st->ref_status = st->status;
+                st->ref_done = 1;
+                st->phase = kPhaseFin;
+            } else {
+                st->refine += 1;
+                st->status = 0;
+                st->u_zero = 0;  // u has been corrected
+                st->phase = kPhaseResid;
+            }
+        }
+        active |= st->phase != kPhaseFin;
+    }
+    if (LOOP) {
+        active = __syncthreads_or(active);
+        if (threadIdx.x == 0) {
+            const bool more = active && loop[0] + 1 < limit && *err == 0;
+            loop[0] = more ? loop[0] + 1 : 0;
+            loop[1] += 1;
+            cudaGraphSetConditional(handle, more ? 1u : 0u);
+        }
     }
 }
 
@@ -2883,19 +2901,6 @@ int make_map(EncodeTiledFn fn, CUtensorMap *m, void *base, uint64_t d0, uint64_t
     return MG_OK;
 }
 
-int read_states(MfBatch &b) {
-    MG_CUDA_TRY(cudaMemcpyAsync(b.states_host, b.states, b.n_probs * sizeof(MfState),
-                                cudaMemcpyDeviceToHost, b.stream));
-    MG_CUDA_TRY(cudaStreamSynchronize(b.stream));
-    int herr = 0;
-    MG_CUDA_TRY(cudaMemcpy(&herr, b.err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) {
-        set_error("tensor-core pipeline wait exceeded its bound (error flag %d)", herr);
-        return MG_ETIMEDOUT;
-    }
-    return MG_OK;
-}
-
 void launch_update(MfBatch &b, float *pnew, bool mg) {
     const int n0 = b.lvl_chunk_hi[0];
     launch_pdl(mf_update_kernel, std::max(1, std::min(n0, b.vec_grid)), kThreads, 0, b.stream, 
@@ -3316,7 +3321,9 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.f64, (size_t)dof));
     MG_TRY(dev_alloc_n(&b.brick_part, (size_t)2 * nb));  // operator partials | ||f||^2 partials
     MG_TRY(dev_alloc_n(&b.chunk_part, (size_t)2 * nc));
-    MG_TRY(dev_alloc_n(&b.err, 1));
+    MG_TRY(dev_alloc_n(&b.err, kErrWords));
+    MG_CUDA_TRY(cudaMallocHost(&b.err_host, kErrWords * sizeof(int)));
+    b.loop_bodies = 0;
     MG_TRY(dev_alloc_n(&b.diag_list, (size_t)b.n_probs + b.h_heads.size()));
     MG_TRY(dev_alloc_n(&b.sens_offs, (size_t)std::max(1, b.n_fine)));
     MG_CUDA_TRY(cudaMallocHost(&b.sens_offs_host, (size_t)std::max(1, b.n_fine) * sizeof(int64_t)));
@@ -3403,7 +3410,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         MG_CUDA_TRY(cudaMemcpyAsync(b.heads, b.h_heads.data(), b.h_heads.size() * sizeof(int),
                                     cudaMemcpyHostToDevice, s));
     MG_CUDA_TRY(cudaMemsetAsync(b.states, 0, b.n_probs * sizeof(MfState), s));
-    MG_CUDA_TRY(cudaMemsetAsync(b.err, 0, sizeof(int), s));
+    MG_CUDA_TRY(cudaMemsetAsync(b.err, 0, kErrWords * sizeof(int), s));
     MG_CUDA_TRY(cudaMemsetAsync(b.u64, 0, dof * 8, s));
     MG_CUDA_TRY(cudaMemsetAsync(b.r64, 0, dof * 8, s));
     MG_CUDA_TRY(cudaMemsetAsync(b.f64, 0, dof * 8, s));
@@ -3700,7 +3707,10 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
 //   FP64 residual + stop test (RESID) | inner CG start (INIT) |
 //   [multigrid z = M r, rz, beta] | p, q = A p, alpha | x, r, stop test |
 //   u += d of stopped inner solves | phase transitions.
-long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity) {
+// loop_end: this step ends the body of a while loop on that handle (nullable).
+constexpr int kLoopBodies = 64;  // bodies of one loop launch at most: the host looks at the clock between launches
+long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
+                       const cudaGraphConditionalHandle *loop_end = nullptr) {
     cudaStream_t s = b.stream;
     const int n0 = b.lvl_chunk_hi[0], nb0 = b.lvl_brick_hi[0];
     const int vg0 = std::max(1, std::min(n0, b.vec_grid));
@@ -3730,30 +3740,62 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity) {
         n += 2;
     }
     launch_pdl(mf_refine_kernel, vg0, kThreads, 0, s, b.chunks, n0, b.x, b.u64, b.states);
-    launch_pdl(mf_phase_kernel, (b.n_fine + 127) / 128, 128, 0, s, b.states, b.n_fine);
+    if (loop_end)
+        launch_pdl(mf_phase_kernel<true>, 1, kPhaseThreads, 0, s, b.states, b.n_fine, *loop_end, b.err + 1, kLoopBodies,
+                   b.err);
+    else
+        launch_pdl(mf_phase_kernel<false>, 1, kPhaseThreads, 0, s, b.states, b.n_fine, cudaGraphConditionalHandle{},
+                   nullptr, 0, nullptr);
     return n + 2;
 }
 
 // CUDA graph of `chunk` solver steps (even: the p0/p1 roles alternate per step),
-// cached per parameter set
-int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk) {
+// cached per parameter set; with `loop` the steps are the body of a while loop that the
+// device ends, else they run once per launch.  A solve to completion that returned to the
+// host after every two steps spent 20 us a round trip on it (16x8x8 2.60 -> 2.24 ms looped,
+// 48x24x24 4.64 -> 4.26, 128x64x64 8.21 -> 7.83); the request loop launches single bodies,
+// between which it admits requests.
+int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop) {
     const std::vector<double> key = {(double)prm.precision, (double)chunk, (double)prm.mg,
                                      (double)prm.smooth_deg, (double)prm.coarse_deg, prm.rtol,
                                      prm.inner_rtol, (double)prm.max_iterations,
                                      (double)prm.max_refinements, (double)b.vec_grid,
-                                     (double)prm.mg_operator};
+                                     (double)prm.mg_operator, loop ? 1.0 : 0.0};
     if (b.graph && b.graph_key == key) return MG_OK;
     if (b.graph) {
         cudaGraphExecDestroy(b.graph);
         b.graph = nullptr;
     }
-    long long n = 0;
     cudaGraph_t g = nullptr;
+    MG_CUDA_TRY(cudaGraphCreate(&g, 0));
+    cudaGraph_t body = g;
+    cudaGraphConditionalHandle handle{};
+    cudaError_t e = cudaSuccess;
+    if (loop) {
+        e = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
+        if (e == cudaSuccess) {
+            cudaGraphNodeParams np = {};
+            np.type = cudaGraphNodeTypeConditional;
+            np.conditional.handle = handle;
+            np.conditional.type = cudaGraphCondTypeWhile;
+            np.conditional.size = 1;
+            cudaGraphNode_t node;
+            e = cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &np);
+            if (e == cudaSuccess) body = np.conditional.phGraph_out[0];
+        }
+    }
+    long long n = 0;
     b.enqueue_error = 0;
-    MG_CUDA_TRY(cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal));
-    for (int it = 0; it < chunk; it++) n += enqueue_step(b, prm, it & 1);
-    cudaError_t e = cudaStreamEndCapture(b.stream, &g);
+    if (e == cudaSuccess)
+        e = cudaStreamBeginCaptureToGraph(b.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        for (int it = 0; it < chunk; it++)
+            n += enqueue_step(b, prm, it & 1, loop && it == chunk - 1 ? &handle : nullptr);
+        cudaGraph_t captured = nullptr;
+        e = cudaStreamEndCapture(b.stream, &captured);  // the same graph as body
+    }
     if (e != cudaSuccess) {
+        cudaGraphDestroy(g);
         set_error("graph capture: %s", cudaGetErrorString(e));
         return MG_ECUDA;
     }
@@ -3782,7 +3824,7 @@ int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk) {
 //   V-cycle preconditioned);  u += ||r|| d.
 // The phases run on the device (enqueue_step); the host only relaunches the
 // step graph until every active problem has finished.
-int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm) {
+int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm, bool loop) {
     const bool use_mg = prm.mg && b.n_levels > 1;
     // launch shape of the vector kernels (captured in the graph)
     int dev = 0, sms = 0;
@@ -3798,7 +3840,7 @@ int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm) {
     const int chunk = prm.graph_chunk > 0 ? (prm.graph_chunk + 1) / 2 * 2 : (use_mg ? 2 : 16);
     MfSolveParams p2 = prm;
     p2.mg = use_mg ? 1 : 0;
-    return build_step_graph(b, p2, chunk);
+    return build_step_graph(b, p2, chunk, loop);
 }
 
 int mf_batch_reset_states(MfBatch &b) {
@@ -3834,32 +3876,24 @@ int mf_batch_activate(MfBatch &b, const std::vector<int> &level0, bool warm_star
     return MG_OK;
 }
 
-int mf_batch_step(MfBatch &b) {
-    if (!b.graph) {
-        set_error("mf_batch_step before mf_batch_prepare");
-        return MG_EINVAL;
-    }
-    MG_CUDA_TRY(cudaGraphLaunch(b.graph, b.stream));
-    count_launches(b.graph_launches);
-    return read_states(b);  // synchronises
-}
-
 int mf_batch_step_begin(MfBatch &b) {
     if (!b.graph) {
         set_error("mf_batch_step before mf_batch_prepare");
         return MG_EINVAL;
     }
-    if (!b.err_host) MG_CUDA_TRY(cudaMallocHost(&b.err_host, sizeof(int)));
     MG_CUDA_TRY(cudaGraphLaunch(b.graph, b.stream));
-    count_launches(b.graph_launches);
-    MG_CUDA_TRY(cudaMemcpyAsync(b.states_host, b.states, b.n_probs * sizeof(MfState), cudaMemcpyDeviceToHost,
+    // only the level-0 problems have a solver state
+    MG_CUDA_TRY(cudaMemcpyAsync(b.states_host, b.states, b.n_fine * sizeof(MfState), cudaMemcpyDeviceToHost,
                                 b.stream));
-    MG_CUDA_TRY(cudaMemcpyAsync(b.err_host, b.err, sizeof(int), cudaMemcpyDeviceToHost, b.stream));
+    MG_CUDA_TRY(cudaMemcpyAsync(b.err_host, b.err, kErrWords * sizeof(int), cudaMemcpyDeviceToHost, b.stream));
     return MG_OK;
 }
 
 int mf_batch_step_end(MfBatch &b) {
     MG_CUDA_TRY(cudaStreamSynchronize(b.stream));
+    // a loop launch reports the bodies it has run
+    count_launches(b.graph_launches * (b.graph_key.back() != 0.0 ? b.err_host[2] - b.loop_bodies : 1));
+    b.loop_bodies = b.err_host[2];
     if (*b.err_host) {
         set_error("tensor-core pipeline wait exceeded its bound (error flag %d)", *b.err_host);
         return MG_ETIMEDOUT;
@@ -3876,14 +3910,15 @@ int mf_batch_finish(MfBatch &b, int i) {
 
 int mf_batch_solve(MfBatch &b, const MfSolveParams &prm, bool warm_start) {
     const double t0 = wall_time();
-    MG_TRY(mf_batch_prepare(b, prm));
+    MG_TRY(mf_batch_prepare(b, prm, true));
     MG_TRY(mf_batch_reset_states(b));
     std::vector<int> act;
     for (int i = 0; i < b.n_fine; i++)
         if (!prm.active || prm.active[i]) act.push_back(i);
     MG_TRY(mf_batch_activate(b, act, warm_start));
     for (;;) {
-        MG_TRY(mf_batch_step(b));
+        MG_TRY(mf_batch_step_begin(b));
+        MG_TRY(mf_batch_step_end(b));
         bool all_done = true;
         for (int i : act) all_done &= b.states_host[i].phase == kPhaseFin;
         if (all_done) break;

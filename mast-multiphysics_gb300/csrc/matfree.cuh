@@ -125,6 +125,8 @@ struct MfState {
     unsigned cnt_apply, cnt_update, cnt_res, pad;
 };
 
+constexpr int kErrWords = 3;
+
 struct MfBatch {
     int n_probs = 0;
     int n_bricks = 0;
@@ -152,7 +154,8 @@ struct MfBatch {
     MfChunkDesc *chunks = nullptr;
     MfState *states = nullptr;
     MfState *states_host = nullptr;  // pinned
-    int *err_host = nullptr;         // pinned copy of *err (step_begin / step_end)
+    int *err_host = nullptr;         // pinned copy of err
+    int loop_bodies = 0;             // loop bodies run up to the last copy
     CUtensorMap *tmaps = nullptr;    // kMapsPerProblem per problem
     // element / node tables
     float *E32 = nullptr;
@@ -189,7 +192,7 @@ struct MfBatch {
     // FP64 refinement vectors (padded layout)
     double *u64 = nullptr, *r64 = nullptr, *f64 = nullptr;
     double *brick_part = nullptr, *chunk_part = nullptr;
-    int *err = nullptr;
+    int *err = nullptr;         // error flags of the bounded waits; loop bodies since a launch; in all
     int *diag_list = nullptr;  // problem list of a partial Jacobi update, then its direct chains
     int *stage_host = nullptr;  // pinned staging of diag_list
     int64_t *sens_offs = nullptr, *sens_offs_host = nullptr;  // dC/drho output offsets (device, pinned)
@@ -241,17 +244,16 @@ int mf_batch_set_bc(MfBatch &b, int i, const uint8_t *node_fix_host, const doubl
 int mf_batch_set_moduli(MfBatch &b, int i, const double *E_dev, const double *dE_dev);
 int mf_batch_solve(MfBatch &b, const MfSolveParams &prm, bool warm_start);
 // stepping interface (mf_batch_solve and the request loop are built on it):
-// prepare captures the step graph for prm; reset puts every problem at FIN;
-// activate starts the listed level-0 problems at the FP64 residual (their
-// Jacobi inverses are refreshed; u is zeroed unless warm_start); step runs one
-// graph launch and refreshes states_host (synchronising); finish returns a
-// FIN problem's status and zeroes u of a zero-load problem.
-int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm);
+// prepare captures the step graph for prm (loop: as a device-side while loop that runs
+// until every problem has finished); reset puts every problem at FIN; activate starts
+// the listed level-0 problems at the FP64 residual (their Jacobi inverses are refreshed;
+// u is zeroed unless warm_start); finish returns a FIN problem's status and zeroes u of a
+// zero-load problem.
+int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm, bool loop = false);
 int mf_batch_reset_states(MfBatch &b);
 int mf_batch_activate(MfBatch &b, const std::vector<int> &level0, bool warm_start);
-int mf_batch_step(MfBatch &b);
-// the same in two halves, so that several batches can run on the GPU at once:
-// begin launches the step graph and the state copy, end waits for them
+// one graph launch, in two halves so that several batches can run on the GPU at once:
+// begin launches the graph and the copy of the states, end waits for them (states_host)
 int mf_batch_step_begin(MfBatch &b);
 int mf_batch_step_end(MfBatch &b);
 int mf_batch_finish(MfBatch &b, int i);
