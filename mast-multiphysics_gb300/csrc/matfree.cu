@@ -194,6 +194,13 @@ __device__ __forceinline__ int64_t dof_index(const MfProblem &P, int gx, int gy,
 }
 
 // --------------------------------------------------------------- block helpers
+// The vector kernels end on FP64 sums that one thread or warp forms alone, and a dependent
+// FP64 addition takes about 75 cycles: the sums are trees of the least depth.
+static_assert(kThreads == 256, "sum_warps adds eight warps' sums");
+__device__ __forceinline__ double sum_warps(const double *sh) {
+    return ((sh[0] + sh[1]) + (sh[2] + sh[3])) + ((sh[4] + sh[5]) + (sh[6] + sh[7]));
+}
+
 __device__ __forceinline__ double block_sum(double v, double *sh) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -201,10 +208,7 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     __syncthreads();
     if (lane == 0) sh[w] = v;
     __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int i = 0; i < kThreads / 32; i++) s += sh[i];
-    return s;  // valid in thread 0
+    return threadIdx.x == 0 ? sum_warps(sh) : 0.0;  // valid in thread 0
 }
 
 // FP32 warp sums, FP64 across the block's warps; valid in thread 0
@@ -215,10 +219,7 @@ __device__ __forceinline__ double block_sum_f(float v, double *sh) {
     __syncthreads();
     if (lane == 0) sh[w] = (double)v;
     __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int i = 0; i < kThreads / 32; i++) s += sh[i];
-    return s;
+    return threadIdx.x == 0 ? sum_warps(sh) : 0.0;
 }
 
 // fixed-order sum of part[begin .. begin+count) over the block; valid in thread 0
@@ -226,14 +227,22 @@ __device__ __forceinline__ double ordered_sum(const double *part, int begin, int
     __shared__ double tree[kThreads];
     double s = 0.0;
     for (int i = threadIdx.x; i < count; i += kThreads) s += __ldcg(part + begin + i);
-    __syncthreads();
-    tree[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = kThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) tree[threadIdx.x] += tree[threadIdx.x + w];
+    if (count > 32) {
         __syncthreads();
+        tree[threadIdx.x] = s;
+        __syncthreads();
+        for (int w = kThreads / 2; w > 32; w >>= 1) {
+            if (threadIdx.x < w) tree[threadIdx.x] += tree[threadIdx.x + w];
+            __syncthreads();
+        }
+        if (threadIdx.x < 32) s = tree[threadIdx.x] + tree[threadIdx.x + 32];
     }
-    return tree[0];
+    if (threadIdx.x < 32) {
+        int w = 16;
+        while (w >= count && w > 0) w >>= 1;  // the lanes from count on hold zeros
+        for (; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+    }
+    return s;
 }
 
 __device__ __forceinline__ bool is_bad(double x) { return !isfinite(x); }
@@ -766,7 +775,7 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
                     last = __shfl_sync(0xffffffffu, last, 0);
                     if (last) {
                         __threadfence();
-                        // eight independent loads in flight per lane, added in column order
+                        // eight independent loads in flight per lane, added in a fixed order
                         double s = 0.0;
                         for (int c0 = lane; c0 < P.col_count; c0 += 32 * 8) {
                             double pv[8];
@@ -775,8 +784,7 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
                                 const int c = c0 + 32 * t;
                                 pv[t] = c < P.col_count ? __ldcg(col_part + P.col_begin + c) : 0.0;
                             }
-#pragma unroll
-                            for (int t = 0; t < 8; t++) s += pv[t];
+                            s += ((pv[0] + pv[1]) + (pv[2] + pv[3])) + ((pv[4] + pv[5]) + (pv[6] + pv[7]));
                         }
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -1123,11 +1131,13 @@ __global__ void __launch_bounds__(kThreads) mf_update_kernel(
     float *__restrict__ x, float *__restrict__ r, float *__restrict__ z,
     const float *__restrict__ p, const float *__restrict__ q, const float *__restrict__ dinv,
     MfState *states, double *__restrict__ chunk_part, int mg) {
-    pdl_enter();
+    pdl_trigger();
     __shared__ double red_sh[kThreads / 32];
     __shared__ int sh_last;
+    MfChunkDesc C = chunks[min((int)blockIdx.x, n_chunks - 1)];
+    pdl_wait();
     for (int ci = blockIdx.x; ci < n_chunks; ci += gridDim.x) {
-        const MfChunkDesc C = chunks[ci];
+        if (ci != (int)blockIdx.x) C = chunks[ci];
         MfState *st = states + C.prob;
         if (st->done) continue;
         const float alpha = (float)st->alpha;
@@ -1152,11 +1162,11 @@ __global__ void __launch_bounds__(kThreads) mf_update_kernel(
             rz = fmaf(rv.x, zv.x, fmaf(rv.y, zv.y, fmaf(rv.z, zv.z, fmaf(rv.w, zv.w, rz))));
             rr = fmaf(rv.x, rv.x, fmaf(rv.y, rv.y, fmaf(rv.z, rv.z, fmaf(rv.w, rv.w, rr))));
         }
-        const double srz = block_sum_f(rz, red_sh);
+        const double srz = mg ? 0.0 : block_sum_f(rz, red_sh);
         const double srr = block_sum_f(rr, red_sh);
         const MfProblem &P = probs[C.prob];
         if (threadIdx.x == 0) {
-            chunk_part[ci] = srz;
+            if (!mg) chunk_part[ci] = srz;
             chunk_part[n_chunks + ci] = srr;
             __threadfence();
             const unsigned t = atomicAdd(&st->cnt_update, 1u);
@@ -1164,7 +1174,7 @@ __global__ void __launch_bounds__(kThreads) mf_update_kernel(
         }
         __syncthreads();
         if (sh_last) {
-            const double trz = ordered_sum(chunk_part, P.chunk_begin, P.chunk_count);
+            const double trz = mg ? 0.0 : ordered_sum(chunk_part, P.chunk_begin, P.chunk_count);
             const double trr = ordered_sum(chunk_part + n_chunks, P.chunk_begin, P.chunk_count);
             if (threadIdx.x == 0) {
                 st->cnt_update = 0;
@@ -1191,11 +1201,13 @@ __global__ void __launch_bounds__(kThreads) mf_dot_rz_kernel(
     const MfChunkDesc *__restrict__ chunks, int n_chunks, const MfProblem *__restrict__ probs,
     const float *__restrict__ r, const float *__restrict__ z, MfState *states,
     double *__restrict__ chunk_part, int init) {
-    pdl_enter();
+    pdl_trigger();
     __shared__ double red_sh[kThreads / 32];
     __shared__ int sh_last;
+    MfChunkDesc C = chunks[min((int)blockIdx.x, n_chunks - 1)];
+    pdl_wait();
     for (int ci = blockIdx.x; ci < n_chunks; ci += gridDim.x) {
-        const MfChunkDesc C = chunks[ci];
+        if (ci != (int)blockIdx.x) C = chunks[ci];
         MfState *st = states + C.prob;
         if (st->done) continue;
         float rz = 0.0f;
@@ -1290,22 +1302,29 @@ __global__ void __launch_bounds__(kThreads) mg_cheb_next_kernel(
     }
 }
 
-// restriction (transpose of trilinear interpolation) into the coarse problems
-// plo..phi-1: mb_c[I] = sum_d w(d) my_f[2I + d], d in {-1,0,1}^3, w = prod (1 - |d|/2);
+// The transfers run over the lists of node blocks of the problems that take part (a grid of
+// the largest problem's blocks times the problems left most blocks of a mixed batch empty: 58
+// problems, prolongation into level 0 97 us a launch, 70 us from the list,
+// restriction 42 and 25).
+//
+// restriction (transpose of trilinear interpolation) into the coarse problems:
+// mb_c[I] = sum_d w(d) my_f[2I + d], d in {-1,0,1}^3, w = prod (1 - |d|/2);
 // z_c = D^-1 mb_c
-__global__ void __launch_bounds__(256) mg_restrict_kernel(const MfProblem *__restrict__ probs, int plo,
+__global__ void __launch_bounds__(kNodeBlk) mg_restrict_kernel(const MfProblem *__restrict__ probs,
+                                                          const MfNodeBlk *__restrict__ blks,
                                                           const MfState *states, const float *__restrict__ my,
                                                           float *__restrict__ mb, float *__restrict__ z,
                                                           const float *__restrict__ dinv) {
-    pdl_enter();
-    const MfProblem C = probs[plo + blockIdx.y];
-    if (states[C.root].done) return;
+    pdl_trigger();
+    const MfNodeBlk B = blks[blockIdx.x];
+    const MfProblem C = probs[B.prob];
     const MfProblem F = probs[C.fine];
-    if (F.bottom) return;  // inside a bottom chain: restricted by the bottom kernel
+    pdl_wait();
+    if (states[C.root].done) return;
     // one coarse node (3 dofs) per thread: its 27 fine neighbours' loads are all
     // issued before the sums (independent, predicated on the grid bounds)
-    const int nn = C.NX * C.NY * C.NZ;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += gridDim.x * blockDim.x) {
+    const int nn = C.NX * C.NY * C.NZ, n = B.node + threadIdx.x;
+    if (n < nn) {
         const int I = n % C.NX, JK = n / C.NX, J = JK % C.NY, K = JK / C.NY;
         const int64_t o = C.dof_off + ((int64_t)K * C.NY + J) * C.pitch + 3 * I;
         float v[27][3];
@@ -1335,19 +1354,22 @@ __global__ void __launch_bounds__(256) mg_restrict_kernel(const MfProblem *__res
     }
 }
 
-// prolongation (trilinear) from the coarse levels into the fine problems
-// plo..phi-1: mx_f[i] += sum_I w mx_c[I] (skips Dirichlet dofs and padding)
-__global__ void __launch_bounds__(256) mg_prolong_kernel(const MfProblem *__restrict__ probs, int plo,
+// prolongation (trilinear) from the coarse levels into the fine problems:
+// mx_f[i] += sum_I w mx_c[I] (skips Dirichlet dofs and padding)
+__global__ void __launch_bounds__(kNodeBlk) mg_prolong_kernel(const MfProblem *__restrict__ probs,
+                                                         const MfNodeBlk *__restrict__ blks,
                                                          const MfState *states, float *__restrict__ mx,
                                                          const float *__restrict__ dinv) {
-    pdl_enter();
-    const MfProblem F = probs[plo + blockIdx.y];
-    if (F.coarse < 0 || F.bottom || states[F.root].done) return;  // nothing to add here
+    pdl_trigger();
+    const MfNodeBlk B = blks[blockIdx.x];
+    const MfProblem F = probs[B.prob];
     const MfProblem C = probs[F.coarse];
+    pdl_wait();
+    if (states[F.root].done) return;
     // one fine node (3 dofs) per thread; its 1, 2, 4 or 8 coarse parents' loads are
     // issued together (the unused ones predicated off)
-    const int nn = F.NX * F.NY * F.NZ;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < nn; n += gridDim.x * blockDim.x) {
+    const int nn = F.NX * F.NY * F.NZ, n = B.node + threadIdx.x;
+    if (n < nn) {
         const int ii = n % F.NX, jk = n / F.NX, j = jk % F.NY, k = jk / F.NY;
         const int64_t o = F.dof_off + ((int64_t)k * F.NY + j) * F.pitch + 3 * ii;
         const float wx = (ii & 1) ? 0.5f : 1.0f, wy = (j & 1) ? 0.5f : 1.0f, wz = (k & 1) ? 0.5f : 1.0f;
@@ -2248,6 +2270,57 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
     }
 }
 
+// The kernels of the refinement phases act on the few problems that are in the phase; their
+// blocks walk only those problems' parts (chunks, bricks).  A walk over every part, each
+// behind its table and state reads, cost a batch of 58 problems about 1 us a part and block.
+//
+// Calls body(part index) for the parts [begin, end) that range(p) gives of the problems p < n
+// with in_phase(p), spread over the grid; every thread of the block (kThreads) calls it.
+// Every block numbers the parts for itself, so in_phase must not change while the kernel runs.
+template <typename InPhase, typename Range, typename Body>
+__device__ __forceinline__ void for_active_parts(int n, InPhase in_phase, Range range, Body body) {
+    if (n == 1) {  // no tables: they cost a single 16x8x8 or 48x24x24 solve 2 %
+        if (!in_phase(0)) return;
+        int begin, end;
+        range(0, begin, end);
+        for (int i = begin + blockIdx.x; i < end; i += gridDim.x) body(i);
+        return;
+    }
+    __shared__ int s_end[kThreads], s_begin[kThreads], s_warp[kThreads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int start = blockIdx.x;  // of this window's numbering
+    for (int p0 = 0; p0 < n; p0 += kThreads) {
+        const int p = p0 + threadIdx.x;
+        const bool in = p < n && in_phase(p);
+        if (!__syncthreads_or(in)) continue;  // also: the previous window's tables are no longer read
+        int begin = 0, end = 0;
+        if (in) range(p, begin, end);
+        int sum = end - begin;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += up;
+        }
+        if (lane == 31) s_warp[w] = sum;
+        __syncthreads();
+        for (int k = 0; k < w; k++) sum += s_warp[k];
+        s_end[threadIdx.x] = sum;
+        s_begin[threadIdx.x] = begin;
+        __syncthreads();
+        const int total = s_end[kThreads - 1];
+        for (; start < total; start += gridDim.x) {
+            int lo = 0, hi = kThreads - 1;  // the first problem whose parts end beyond start
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (s_end[mid] > start) hi = mid;
+                else lo = mid + 1;
+            }
+            body(s_begin[lo] + start - (lo ? s_end[lo - 1] : 0));
+        }
+        start -= total;
+    }
+}
+
 // inner CG start (problems in INIT): b = scale r64 (unit norm), x = 0, r = b,
 // z = D^-1 r, p0 = p1 = 0; moves the problem to CG
 __global__ void __launch_bounds__(kThreads) mf_inner_init_kernel(
@@ -2255,14 +2328,18 @@ __global__ void __launch_bounds__(kThreads) mf_inner_init_kernel(
     const double *__restrict__ r64, float *__restrict__ x, float *__restrict__ r,
     float *__restrict__ z, float *__restrict__ p0, float *__restrict__ p1,
     const float *__restrict__ dinv, MfState *states, double *__restrict__ chunk_part,
-    double inner_rtol2, int maxit) {
+    double inner_rtol2, int maxit, int n_fine) {
     pdl_enter();
     __shared__ double red_sh[kThreads / 32];
     __shared__ int sh_last;
-    for (int ci = blockIdx.x; ci < n_chunks; ci += gridDim.x) {
+    for_active_parts(n_fine, [&](int p) { return states[p].resid != 0; },
+                     [&](int p, int &begin, int &end) {
+                         begin = probs[p].chunk_begin;
+                         end = begin + probs[p].chunk_count;
+                     }, [&](int ci) {
         const MfChunkDesc C = chunks[ci];
         MfState *st = states + C.prob;
-        if (st->phase != kPhaseInit) continue;
+        if (st->phase != kPhaseInit) return;  // finished by its residual
         const double scale = st->scale;
         float rz = 0.0f, rr = 0.0f;
         for (int64_t i = C.begin + threadIdx.x; i < C.end; i += kThreads) {
@@ -2307,7 +2384,7 @@ __global__ void __launch_bounds__(kThreads) mf_inner_init_kernel(
             }
         }
         __syncthreads();
-    }
+    });
 }
 
 // a problem whose inner CG has just stopped and whose correction is usable
@@ -2317,18 +2394,20 @@ __device__ __forceinline__ bool inner_finished(const MfState *st) {
 
 // refinement update u += x / scale (x is 0 on Dirichlet dofs and padding) for
 // the problems whose inner CG has stopped
-__global__ void mf_refine_kernel(const MfChunkDesc *__restrict__ chunks, int n_chunks,
-                                 const float *__restrict__ x, double *__restrict__ u64,
-                                 const MfState *states) {
+__global__ void __launch_bounds__(kThreads) mf_refine_kernel(
+    const MfChunkDesc *__restrict__ chunks, const MfProblem *__restrict__ probs, int n_fine,
+    const float *__restrict__ x, double *__restrict__ u64, const MfState *states) {
     pdl_enter();
-    for (int ci = blockIdx.x; ci < n_chunks; ci += gridDim.x) {
+    for_active_parts(n_fine, [&](int p) { return inner_finished(states + p); },
+                     [&](int p, int &begin, int &end) {
+                         begin = probs[p].chunk_begin;
+                         end = begin + probs[p].chunk_count;
+                     }, [&](int ci) {
         const MfChunkDesc C = chunks[ci];
-        const MfState *st = states + C.prob;
-        if (!inner_finished(st)) continue;
-        const double inv = 1.0 / st->scale;
-        for (int64_t i = C.begin + threadIdx.x; i < C.end; i += blockDim.x)
+        const double inv = 1.0 / states[C.prob].scale;
+        for (int64_t i = C.begin + threadIdx.x; i < C.end; i += kThreads)
             u64[i] = fma((double)x[i], inv, u64[i]);
-    }
+    });
 }
 
 // after the refinement update: a stopped inner CG sends its problem back to the
@@ -2356,6 +2435,7 @@ __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states
                 st->phase = kPhaseResid;
             }
         }
+        st->resid = st->phase == kPhaseResid;
         active |= st->phase != kPhaseFin;
     }
     if (LOOP) {
@@ -2389,7 +2469,7 @@ __global__ void __launch_bounds__(kThreads) mf_residual64_kernel(
     const dfloat *__restrict__ Edf, const uint8_t *__restrict__ node_fix,
     const double *__restrict__ u64, const double *__restrict__ f64, const FacK<dfloat> K,
     double *__restrict__ r64, MfState *states, double *__restrict__ brick_part, double rtol2,
-    int max_ref) {
+    int max_ref, int n_fine) {
     pdl_enter();
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ double red_sh[kThreads / 32];
@@ -2397,11 +2477,14 @@ __global__ void __launch_bounds__(kThreads) mf_residual64_kernel(
     dfloat *su = reinterpret_cast<dfloat *>(smem + kOffU64);
     dfloat *sE = reinterpret_cast<dfloat *>(smem + kOffE64);
     dfloat(*sY)[kRGroupEl] = reinterpret_cast<dfloat(*)[kRGroupEl]>(smem + kOffY64);  // [b * 3 + c][element]
-    for (int bi = blockIdx.x; bi < n_bricks; bi += gridDim.x) {
+    for_active_parts(n_fine, [&](int p) { return states[p].resid != 0; },
+                     [&](int p, int &begin, int &end) {
+                         begin = probs[p].brick_begin;
+                         end = begin + probs[p].brick_count;
+                     }, [&](int bi) {
         const MfBrick br = bricks[bi];
         const MfProblem P = probs[br.prob];
         MfState *st = states + br.prob;
-        if (st->phase != kPhaseResid) continue;
         const bool need_ff = st->ff64 == 0.0;  // first residual of a solve: also ||f||^2
         const bool u_zero = st->u_zero != 0;    // cold start: r = f, no operator pass
         const int gx0 = br.bx * kBN, gy0 = br.by * kBN, gz0 = br.bz * kBN;
@@ -2520,7 +2603,7 @@ __global__ void __launch_bounds__(kThreads) mf_residual64_kernel(
             }
         }
         __syncthreads();
-    }
+    });
 }
 
 // Jacobi inverse of the mixed operator: 1 / sum_e E_e K0[3a+c][3a+c];
@@ -3098,6 +3181,11 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.h_fac_tiles.clear();
     std::vector<int64_t> level_count(b.n_levels + 1, 0);  // problems per multigrid level
     for (const MfProblem &P : b.h_probs) level_count[P.level]++;
+    int64_t dofs0 = 0;  // of the designs' own grids, which the vector kernels run over
+    for (const MfProblem &P : b.h_probs)
+        if (P.level == 0) dofs0 += (int64_t)((3 * (P.nx + 1) + 3) / 4 * 4) * (P.ny + 1) * (P.nz + 1);
+    int chunk = kMinChunk;
+    while (chunk < kMaxChunk && dofs0 > (int64_t)chunk * kWaveBlocks) chunk *= 2;
     for (size_t pi = 0; pi < b.h_probs.size(); pi++) {
         MfProblem &P = b.h_probs[pi];
         if (P.nx <= 0 || P.ny <= 0 || P.nz <= 0 || P.nx >= 32767 * kBN || P.ny >= 32767 * kBN ||
@@ -3164,13 +3252,13 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
                         b.h_fac_tiles.push_back(MfCol{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
         }
         P.chunk_begin = nc;
-        P.chunk_count = (int)((P.n_pad + kChunk - 1) / kChunk);
+        P.chunk_count = (int)((P.n_pad + chunk - 1) / chunk);
         for (int c = 0; c < P.chunk_count; c++) {
             MfChunkDesc C;
             C.prob = (int)pi;
             C.pad = 0;
-            C.begin = P.dof_off + (int64_t)c * kChunk;
-            C.end = std::min(P.dof_off + P.n_pad, C.begin + kChunk);
+            C.begin = P.dof_off + (int64_t)c * chunk;
+            C.end = std::min(P.dof_off + P.n_pad, C.begin + chunk);
             b.h_chunks.push_back(C);
         }
         nc += P.chunk_count;
@@ -3290,6 +3378,31 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
             }
         }
         if (b.bottom_cluster) break;
+    }
+    // node blocks of the transfers, by level: the problems restricted into (their fine level
+    // is not inside a bottom chain) and the problems prolonged into
+    {
+        std::vector<MfNodeBlk> blks;
+        auto add = [&](int pi) {
+            const MfProblem &P = b.h_probs[pi];
+            for (int n = 0; n < P.NX * P.NY * P.NZ; n += kNodeBlk) blks.push_back(MfNodeBlk{pi, n});
+        };
+        b.lvl_restrict_lo.clear(); b.lvl_restrict_hi.clear(); b.lvl_prolong_lo.clear(); b.lvl_prolong_hi.clear();
+        for (int l = 0; l < b.n_levels; l++) {
+            b.lvl_restrict_lo.push_back((int)blks.size());
+            for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++)
+                if (b.h_probs[pi].fine >= 0 && !b.h_probs[b.h_probs[pi].fine].bottom) add(pi);
+            b.lvl_restrict_hi.push_back((int)blks.size());
+            b.lvl_prolong_lo.push_back((int)blks.size());
+            for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++)
+                if (b.h_probs[pi].coarse >= 0 && !b.h_probs[pi].bottom) add(pi);
+            b.lvl_prolong_hi.push_back((int)blks.size());
+        }
+        MG_TRY(dev_alloc_n(&b.node_blks, std::max<size_t>(1, blks.size())));
+        if (!blks.empty())
+            MG_CUDA_TRY(cudaMemcpyAsync(b.node_blks, blks.data(), blks.size() * sizeof(MfNodeBlk),
+                                        cudaMemcpyHostToDevice, b.stream));
+        MG_CUDA_TRY(cudaStreamSynchronize(b.stream));  // blks is a host temporary
     }
     MG_TRY(dev_alloc_n(&b.coarse_off, std::max<size_t>(1, b.h_coarse_off.size())));
     MG_TRY(dev_alloc_n(&b.coarse_inv, (size_t)std::max<int64_t>(1, inv_floats)));
@@ -3430,7 +3543,7 @@ void mf_batch_free(MfBatch &b) {
     void *ptrs[] = {b.probs, b.bricks, b.chunks, b.states, b.tmaps, b.E32, b.Edf, b.dE64,
                     b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
-                    b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_part, b.Bop2, b.fac_tiles, b.fac_maps,
+                    b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_part, b.Bop2, b.fac_tiles, b.fac_maps, b.node_blks,
                     b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_chains, b.cl_k0, b.sens_offs};
     for (void *q : ptrs) dev_free(q);
     if (b.stage_host) cudaFreeHost(b.stage_host);
@@ -3654,12 +3767,9 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
         const float *rin = (l == 0) ? b.r : b.mb;
         n += enqueue_smooth(b, fac, prec, l, rin, 1, sdeg, cs, 0);
         launch_level_op<2>(b, fac, prec, l, 4, b.mx, rin, b.my, 0);  // my = rin - A mx
-        const int clo = b.lvl_prob_lo[l + 1], chi = b.lvl_prob_hi[l + 1];
-        int64_t maxnodes = 1;
-        for (int pi = clo; pi < chi; pi++)
-            maxnodes = std::max<int64_t>(maxnodes, (int64_t)b.h_probs[pi].NX * b.h_probs[pi].NY * b.h_probs[pi].NZ);
-        dim3 grid(std::max(1u, std::min(blocks_for(maxnodes, 256), 4096u)), chi - clo);
-        launch_pdl(mg_restrict_kernel, grid, 256, 0, b.stream, b.probs, clo, b.states, b.my, b.mb, b.z, b.dinv);
+        if (const int blks = b.lvl_restrict_hi[l + 1] - b.lvl_restrict_lo[l + 1])
+            launch_pdl(mg_restrict_kernel, blks, kNodeBlk, 0, b.stream, b.probs, b.node_blks + b.lvl_restrict_lo[l + 1],
+                       b.states, b.my, b.mb, b.z, b.dinv);
         n += 2;
         if (own_coarsest(l)) n += enqueue_smooth(b, fac, prec, l, rin, 1, cdeg, cc, 1);
     }
@@ -3686,13 +3796,9 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
     for (int l = L - 2; l >= 0; l--) {
         if (!any_level(l)) continue;
         const float *rin = (l == 0) ? b.r : b.mb;
-        const int flo = b.lvl_prob_lo[l], fhi = b.lvl_prob_hi[l];
-        int64_t maxnodes = 1;
-        for (int pi = flo; pi < fhi; pi++)
-            if (b.h_probs[pi].coarse >= 0)
-                maxnodes = std::max<int64_t>(maxnodes, (int64_t)b.h_probs[pi].NX * b.h_probs[pi].NY * b.h_probs[pi].NZ);
-        dim3 grid(std::max(1u, std::min(blocks_for(maxnodes, 256), 4096u)), fhi - flo);
-        launch_pdl(mg_prolong_kernel, grid, 256, 0, b.stream, b.probs, flo, b.states, b.mx, b.dinv);
+        if (const int blks = b.lvl_prolong_hi[l] - b.lvl_prolong_lo[l])
+            launch_pdl(mg_prolong_kernel, blks, kNodeBlk, 0, b.stream, b.probs, b.node_blks + b.lvl_prolong_lo[l],
+                       b.states, b.mx, b.dinv);
         // my = rin - A mx; the fused smoother starts from z = D^-1 my (and of degree 2 needs no more)
         const bool from_z = fac && sdeg >= 2;
         launch_level_op<2>(b, fac, prec, l, 4, b.mx, rin, from_z && sdeg == 2 ? nullptr : b.my, 0,
@@ -3719,10 +3825,10 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
     const int max_ref = prm.max_refinements > 0 ? prm.max_refinements : 30;
     launch_pdl(mf_residual64_kernel, std::max(1, std::min(nb0, b.apply_grid)), kThreads, kResidSmem, s, 
         b.probs, b.bricks, nb0, b.Edf, b.node_fix, b.u64, b.f64, b.facdf, b.r64, b.states,
-        b.brick_part, prm.rtol * prm.rtol, max_ref);
+        b.brick_part, prm.rtol * prm.rtol, max_ref, b.n_fine);
     launch_pdl(mf_inner_init_kernel, vg0, kThreads, 0, s, 
         b.chunks, n0, b.probs, b.r64, b.x, b.r, b.z, b.p0, b.p1, b.dinv, b.states, b.chunk_part,
-        prm.inner_rtol * prm.inner_rtol, maxit);
+        prm.inner_rtol * prm.inner_rtol, maxit, b.n_fine);
     long long n = 2;
     float *pnew = parity ? b.p0 : b.p1;
     if (use_mg) {
@@ -3739,7 +3845,7 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
         launch_update(b, pnew, false);                 // also z = D^-1 r, beta
         n += 2;
     }
-    launch_pdl(mf_refine_kernel, vg0, kThreads, 0, s, b.chunks, n0, b.x, b.u64, b.states);
+    launch_pdl(mf_refine_kernel, vg0, kThreads, 0, s, b.chunks, b.probs, b.n_fine, b.x, b.u64, b.states);
     if (loop_end)
         launch_pdl(mf_phase_kernel<true>, 1, kPhaseThreads, 0, s, b.states, b.n_fine, *loop_end, b.err + 1, kLoopBodies,
                    b.err);
@@ -3870,6 +3976,7 @@ int mf_batch_activate(MfBatch &b, const std::vector<int> &level0, bool warm_star
         memset(&h, 0, sizeof(MfState));
         h.done = 1;
         h.phase = kPhaseResid;  // its first residual pass also forms ||f||^2
+        h.resid = 1;
         h.u_zero = warm_start ? 0 : 1;
         MG_CUDA_TRY(cudaMemcpyAsync(b.states + i, &h, sizeof(MfState), cudaMemcpyHostToDevice, b.stream));
     }

@@ -21,7 +21,11 @@ constexpr int kBE = kBN + 1;
 constexpr int kBU = kBN + 2;
 constexpr int kNEL = kBE * kBE * kBE;          // 729 elements per brick
 constexpr int kNTILE = (kNEL + 127) / 128;     // 6 MMA tiles of 128 elements
-constexpr int kChunk = 4096;                   // dofs per vector-kernel chunk (four float4 per thread)
+// Dofs per vector-kernel chunk, one to four float4 per thread: the fewest that leave no more
+// chunks than one wave of blocks (8 on each of 152 SMs).  With 4096 throughout, the two
+// vector kernels of a 16x8x8 iteration ran on two blocks each; the rule and the shorter sums
+// took its solve and sensitivities from 3.02 to 2.81 ms, 64x32x32 from 7.52 to 7.03 ms.
+constexpr int kMinChunk = 1024, kMaxChunk = 4096, kWaveBlocks = 8 * 152;
 constexpr int kMapsPerProblem = 6;             // z, p0, p1, E, mg x, mg d (column operator boxes)
 // Column operator: a column owns kCX x kCY nodes in x, y and up to kCZ node
 // planes in z; it streams through its element planes (8 x 16 elements each,
@@ -97,6 +101,11 @@ struct MfCol {
     int16_t cx, cy, cz, pad;
 };
 
+constexpr int kNodeBlk = 256;  // nodes per block of the level transfers
+struct MfNodeBlk {
+    int prob, node;  // nodes [node, node + kNodeBlk) of the problem
+};
+
 struct MfChunkDesc {
     int prob;
     int pad;
@@ -120,8 +129,9 @@ struct MfState {
     double rr64, ff64, scale;
     int iter, done, status, maxit;
     int total_iter, refine, ref_done, ref_status;
-    int phase, first, u_zero, pad1; // first: the next dot_rz starts the inner CG (beta = 0);
-                                    // u_zero: u is still 0 (the residual is f)
+    int phase, first, u_zero, resid;  // first: the next dot_rz starts the inner CG (beta = 0);
+                                      // u_zero: u is still 0 (the residual is f); resid: this step
+                                      // forms the residual (set before the step, fixed within it)
     unsigned cnt_apply, cnt_update, cnt_res, pad;
 };
 
@@ -143,6 +153,8 @@ struct MfBatch {
     std::vector<int> lvl_col_lo, lvl_col_hi;
     double *col_part = nullptr;   // per-column partial of p.q
     uint32_t *Bop2 = nullptr;     // K0 as the column operator's four (dy, dz) B tiles
+    MfNodeBlk *node_blks = nullptr;  // of the level transfers: per level restricted into, prolonged into
+    std::vector<int> lvl_restrict_lo, lvl_restrict_hi, lvl_prolong_lo, lvl_prolong_hi;
     MfCol *fac_tiles = nullptr;   // tiles of the factored CUDA-core operator (cx, cy, cz)
     CUtensorMap *fac_maps = nullptr;  // its tensor maps per problem (node vectors, moduli)
     std::vector<MfCol> h_fac_tiles;
