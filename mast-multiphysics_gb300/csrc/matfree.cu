@@ -1196,11 +1196,24 @@ __global__ void __launch_bounds__(kThreads) mf_update_kernel(
     }
 }
 
-// rz = r . z after the V-cycle; init: beta = 0, else beta = rz / rz_old
+// r . z of the new residual and its preconditioned form: beta
+__device__ __forceinline__ void finish_rz(MfState *st, double rz) {
+    if (is_bad(rz) || !(rz > 0.0)) {
+        // a preconditioner that is not positive on r: stop with breakdown
+        st->status = is_bad(rz) ? MG_ENAN : MG_EBREAKDOWN;
+        st->done = 1;
+    } else {
+        st->beta = st->first ? 0.0 : rz / st->rz;
+        st->rz = rz;
+        st->first = 0;
+    }
+}
+
+// rz = r . z after the V-cycle
 __global__ void __launch_bounds__(kThreads) mf_dot_rz_kernel(
     const MfChunkDesc *__restrict__ chunks, int n_chunks, const MfProblem *__restrict__ probs,
     const float *__restrict__ r, const float *__restrict__ z, MfState *states,
-    double *__restrict__ chunk_part, int init) {
+    double *__restrict__ chunk_part) {
     pdl_trigger();
     __shared__ double red_sh[kThreads / 32];
     __shared__ int sh_last;
@@ -1230,15 +1243,7 @@ __global__ void __launch_bounds__(kThreads) mf_dot_rz_kernel(
             const double trz = ordered_sum(chunk_part, P.chunk_begin, P.chunk_count);
             if (threadIdx.x == 0) {
                 st->cnt_update = 0;
-                if (is_bad(trz) || !(trz > 0.0)) {
-                    // a preconditioner that is not positive on r: stop with breakdown
-                    st->status = is_bad(trz) ? MG_ENAN : MG_EBREAKDOWN;
-                    st->done = 1;
-                } else {
-                    st->beta = (init || st->first) ? 0.0 : trz / st->rz;
-                    st->rz = trz;
-                    st->first = 0;
-                }
+                finish_rz(st, trz);
             }
         }
         __syncthreads();
@@ -1879,19 +1884,25 @@ __global__ void __launch_bounds__(kCoarseInvThreads, 1) mg_coarse_inverse_kernel
 
 // ------------------------------------------------- bottom V-cycle on a cluster
 // The same bottom V-cycle as mg_bottom_kernel, spread over a thread-block
-// cluster of up to 16 CTAs (one cluster per chain) so that a single design's
-// chain can start at a larger level.  CTA r owns the nodes [r chunk, (r + 1) chunk)
-// of every level of the chain and keeps their x, b, r, d, y in its shared memory
-// (with D^-1 and the moduli of whole levels); a phase reads other CTAs' nodes
-// through distributed shared memory (mapa + ld.shared::cluster) and a cluster
-// barrier (release / acquire) separates the phases.  Global memory is touched only
-// at the start (rhs, tables) and at the end (the head's correction).  Every dof is
-// computed by one thread in a fixed order whatever the cluster size, so the result
-// does not depend on it.
+// cluster of up to 16 CTAs so that a single design's chain can start at a larger
+// level, for a small design at its own grid: the whole V-cycle and r.z are then
+// one kernel (16x8x8, solve with sensitivities: 2.80 -> 2.24 ms).  CTA r owns the
+// nodes [r chunk, (r + 1) chunk) of every level of the chain and keeps their x, b,
+// r, d, y in its shared memory, with D^-1 of the nodes and the moduli of the
+// elements around them; a phase reads other CTAs' nodes through distributed shared
+// memory (mapa + ld.shared::cluster) and a cluster barrier (release / acquire)
+// separates the phases.  Global memory is touched only at the start (rhs, tables)
+// and at the end (the head's correction).  Every dof is computed by one thread in a
+// fixed order whatever the cluster size, so the correction does not depend on it
+// (r.z of a chain from the own grid does, in its rounding).
 constexpr int kClusterThreads = 512;
-constexpr int kClusterMaxHeadNodes = 4096;
+// Nodes of the largest level that a chain may start at, the design's own grid included: up to here
+// the cluster's phases on 16 SMs beat the level kernels on all of them (us an iteration of single
+// designs, chain from the own grid / level by level: 1,377 nodes 57.5 / 72.1, 3,509 78.5 / 80.6,
+// 4,225 76.3 / 80.3, 4,913 77.6 / 83.0; 5,577 85.3 / 84.8).
+constexpr int kClusterMaxHeadNodes = 5000;
 constexpr int kClusterMax = 16;
-constexpr int kClusterK0 = 576 + 800;  // K0 and its regrouped copy (floats)
+constexpr int kClusterK0 = 576;  // K0 regrouped by the lanes' corners (floats)
 
 __device__ __forceinline__ unsigned cluster_ctarank() {
     unsigned r;
@@ -1923,82 +1934,106 @@ __device__ __forceinline__ void cl_ijk(const ClusterLevel &L, int n, int &i, int
     j = cl_div(rem, L.rNX);
     i = rem - j * L.NX;
 }
-// component c of node n of a vector whose slabs sit at `slab` in every CTA: a
-// plain load through the generic window, so that independent loads overlap
-__device__ __forceinline__ float cl_get(const float *slab, const ClusterLevel &L, int n, int c, int rank) {
+// address in the cluster's shared memory of word `off` of CTA `rank`'s dynamic shared memory, and a
+// load from it (volatile: the barriers between the phases order the loads, and loads that follow one
+// another are in flight together)
+__device__ __forceinline__ uint32_t cl_addr(const float *sm, int off, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(sm + off)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float cl_load(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+// component c of node n of the vector whose slabs sit at offset `slab` in every CTA
+__device__ __forceinline__ float cl_get(const float *sm, int slab, const ClusterLevel &L, int n, int c) {
     const int owner = cl_div(n, L.rchunk);
-    const float *p = slab + (n - owner * L.chunk) * 3 + c;
-    return owner == rank ? *p : *cl_map(p, owner);
+    return cl_load(cl_addr(sm, slab + (n - owner * L.chunk) * 3 + c, owner));
 }
 
 enum { kClX = 0, kClB, kClR, kClD, kClY };
-__device__ __forceinline__ float *cl_slab(float *sm, const ClusterLevel &L, int v) {
-    return sm + L.s_vec + v * 3 * L.chunk;
-}
+__device__ __forceinline__ int cl_slab(const ClusterLevel &L, int v) { return L.s_vec + v * 3 * L.chunk; }
 
 // One phase of the cluster V-cycle on level L: y = A in with eight lanes per node
 // (as bottom_apply), the elementwise update that follows it done by the lanes that
 // hold each dof's sum, so that the phase needs no second barrier:
-//   STEP 0, residual:             in = x;   r = b - y
-//   STEP 1, first smoothing step: in = D^-1 rin theta (formed while staging rin);
+//   step 0, residual:             in = x;   r = b - y
+//   step 1, first smoothing step: in = D^-1 rin theta (formed while staging rin);
 //           r0 = rin, d0 = D^-1 r0 theta, x0 = d0 or x + d0, then the step-1 update
-//   STEP 2, later smoothing step: in = d;   r -= y, d' = c1 d + c2 D^-1 r, x += d'
+//   step 2, later smoothing step: in = d;   r -= y, d' = c1 d + c2 D^-1 r, x += d'
 // (0 on Dirichlet dofs throughout).  The operand over the CTA's nodes and their
 // one-layer halo (nodes n0 - H .. n1 - 1 + H, H = NX NY + NX + 1) is first staged
 // in shared memory; no phase writes a slab that another CTA reads in it (the
 // callers rotate r, d and y).
 struct ClusterStep {
-    const float *in, *b, *r_src, *d_src;  // slabs (this CTA's shared memory)
-    float *r_dst, *d_dst, *x;
-    bool x0_zero;
+    int in, b, r_src, d_src, r_dst, d_dst, x;  // slabs (offsets in the CTA's shared memory)
+    bool x0_zero, staged;                      // staged: the operand is in place already
     float inv_theta, c1, c2;
 };
 
+// The phases are short (one to four nodes a lane) and follow one another through a cluster barrier, so
+// each is bound by its chain of dependent instructions, and what is the same in every phase is formed
+// once, before the kernel waits for its predecessor: a lane's corner, and with it its 3 x 24 row block
+// Kr of K0 (registers: 24 shared-memory loads a node and lane where there were 48); per level the
+// cluster addresses that the staging reads and each node's elements (shared memory).  Inlined once
+// per kind of phase: the V-cycle below is one loop over its phases.  With K0 and the operand both read
+// from shared memory and the indices formed in every phase, 90x46x38 (a chain from 3,432 nodes) took
+// 7.30 ms a solve with sensitivities where it takes 6.52, 64x32x32 (from 1,377) 7.21 and 6.91.
 template <int STEP>
-__device__ void cl_step(const ClusterLevel &L, float *sm, const float *sK, float *stage, const ClusterStep &S,
-                        int rank) {
-    const int nn = L.NX * L.NY * L.NZ;
+__device__ __forceinline__ void cl_step(const ClusterLevel &L, float *sm, const float (&Kr)[72], float *stage,
+                                        const ClusterStep &S, int rank) {
+    const int nn = L.NXY * L.NZ, NX = L.NX, NXY = L.NXY;
     const int n0 = rank * L.chunk, n1 = min(nn, n0 + L.chunk);
-    const int H = L.NX * L.NY + L.NX + 1;
+    const int H = NXY + NX + 1, nlo = max(0, n0 - H);
     const float *dinvL = sm + L.s_dinv, *EL = sm + L.s_E;
-    const int nlo = max(0, n0 - H);
-    if (n0 < n1) {
-        const int cnt = 3 * (min(nn - 1, n1 - 1 + H) - nlo + 1);
-        for (int t = threadIdx.x; t < cnt; t += kClusterThreads) {
-            const int n = nlo + t / 3, c = t - 3 * (t / 3);
-            const float v = cl_get(S.in, L, n, c, rank);
-            stage[t] = STEP == 1 ? dinvL[3 * n + c] * v * S.inv_theta : v;
+    if (n0 < n1 && !S.staged) {
+        const int cnt = 3 * (min(nn, n1 + H) - nlo), slab = 4 * (S.in - L.s_vec);
+        const int *addr = reinterpret_cast<const int *>(sm) + L.s_addr;
+        // up to three words a thread in flight together: one round trip through the cluster's network
+        for (int t = threadIdx.x; t < cnt; t += 3 * kClusterThreads) {
+            const int t1 = t + kClusterThreads, t2 = t1 + kClusterThreads;
+            float v0 = cl_load(addr[t] + slab), v1 = 0.0f, v2 = 0.0f;
+            if (t1 < cnt) v1 = cl_load(addr[t1] + slab);
+            if (t2 < cnt) v2 = cl_load(addr[t2] + slab);
+            stage[t] = STEP == 1 ? dinvL[t] * v0 * S.inv_theta : v0;
+            if (t1 < cnt) stage[t1] = STEP == 1 ? dinvL[t1] * v1 * S.inv_theta : v1;
+            if (t2 < cnt) stage[t2] = STEP == 1 ? dinvL[t2] * v2 * S.inv_theta : v2;
         }
     }
     __syncthreads();
-    const int corner = threadIdx.x & 7;
-    const int dx = corner & 1, dy = (corner >> 1) & 1, dz = corner >> 2;
-    const float4 *Kt = reinterpret_cast<const float4 *>(sK + 576 + 100 * corner_index(dx, dy, dz));
-    for (int base = n0; base < n1; base += kClusterThreads / 8) {
-        const int n = base + (threadIdx.x >> 3);
+    const int *elems = reinterpret_cast<const int *>(sm) + L.s_elem;
+    const int corner = threadIdx.x & 7, dx = corner & 1, dy = (corner >> 1) & 1, dz = corner >> 2;
+    const int corner_u = 3 * (dx + NX * dy + NXY * dz), corner_e = dx + L.nx * (dy + L.ny * dz);
+    const int own = n1 - n0;
+    for (int w = (threadIdx.x >> 5) * 4; w < own; w += kClusterThreads / 8) {  // four nodes a warp
+        const int n = w + ((threadIdx.x >> 3) & 3);
+        const int el = n < own ? elems[n] : 0;
+        const bool mine = n < own && corner < 3;
+        const int lo = mine ? 3 * n + corner : 0;
+        const float dn = dinvL[3 * (n0 - nlo) + lo];
+        const float rv0 = sm[(STEP == 0 ? S.b : S.r_src) + lo];
+        const float xv = STEP == 0 || (STEP == 1 && S.x0_zero) ? 0.0f : sm[S.x + lo];
+        const float dv0 = STEP == 2 ? sm[S.d_src + lo] : 0.0f;
         float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-        if (n < n1) {
-            int i, j, k;
-            cl_ijk(L, n, i, j, k);
-            const int ex = i - dx, ey = j - dy, ez = k - dz;
-            if (ex >= 0 && ey >= 0 && ez >= 0 && ex < L.nx && ey < L.ny && ez < L.nz) {
-                const float e = EL[ex + L.nx * (ey + L.ny * ez)];
-                const float *u0p = stage + 3 * (ex + L.NX * (ey + L.NY * ez) - nlo);
-                float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
+        if ((el >> corner) & 1) {
+            const float e = EL[(el >> 8) - corner_e];
+            const float *u0p = stage + 3 * (n0 - nlo + n) - corner_u;
+            float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
 #pragma unroll
-                for (int bc = 0; bc < 8; bc++) {
-                    int bx, by, bz;
-                    corner_bits(bc, bx, by, bz);
-                    const float *u = u0p + 3 * (bx + L.NX * (by + L.NY * bz));
-                    const float4 k0 = Kt[3 * bc], k1 = Kt[3 * bc + 1], k2 = Kt[3 * bc + 2];
-                    s0 = fmaf(k0.z, u[2], fmaf(k0.y, u[1], fmaf(k0.x, u[0], s0)));
-                    s1 = fmaf(k1.y, u[2], fmaf(k1.x, u[1], fmaf(k0.w, u[0], s1)));
-                    s2 = fmaf(k2.x, u[2], fmaf(k1.w, u[1], fmaf(k1.z, u[0], s2)));
-                }
-                a0 = e * s0;
-                a1 = e * s1;
-                a2 = e * s2;
+            for (int bc = 0; bc < 8; bc++) {
+                int bx, by, bz;
+                corner_bits(bc, bx, by, bz);
+                const float *u = u0p + 3 * (bx + NX * by + NXY * bz);
+                const float *kb = Kr + 9 * bc;
+                s0 = fmaf(kb[2], u[2], fmaf(kb[1], u[1], fmaf(kb[0], u[0], s0)));
+                s1 = fmaf(kb[5], u[2], fmaf(kb[4], u[1], fmaf(kb[3], u[0], s1)));
+                s2 = fmaf(kb[8], u[2], fmaf(kb[7], u[1], fmaf(kb[6], u[0], s2)));
             }
+            a0 = e * s0;
+            a1 = e * s1;
+            a2 = e * s2;
         }
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) {
@@ -2006,136 +2041,132 @@ __device__ void cl_step(const ClusterLevel &L, float *sm, const float *sK, float
             a1 += __shfl_xor_sync(0xffffffffu, a1, off);
             a2 += __shfl_xor_sync(0xffffffffu, a2, off);
         }
-        if (n < n1 && corner < 3) {
-            const int lo = 3 * (n - n0) + corner;
-            const float dn = dinvL[3 * n + corner];
+        if (mine) {
             const float y = dn == 0.0f ? 0.0f : (corner == 0 ? a0 : (corner == 1 ? a1 : a2));
             if (STEP == 0) {
-                S.r_dst[lo] = dn == 0.0f ? 0.0f : S.b[lo] - y;
+                sm[S.r_dst + lo] = dn == 0.0f ? 0.0f : rv0 - y;
             } else {
-                const float rv0 = S.r_src[lo];
-                float d0, x0;
-                if (STEP == 1) {
-                    d0 = dn * rv0 * S.inv_theta;
-                    x0 = S.x0_zero ? d0 : S.x[lo] + d0;
-                } else {
-                    d0 = S.d_src[lo];
-                    x0 = S.x[lo];
-                }
+                const float d0 = STEP == 1 ? dn * rv0 * S.inv_theta : dv0;
+                const float x0 = STEP == 1 ? (S.x0_zero ? d0 : xv + d0) : xv;
                 const float rv = rv0 - y;
                 const float dv = fmaf(S.c1, d0, S.c2 * dn * rv);
-                S.r_dst[lo] = rv;
-                S.d_dst[lo] = dv;
-                S.x[lo] = x0 + dv;
+                sm[S.r_dst + lo] = rv;
+                sm[S.d_dst + lo] = dv;
+                sm[S.x + lo] = x0 + dv;
             }
         }
     }
 }
 
-// x (+)= Chebyshev-Jacobi smoothing of degree deg for rhs rin (as bottom_smooth):
-// deg - 1 phases (one for deg = 1); r, d and y are rotated so that no phase
-// writes what other CTAs read in it
-__device__ void cl_smooth(const ClusterLevel &L, float *sm, const float *sK, float *stage, const float *rin,
-                          bool x0_zero, int deg, float inv_theta, const float *c1, const float *c2, int rank) {
-    float *x = cl_slab(sm, L, kClX), *r = cl_slab(sm, L, kClR), *d = cl_slab(sm, L, kClD),
-          *sp = cl_slab(sm, L, kClY);
-    if (deg <= 1) {
-        const int nn = L.NX * L.NY * L.NZ;
-        const int n0 = rank * L.chunk, nown = max(0, min(nn, n0 + L.chunk) - n0);
-        const float *dinvL = sm + L.s_dinv + 3 * n0;
-        for (int q = threadIdx.x; q < 3 * nown; q += kClusterThreads) {
-            const float rv = rin[q], dv = dinvL[q] * rv * inv_theta;
-            r[q] = rv;
-            d[q] = dv;
-            x[q] = x0_zero ? dv : x[q] + dv;
-        }
-        cluster_barrier();
-        return;
+// Chebyshev-Jacobi smoothing of degree 1 for rhs rin: x (+)= D^-1 rin theta, no phase
+__device__ __noinline__ void cl_smooth1(const ClusterLevel &L, float *sm, int rin, bool x0_zero,
+                                        float inv_theta, int rank) {
+    float *x = sm + cl_slab(L, kClX);
+    const int nn = L.NXY * L.NZ;
+    const int n0 = rank * L.chunk, nown = max(0, min(nn, n0 + L.chunk) - n0);
+    const float *dinvL = sm + L.s_dinv + 3 * (n0 - max(0, n0 - (L.NXY + L.NX + 1)));
+    for (int q = threadIdx.x; q < 3 * nown; q += kClusterThreads) {
+        const float dv = dinvL[q] * sm[rin + q] * inv_theta;
+        x[q] = x0_zero ? dv : x[q] + dv;
     }
-    ClusterStep S{};
-    S.x = x;
-    S.inv_theta = inv_theta;
-    S.x0_zero = x0_zero;
-    // step 1 reads rin at the neighbours: its residual goes to the spare slab when rin is r
-    S.in = rin;
-    S.r_src = rin;
-    S.r_dst = rin == r ? sp : r;
-    S.d_dst = d;
-    S.c1 = c1[1];
-    S.c2 = c2[1];
-    cl_step<1>(L, sm, sK, stage, S, rank);
     cluster_barrier();
-    if (rin == r) {
-        float *t = r; r = sp; sp = t;
-    }
-    for (int k = 2; k < deg; k++) {
-        // reads d at the neighbours: the new direction goes to the spare slab
-        S.in = d;
-        S.r_src = r;
-        S.r_dst = r;
-        S.d_src = d;
-        S.d_dst = sp;
-        S.c1 = c1[k];
-        S.c2 = c2[k];
-        cl_step<2>(L, sm, sK, stage, S, rank);
-        cluster_barrier();
-        float *t = d; d = sp; sp = t;
-    }
 }
 
-// r = b - A x (0 on Dirichlet dofs), one phase
-__device__ void cl_residual(const ClusterLevel &L, float *sm, const float *sK, float *stage, int rank) {
-    ClusterStep S{};
-    S.in = cl_slab(sm, L, kClX);
-    S.b = cl_slab(sm, L, kClB);
-    S.r_dst = cl_slab(sm, L, kClR);
-    cl_step<0>(L, sm, sK, stage, S, rank);
-    cluster_barrier();
+// restriction: cluster address of the residual at fine neighbour `lane` (< 27) of coarse node n, 0 if none
+__device__ __forceinline__ int cl_fine_addr(const float *sm, const ClusterLevel &F, const ClusterLevel &C, int n, int lane) {
+    int I, J, K;
+    cl_ijk(C, n, I, J, K);
+    const int ii = 2 * I + lane % 3 - 1, jj = 2 * J + lane / 3 % 3 - 1, kk = 2 * K + lane / 9 - 1;
+    if (lane >= 27 || ii < 0 || ii >= F.NX || jj < 0 || jj >= F.NY || kk < 0 || kk >= F.NZ) return 0;
+    const int nf = ii + F.NX * (jj + F.NY * kk), owner = cl_div(nf, F.rchunk);
+    return (int)cl_addr(sm, cl_slab(F, kClR) + 3 * (nf - owner * F.chunk), owner);
 }
 
 __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
-    const ClusterChain *__restrict__ chains, const MfState *states, const float *__restrict__ E32,
-    const float *__restrict__ dinv, const float *__restrict__ mb, float *__restrict__ mx,
-    const float *__restrict__ k0f, BottomCheb cc, int sdeg, int cdeg, const int64_t *__restrict__ coarse_off,
-    const float *__restrict__ coarse_inv, const int *__restrict__ coarse_ok) {
+    const ClusterChain *__restrict__ chain, MfState *states, const float *__restrict__ E32,
+    const float *__restrict__ dinv, const float *__restrict__ rhs, float *__restrict__ mx, bool from_root,
+    const float *__restrict__ k0f, const __grid_constant__ BottomCheb cc, int sdeg, int cdeg,
+    const int64_t *__restrict__ coarse_off, const float *__restrict__ coarse_inv, const int *__restrict__ coarse_ok) {
     // D^-1, the moduli and the coarse inverse were formed before this graph ran
     // (activation); they are loaded while the preceding kernel finishes, the
     // head's rhs and the solver state only after it
     pdl_trigger();
-    extern __shared__ __align__(16) float sm[];  // K0 tables, stage, per level: D^-1, E, slabs
-    __shared__ ClusterChain sc;
+    extern __shared__ __align__(16) float sm[];  // stage, per level: D^-1, E, slabs, tables
+    __shared__ double s_rz[kClusterMax], s_red[kClusterThreads / 32];
     const int csize = (int)cluster_nctarank(), rank = (int)cluster_ctarank();
-    const int chain = blockIdx.x / csize;
-    {
-        const int *src = reinterpret_cast<const int *>(chains + chain);
-        int *dst = reinterpret_cast<int *>(&sc);
-        for (int i = threadIdx.x; i < (int)(sizeof(ClusterChain) / 4); i += kClusterThreads) dst[i] = src[i];
-    }
-    for (int i = threadIdx.x; i < kClusterK0; i += kClusterThreads) sm[i] = k0f[i];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (in shared memory: read by level from the constant bank, the tables slowed every phase)
+    __shared__ ClusterChain ch;
+    for (int i = threadIdx.x; i < (int)(sizeof(ClusterChain) / 4); i += kClusterThreads)
+        reinterpret_cast<int *>(&ch)[i] = reinterpret_cast<const int *>(chain)[i];
     __syncthreads();
-    const int m = sc.m;
-    const float *sK = sm;
-    float *stage = sm + sc.s_stage;
-    // D^-1 and E of every level (compact order), the head's rhs over this CTA's nodes
+    const int m = ch.m;
+    int *smi = reinterpret_cast<int *>(sm);
+    // D^-1 and E of every level (compact order) as far as this CTA's phases read them: its
+    // nodes and their halo, the elements around its nodes.  Copied asynchronously: the round
+    // trips of all levels overlap (one after another they took 9 to 12 thousand cycles).
+    auto copy_word = [&](int off, const float *src) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(sm + off)), "l"(src) : "memory");
+    };
     for (int l = 0; l < m; l++) {
-        const ClusterLevel &L = sc.L[l];
-        const int nn = L.NX * L.NY * L.NZ, ne = L.nx * L.ny * L.nz;
-        for (int q = threadIdx.x; q < 3 * nn; q += kClusterThreads) {
-            const int n = q / 3, c = q - 3 * n;
-            const int i = n % L.NX, j = (n / L.NX) % L.NY, k = n / (L.NX * L.NY);
-            sm[L.s_dinv + q] = dinv[L.dof_off + ((int64_t)k * L.NY + j) * L.pitch + 3 * i + c];
+        const ClusterLevel &L = ch.L[l];
+        const int nn = L.NXY * L.NZ, H = L.NXY + L.NX + 1;
+        const int n0 = rank * L.chunk, n1 = min(nn, n0 + L.chunk), nlo = max(0, n0 - H);
+        if (n0 >= n1) continue;
+        const int cnt = 3 * (min(nn, n1 + H) - nlo);
+#pragma unroll 2
+        for (int t = threadIdx.x; t < cnt; t += kClusterThreads) {
+            const int n = nlo + t / 3, c = t - 3 * (t / 3);
+            int i, j, k;
+            cl_ijk(L, n, i, j, k);
+            const int idx = (k * L.NY + j) * L.pitch + 3 * i + c;
+            copy_word(L.s_dinv + t, dinv + L.dof_off + idx);
+            if (l == 0) smi[ch.s_idx + t] = idx;
+            const int owner = cl_div(n, L.rchunk);
+            smi[L.s_addr + t] = (int)cl_addr(sm, L.s_vec + 3 * (n - owner * L.chunk) + c, owner);
         }
-        for (int e = threadIdx.x; e < ne; e += kClusterThreads) {
-            const int ex = e % L.nx, ey = (e / L.nx) % L.ny, ez = e / (L.nx * L.ny);
-            sm[L.s_E + e] = E32[L.elem_off + ((int64_t)ez * L.ny + ey) * L.pitch_e + ex];
+        const int nxy = L.nx * L.ny;
+        const float rnx = 1.0f / (float)L.nx, rnxy = 1.0f / (float)nxy;  // exact quotients: fewer than 2^13 elements
+        const int e1 = nxy * min(L.nz, cl_div(n1 - 1, L.rNXY) + 1);
+        for (int e = nxy * max(0, cl_div(n0, L.rNXY) - 1) + threadIdx.x; e < e1; e += kClusterThreads) {
+            const int ez = cl_div(e, rnxy), er = e - ez * nxy, ey = cl_div(er, rnx), ex = er - ey * L.nx;
+            copy_word(L.s_E + e, E32 + L.elem_off + ((int64_t)ez * L.ny + ey) * L.pitch_e + ex);
+        }
+        for (int n = n0 + threadIdx.x; n < n1; n += kClusterThreads) {
+            // the element at corner 0 and which of the eight lie in the grid
+            int i, j, k;
+            cl_ijk(L, n, i, j, k);
+            const int mx = (i < L.nx ? 0x55 : 0) | (i > 0 ? 0xaa : 0);
+            const int my = (j < L.ny ? 0x33 : 0) | (j > 0 ? 0xcc : 0);
+            const int mz = (k < L.nz ? 0x0f : 0) | (k > 0 ? 0xf0 : 0);
+            smi[L.s_elem + n - n0] = (i + L.nx * (j + L.ny * k)) << 8 | (mx & my & mz);
+            if (l < m - 1) {  // its first parent among those this CTA stages, and which others it has
+                const ClusterLevel &C = ch.L[l + 1];
+                const int kc = (k >> 1) - (cl_div(n0, L.rNXY) >> 1);
+                smi[L.s_par + n - n0] = ((i >> 1) + C.NX * (j >> 1) + C.NXY * kc) << 3 | (k & 1) << 2 | (j & 1) << 1 | (i & 1);
+            }
+        }
+        if (l < m - 1) {  // where each warp's lanes read for its first coarse node
+            const ClusterLevel &C = ch.L[l + 1];
+            const int n = rank * C.chunk + warp;
+            smi[L.s_fine + threadIdx.x] =
+                n < min(C.NXY * C.NZ, (rank + 1) * C.chunk) ? cl_fine_addr(sm, L, C, n, lane) : 0;
+        }
+    }
+    float Kr[72];  // rows of this lane's corner, [node][row][component]
+    {
+        const float4 *src = reinterpret_cast<const float4 *>(k0f + 72 * (threadIdx.x & 7));
+#pragma unroll
+        for (int i = 0; i < 18; i++) {
+            const float4 v = __ldg(src + i);
+            Kr[4 * i] = v.x; Kr[4 * i + 1] = v.y; Kr[4 * i + 2] = v.z; Kr[4 * i + 3] = v.w;
         }
     }
     // the direct solve's rows of this CTA (one warp per row), loaded now
-    const ClusterLevel &Lc = sc.L[m - 1];
-    const int64_t inv_off = coarse_ok[chain] ? coarse_off[chain] : -1;
-    const int nnc = Lc.NX * Lc.NY * Lc.NZ, ndc = 3 * nnc;
+    const ClusterLevel &Lc = ch.L[m - 1];
+    const int64_t inv_off = coarse_ok[0] ? coarse_off[0] : -1;
+    const int nnc = Lc.NXY * Lc.NZ, ndc = 3 * nnc;
     const int c0 = rank * Lc.chunk, crows = 3 * max(0, min(nnc, c0 + Lc.chunk) - c0);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kInvPer = (kCoarseDirectMax + 31) / 32;
     float inv[kInvPer];
 #pragma unroll
@@ -2145,128 +2176,205 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
                      ? __ldg(coarse_inv + inv_off + (int64_t)(3 * c0 + warp) * ndc + r)
                      : 0.0f;
     }
-    const ClusterLevel &L0 = sc.L[0];
+    const ClusterLevel &L0 = ch.L[0];
+    const int own0 = rank * L0.chunk, nown0 = max(0, min(L0.NXY * L0.NZ, own0 + L0.chunk) - own0);
+    const int *idx0 = smi + ch.s_idx + 3 * (own0 - max(0, own0 - (L0.NXY + L0.NX + 1)));  // of the own dofs
+    rhs += L0.dof_off;
+    mx += L0.dof_off;
+    float *b0 = sm + cl_slab(L0, kClB);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
     pdl_wait();
-    // the same state in every CTA of the cluster: all return, or none
-    if (states[sc.root].done) return;
+    // The first phase's operand comes from the rhs in global memory and not from other CTAs, with
+    // the CTA's own rhs among it; loaded along with the state
+    const bool first_staged = m > 1 ? sdeg >= 2 : inv_off < 0 && cdeg >= 2;
     {
-        const int nn = L0.NX * L0.NY * L0.NZ, n0 = rank * L0.chunk, nown = max(0, min(nn, n0 + L0.chunk) - n0);
-        float *b0 = cl_slab(sm, L0, kClB);
-        for (int q = threadIdx.x; q < 3 * nown; q += kClusterThreads) {
-            const int n = n0 + q / 3, c = q - 3 * (q / 3);
-            int i, j, k;
-            cl_ijk(L0, n, i, j, k);
-            b0[q] = __ldcg(mb + L0.dof_off + ((int64_t)k * L0.NY + j) * L0.pitch + 3 * i + c);
-        }
-    }
-    cluster_barrier();  // every CTA's tables and rhs are in place
-    // down: smooth, residual, restrict
-    for (int l = 0; l < m - 1; l++) {
-        const ClusterLevel &F = sc.L[l], &C = sc.L[l + 1];
-        cl_smooth(F, sm, sK, stage, cl_slab(sm, F, kClB), true, sdeg, cc.inv_theta_s, cc.c1s, cc.c2s, rank);
-        cl_residual(F, sm, sK, stage, rank);
-        // one warp per coarse node: lane t < 27 takes fine neighbour t (all three
-        // components), the weighted values meet in a fixed xor butterfly
-        const int nnC = C.NX * C.NY * C.NZ, n0 = rank * C.chunk, n1 = min(nnC, n0 + C.chunk);
-        const float *rF = cl_slab(sm, F, kClR);
-        float *bC = cl_slab(sm, C, kClB);
-        const int warp_r = threadIdx.x >> 5, lane_r = threadIdx.x & 31;
-        for (int n = n0 + warp_r; n < n1; n += kClusterThreads / 32) {
-            int I, J, K;
-            cl_ijk(C, n, I, J, K);
-            const int dx = lane_r % 3 - 1, dy = (lane_r / 3) % 3 - 1, dz = lane_r / 9 - 1;
-            const int ii = 2 * I + dx, jj = 2 * J + dy, kk = 2 * K + dz;
-            float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
-            if (lane_r < 27 && ii >= 0 && ii < F.NX && jj >= 0 && jj < F.NY && kk >= 0 && kk < F.NZ) {
-                const int nf = ii + F.NX * (jj + F.NY * kk);
-                const float w = (dz ? 0.5f : 1.0f) * (dy ? 0.5f : 1.0f) * (dx ? 0.5f : 1.0f);
-                v0 = w * cl_get(rF, F, nf, 0, rank);
-                v1 = w * cl_get(rF, F, nf, 1, rank);
-                v2 = w * cl_get(rF, F, nf, 2, rank);
-            }
+        const int nlo = max(0, own0 - (L0.NXY + L0.NX + 1)), at = 3 * (own0 - nlo);
+        const int cnt = nown0 ? 3 * (min(L0.NXY * L0.NZ, own0 + L0.chunk + L0.NXY + L0.NX + 1) - nlo) : 0;
+        const float inv_theta = m > 1 ? cc.inv_theta_s : cc.inv_theta_c;
+        const int *idx = smi + ch.s_idx;
+        const int done = states[ch.root].done;
+        float v[3];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                v0 += __shfl_xor_sync(0xffffffffu, v0, off);
-                v1 += __shfl_xor_sync(0xffffffffu, v1, off);
-                v2 += __shfl_xor_sync(0xffffffffu, v2, off);
-            }
-            if (lane_r < 3) {
-                const float v = lane_r == 0 ? v0 : (lane_r == 1 ? v1 : v2);
-                bC[3 * (n - n0) + lane_r] = sm[C.s_dinv + 3 * n + lane_r] != 0.0f ? v : 0.0f;
-            }
+        for (int k = 0; k < 3; k++) {
+            const int t = threadIdx.x + k * kClusterThreads;
+            v[k] = t < cnt ? __ldcg(rhs + idx[t]) : 0.0f;
         }
-        cluster_barrier();
-    }
-    // coarsest grid of the chain: exact solve with the stored inverse, or smoothing
-    if (inv_off >= 0) {
-        // one warp per own row, partial sums met by a fixed xor butterfly; the
-        // first pass uses the rows loaded at the start
-        const float *bc = cl_slab(sm, Lc, kClB);
-        float *xc = cl_slab(sm, Lc, kClX);
-        for (int w0 = 0; w0 < crows; w0 += kClusterThreads / 32) {
-            const int w = w0 + warp;
-            if (w >= crows) break;  // whole warps leave together
-            float sacc = 0.0f;
+        // the same state in every CTA of the cluster: all return, or none
+        if (done) return;
+        auto place = [&](int t, float w) {
+            sm[ch.s_stage + t] = sm[L0.s_dinv + t] * w * inv_theta;
+            if ((unsigned)(t - at) < (unsigned)(3 * nown0)) b0[t - at] = w;
+        };
 #pragma unroll
-            for (int t = 0; t < kInvPer; t++) {
-                const int r = lane + 32 * t;
-                if (r < ndc) {
-                    const float a = w0 == 0 ? inv[t] : __ldg(coarse_inv + inv_off + (int64_t)(3 * c0 + w) * ndc + r);
-                    sacc = fmaf(a, cl_get(bc, Lc, r / 3, r - 3 * (r / 3), rank), sacc);
+        for (int k = 0; k < 3; k++)
+            if (const int t = threadIdx.x + k * kClusterThreads; t < cnt) place(t, v[k]);
+        for (int t = threadIdx.x + 3 * kClusterThreads; t < cnt; t += kClusterThreads) place(t, __ldcg(rhs + idx[t]));
+    }
+    if (!first_staged) cluster_barrier();
+    // down the chain: smooth, residual, restrict; the coarsest grid; up: prolong, residual, smooth
+    for (int it = 0; it < 2 * m - 1; it++) {
+        const int l = it < m ? it : 2 * m - 2 - it;
+        const bool down = it < m - 1, up = it >= m;
+        const ClusterLevel &F = ch.L[l], &C = ch.L[min(l + 1, m - 1)];
+        const int nnF = F.NXY * F.NZ, n0 = rank * F.chunk, nown = max(0, min(nnF, n0 + F.chunk) - n0);
+        const float *dinvF = sm + F.s_dinv + 3 * (n0 - max(0, n0 - (F.NXY + F.NX + 1)));  // own dofs
+        if (up) {
+            // the coarse planes around the own nodes first (the address of a parent by itself, up to
+            // eight a dof, cost more than this copy)
+            const int kc0 = cl_div(n0, F.rNXY) >> 1, kc1 = min((cl_div(n0 + max(nown, 1) - 1, F.rNXY) + 1) >> 1, C.NZ - 1);
+            float *stage = sm + ch.s_stage, *xF = sm + cl_slab(F, kClX);
+            const int cnt = nown > 0 ? 3 * C.NXY * (kc1 - kc0 + 1) : 0;
+            for (int t = threadIdx.x; t < cnt; t += kClusterThreads)
+                stage[t] = cl_get(sm, cl_slab(C, kClX), C, C.NXY * kc0 + t / 3, t - 3 * (t / 3));
+            __syncthreads();
+            for (int q = threadIdx.x; q < 3 * nown; q += kClusterThreads) {
+                if (dinvF[q] == 0.0f) continue;
+                const int par = smi[F.s_par + q / 3], ox = par & 1, oy = (par >> 1) & 1, oz = (par >> 2) & 1;
+                const float w = (ox ? 0.5f : 1.0f) * (oy ? 0.5f : 1.0f) * (oz ? 0.5f : 1.0f);
+                const float *xc = stage + 3 * (par >> 3) + q % 3;
+                float acc = 0.0f;
+#pragma unroll
+                for (int t = 0; t < 8; t++) {  // the 1, 2, 4 or 8 parents in a fixed order
+                    const int a = t >> 2, bb = (t >> 1) & 1, cc2 = t & 1;
+                    if ((a == 0 || oz) && (bb == 0 || oy) && (cc2 == 0 || ox))
+                        acc = fmaf(w, xc[3 * (cc2 + C.NX * bb + C.NXY * a)], acc);
+                }
+                xF[q] += acc;
+            }
+            cluster_barrier();
+        } else if (!down && inv_off >= 0) {
+            // the coarsest grid by the stored inverse: one warp per own row, partial sums met by
+            // a fixed xor butterfly; the first pass uses the rows loaded at the start
+            float *bc = sm + ch.s_stage, *xc = sm + cl_slab(Lc, kClX);
+            for (int r = threadIdx.x; r < ndc; r += kClusterThreads) bc[r] = cl_get(sm, cl_slab(Lc, kClB), Lc, r / 3, r % 3);
+            __syncthreads();
+            for (int w0 = 0; w0 < crows; w0 += kClusterThreads / 32) {
+                const int w = w0 + warp;
+                if (w >= crows) break;  // whole warps leave together
+                float sacc = 0.0f;
+#pragma unroll
+                for (int t = 0; t < kInvPer; t++) {
+                    const int r = lane + 32 * t;
+                    if (r < ndc) {
+                        const float a = w0 == 0 ? inv[t] : __ldg(coarse_inv + inv_off + (int64_t)(3 * c0 + w) * ndc + r);
+                        sacc = fmaf(a, bc[r], sacc);
+                    }
+                }
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, off);
+                if (lane == 0) xc[w] = dinvF[w] == 0.0f ? 0.0f : sacc;
+            }
+            cluster_barrier();
+            continue;
+        }
+        const bool coarsest = !down && !up;
+        const int deg = coarsest ? cdeg : sdeg;
+        const int n_smooth = max(deg, 1) - 1, n_steps = n_smooth + (coarsest ? 0 : 1);
+        const float inv_theta = coarsest ? cc.inv_theta_c : cc.inv_theta_s;
+        const int bF = cl_slab(F, kClB);
+        int r = cl_slab(F, kClR), d = cl_slab(F, kClD), sp = cl_slab(F, kClY);
+        if (deg <= 1 && !up) cl_smooth1(F, sm, bF, true, inv_theta, rank);
+        for (int s = 0; s < n_steps; s++) {
+            const bool residual = down ? s == n_smooth : (up && s == 0);
+            const int k = up ? s : s + 1;  // smoothing step
+            ClusterStep S;
+            S.x = cl_slab(F, kClX);
+            S.inv_theta = inv_theta;
+            S.x0_zero = !up;
+            S.staged = it == 0 && s == 0 && first_staged;
+            S.r_dst = S.r_src = r;
+            S.d_dst = S.d_src = d;
+            if (residual) {
+                S.in = S.x;
+                S.b = bF;
+                S.r_dst = cl_slab(F, kClR);
+                if (up) r = S.r_dst;
+                cl_step<0>(F, sm, Kr, sm + ch.s_stage, S, rank);
+            } else {
+                S.c1 = coarsest ? cc.c1c[k] : cc.c1s[k];
+                S.c2 = coarsest ? cc.c2c[k] : cc.c2s[k];
+                if (k == 1) {
+                    // reads the rhs at the neighbours: where it is r (post-smoothing on the residual),
+                    // the new residual goes to the spare slab
+                    S.in = S.r_src = up ? r : bF;
+                    if (up) {
+                        S.r_dst = sp;
+                        sp = r;
+                        r = S.r_dst;
+                    }
+                    cl_step<1>(F, sm, Kr, sm + ch.s_stage, S, rank);
+                } else {
+                    // reads d at the neighbours: the new direction goes to the spare slab
+                    S.in = d;
+                    S.d_dst = sp;
+                    sp = d;
+                    d = S.d_dst;
+                    cl_step<2>(F, sm, Kr, sm + ch.s_stage, S, rank);
                 }
             }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) sacc += __shfl_xor_sync(0xffffffffu, sacc, off);
-            if (lane == 0) xc[w] = sm[Lc.s_dinv + 3 * c0 + w] == 0.0f ? 0.0f : sacc;
+            cluster_barrier();
         }
-        cluster_barrier();
-    } else {
-        cl_smooth(Lc, sm, sK, stage, cl_slab(sm, Lc, kClB), true, cdeg, cc.inv_theta_c, cc.c1c, cc.c2c, rank);
-    }
-    // up: prolong, residual, post-smooth
-    for (int l = m - 2; l >= 0; l--) {
-        const ClusterLevel &F = sc.L[l], &C = sc.L[l + 1];
-        const int nnF = F.NX * F.NY * F.NZ, n0 = rank * F.chunk, nown = max(0, min(nnF, n0 + F.chunk) - n0);
-        const float *xC = cl_slab(sm, C, kClX);
-        float *xF = cl_slab(sm, F, kClX);
-        for (int q = threadIdx.x; q < 3 * nown; q += kClusterThreads) {
-            const int n = n0 + q / 3, c = q - 3 * (q / 3);
-            if (sm[F.s_dinv + 3 * n + c] == 0.0f) continue;
-            int ii, jj, kk;
-            cl_ijk(F, n, ii, jj, kk);
-            const float w = ((ii & 1) ? 0.5f : 1.0f) * ((jj & 1) ? 0.5f : 1.0f) * ((kk & 1) ? 0.5f : 1.0f);
-            // the 1, 2, 4 or 8 parents' loads first, then the sums in a fixed order
-            float v[8];
+        if (deg <= 1 && up) cl_smooth1(F, sm, r, false, inv_theta, rank);
+        if (down) {
+            // one warp per coarse node: lane t < 27 takes fine neighbour t (all three
+            // components), the weighted values meet in a fixed xor butterfly
+            const int nnC = C.NXY * C.NZ, m0 = rank * C.chunk, m1 = min(nnC, m0 + C.chunk);
+            const float *dinvC = sm + C.s_dinv + 3 * (m0 - max(0, m0 - (C.NXY + C.NX + 1)));
+            float *bC = sm + cl_slab(C, kClB);
+            const int dx = lane % 3 - 1, dy = (lane / 3) % 3 - 1, dz = lane / 9 - 1;
+            const float w = (dz ? 0.5f : 1.0f) * (dy ? 0.5f : 1.0f) * (dx ? 0.5f : 1.0f);
+            for (int n = m0 + warp; n < m1; n += kClusterThreads / 32) {
+                const uint32_t a = n == m0 + warp ? smi[F.s_fine + threadIdx.x] : cl_fine_addr(sm, F, C, n, lane);
+                float v0 = 0.0f, v1 = 0.0f, v2 = 0.0f;
+                if (a) {
+                    v0 = w * cl_load(a);
+                    v1 = w * cl_load(a + 4);
+                    v2 = w * cl_load(a + 8);
+                }
 #pragma unroll
-            for (int t = 0; t < 8; t++) {
-                const int a = t >> 2, bb = (t >> 1) & 1, cc2 = t & 1;
-                const bool use = (a == 0 || (kk & 1)) && (bb == 0 || (jj & 1)) && (cc2 == 0 || (ii & 1));
-                v[t] = use ? cl_get(xC, C, ((ii + cc2) >> 1) + C.NX * (((jj + bb) >> 1) + C.NY * ((kk + a) >> 1)), c, rank)
-                           : 0.0f;
+                for (int off = 16; off > 0; off >>= 1) {
+                    v0 += __shfl_xor_sync(0xffffffffu, v0, off);
+                    v1 += __shfl_xor_sync(0xffffffffu, v1, off);
+                    v2 += __shfl_xor_sync(0xffffffffu, v2, off);
+                }
+                if (lane < 3) {
+                    const float v = lane == 0 ? v0 : (lane == 1 ? v1 : v2);
+                    bC[3 * (n - m0) + lane] = dinvC[3 * (n - m0) + lane] != 0.0f ? v : 0.0f;
+                }
             }
-            float acc = 0.0f;
-#pragma unroll
-            for (int t = 0; t < 8; t++) {
-                const int a = t >> 2, bb = (t >> 1) & 1, cc2 = t & 1;
-                if ((a == 0 || (kk & 1)) && (bb == 0 || (jj & 1)) && (cc2 == 0 || (ii & 1))) acc = fmaf(w, v[t], acc);
-            }
-            xF[q] += acc;
+            cluster_barrier();
         }
-        cluster_barrier();
-        cl_residual(F, sm, sK, stage, rank);
-        // post-smoothing on the residual: x += S(r) (the smoother starts from r in place)
-        cl_smooth(F, sm, sK, stage, cl_slab(sm, F, kClR), false, sdeg, cc.inv_theta_s, cc.c1s, cc.c2s, rank);
     }
     // the head's correction over this CTA's nodes back to the padded global layout
-    {
-        const int nn = L0.NX * L0.NY * L0.NZ, n0 = rank * L0.chunk, nown = max(0, min(nn, n0 + L0.chunk) - n0);
-        const float *x0 = cl_slab(sm, L0, kClX);
-        for (int q = threadIdx.x; q < 3 * nown; q += kClusterThreads) {
-            const int n = n0 + q / 3, c = q - 3 * (q / 3);
-            int i, j, k;
-            cl_ijk(L0, n, i, j, k);
-            mx[L0.dof_off + ((int64_t)k * L0.NY + j) * L0.pitch + 3 * i + c] = x0[q];
+    const float *x0 = sm + cl_slab(L0, kClX);
+    float rz = 0.0f;
+    for (int q = threadIdx.x; q < 3 * nown0; q += kClusterThreads) {
+        mx[idx0[q]] = x0[q];
+        rz = fmaf(b0[q], x0[q], rz);
+    }
+    if (!from_root) return;
+    // the whole V-cycle ran here: r.z and beta too (as mf_dot_rz_kernel)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) rz += __shfl_xor_sync(0xffffffffu, rz, off);
+    if (lane == 0) s_red[warp] = (double)rz;
+    __syncthreads();
+    if (warp == 0) {
+        double s = lane < kClusterThreads / 32 ? s_red[lane] : 0.0;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (lane == 0) {
+            uint32_t at_first;  // the same word of the cluster's first CTA
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at_first) : "r"(smem_u32(s_rz + rank)));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at_first), "d"(s) : "memory");
         }
+    }
+    cluster_barrier();
+    if (rank == 0 && warp == 0) {
+        double s = lane < csize ? s_rz[lane] : 0.0;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (lane == 0) finish_rz(states + ch.root, s);
     }
 }
 
@@ -3092,6 +3200,7 @@ int64_t cluster_layout(const MfBatch &b, int cs, std::vector<ClusterChain> &chai
             L.pitch = T.pitch; L.pitch_e = T.pitch_e;
             L.dof_off = T.dof_off; L.elem_off = T.elem_off;
             const int nn = T.NX * T.NY * T.NZ, H = T.NX * T.NY + T.NX + 1;
+            int64_t staged = 0;  // words staged by one CTA
             L.chunk = (nn + cs - 1) / cs;
             L.NXY = T.NX * T.NY;
             L.rNX = 1.0f / (float)T.NX;
@@ -3105,22 +3214,41 @@ int64_t cluster_layout(const MfBatch &b, int cs, std::vector<ClusterChain> &chai
                     return -1;
             for (int r = 0; r < cs; r++) {
                 const int n0 = r * L.chunk, n1 = std::min(nn, n0 + L.chunk);
-                if (n0 < n1) stage = std::max<int64_t>(stage, 3LL * (std::min(nn - 1, n1 - 1 + H) - std::max(0, n0 - H) + 1));
+                if (n0 < n1) staged = std::max<int64_t>(staged, 3LL * (std::min(nn, n1 + H) - std::max(0, n0 - H)));
             }
+            staged = (staged + 3) / 4 * 4;
+            stage = std::max(stage, staged);
+            if (m > 0) {  // prolongation to the level above stages the coarse planes around its nodes
+                const ClusterLevel &F = ch.L[m - 1];
+                const int nf = F.NXY * F.NZ;
+                for (int n0 = 0; n0 < nf; n0 += F.chunk) {
+                    const int k0 = n0 / F.NXY >> 1;
+                    const int k1 = std::min(((std::min(nf, n0 + F.chunk) - 1) / F.NXY + 1) >> 1, T.NZ - 1);
+                    stage = std::max<int64_t>(stage, 3LL * L.NXY * (k1 - k0 + 1));
+                }
+            }
+            stage = std::max<int64_t>(stage, 3LL * nn <= kCoarseDirectMax ? 3LL * nn : 0);  // rhs of a direct solve
+            L.s_dinv = (int)staged;  // words, until the offsets are given below
         }
         ch.m = m;
-        int64_t off = kClusterK0;
-        ch.s_stage = (int)off;
-        off += (stage + 3) / 4 * 4;
+        int64_t off = 0;
+        auto take = [&](int64_t words) {
+            const int at = (int)off;
+            off += (words + 3) / 4 * 4;
+            return at;
+        };
+        ch.s_stage = take(stage);
+        ch.s_idx = take(m > 0 ? ch.L[0].s_dinv : 0);
         for (int l = 0; l < m; l++) {
             ClusterLevel &L = ch.L[l];
-            const int64_t nn = (int64_t)L.NX * L.NY * L.NZ, ne = (int64_t)L.nx * L.ny * L.nz;
-            L.s_dinv = (int)off;
-            off += (3 * nn + 3) / 4 * 4;
-            L.s_E = (int)off;
-            off += (ne + 3) / 4 * 4;
-            L.s_vec = (int)off;
-            off += 15LL * L.chunk;
+            const int staged = L.s_dinv;
+            L.s_dinv = take(staged);
+            L.s_addr = take(staged);
+            L.s_E = take((int64_t)L.nx * L.ny * L.nz);
+            L.s_vec = take(15LL * L.chunk);
+            L.s_elem = take(L.chunk);
+            L.s_par = take(L.chunk);
+            L.s_fine = take(kClusterThreads);
         }
         most = std::max(most, off * 4);
     }
@@ -3287,20 +3415,23 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     // most kBottomMaxHeadNodes nodes whose chain (it and all coarser levels) fits
     // the bottom kernel's shared memory; larger levels run level by level on the
     // whole GPU (the one-CTA kernel is bound by one SM's shared-memory pipe there).
-    // With a cluster per chain (bottom_cluster: single-design solves), the first
-    // level with at most kClusterMaxHeadNodes nodes.
+    // On a cluster (bottom_cluster: single-design solves), the first level with at
+    // most kClusterMaxHeadNodes nodes, the finest included.
     // (a device on which no cluster of the bottom kernel can be placed falls back
     // to the one-CTA chains)
     int64_t inv_floats = 0;
-    for (int attempt = bottom_cluster ? 0 : 1; attempt < 2; attempt++) {
+    for (int attempt = bottom_cluster && b.n_fine == 1 ? 0 : 1; attempt < 2; attempt++) {
         const bool use_cluster = attempt == 0;
         b.h_heads.clear();
         b.h_head_root.clear();
         b.bottom_smem = 0;
         b.bottom_cluster = 0;
+        b.chains_from_root = false;
         for (MfProblem &T : b.h_probs) T.bottom = 0;
         for (int r = 0; r < b.n_fine; r++) {
-            for (int q = b.h_probs[r].coarse; q >= 0; q = b.h_probs[q].coarse) {
+            // the cluster's chain may start at the design's own grid
+            const bool try_root = use_cluster && b.h_probs[r].coarse >= 0;
+            for (int q = try_root ? r : b.h_probs[r].coarse; q >= 0; q = b.h_probs[q].coarse) {
                 int64_t floats = 576 + 800, depth = 0;
                 for (int t = q; t >= 0; t = b.h_probs[t].coarse, depth++) {
                     const MfProblem &T = b.h_probs[t];
@@ -3315,8 +3446,9 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
                 if (depth <= kBottomMaxLevels && fits) {
                     b.h_heads.push_back(q);
                     b.h_head_root.push_back(r);
-                    b.bottom_smem = use_cluster ? (576 + 800) * 4 : std::max(b.bottom_smem, (int)bytes);
-                    for (int t = q; t >= 0; t = b.h_probs[t].coarse) b.h_probs[t].bottom = 1;
+                    b.bottom_smem = use_cluster ? 0 : std::max(b.bottom_smem, (int)bytes);
+                    for (int t = q; t >= 0; t = b.h_probs[t].coarse) b.h_probs[t].bottom = t != r;
+                    b.chains_from_root = q == r;
                     break;
                 }
             }
@@ -3347,7 +3479,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         {
             // the largest cluster (16 CTAs: non-portable size) the device can place
             // MASTGPU_BOTTOM_CLUSTER caps the cluster (1, 2, 4, 8 or 16 CTAs): a test knob,
-            // the result does not depend on the cluster size
+            // the correction does not depend on the cluster size
             int cap = kClusterMax;
             if (const char *env = std::getenv("MASTGPU_BOTTOM_CLUSTER")) cap = std::max(1, std::min(kClusterMax, std::atoi(env)));
             int first = 1;
@@ -3500,18 +3632,18 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_CUDA_TRY(cudaMemcpyAsync(b.chunks, b.h_chunks.data(), b.h_chunks.size() * sizeof(MfChunkDesc), cudaMemcpyHostToDevice, s));
     MG_CUDA_TRY(cudaMemcpyAsync(b.K0, K0, 576 * 8, cudaMemcpyHostToDevice, s));
     if (b.bottom_cluster) {
-        // K0 and its regrouped copy in FP32 (as mg_bottom_kernel forms them), the chains' level tables
+        // K0 in FP32, the three rows of the corner (dx, dy, dz) at 72 (dx + 2 dy + 4 dz) as
+        // [node][row][component]
         std::vector<float> k0f(kClusterK0);
-        for (int i = 0; i < 576; i++) k0f[i] = (float)K0[i];
-        for (int i = 0; i < 800; i++) {
-            const int a = i / 100, t = i % 100, bc = t / 12, q = t % 12, r = q / 3, c = q % 3;
-            k0f[576 + i] = (t < 96 && q < 9) ? (float)K0[(3 * a + r) * 24 + 3 * bc + c] : 0.0f;
+        for (int i = 0; i < kClusterK0; i++) {
+            const int lex = i / 72, bc = i % 72 / 9, r = i % 9 / 3, c = i % 3;
+            const int a = corner_index(lex & 1, (lex >> 1) & 1, lex >> 2);
+            k0f[i] = (float)K0[(3 * a + r) * 24 + 3 * bc + c];
         }
         MG_TRY(dev_alloc_n(&b.cl_k0, (size_t)kClusterK0));
-        MG_TRY(dev_alloc_n(&b.cl_chains, b.h_cl_chains.size()));
         MG_CUDA_TRY(cudaMemcpyAsync(b.cl_k0, k0f.data(), k0f.size() * 4, cudaMemcpyHostToDevice, s));
-        MG_CUDA_TRY(cudaMemcpyAsync(b.cl_chains, b.h_cl_chains.data(), b.h_cl_chains.size() * sizeof(ClusterChain),
-                                    cudaMemcpyHostToDevice, s));
+        MG_TRY(dev_alloc_n(&b.cl_chain, 1));
+        MG_CUDA_TRY(cudaMemcpyAsync(b.cl_chain, b.h_cl_chains.data(), sizeof(ClusterChain), cudaMemcpyHostToDevice, s));
         MG_CUDA_TRY(cudaStreamSynchronize(s));  // k0f is a host temporary
     }
     if (!b.h_coarse_off.empty()) {
@@ -3544,7 +3676,7 @@ void mf_batch_free(MfBatch &b) {
                     b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
                     b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_part, b.Bop2, b.fac_tiles, b.fac_maps, b.node_blks,
-                    b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_chains, b.cl_k0, b.sens_offs};
+                    b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chain, b.sens_offs};
     for (void *q : ptrs) dev_free(q);
     if (b.stage_host) cudaFreeHost(b.stage_host);
     if (b.sens_offs_host) cudaFreeHost(b.sens_offs_host);
@@ -3752,6 +3884,7 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
     const Cheb cs = cheb_coeffs(b.cheb_lmax, sdeg), cc = cheb_coeffs(b.cheb_lmax, cdeg);
     const int L = b.n_levels;
     auto any_level = [&](int l) {  // some problem of level l is solved level by level
+        if (l == 0 && b.chains_from_root) return false;
         for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++)
             if (!b.h_probs[pi].bottom) return true;
         return false;
@@ -3783,10 +3916,10 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
             bc.c1c[k] = cc.c1[k]; bc.c2c[k] = cc.c2[k];
         }
         if (b.bottom_cluster)
-            launch_cluster_pdl(mg_bottom_cluster_kernel, (unsigned)(b.h_heads.size() * b.bottom_cluster),
-                               kClusterThreads, b.bottom_smem, b.bottom_cluster, b.stream, b.cl_chains, b.states,
-                               b.E32, b.dinv, b.mb, b.mx, b.cl_k0, bc, sdeg, cdeg, b.coarse_off, b.coarse_inv,
-                               b.coarse_ok);
+            launch_cluster_pdl(mg_bottom_cluster_kernel, (unsigned)b.bottom_cluster,
+                               kClusterThreads, b.bottom_smem, b.bottom_cluster, b.stream, b.cl_chain, b.states,
+                               b.E32, b.dinv, b.chains_from_root ? b.r : b.mb, b.mx, b.chains_from_root, b.cl_k0, bc, sdeg,
+                               cdeg, b.coarse_off, b.coarse_inv, b.coarse_ok);
         else
             launch_pdl(mg_bottom_kernel, (unsigned)b.h_heads.size(), kBottomThreads, b.bottom_smem, b.stream,
                 b.probs, b.heads, b.states, b.E32, b.dinv, b.mb, b.mx, b.K0, bc, sdeg, cdeg, b.coarse_off,
@@ -3835,11 +3968,13 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
         const int sdeg = prm.smooth_deg > 0 ? prm.smooth_deg : 2;
         const int cdeg = prm.coarse_deg > 0 ? prm.coarse_deg : 8;
         n += enqueue_vcycle(b, prm.mg_operator == 0, mg_precision(prm.precision), sdeg, cdeg);
-        launch_pdl(mf_dot_rz_kernel, vg0, kThreads, 0, s, b.chunks, n0, b.probs, b.r, b.mx, b.states,
-                                                 b.chunk_part, 0);
+        if (!b.chains_from_root) {
+            launch_pdl(mf_dot_rz_kernel, vg0, kThreads, 0, s, b.chunks, n0, b.probs, b.r, b.mx, b.states, b.chunk_part);
+            n += 1;
+        }
         launch_cg_apply(b, prm.precision, 4, parity);  // p = z + beta p_old, q = A p, alpha
         launch_update(b, pnew, true);                  // x, r, stop test
-        n += 3;
+        n += 2;
     } else {
         launch_cg_apply(b, prm.precision, 0, parity);
         launch_update(b, pnew, false);                 // also z = D^-1 r, beta

@@ -56,12 +56,14 @@ struct ClusterLevel {
     int pitch, pitch_e;
     int64_t dof_off, elem_off;
     int chunk;                // nodes per CTA (CTA r owns nodes [r chunk, (r + 1) chunk))
-    int s_dinv, s_E, s_vec;   // shared-memory offsets (floats): D^-1 and E of the level, the CTA's slabs
+    int s_dinv, s_E, s_vec;   // shared-memory offsets (words): D^-1 of the staged nodes, E of the level, the CTA's slabs
+    int s_addr, s_elem;       // cluster addresses of the staged words; the nodes' elements (first, mask of eight)
+    int s_par, s_fine;        // the nodes' parents; cluster addresses that restriction from here reads
     int NXY;                  // NX NY
     float rNX, rNXY, rchunk;  // 1 / NX, 1 / NXY, 1 / chunk: n / d = trunc((n + 1/2) (1 / d)) (checked on the host)
 };
 struct ClusterChain {
-    int m, root, s_stage, pad;
+    int m, root, s_stage, s_idx;  // s_idx: the staged words' places in the head's padded vectors
     ClusterLevel L[kBottomMaxLevels];
 };
 
@@ -198,9 +200,10 @@ struct MfBatch {
     int *coarse_ok = nullptr;
     int bottom_smem = 0;        // dynamic shared memory of the bottom kernel
     int bottom_cluster = 0;     // CTAs per chain of the cluster bottom kernel (0: one-CTA kernel)
-    std::vector<ClusterChain> h_cl_chains;  // its per-chain level tables
-    ClusterChain *cl_chains = nullptr;
-    float *cl_k0 = nullptr;     // K0 and its regrouped copy in FP32
+    bool chains_from_root = false;  // the cluster chain starts at the design's own grid: the whole V-cycle
+    std::vector<ClusterChain> h_cl_chains;  // its chain's level tables (one: a single design)
+    ClusterChain *cl_chain = nullptr;
+    float *cl_k0 = nullptr;     // K0 in FP32, regrouped by corners
     // FP64 refinement vectors (padded layout)
     double *u64 = nullptr, *r64 = nullptr, *f64 = nullptr;
     double *brick_part = nullptr, *chunk_part = nullptr;
@@ -243,9 +246,9 @@ void hex8_box_stiffness(double hx, double hy, double hz, double nu, double K[576
 
 // shapes: the designs' own grids (level 0); max_levels > 1 adds the coarse
 // multigrid levels of every design (mg_coarsens);
-// bottom_cluster: each chain's bottom V-cycle on a thread-block cluster from a
-// larger level on (single-design solves; batches keep the one-CTA form, so a
-// design's preconditioner is the same in every batch)
+// bottom_cluster: the bottom V-cycle on a thread-block cluster from a larger level
+// on, the design's own grid included (one design only; batches keep the one-CTA
+// form, so a design's preconditioner is the same in every batch)
 int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, double hy,
                   double hz, double nu, cudaStream_t stream, int max_levels = kMaxLevels,
                   bool bottom_cluster = false);
