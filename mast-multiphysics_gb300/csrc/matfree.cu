@@ -1307,10 +1307,9 @@ __global__ void __launch_bounds__(kThreads) mg_cheb_next_kernel(
     }
 }
 
-// The transfers run over the lists of node blocks of the problems that take part (a grid of
-// the largest problem's blocks times the problems left most blocks of a mixed batch empty: 58
-// problems, prolongation into level 0 97 us a launch, 70 us from the list,
-// restriction 42 and 25).
+// The transfers run over the list of node blocks of the coarse problems that take part (a grid
+// of the largest problem's blocks times the problems left most blocks of a mixed batch empty: 58
+// problems, restriction from level 0 42 us a launch, 21 us from the list).
 //
 // restriction (transpose of trilinear interpolation) into the coarse problems:
 // mb_c[I] = sum_d w(d) my_f[2I + d], d in {-1,0,1}^3, w = prod (1 - |d|/2);
@@ -1359,47 +1358,78 @@ __global__ void __launch_bounds__(kNodeBlk) mg_restrict_kernel(const MfProblem *
     }
 }
 
-// prolongation (trilinear) from the coarse levels into the fine problems:
-// mx_f[i] += sum_I w mx_c[I] (skips Dirichlet dofs and padding)
+// prolongation (trilinear) from the coarse problems into their fine ones:
+// mx_f[i] += sum_I w mx_c[I] (skips Dirichlet dofs and padding).  One coarse node (I, J, K) per
+// thread: it reads the cell's eight coarse nodes once and updates the fine nodes 2I..2I+1, 2J..2J+1,
+// 2K..2K+1, each from its 1, 2, 4 or 8 parents; all loads are issued before the first sum.  Bound by
+// DRAM and L2 (20 bytes a fine dof).  With a fine node per thread its up to eight parents were read
+// for every node: 58 problems, level 0 (10.9 M dofs) 70 us a launch, 20 us by cells.
 __global__ void __launch_bounds__(kNodeBlk) mg_prolong_kernel(const MfProblem *__restrict__ probs,
                                                          const MfNodeBlk *__restrict__ blks,
-                                                         const MfState *states, float *__restrict__ mx,
+                                                         const MfState *states, float *mx,
                                                          const float *__restrict__ dinv) {
     pdl_trigger();
     const MfNodeBlk B = blks[blockIdx.x];
-    const MfProblem F = probs[B.prob];
-    const MfProblem C = probs[F.coarse];
+    const MfProblem C = probs[B.prob];
+    const MfProblem F = probs[C.fine];
+    const int n = B.node + threadIdx.x;
+    const bool in = n < C.NX * C.NY * C.NZ;
+    const int I = n % C.NX, JK = n / C.NX, J = JK % C.NY, K = JK / C.NY;
     pdl_wait();
-    if (states[F.root].done) return;
-    // one fine node (3 dofs) per thread; its 1, 2, 4 or 8 coarse parents' loads are
-    // issued together (the unused ones predicated off)
-    const int nn = F.NX * F.NY * F.NZ, n = B.node + threadIdx.x;
-    if (n < nn) {
-        const int ii = n % F.NX, jk = n / F.NX, j = jk % F.NY, k = jk / F.NY;
-        const int64_t o = F.dof_off + ((int64_t)k * F.NY + j) * F.pitch + 3 * ii;
-        const float wx = (ii & 1) ? 0.5f : 1.0f, wy = (j & 1) ? 0.5f : 1.0f, wz = (k & 1) ? 0.5f : 1.0f;
-        const float w = wx * wy * wz;
-        float v[8][3];
+    if (states[F.root].done || !in) return;
+    const bool has_x = 2 * I + 1 < F.NX, has_y = 2 * J + 1 < F.NY, has_z = 2 * K + 1 < F.NZ;
+    if (2 * I >= F.NX || 2 * J >= F.NY || 2 * K >= F.NZ) return;  // beyond an odd side
+    float v[8][3];  // the cell's coarse nodes
+    const float *src = mx + C.dof_off + ((int64_t)K * C.NY + J) * C.pitch + 3 * I;
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const int a = q >> 2, bb = (q >> 1) & 1, cc = q & 1;
-            const bool use = (a == 0 || (k & 1)) && (bb == 0 || (j & 1)) && (cc == 0 || (ii & 1));
-            const int I = (ii + cc) >> 1, J = (j + bb) >> 1, K = (k + a) >> 1;
-            const float *src = mx + C.dof_off + (use ? ((int64_t)K * C.NY + J) * C.pitch + 3 * I : 0);
+    for (int q = 0; q < 8; q++) {
+        const bool use = (!(q & 1) || has_x) && (!(q & 2) || has_y) && (!(q & 4) || has_z);
+        const int64_t o = use ? ((int64_t)(q >> 2) * C.NY + ((q >> 1) & 1)) * C.pitch + 3 * (q & 1) : 0;
 #pragma unroll
-            for (int c = 0; c < 3; c++) v[q][c] = use ? src[c] : 0.0f;
-        }
+        for (int c = 0; c < 3; c++) v[q][c] = use ? src[o + c] : 0.0f;
+    }
+    // two neighbouring fine nodes are six floats from an even place on: three pairs, the last
+    // pair and a half left out where the second node does not exist
+    float m[4][6], d[4][6];
+    const int64_t o0 = F.dof_off + ((int64_t)2 * K * F.NY + 2 * J) * F.pitch + 6 * I;
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            if (dinv[o + c] == 0.0f) continue;
-            float acc = 0.0f;
+    for (int row = 0; row < 4; row++) {
+        const bool use = (!(row & 1) || has_y) && (!(row & 2) || has_z);
+        const int64_t o = o0 + (use ? ((int64_t)(row >> 1) * F.NY + (row & 1)) * F.pitch : 0);
 #pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const int a = q >> 2, bb = (q >> 1) & 1, cc = q & 1;
-                const bool use = (a == 0 || (k & 1)) && (bb == 0 || (j & 1)) && (cc == 0 || (ii & 1));
-                if (use) acc = fmaf(w, v[q][c], acc);
+        for (int h = 0; h < 3; h++) {
+            if (has_x || h == 0) {
+                const float2 mv = *reinterpret_cast<const float2 *>(mx + o + 2 * h);
+                const float2 dv = *reinterpret_cast<const float2 *>(dinv + o + 2 * h);
+                m[row][2 * h] = mv.x; m[row][2 * h + 1] = mv.y;
+                d[row][2 * h] = dv.x; d[row][2 * h + 1] = dv.y;
             }
-            mx[o + c] += acc;
+        }
+        if (!has_x) { m[row][2] = mx[o + 2]; d[row][2] = dinv[o + 2]; }
+    }
+#pragma unroll
+    for (int row = 0; row < 4; row++) {
+        const int b = row & 1, a = row >> 1;
+        if ((b && !has_y) || (a && !has_z)) continue;
+        const int64_t o = o0 + ((int64_t)a * F.NY + b) * F.pitch;
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float w = (x ? 0.5f : 1.0f) * (b ? 0.5f : 1.0f) * (a ? 0.5f : 1.0f);
+                float acc = 0.0f;
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if ((!(q & 1) || x) && (!(q & 2) || b) && (!(q & 4) || a)) acc = fmaf(w, v[q][c], acc);
+                if (d[row][3 * x + c] != 0.0f) m[row][3 * x + c] += acc;
+            }
+        if (has_x) {
+#pragma unroll
+            for (int h = 0; h < 3; h++)
+                *reinterpret_cast<float2 *>(mx + o + 2 * h) = make_float2(m[row][2 * h], m[row][2 * h + 1]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) mx[o + c] = m[row][c];
         }
     }
 }
@@ -1731,32 +1761,37 @@ __global__ void __launch_bounds__(kBottomThreads, 1) mg_bottom_kernel(
 // "A tutorial on the SWEEP operator", 1979): sweeping pivot k maps
 // a_ij -> a_ij - a_ik a_kj / a_kk (i, j != k), a_ik -> a_ik / a_kk and
 // a_kk -> -1 / a_kk; sweeping every pivot leaves -A^-1.  Each thread keeps a 6 x 6
-// tile in registers and forms a_ik a_kj as one product, so the tiles stay bitwise
-// symmetric and the stored inverse is exactly symmetric (the V-cycle stays a
-// fixed symmetric preconditioner).  No pivoting: the pivots of a symmetric
-// positive definite matrix are positive.  A pivot that is not (a singular or
-// indefinite coarse operator) clears coarse_ok and the bottom kernel smooths that
-// chain's coarsest grid instead.
+// tile of the lower triangle in registers (the upper one is its mirror image, so
+// the stored inverse is exactly symmetric and the V-cycle stays a fixed symmetric
+// preconditioner).  A node's three pivots are swept between two barriers: every
+// thread forms the second and third pivot row at its rows and columns from the
+// three rows as they were before the node (the same operations in the same order
+// as pivot by pivot).  Bound by the barriers and the chain of three reciprocals:
+// 135 dofs 137 us with a barrier per pivot and both triangles kept, 76 us so.
+// No pivoting: the pivots of a symmetric positive definite matrix are positive.  A
+// pivot that is not (a singular or indefinite coarse operator) clears coarse_ok and
+// the bottom kernel smooths that chain's coarsest grid instead.
 constexpr int kCoarseTile = 6;
 constexpr int kCoarseTiles = kCoarseDirectMax / kCoarseTile;
-constexpr int kCoarseInvThreads = kCoarseTiles * kCoarseTiles;
+constexpr int kCoarseInvTiles = kCoarseTiles * (kCoarseTiles + 1) / 2;
+constexpr int kCoarseInvThreads = (kCoarseInvTiles + 31) / 32 * 32;
 constexpr int kCoarseMaxElems = 64;  // nodes <= kCoarseDirectMax / 3 = 48, so elements < 48
+constexpr int kCoarsePitch = kCoarseDirectMax + 1;  // odd: a column's words lie in different banks
 constexpr int kCoarseInvSmem =
-    (kCoarseDirectMax * kCoarseDirectMax + 576 + kCoarseMaxElems + 3 * kCoarseDirectMax) * 4;
-static_assert(kCoarseDirectMax % kCoarseTile == 0, "the sweep tiles cover the padded operator");
+    (kCoarseDirectMax * kCoarsePitch + 576 + kCoarseMaxElems + 7 * kCoarseDirectMax) * 4;
+static_assert(kCoarseDirectMax % kCoarseTile == 0 && kCoarseTile % 3 == 0, "whole nodes per tile, whole tiles");
 
 __global__ void __launch_bounds__(kCoarseInvThreads, 1) mg_coarse_inverse_kernel(
     const MfProblem *__restrict__ probs, const int *__restrict__ heads, const int *__restrict__ list,
     const float *__restrict__ E32, const float *__restrict__ dinv, const double *__restrict__ K0,
     const int64_t *__restrict__ coarse_off, float *__restrict__ coarse_inv, int *__restrict__ coarse_ok) {
-    constexpr int NP = kCoarseDirectMax, T = kCoarseTile;
+    constexpr int NP = kCoarseDirectMax, T = kCoarseTile, LD = kCoarsePitch;
     extern __shared__ __align__(16) float sci[];
-    float *sA = sci;              // NP x NP assembled operator
-    float *sK = sA + NP * NP;     // K0 (576)
+    float *sA = sci;              // assembled operator, rows of LD words
+    float *sK = sA + NP * LD;     // K0 (576)
     float *sE = sK + 576;         // the level's moduli
-    float *sv = sE + kCoarseMaxElems;  // pivot rows, double-buffered (2 x NP)
-    int *sfix = reinterpret_cast<int *>(sv + 2 * NP);
-    __shared__ float s_rcp[2];         // 1 / pivot of each buffered row, formed once by its writer
+    float *sv = sE + kCoarseMaxElems;  // three pivot rows, double-buffered (2 x 3 x NP)
+    int *sfix = reinterpret_cast<int *>(sv + 6 * NP);
     const int h = list[blockIdx.x];
     const int64_t off = coarse_off[h];
     if (off < 0) return;
@@ -1779,10 +1814,12 @@ __global__ void __launch_bounds__(kCoarseInvThreads, 1) mg_coarse_inverse_kernel
         const int i = n % C.NX, j = (n / C.NX) % C.NY, k = n / (C.NX * C.NY);
         sfix[q] = dinv[dof_index(C, i, j, k, cq)] == 0.0f;
     }
+    for (int i = tid; i < nd * LD; i += kCoarseInvThreads) sA[i] = 0.0f;
     __syncthreads();
-    for (int q = tid; q < nd; q += kCoarseInvThreads) {
-        float *row = sA + q * NP;
-        for (int r = 0; r < NP; r++) row[r] = 0.0f;
+    // a thread per row and column component
+    for (int t = tid; t < 3 * nd; t += kCoarseInvThreads) {
+        const int cb = t / nd, q = t - cb * nd;
+        float *row = sA + q * LD + cb;
         const int n = q / 3, cq = q - 3 * n;
         const int i = n % C.NX, jj = (n / C.NX) % C.NY, k = n / (C.NX * C.NY);
         for (int a = 0; a < 8; a++) {
@@ -1791,94 +1828,136 @@ __global__ void __launch_bounds__(kCoarseInvThreads, 1) mg_coarse_inverse_kernel
             const int ex = i - dx, ey = jj - dy, ez = k - dz;
             if (ex < 0 || ey < 0 || ez < 0 || ex >= C.nx || ey >= C.ny || ez >= C.nz) continue;
             const float e = sE[ex + C.nx * (ey + C.ny * ez)];
+#pragma unroll
             for (int bc = 0; bc < 8; bc++) {
                 int bx, by, bz;
                 corner_bits(bc, bx, by, bz);
                 const int m = (ex + bx) + C.NX * ((ey + by) + C.NY * (ez + bz));
-                for (int cb = 0; cb < 3; cb++)
-                    row[3 * m + cb] = fmaf(e, sK[(3 * a + cq) * 24 + 3 * bc + cb], row[3 * m + cb]);
+                row[3 * m] = fmaf(e, sK[(3 * a + cq) * 24 + 3 * bc + cb], row[3 * m]);
             }
         }
     }
     __syncthreads();
-    const int ti = tid / kCoarseTiles, tj = tid - ti * kCoarseTiles;
-    const int i0 = ti * T, j0 = tj * T;
-    float a[T][T];
+    // tile (ti, tj), tj <= ti, of the lower triangle, numbered row by row
+    int ti = (int)((sqrtf(8.0f * tid + 1.0f) - 1.0f) * 0.5f);
+    while (ti * (ti + 1) / 2 > tid) ti--;
+    while ((ti + 1) * (ti + 2) / 2 <= tid) ti++;
+    const int tj = tid - ti * (ti + 1) / 2, i0 = ti * T, j0 = tj * T;
+    const bool mine = tid < kCoarseInvTiles;
+    float2 a[T][T / 2];
 #pragma unroll
     for (int r = 0; r < T; r++)
 #pragma unroll
         for (int cc = 0; cc < T; cc++) {
             const int i = i0 + r, j = j0 + cc;
             float v = i == j ? 1.0f : 0.0f;
-            if (i < nd && j < nd && !sfix[i] && !sfix[j]) v = i <= j ? sA[i * NP + j] : sA[j * NP + i];
-            a[r][cc] = v;
+            if (mine && i < nd && j < nd && !sfix[i] && !sfix[j]) v = i <= j ? sA[i * LD + j] : sA[j * LD + i];
+            (cc & 1 ? a[r][cc / 2].y : a[r][cc / 2].x) = v;
         }
-    if (ti == 0)
+    // the three rows from pivot k on into buffer `buf`: from the tiles of the row and, mirrored, of the column
+    auto publish = [&](int k, int buf) {
+        float *v = sv + buf * 3 * NP;
+        const int kr = k - i0, kc = k - j0;
+        if (!mine) return;
+        if (kr == 0 || kr == 3) {
 #pragma unroll
-        for (int cc = 0; cc < T; cc++) sv[j0 + cc] = a[0][cc];
-    if (tid == 0) s_rcp[0] = 1.0f / a[0][0];
+            for (int q = 0; q < 3; q++)
+#pragma unroll
+                for (int cc = 0; cc < T / 2; cc++) {
+                    const float2 w = kr == 0 ? a[q][cc] : a[q + 3][cc];
+                    v[q * NP + j0 + 2 * cc] = w.x;
+                    v[q * NP + j0 + 2 * cc + 1] = w.y;
+                }
+        } else if (kc == 0 || kc == 3) {
+#pragma unroll
+            for (int r = 0; r < T; r++) {
+                v[i0 + r] = kc == 0 ? a[r][0].x : a[r][1].y;
+                v[NP + i0 + r] = kc == 0 ? a[r][0].y : a[r][2].x;
+                v[2 * NP + i0 + r] = kc == 0 ? a[r][1].x : a[r][2].y;
+            }
+        }
+    };
+    publish(0, 0);
     __syncthreads();
     int ok = 1, cur = 0;
-    for (int k = 0; k < nd; k++) {
-        const float *v = sv + cur * NP;
-        const float d = v[k];  // the same value in every thread: the exit below is uniform
-        if (!(d > 0.0f) || !isfinite(d)) {
+    for (int k = 0; k < nd; k += 3) {
+        const float *v0 = sv + cur * 3 * NP, *v1 = v0 + NP, *v2 = v1 + NP;
+        // the node's 3 x 3 block: its pivots, the same values in every thread (the exit is uniform)
+        const float c01 = v0[k + 1], c02 = v0[k + 2];
+        const float d0 = v0[k], p0 = 1.0f / d0;
+        const float d1 = fmaf(-(c01 * c01), p0, v1[k + 1]), p1 = 1.0f / d1;
+        const float c12 = fmaf(-(c01 * c02), p0, v1[k + 2]);
+        const float d2 = fmaf(-(c12 * c12), p1, fmaf(-(c02 * c02), p0, v2[k + 2])), p2 = 1.0f / d2;
+        if (!(d0 > 0.0f) || !isfinite(d0) || !(d1 > 0.0f) || !isfinite(d1) || !(d2 > 0.0f) || !isfinite(d2)) {
             ok = 0;
             break;
         }
-        const float p = s_rcp[cur];
-        float vi[T], vj[T];
+        if (mine) {
+            // the pivot rows at index i, each as it is when its pivot is swept
+            auto rows_at = [&](int i, float &x0, float &x1, float &x2) {
+                x0 = v0[i];
+                x1 = i == k ? c01 * p0 : fmaf(-(c01 * x0), p0, v1[i]);
+                x2 = i == k ? c02 * p0 : fmaf(-(c02 * x0), p0, v2[i]);
+                x2 = i == k + 1 ? c12 * p1 : fmaf(-(c12 * x1), p1, x2);
+            };
+            // a swept row or column becomes v p: 0 - (-1 v) p, with the factor -1 at the swept
+            // index and the tile's entries there set to 0 (few threads, in nearly every warp)
+            const int kr = k - i0, kc = k - j0;
+            float vi[3][T];
+            float2 vj[3][T / 2];
 #pragma unroll
-        for (int r = 0; r < T; r++) {
-            vi[r] = v[i0 + r];
-            vj[r] = v[j0 + r];
-        }
+            for (int r = 0; r < T; r++) {
+                rows_at(i0 + r, vi[0][r], vi[1][r], vi[2][r]);
+                vi[r % 3][r] = kr == r - r % 3 ? -1.0f : vi[r % 3][r];
+            }
 #pragma unroll
-        for (int r = 0; r < T; r++)
+            for (int cc = 0; cc < T; cc++) {
+                float x[3];
+                rows_at(j0 + cc, x[0], x[1], x[2]);
+                x[cc % 3] = kc == cc - cc % 3 ? -1.0f : x[cc % 3];
 #pragma unroll
-            for (int cc = 0; cc < T; cc++) a[r][cc] = fmaf(-(vi[r] * vj[cc]), p, a[r][cc]);
-        const int kr = k - i0, kc = k - j0;
-        // row and column k: a_kj = v_j / d, a_ik = v_i / d, a_kk = -1 / d
-        if ((unsigned)kr < (unsigned)T) {
+                for (int q = 0; q < 3; q++) (cc & 1 ? vj[q][cc / 2].y : vj[q][cc / 2].x) = x[q];
+            }
+            const bool swept = kr == 0 || kr == 3 || kc == 0 || kc == 3;
 #pragma unroll
-            for (int r = 0; r < T; r++)
-                if (r == kr)
+            for (int q = 0; q < 3; q++) {
+                if (swept) {
 #pragma unroll
-                    for (int cc = 0; cc < T; cc++) a[r][cc] = cc == kc ? -p : vj[cc] * p;
-        }
-        if ((unsigned)kc < (unsigned)T) {
+                    for (int half = 0; half < 2; half++) {
+                        const int at = 3 * half + q;
+                        if (kr == 3 * half)
 #pragma unroll
-            for (int cc = 0; cc < T; cc++)
-                if (cc == kc)
+                            for (int cc = 0; cc < T / 2; cc++) a[at][cc] = make_float2(0.0f, 0.0f);
+                        if (kc == 3 * half)
 #pragma unroll
-                    for (int r = 0; r < T; r++)
-                        if (r != kr) a[r][cc] = vi[r] * p;
-        }
-        const int nr = k + 1 - i0;  // the next pivot row (and its reciprocal pivot)
-        if ((unsigned)nr < (unsigned)T) {
-            float *vn = sv + (cur ^ 1) * NP;
-            const int nc = k + 1 - j0;
-#pragma unroll
-            for (int r = 0; r < T; r++)
-                if (r == nr)
-#pragma unroll
-                    for (int cc = 0; cc < T; cc++) {
-                        vn[j0 + cc] = a[r][cc];
-                        if (cc == nc) s_rcp[cur ^ 1] = 1.0f / a[r][cc];
+                            for (int r = 0; r < T; r++) (at & 1 ? a[r][at / 2].y : a[r][at / 2].x) = 0.0f;
                     }
+                }
+                const float p = q == 0 ? p0 : q == 1 ? p1 : p2;
+                const float2 np = make_float2(-p, -p);
+#pragma unroll
+                for (int r = 0; r < T; r++)
+#pragma unroll
+                    for (int cc = 0; cc < T / 2; cc++)
+                        a[r][cc] = __ffma2_rn(__fmul2_rn(make_float2(vi[q][r], vi[q][r]), vj[q][cc]), np, a[r][cc]);
+            }
         }
-        __syncthreads();
         cur ^= 1;
+        if (k + 3 < nd) publish(k + 3, cur);
+        __syncthreads();
     }
     if (tid == 0) coarse_ok[h] = ok;
-    if (!ok) return;
+    if (!ok || !mine) return;
     float *out = coarse_inv + off;
 #pragma unroll
     for (int r = 0; r < T; r++)
 #pragma unroll
         for (int cc = 0; cc < T; cc++) {
             const int i = i0 + r, j = j0 + cc;
-            if (i < nd && j < nd) out[i * nd + j] = -a[r][cc];
+            if (i >= nd || j >= nd) continue;
+            const float w = cc & 1 ? a[r][cc / 2].y : a[r][cc / 2].x;
+            out[i * nd + j] = -w;
+            if (ti != tj) out[j * nd + i] = -w;
         }
 }
 
@@ -3511,24 +3590,20 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         }
         if (b.bottom_cluster) break;
     }
-    // node blocks of the transfers, by level: the problems restricted into (their fine level
-    // is not inside a bottom chain) and the problems prolonged into
+    // node blocks of the transfers, by level: the coarse problems whose fine one is not inside a
+    // bottom chain
     {
         std::vector<MfNodeBlk> blks;
-        auto add = [&](int pi) {
-            const MfProblem &P = b.h_probs[pi];
-            for (int n = 0; n < P.NX * P.NY * P.NZ; n += kNodeBlk) blks.push_back(MfNodeBlk{pi, n});
-        };
-        b.lvl_restrict_lo.clear(); b.lvl_restrict_hi.clear(); b.lvl_prolong_lo.clear(); b.lvl_prolong_hi.clear();
+        b.lvl_blk_lo.clear();
+        b.lvl_blk_hi.clear();
         for (int l = 0; l < b.n_levels; l++) {
-            b.lvl_restrict_lo.push_back((int)blks.size());
-            for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++)
-                if (b.h_probs[pi].fine >= 0 && !b.h_probs[b.h_probs[pi].fine].bottom) add(pi);
-            b.lvl_restrict_hi.push_back((int)blks.size());
-            b.lvl_prolong_lo.push_back((int)blks.size());
-            for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++)
-                if (b.h_probs[pi].coarse >= 0 && !b.h_probs[pi].bottom) add(pi);
-            b.lvl_prolong_hi.push_back((int)blks.size());
+            b.lvl_blk_lo.push_back((int)blks.size());
+            for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++) {
+                const MfProblem &P = b.h_probs[pi];
+                if (P.fine < 0 || b.h_probs[P.fine].bottom) continue;
+                for (int n = 0; n < P.NX * P.NY * P.NZ; n += kNodeBlk) blks.push_back(MfNodeBlk{pi, n});
+            }
+            b.lvl_blk_hi.push_back((int)blks.size());
         }
         MG_TRY(dev_alloc_n(&b.node_blks, std::max<size_t>(1, blks.size())));
         if (!blks.empty())
@@ -3900,8 +3975,8 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
         const float *rin = (l == 0) ? b.r : b.mb;
         n += enqueue_smooth(b, fac, prec, l, rin, 1, sdeg, cs, 0);
         launch_level_op<2>(b, fac, prec, l, 4, b.mx, rin, b.my, 0);  // my = rin - A mx
-        if (const int blks = b.lvl_restrict_hi[l + 1] - b.lvl_restrict_lo[l + 1])
-            launch_pdl(mg_restrict_kernel, blks, kNodeBlk, 0, b.stream, b.probs, b.node_blks + b.lvl_restrict_lo[l + 1],
+        if (const int blks = b.lvl_blk_hi[l + 1] - b.lvl_blk_lo[l + 1])
+            launch_pdl(mg_restrict_kernel, blks, kNodeBlk, 0, b.stream, b.probs, b.node_blks + b.lvl_blk_lo[l + 1],
                        b.states, b.my, b.mb, b.z, b.dinv);
         n += 2;
         if (own_coarsest(l)) n += enqueue_smooth(b, fac, prec, l, rin, 1, cdeg, cc, 1);
@@ -3929,8 +4004,8 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
     for (int l = L - 2; l >= 0; l--) {
         if (!any_level(l)) continue;
         const float *rin = (l == 0) ? b.r : b.mb;
-        if (const int blks = b.lvl_prolong_hi[l] - b.lvl_prolong_lo[l])
-            launch_pdl(mg_prolong_kernel, blks, kNodeBlk, 0, b.stream, b.probs, b.node_blks + b.lvl_prolong_lo[l],
+        if (const int blks = b.lvl_blk_hi[l + 1] - b.lvl_blk_lo[l + 1])
+            launch_pdl(mg_prolong_kernel, blks, kNodeBlk, 0, b.stream, b.probs, b.node_blks + b.lvl_blk_lo[l + 1],
                        b.states, b.mx, b.dinv);
         // my = rin - A mx; the fused smoother starts from z = D^-1 my (and of degree 2 needs no more)
         const bool from_z = fac && sdeg >= 2;

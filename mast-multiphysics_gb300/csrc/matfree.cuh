@@ -103,7 +103,7 @@ struct MfCol {
     int16_t cx, cy, cz, pad;
 };
 
-constexpr int kNodeBlk = 256;  // nodes per block of the level transfers
+constexpr int kNodeBlk = 64;  // nodes per block of the level transfers (256: 48x24x24 prolonged on 17 SMs)
 struct MfNodeBlk {
     int prob, node;  // nodes [node, node + kNodeBlk) of the problem
 };
@@ -155,8 +155,8 @@ struct MfBatch {
     std::vector<int> lvl_col_lo, lvl_col_hi;
     double *col_part = nullptr;   // per-column partial of p.q
     uint32_t *Bop2 = nullptr;     // K0 as the column operator's four (dy, dz) B tiles
-    MfNodeBlk *node_blks = nullptr;  // of the level transfers: per level restricted into, prolonged into
-    std::vector<int> lvl_restrict_lo, lvl_restrict_hi, lvl_prolong_lo, lvl_prolong_hi;
+    MfNodeBlk *node_blks = nullptr;  // of the level transfers, by coarse level
+    std::vector<int> lvl_blk_lo, lvl_blk_hi;
     MfCol *fac_tiles = nullptr;   // tiles of the factored CUDA-core operator (cx, cy, cz)
     CUtensorMap *fac_maps = nullptr;  // its tensor maps per problem (node vectors, moduli)
     std::vector<MfCol> h_fac_tiles;
