@@ -2190,6 +2190,13 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
     for (int l = 0; l < m; l++) {
         const ClusterLevel &L = ch.L[l];
         const int nn = L.NXY * L.NZ, H = L.NXY + L.NX + 1;
+        if (l < m - 1) {  // where each warp's lanes read for its first coarse node (a CTA without
+                          // nodes of this level may own coarse ones)
+            const ClusterLevel &C = ch.L[l + 1];
+            const int n = rank * C.chunk + warp;
+            smi[L.s_fine + threadIdx.x] =
+                n < min(C.NXY * C.NZ, (rank + 1) * C.chunk) ? cl_fine_addr(sm, L, C, n, lane) : 0;
+        }
         const int n0 = rank * L.chunk, n1 = min(nn, n0 + L.chunk), nlo = max(0, n0 - H);
         if (n0 >= n1) continue;
         const int cnt = 3 * (min(nn, n1 + H) - nlo);
@@ -2224,12 +2231,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
                 const int kc = (k >> 1) - (cl_div(n0, L.rNXY) >> 1);
                 smi[L.s_par + n - n0] = ((i >> 1) + C.NX * (j >> 1) + C.NXY * kc) << 3 | (k & 1) << 2 | (j & 1) << 1 | (i & 1);
             }
-        }
-        if (l < m - 1) {  // where each warp's lanes read for its first coarse node
-            const ClusterLevel &C = ch.L[l + 1];
-            const int n = rank * C.chunk + warp;
-            smi[L.s_fine + threadIdx.x] =
-                n < min(C.NXY * C.NZ, (rank + 1) * C.chunk) ? cl_fine_addr(sm, L, C, n, lane) : 0;
         }
     }
     float Kr[72];  // rows of this lane's corner, [node][row][component]

@@ -22,8 +22,9 @@ def reference(shape):
 
 # 4 x 4 x 4: the smallest chain of two levels; 16^3 (4,913 nodes): the largest cube solved from its
 # own grid; 17 x 16 x 16 (5,202 nodes): level by level; 30/31/32 x 14/15/16: one node short of a tile,
-# a whole one, one node over
-SHAPES = [(4, 4, 4), (9, 8, 3), (16, 16, 16), (17, 16, 16), (30, 14, 9), (31, 15, 10), (32, 16, 9)]
+# a whole one, one node over; 2 x 1 x 26: the second level (56 nodes) leaves two of sixteen CTAs
+# without nodes, the third (32) none
+SHAPES = [(4, 4, 4), (9, 8, 3), (16, 16, 16), (17, 16, 16), (30, 14, 9), (31, 15, 10), (32, 16, 9), (2, 1, 26)]
 
 
 @pytest.mark.parametrize("degree", [1, 2, 3, 5])
