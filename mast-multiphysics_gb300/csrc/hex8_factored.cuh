@@ -130,7 +130,6 @@ __device__ __forceinline__ dfloat operator*(dfloat a, dfloat b) {
     return df_renorm(p, e);
 }
 __device__ __forceinline__ dfloat &operator+=(dfloat &a, dfloat b) { return a = a + b; }
-__device__ __forceinline__ dfloat &operator*=(dfloat &a, dfloat b) { return a = a * b; }
 __device__ __forceinline__ dfloat fma_t(dfloat a, dfloat b, dfloat c) { return a * b + c; }
 __device__ __forceinline__ dfloat df_from(double x) {
     dfloat r;
@@ -175,11 +174,6 @@ __device__ __forceinline__ dfloat df_zero() {
     r.lo = 0.0f;
     return r;
 }
-template <typename T>
-__device__ __forceinline__ T zero_t() { return T(0); }
-template <>
-__device__ __forceinline__ dfloat zero_t<dfloat>() { return df_zero(); }
-
 // v[c][b]: component c at lexicographic corner b; on return its sum/difference
 // modes u~ = H^T u (per component, the 8-point Walsh-Hadamard butterfly)
 template <typename T>
@@ -249,31 +243,60 @@ __device__ __forceinline__ void hex8_factored_khat(const FacK<T> &K, const T (&v
     yh[2][7] = K.v[44] * v[2][7];
 }
 
-// v[c][b]: component c at lexicographic corner b; on return e * (K0 u_e) in the
-// same layout.  Fixed operation order (deterministic).
-template <typename T>
-__device__ __forceinline__ void hex8_factored_apply(const FacK<T> &K, T e, T (&v)[3][8]) {
-    hex8_factored_forward(v);
-    T yh[3][8];
-    hex8_factored_khat(K, v, yh);
-    // back to the corners: the transpose butterflies, mode 0 is zero
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        yh[c][0] = zero_t<T>();
-#pragma unroll
-        for (int m = 1; m < 8; m++) yh[c][m] *= e;
-#pragma unroll
-        for (int t = 1; t < 8; t <<= 1)
-#pragma unroll
-            for (int b = 0; b < 8; b++)
-                if (!(b & t)) {
-                    const T a = yh[c][b], bb = yh[c][b | t];
-                    yh[c][b] = a - bb;
-                    yh[c][b | t] = a + bb;
-                }
-#pragma unroll
-        for (int b = 0; b < 8; b++) v[c][b] = yh[c][b];
-    }
+// A product of two double-floats before its renormalisation: p + err
+struct DfTerm {
+    float p, err;
+};
+__device__ __forceinline__ DfTerm df_term(dfloat a, dfloat b) {
+    DfTerm t;
+    t.p = __fmul_rn(a.hi, b.hi);
+    t.err = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.hi, -t.p)));
+    return t;
+}
+__device__ __forceinline__ DfTerm operator+(DfTerm a, DfTerm b) {
+    DfTerm t;
+    t.p = __fadd_rn(a.p, b.p);
+    const float bb = __fsub_rn(t.p, a.p);
+    const float e = __fadd_rn(__fsub_rn(a.p, __fsub_rn(t.p, bb)), __fsub_rn(b.p, bb));
+    t.err = __fadd_rn(e, __fadd_rn(a.err, b.err));
+    return t;
+}
+__device__ __forceinline__ dfloat operator*(DfTerm a, dfloat b) {
+    const float p = __fmul_rn(a.p, b.hi);
+    const float e = __fmaf_rn(a.p, b.lo, __fmaf_rn(a.err, b.hi, __fmaf_rn(a.p, b.hi, -p)));
+    return df_renorm(p, e);
+}
+
+// v[c][m]: the modes u~ -> e Khat/64 u~ in place in double-floats (modes 1..7; mode 0 is not read or
+// written), group by group as hex8_factored_khat2.  The products of a sum are renormalised once, with
+// the factor e: 520 instructions where products and additions each by itself take 726.
+__device__ __forceinline__ void hex8_factored_khat_df(const FacK<dfloat> &K, dfloat e, dfloat (&v)[3][8]) {
+    auto group3 = [&](dfloat &a, dfloat &b, dfloat &c, int aa, int ab, int ac, int ba, int bb, int bc, int ca, int cb,
+                      int cc) {
+        const dfloat x = ((df_term(K.v[aa], a) + df_term(K.v[ab], b)) + df_term(K.v[ac], c)) * e;
+        const dfloat y = ((df_term(K.v[ba], a) + df_term(K.v[bb], b)) + df_term(K.v[bc], c)) * e;
+        const dfloat z = ((df_term(K.v[ca], a) + df_term(K.v[cb], b)) + df_term(K.v[cc], c)) * e;
+        a = x;
+        b = y;
+        c = z;
+    };
+    auto group2 = [&](dfloat &a, dfloat &b, int aa, int ab, int ba, int bb) {
+        const dfloat x = (df_term(K.v[aa], a) + df_term(K.v[ab], b)) * e;
+        const dfloat y = (df_term(K.v[ba], a) + df_term(K.v[bb], b)) * e;
+        a = x;
+        b = y;
+    };
+    group3(v[0][1], v[1][2], v[2][4], 0, 1, 2, 17, 18, 19, 37, 38, 39);
+    group2(v[0][2], v[1][1], 3, 4, 15, 16);
+    group2(v[0][3], v[2][6], 5, 6, 42, 43);
+    group2(v[0][4], v[2][1], 7, 8, 30, 31);
+    group2(v[0][5], v[1][6], 9, 10, 27, 28);
+    group3(v[0][6], v[1][5], v[2][3], 11, 12, 13, 24, 25, 26, 34, 35, 36);
+    group2(v[1][3], v[2][5], 20, 21, 40, 41);
+    group2(v[1][4], v[2][2], 22, 23, 32, 33);
+    v[0][7] = df_term(K.v[14], v[0][7]) * e;
+    v[1][7] = df_term(K.v[29], v[1][7]) * e;
+    v[2][7] = df_term(K.v[44], v[2][7]) * e;
 }
 
 // Two elements at once in packed FP32x2 arithmetic (each component of a float2 is one

@@ -8,28 +8,15 @@
 // eliminated (identity rows, zero columns) as in the plain form; they are
 // marked by a zero Jacobi inverse, which keeps r, z and p zero there.
 //
-// Brick kernel (one CTA per 8x8x8 block of owned nodes, persistent grid,
-// two CTAs per SM):
-//   1. one thread issues three TMA tile loads (cp.async.bulk.tensor.3d) into
-//      shared memory: the (8+2)^3 node halo of z and of p_old, and the 9^3
-//      element moduli around the owned nodes; out-of-grid parts arrive as 0;
-//   2. per 128-element tile, all threads write the element displacement rows
-//      U = z + beta p_old (128 x 24) as TF32 or BF16 in the canonical
-//      no-swizzle K-major UMMA layout (the split variants also write the
-//      rounding remainder U_lo), and one thread issues tcgen05.mma:
-//      D(128 x 32, FP32, TMEM) = U K0^T [+ U_lo K0^T + U K0_lo^T];
-//      two A buffers and two TMEM accumulators let tile t's MMA run while
-//      tile t-1 is drained;
-//   3. tcgen05.ld drains D, each row is scaled by E_e (the rho^p epilogue) and
-//      parked in a 128-row shared buffer;
-//   4. every owned dof adds the contributions of its (up to 8) elements found
-//      in that tile, in a fixed order, into a register accumulator: no atomics,
-//      no colouring, deterministic, one global write per output dof.
-// Elements in the one-element halo are evaluated by both neighbouring bricks
-// (729 evaluations per 512 owned nodes).
+// The CG operator runs on the tensor cores by columns of nodes (mf_col_kernel), the
+// multigrid levels on the CUDA cores with the factored element stiffness
+// (mf_fac_kernel), the small levels in one CTA or one cluster per chain, and the
+// FP64 residual in double-float arithmetic (mf_residual64_kernel).  Every owned dof
+// adds its elements' contributions in a fixed order: no atomics, no colouring, one
+// global write per dof; tiles evaluate the elements of their one-element halo anew.
 //
-// Reductions are per problem and deterministic: every brick (chunk) writes a
-// partial and the last brick (chunk) of a problem -- found with a per-problem
+// Reductions are per problem and deterministic: every tile (chunk) writes a
+// partial and the last tile (chunk) of a problem -- found with a per-problem
 // counter -- sums that problem's partials in index order.  A problem's result
 // is therefore bitwise independent of which other problems share the batch.
 #include <cstdlib>
@@ -2463,9 +2450,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
 // behind its table and state reads, cost a batch of 58 problems about 1 us a part and block.
 //
 // Calls body(part index) for the parts [begin, end) that range(p) gives of the problems p < n
-// with in_phase(p), spread over the grid; every thread of the block (kThreads) calls it.
+// with in_phase(p), spread over the grid; every one of the block's NT threads calls it.
 // Every block numbers the parts for itself, so in_phase must not change while the kernel runs.
-template <typename InPhase, typename Range, typename Body>
+template <int NT, typename InPhase, typename Range, typename Body>
 __device__ __forceinline__ void for_active_parts(int n, InPhase in_phase, Range range, Body body) {
     if (n == 1) {  // no tables: they cost a single 16x8x8 or 48x24x24 solve 2 %
         if (!in_phase(0)) return;
@@ -2474,10 +2461,10 @@ __device__ __forceinline__ void for_active_parts(int n, InPhase in_phase, Range 
         for (int i = begin + blockIdx.x; i < end; i += gridDim.x) body(i);
         return;
     }
-    __shared__ int s_end[kThreads], s_begin[kThreads], s_warp[kThreads / 32];
+    __shared__ int s_end[NT], s_begin[NT], s_warp[NT / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int start = blockIdx.x;  // of this window's numbering
-    for (int p0 = 0; p0 < n; p0 += kThreads) {
+    for (int p0 = 0; p0 < n; p0 += NT) {
         const int p = p0 + threadIdx.x;
         const bool in = p < n && in_phase(p);
         if (!__syncthreads_or(in)) continue;  // also: the previous window's tables are no longer read
@@ -2495,9 +2482,9 @@ __device__ __forceinline__ void for_active_parts(int n, InPhase in_phase, Range 
         s_end[threadIdx.x] = sum;
         s_begin[threadIdx.x] = begin;
         __syncthreads();
-        const int total = s_end[kThreads - 1];
+        const int total = s_end[NT - 1];
         for (; start < total; start += gridDim.x) {
-            int lo = 0, hi = kThreads - 1;  // the first problem whose parts end beyond start
+            int lo = 0, hi = NT - 1;  // the first problem whose parts end beyond start
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
                 if (s_end[mid] > start) hi = mid;
@@ -2520,7 +2507,7 @@ __global__ void __launch_bounds__(kThreads) mf_inner_init_kernel(
     pdl_enter();
     __shared__ double red_sh[kThreads / 32];
     __shared__ int sh_last;
-    for_active_parts(n_fine, [&](int p) { return states[p].resid != 0; },
+    for_active_parts<kThreads>(n_fine, [&](int p) { return states[p].resid != 0; },
                      [&](int p, int &begin, int &end) {
                          begin = probs[p].chunk_begin;
                          end = begin + probs[p].chunk_count;
@@ -2586,7 +2573,7 @@ __global__ void __launch_bounds__(kThreads) mf_refine_kernel(
     const MfChunkDesc *__restrict__ chunks, const MfProblem *__restrict__ probs, int n_fine,
     const float *__restrict__ x, double *__restrict__ u64, const MfState *states) {
     pdl_enter();
-    for_active_parts(n_fine, [&](int p) { return inner_finished(states + p); },
+    for_active_parts<kThreads>(n_fine, [&](int p) { return inner_finished(states + p); },
                      [&](int p, int &begin, int &end) {
                          begin = probs[p].chunk_begin;
                          end = begin + probs[p].chunk_count;
@@ -2637,146 +2624,241 @@ __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states
     }
 }
 
-// FP64 outer residual r = f - K u (CUDA-core FP64, factored element stiffness,
-// hex8_factored.cuh), per-problem ||r||^2 -> scale.  A brick of kBN^3 owned
-// nodes evaluates its (kBN+1)^3 surrounding elements in three groups of kBE/3
-// element layers: each element's 24 corner results go to shared memory, then
-// every owned node adds the results of its elements in that group to register
-// accumulators, in a fixed order (deterministic, atomic-free).
-constexpr int kRGroupLayers = kBE / 3;                      // 3 element layers per group
-constexpr int kRGroupEl = kBE * kBE * kRGroupLayers;        // 243 elements
-constexpr int kRNodesPerThread = (kBN * kBN * kBN + kThreads - 1) / kThreads;  // 2
-constexpr int kOffU64 = 0;
-constexpr int kOffE64 = kBU * kBU * kBU * 3 * 8;            // 24000
-constexpr int kOffY64 = kOffE64 + kNEL * 8;                 // +5832
-constexpr int kResidSmem = kOffY64 + 24 * kRGroupEl * 8;    // +46656
-static_assert(kBE % 3 == 0 && kRGroupEl <= kThreads, "one element per thread and group");
+// FP64 outer residual r = f - K u (double-float arithmetic, factored element
+// stiffness, hex8_factored.cuh), per-problem ||r||^2 -> scale.  A tile owns
+// kROwnX x kROwnY nodes in x, y (to the end of the side in the last tile) and
+// P.res_z node planes, evaluates the kREX x kREY elements around them, a thread
+// each, and streams through the element layers as mf_fac_kernel does: the x, y part
+// of the transform belongs to a node plane and is formed once for the two layers
+// that meet there, and the results of the two layers are added in mode space before
+// one inverse x, y transform per node plane.  Its four corner values go to shared
+// memory, from where every owned node adds those of its four elements in a fixed
+// order (deterministic, atomic-free).  u's planes arrive by asynchronous copies two
+// layers ahead and are split into double-floats once per tile.
+// Bound by the FP32 pipe (an addition of two double-floats is 11 instructions):
+// 128x64x64 169 us with bricks of 8^3 nodes that evaluated 1.9 elements for each one
+// and 24 corner values apiece, 102 us so; the z overlap and the tiles' edges leave 1.3.
+constexpr int kROwnX = 16, kROwnY = 8;
+constexpr int kREX = kROwnX + 1, kREY = kROwnY + 1;   // elements per tile layer
+constexpr int kRNX = kREX + 1, kRNY = kREY + 1;       // nodes per tile plane
+constexpr int kRThreads = 160;                        // 153 elements, 153 nodes at most
+constexpr int kRPlane = 3 * kRNX * kRNY;              // 540 words of a node plane
+constexpr int kRLoads = (kRPlane + kRThreads - 1) / kRThreads;
+constexpr int kRMaxZ = 12;
+constexpr int kResidSmem = (2 * kRPlane + 2 * kRPlane + 2 * 12 * kRThreads) * 8;  // planes, raw planes, exchange
+static_assert(kREX * kREY <= kRThreads, "one element and one node per thread");
 
-__global__ void __launch_bounds__(kThreads) mf_residual64_kernel(
+// block sum of kRThreads threads; valid in thread 0
+__device__ __forceinline__ double resid_sum(double v, double *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return threadIdx.x == 0 ? ((sh[0] + sh[1]) + (sh[2] + sh[3])) + sh[4] : 0.0;
+}
+static_assert(kRThreads == 5 * 32, "resid_sum adds five warps");
+
+__global__ void __launch_bounds__(kRThreads, 3) mf_residual64_kernel(
     const MfProblem *__restrict__ probs, const MfBrick *__restrict__ bricks, int n_bricks,
     const dfloat *__restrict__ Edf, const uint8_t *__restrict__ node_fix,
-    const double *__restrict__ u64, const double *__restrict__ f64, const FacK<dfloat> K,
+    const double *__restrict__ u64, const double *__restrict__ f64, const __grid_constant__ FacK<dfloat> K,
     double *__restrict__ r64, MfState *states, double *__restrict__ brick_part, double rtol2,
     int max_ref, int n_fine) {
     pdl_enter();
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ double red_sh[kThreads / 32];
+    __shared__ double red_sh[kRThreads / 32];
     __shared__ int sh_last;
-    dfloat *su = reinterpret_cast<dfloat *>(smem + kOffU64);
-    dfloat *sE = reinterpret_cast<dfloat *>(smem + kOffE64);
-    dfloat(*sY)[kRGroupEl] = reinterpret_cast<dfloat(*)[kRGroupEl]>(smem + kOffY64);  // [b * 3 + c][element]
-    for_active_parts(n_fine, [&](int p) { return states[p].resid != 0; },
+    dfloat *planes = reinterpret_cast<dfloat *>(smem);                // [2][kRPlane]
+    double *raws = reinterpret_cast<double *>(planes + 2 * kRPlane);  // [2][kRPlane]
+    dfloat *xchg = reinterpret_cast<dfloat *>(raws + 2 * kRPlane);    // [2][12][kRThreads]
+    const int tid = threadIdx.x;
+    const bool active = tid < kREX * kREY;
+    const int tx = active ? tid % kREX : 0, ty = active ? tid / kREX : 0;  // of the thread's element and node
+    for_active_parts<kRThreads>(n_fine, [&](int p) { return states[p].resid != 0; },
                      [&](int p, int &begin, int &end) {
                          begin = probs[p].brick_begin;
                          end = begin + probs[p].brick_count;
                      }, [&](int bi) {
         const MfBrick br = bricks[bi];
-        const MfProblem P = probs[br.prob];
+        const MfProblem &P = probs[br.prob];
         MfState *st = states + br.prob;
         const bool need_ff = st->ff64 == 0.0;  // first residual of a solve: also ||f||^2
         const bool u_zero = st->u_zero != 0;    // cold start: r = f, no operator pass
-        const int gx0 = br.bx * kBN, gy0 = br.by * kBN, gz0 = br.bz * kBN;
-        __syncthreads();
-        for (int i = threadIdx.x; i < (u_zero ? 0 : kBU * kBU * kBU * 3); i += kThreads) {
-            const int node = i / 3, c = i - node * 3;
-            const int ux = node % kBU, uy = (node / kBU) % kBU, uz = node / (kBU * kBU);
-            const int gx = gx0 - 1 + ux, gy = gy0 - 1 + uy, gz = gz0 - 1 + uz;
-            double v = 0.0;
-            if (gx >= 0 && gx < P.NX && gy >= 0 && gy < P.NY && gz >= 0 && gz < P.NZ) {
-                const int64_t gn = gx + (int64_t)P.NX * (gy + (int64_t)P.NY * gz);
-                if (!((node_fix[P.node_off + gn] >> c) & 1)) v = u64[dof_index(P, gx, gy, gz, c)];
-            }
-            su[i] = df_split(v);
-        }
-        for (int l = threadIdx.x; l < (u_zero ? 0 : kNEL); l += kThreads) {
-            const int ex = l % kBE, ey = (l / kBE) % kBE, ez = l / (kBE * kBE);
-            const int gx = gx0 - 1 + ex, gy = gy0 - 1 + ey, gz = gz0 - 1 + ez;
-            dfloat e = df_zero();
-            if (gx >= 0 && gx < P.nx && gy >= 0 && gy < P.ny && gz >= 0 && gz < P.nz)
-                e = Edf[P.elem_off + ((int64_t)gz * P.ny + gy) * P.pitch_e + gx];
-            sE[l] = e;
-        }
-        dfloat acc[kRNodesPerThread][3];
+        const int NX = P.NX, NY = P.NY, NZ = P.NZ, nx = P.nx, ny = P.ny, nz = P.nz, pitch = P.pitch;
+        const int gx0 = br.bx * kROwnX, gy0 = br.by * kROwnY, z0 = br.bz * P.res_z, z1 = min(z0 + P.res_z, NZ);
+        const int ownx = gx0 + kROwnX >= nx ? NX - gx0 : kROwnX, owny = gy0 + kROwnY >= ny ? NY - gy0 : kROwnY;
+        const int S = z1 - z0 + 1;  // element layers z0 - 1 .. z1 - 1; node planes z0 - 1 .. z1
+        const uint8_t *fix = node_fix + P.node_off;
+        const double *u = u64 + P.dof_off;
+        // node plane p (z0 - 1 + p): the words of this thread, copied into raw buffer p & 1, and
+        // split from there (0 beyond the grid and on Dirichlet dofs) into plane buffer p & 1
+        auto word = [&](int k, int p, int &t, int &gx, int64_t &line, int &c) {
+            t = tid + k * kRThreads;
+            const int row = t / (3 * kRNX), col = t - row * (3 * kRNX), i = col / 3;
+            const int gy = gy0 - 1 + row, gz = z0 - 1 + p;
+            gx = gx0 - 1 + i;
+            c = col - 3 * i;
+            line = (int64_t)gz * NY + gy;
+            return t < kRPlane && (unsigned)gx < (unsigned)NX && (unsigned)gy < (unsigned)NY && (unsigned)gz < (unsigned)NZ;
+        };
+        auto load = [&](int p, unsigned (&fb)[kRLoads]) {  // fb: 1 where the word is 0
 #pragma unroll
-        for (int k = 0; k < kRNodesPerThread; k++) acc[k][0] = acc[k][1] = acc[k][2] = df_zero();
-        for (int g = 0; g < (u_zero ? 0 : 3); g++) {
-            __syncthreads();  // su / sE loaded; the previous group's readers of sY are done
-            const int l = threadIdx.x;
-            if (l < kRGroupEl) {
-                const int ex = l % kBE, ey = (l / kBE) % kBE, ez = g * kRGroupLayers + l / (kBE * kBE);
-                const dfloat e = sE[ex + kBE * (ey + kBE * ez)];
-                dfloat v[3][8];
-#pragma unroll
-                for (int b = 0; b < 8; b++) {
-                    const dfloat *ub = su + (((ez + (b >> 2)) * kBU + ey + ((b >> 1) & 1)) * kBU + ex + (b & 1)) * 3;
-                    v[0][b] = ub[0]; v[1][b] = ub[1]; v[2][b] = ub[2];
-                }
-                if (e.hi != 0.0f) {
-                    hex8_factored_apply(K, e, v);
-                } else {
-#pragma unroll
-                    for (int b = 0; b < 8; b++) v[0][b] = v[1][b] = v[2][b] = df_zero();
-                }
-#pragma unroll
-                for (int b = 0; b < 8; b++) {
-                    sY[b * 3][l] = v[0][b];
-                    sY[b * 3 + 1][l] = v[1][b];
-                    sY[b * 3 + 2][l] = v[2][b];
+            for (int k = 0; k < kRLoads; k++) {
+                int t, gx, c;
+                int64_t line;
+                fb[k] = 1;
+                if (word(k, p, t, gx, line, c)) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(raws + (p & 1) * kRPlane + t)),
+                                 "l"(u + line * pitch + 3 * gx + c) : "memory");
+                    fb[k] = (unsigned)fix[line * NX + gx] >> c;
                 }
             }
+        };
+        auto split = [&](int p, const unsigned (&fb)[kRLoads]) {
+#pragma unroll
+            for (int k = 0; k < kRLoads; k++) {
+                const int t = tid + k * kRThreads;
+                if (t >= kRPlane) continue;
+                planes[(p & 1) * kRPlane + t] = fb[k] & 1 ? df_zero() : df_split(raws[(p & 1) * kRPlane + t]);
+            }
+        };
+        // the element's modulus in layer s
+        const int gex = gx0 - 1 + tx, gey = gy0 - 1 + ty;
+        const bool in_grid = active && (unsigned)gex < (unsigned)nx && (unsigned)gey < (unsigned)ny;
+        const dfloat *Ecol = Edf + P.elem_off + (in_grid ? (int64_t)gey * P.pitch_e + gex : 0);
+        const int64_t Elayer = (int64_t)ny * P.pitch_e;
+        auto modulus = [&](int s) {
+            const int k = z0 - 1 + s;
+            return in_grid && s < S && k >= 0 && k < nz ? Ecol[k * Elayer] : df_zero();
+        };
+        // x, y modes (q = mx + 2 my) of plane p at the element
+        auto modes = [&](int p, int c, dfloat (&m)[4]) {
+            const dfloat *n0 = planes + (p & 1) * kRPlane + 3 * (ty * kRNX + tx) + c;
+            const dfloat a = n0[0], b = n0[3], cc = n0[3 * kRNX], d = n0[3 * kRNX + 3];
+            const dfloat s0 = a + b, s1 = cc + d, d0 = b - a, d1 = d - cc;
+            m[0] = s0 + s1;
+            m[1] = d0 + d1;
+            m[2] = s1 - s0;
+            m[3] = d1 - d0;
+        };
+        unsigned fb[kRLoads];
+        dfloat low[3][4], car[3][4], e = df_zero();  // modes of plane s; results of layer s - 1 on it
+        if (!u_zero) {
+            unsigned fb1[kRLoads];
+            load(0, fb);
+            load(1, fb1);
+            e = modulus(0);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            split(0, fb);
+            split(1, fb1);
+            load(2, fb);  // a tile has two layers at least
             __syncthreads();
 #pragma unroll
-            for (int k = 0; k < kRNodesPerThread; k++) {
-                const int node = threadIdx.x + k * kThreads;
-                if (node >= kBN * kBN * kBN) continue;
-                const int ox = node % kBN, oy = (node / kBN) % kBN, oz = node / (kBN * kBN);
+            for (int c = 0; c < 3; c++) {
+                modes(0, c, low[c]);
 #pragma unroll
-                for (int b = 0; b < 8; b++) {  // the node is corner b of element (o + 1 - d)
-                    const int dx = b & 1, dy = (b >> 1) & 1, dz = b >> 2;
-                    const int lz = oz + 1 - dz - g * kRGroupLayers;
-                    if (lz < 0 || lz >= kRGroupLayers) continue;
-                    const int el = (ox + 1 - dx) + kBE * ((oy + 1 - dy) + kBE * lz);
-                    acc[k][0] += sY[b * 3][el];
-                    acc[k][1] += sY[b * 3 + 1][el];
-                    acc[k][2] += sY[b * 3 + 2][el];
+                for (int q = 0; q < 4; q++) car[c][q] = df_zero();
+            }
+            __syncthreads();  // plane 0 is read; plane 2 takes its buffer in the first layer
+        }
+        const bool own = active && tx < ownx && ty < owny;
+        const int64_t line0 = (int64_t)(z0 - 1) * NY + gy0 + ty, fix0 = line0 * NX + gx0 + tx;
+        const int64_t g0 = P.dof_off + line0 * pitch + 3 * (gx0 + tx);
+        double part = 0.0, fpart = 0.0;
+        for (int s = 0; s < S; s++) {
+            dfloat *X = xchg + (s & 1) * 12 * kRThreads;
+            if (!u_zero) {
+                const dfloat e_next = modulus(s + 1);
+                dfloat v[3][8];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    dfloat high[4];
+                    modes(s + 1, c, high);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (q) v[c][q] = low[c][q] + high[q];  // mode 0 has no part in the result
+                        v[c][q + 4] = high[q] - low[c][q];
+                        low[c][q] = high[q];
+                    }
+                }
+                hex8_factored_khat_df(K, e, v);
+                e = e_next;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    dfloat node[4];  // plane s: the layer below's part and this layer's
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        node[q] = q ? car[c][q] + (v[c][q] - v[c][q + 4]) : car[c][0] - v[c][4];
+                        car[c][q] = q ? v[c][q] + v[c][q + 4] : v[c][4];
+                    }
+                    if (s >= 1) {  // back to the corners; plane 0 is the tile below's
+                        const dfloat y0 = node[0] - node[2], y1 = node[0] + node[2];
+                        const dfloat d0 = node[1] - node[3], d1 = node[1] + node[3];
+                        X[(4 * c) * kRThreads + tid] = y0 - d0;  // corner bx + 2 by
+                        X[(4 * c + 1) * kRThreads + tid] = y0 + d0;
+                        X[(4 * c + 2) * kRThreads + tid] = y1 - d1;
+                        X[(4 * c + 3) * kRThreads + tid] = y1 + d1;
+                    }
+                }
+                // plane s + 2 into the buffer of plane s, whose readers are behind the last barrier
+                if (s + 2 <= S) {
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    split(s + 2, fb);
+                    if (s + 3 <= S) load(s + 3, fb);
+                }
+            }
+            double fv[3] = {0.0, 0.0, 0.0};
+            const int64_t g = g0 + (int64_t)s * NY * pitch;
+            uint8_t fixed = 0;
+            if (s >= 1 && own) {
+                fixed = fix[fix0 + (int64_t)s * NY * NX];
+#pragma unroll
+                for (int c = 0; c < 3; c++) fv[c] = f64[g + c];
+            }
+            __syncthreads();
+            if (s >= 1 && own) {
+                // the node is corner (0, 0) of element (tx + 1, ty + 1), ...; the tile's last node
+                // of a side has no element beyond it
+                const bool right = tx + 1 < kREX, back = ty + 1 < kREY;
+                const dfloat *Xn = X + tid;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    double yv = 0.0;
+                    if (!u_zero) {
+                        dfloat y = Xn[(4 * c + 3) * kRThreads];
+                        if (right) y += Xn[(4 * c + 2) * kRThreads + 1];
+                        if (back) y += Xn[(4 * c + 1) * kRThreads + kREX];
+                        if (right && back) y += Xn[(4 * c) * kRThreads + kREX + 1];
+                        yv = df_to(y);
+                    }
+                    double rv = fv[c] - yv;
+                    if ((fixed >> c) & 1) rv = 0.0;
+                    r64[g + c] = rv;
+                    part = fma(rv, rv, part);
+                    if (need_ff) fpart = fma(fv[c], fv[c], fpart);
                 }
             }
         }
-        double part = 0.0, fpart = 0.0;
-#pragma unroll
-        for (int k = 0; k < kRNodesPerThread; k++) {
-            const int node = threadIdx.x + k * kThreads;
-            if (node >= kBN * kBN * kBN) continue;
-            const int ox = node % kBN, oy = (node / kBN) % kBN, oz = node / (kBN * kBN);
-            const int gx = gx0 + ox, gy = gy0 + oy, gz = gz0 + oz;
-            if (gx >= P.NX || gy >= P.NY || gz >= P.NZ) continue;
-            const int64_t gn = gx + (int64_t)P.NX * (gy + (int64_t)P.NY * gz);
-            const uint8_t fix = node_fix[P.node_off + gn];
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const int64_t gd = dof_index(P, gx, gy, gz, c);
-                const double fv = f64[gd];
-                double rv = fv - df_to(acc[k][c]);
-                if ((fix >> c) & 1) rv = 0.0;
-                r64[gd] = rv;
-                part = fma(rv, rv, part);
-                fpart = fma(fv, fv, fpart);
-            }
-        }
-        const double s = block_sum(part, red_sh);
-        const double sf = need_ff ? block_sum(fpart, red_sh) : 0.0;
-        if (threadIdx.x == 0) {
+        const double s = resid_sum(part, red_sh);
+        const double sf = need_ff ? resid_sum(fpart, red_sh) : 0.0;
+        if (tid == 0) {
             brick_part[bi] = s;
             brick_part[n_bricks + bi] = sf;
             __threadfence();
             const unsigned t = atomicAdd(&st->cnt_res, 1u);
             sh_last = (t == (unsigned)P.brick_count - 1);
         }
-        __syncthreads();
+        __syncthreads();  // also: the tile's last reads of the buffers are done
         if (sh_last) {
-            const double rr = ordered_sum(brick_part, P.brick_begin, P.brick_count);
-            const double ff = need_ff ? ordered_sum(brick_part + n_bricks, P.brick_begin, P.brick_count) : 0.0;
-            if (threadIdx.x == 0) {
+            auto total = [&](const double *v) {
+                double w = 0.0;
+                for (int i = tid; i < P.brick_count; i += kRThreads) w += __ldcg(v + P.brick_begin + i);
+                return resid_sum(w, red_sh);
+            };
+            const double rr = total(brick_part);
+            const double ff = need_ff ? total(brick_part + n_bricks) : 0.0;
+            if (tid == 0) {
                 st->cnt_res = 0;
                 if (need_ff) st->ff64 = ff > 0.0 ? ff : -1.0;  // -1: zero load (u = 0)
                 st->rr64 = rr;
@@ -3396,8 +3478,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     while (chunk < kMaxChunk && dofs0 > (int64_t)chunk * kWaveBlocks) chunk *= 2;
     for (size_t pi = 0; pi < b.h_probs.size(); pi++) {
         MfProblem &P = b.h_probs[pi];
-        if (P.nx <= 0 || P.ny <= 0 || P.nz <= 0 || P.nx >= 32767 * kBN || P.ny >= 32767 * kBN ||
-            P.nz >= 32767 * kBN) {
+        if (P.nx <= 0 || P.ny <= 0 || P.nz <= 0 || P.nx >= kMaxSide || P.ny >= kMaxSide || P.nz >= kMaxSide) {
             set_error("bad grid %dx%dx%d", P.nx, P.ny, P.nz);
             return MG_EINVAL;
         }
@@ -3422,7 +3503,15 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         P.node_off = nd;
         dof += P.n_pad;
         nd += (int64_t)P.NX * P.NY * P.NZ;
-        const int bx = (P.NX + kBN - 1) / kBN, by = (P.NY + kBN - 1) / kBN, bz = (P.NZ + kBN - 1) / kBN;
+        // tiles of the FP64 residual: as deep as one wave of resident tiles allows, up to kRMaxZ
+        // node planes (a layer more is evaluated than planes are owned).  In a batch several
+        // problems form their residual in the same step: an eighth of the slots each, whatever
+        // the others are (the tiles decide the order of the sum ||r||^2)
+        const int bx = (P.nx + kROwnX - 1) / kROwnX, by = (P.ny + kROwnY - 1) / kROwnY;
+        const int64_t res_slots = bottom_cluster ? 3LL * sms : 3LL * sms / 8;
+        const int64_t res_per = std::max<int64_t>(1, res_slots / ((int64_t)bx * by));
+        P.res_z = (int)std::max<int64_t>((P.NZ + 32766) / 32767, std::min<int64_t>(kRMaxZ, (P.NZ + res_per - 1) / res_per));
+        const int bz = (P.NZ + P.res_z - 1) / P.res_z;
         P.brick_begin = nb;
         P.brick_count = bx * by * bz;
         for (int k = 0; k < bz; k++)
@@ -3615,7 +3704,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.coarse_off, std::max<size_t>(1, b.h_coarse_off.size())));
     MG_TRY(dev_alloc_n(&b.coarse_inv, (size_t)std::max<int64_t>(1, inv_floats)));
     MG_TRY(dev_alloc_n(&b.coarse_ok, std::max<size_t>(1, b.h_coarse_off.size())));
-    b.apply_grid = std::max(1, std::min(nb, 2 * sms));  // FP64 residual: two CTAs per SM
+    b.res_grid = std::max(1, std::min(nb, 3 * sms));    // FP64 residual: three CTAs per SM
     b.col_grid = std::max(1, std::min(b.n_cols, kColCtas * sms));  // column CTAs per SM
     b.fac_grid = 2 * sms;                                     // two factored-operator CTAs per SM
     b.vec_grid = std::max(1, std::min(nc, 8 * sms));
@@ -4032,7 +4121,7 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
     const bool use_mg = prm.mg && b.n_levels > 1;
     const int maxit = prm.max_iterations > 0 ? prm.max_iterations : 100000;
     const int max_ref = prm.max_refinements > 0 ? prm.max_refinements : 30;
-    launch_pdl(mf_residual64_kernel, std::max(1, std::min(nb0, b.apply_grid)), kThreads, kResidSmem, s, 
+    launch_pdl(mf_residual64_kernel, std::max(1, std::min(nb0, b.res_grid)), kRThreads, kResidSmem, s, 
         b.probs, b.bricks, nb0, b.Edf, b.node_fix, b.u64, b.f64, b.facdf, b.r64, b.states,
         b.brick_part, prm.rtol * prm.rtol, max_ref, b.n_fine);
     launch_pdl(mf_inner_init_kernel, vg0, kThreads, 0, s, 

@@ -14,13 +14,7 @@
 
 namespace mg {
 
-// Owned-node brick edge; a brick reads the (kBN+2)^3 node halo and evaluates
-// the (kBN+1)^3 elements around its kBN^3 owned nodes.
-constexpr int kBN = 8;
-constexpr int kBE = kBN + 1;
-constexpr int kBU = kBN + 2;
-constexpr int kNEL = kBE * kBE * kBE;          // 729 elements per brick
-constexpr int kNTILE = (kNEL + 127) / 128;     // 6 MMA tiles of 128 elements
+constexpr int kMaxSide = 8 * 32767;            // elements a side (tile numbers are 16 bits)
 // Dofs per vector-kernel chunk, one to four float4 per thread: the fewest that leave no more
 // chunks than one wave of blocks (8 on each of 152 SMs).  With 4096 throughout, the two
 // vector kernels of a 16x8x8 iteration ran on two blocks each; the rule and the shorter sums
@@ -80,7 +74,8 @@ struct MfProblem {
     int64_t dof_off;      // offset into the concatenated padded dof vectors
     int64_t elem_off;     // offset into the padded element tables (E32, Edf, dE64)
     int64_t node_off;     // offset into the node Dirichlet masks (unpadded)
-    int brick_begin, brick_count;
+    int brick_begin, brick_count;  // tiles of the FP64 residual
+    int res_z;            // node planes per tile
     int chunk_begin, chunk_count;
     int col_begin, col_count;
     int col_z;            // node planes per column (kCZ or fewer for small grids)
@@ -220,7 +215,7 @@ struct MfBatch {
     std::vector<double> graph_key;    // parameters the graph was captured with
     long long graph_launches = 0;     // kernel nodes in the graph
     int enqueue_error = 0;            // an operator asked for a vector without a tensor map
-    int apply_grid = 0, vec_grid = 0, col_grid = 0, fac_grid = 0;
+    int res_grid = 0, vec_grid = 0, col_grid = 0, fac_grid = 0;
     cudaStream_t stream = nullptr;
 };
 
