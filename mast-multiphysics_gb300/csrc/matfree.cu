@@ -10,7 +10,7 @@
 //
 // The CG operator runs on the tensor cores by columns of nodes (mf_col_kernel), the
 // multigrid levels on the CUDA cores with the factored element stiffness
-// (mf_fac_kernel), the small levels in one CTA or one cluster per chain, and the
+// (mf_fac_kernel), the small levels of a chain on one thread-block cluster, and the
 // FP64 residual in double-float arithmetic (mf_residual64_kernel).  Every owned dof
 // adds its elements' contributions in a fixed order: no atomics, no colouring, one
 // global write per dof; tiles evaluate the elements of their one-element halo anew.
@@ -1443,301 +1443,30 @@ __global__ void mg_coarsen_kernel(const MfProblem *__restrict__ probs, int plo,
     }
 }
 
-// ------------------------------------------------------ bottom V-cycle (one CTA)
-// The small coarse levels of a design (from its chain head down to its
-// coarsest grid) are solved by one CTA per chain, entirely in shared memory,
-// in FP32 on the CUDA cores: the same Chebyshev-Jacobi smoothers, residuals,
-// restriction and prolongation as the level-by-level launches above, without
-// one launch per level operation.  Per level the shared memory holds x, b, r,
-// d, y, D^-1 (per dof, compact node-interleaved order) and E (per element).
-constexpr int kBottomThreads = 512;
-constexpr int kBottomSmemMax = 200 * 1024;  // per chain: 576 + sum over levels (18 NN + ne) floats
-constexpr int kBottomMaxHeadNodes = 2 * kBottomThreads;
-
-struct BottomLevel {
-    int NX, NY, NZ, nx, ny, nz;
-    float *x, *b, *r, *d, *y, *dinv, *E;
-};
-
-// y = A in on level L (0 on Dirichlet dofs; `in` is 0 there): node-centric
-// gather over the node's elements in a fixed order.  Levels of at most
-// kBottomLaneNodes nodes use eight lanes per node instead (lane d = dx + 2 dy +
-// 4 dz forms the node's rows of element node - d; the partial sums meet in a
-// fixed xor butterfly), which shortens the dependent chain per pass eightfold.
-constexpr int kBottomLaneNodes = kBottomThreads / 2;
-__device__ void bottom_apply(const BottomLevel &L, const float *sK, const float *in, float *out) {
-    const int nn = L.NX * L.NY * L.NZ;
-    if (nn <= kBottomLaneNodes) {
-        const int corner = threadIdx.x & 7;
-        const int dx = corner & 1, dy = (corner >> 1) & 1, dz = corner >> 2;
-        // this corner's 3 x 24 rows of K0 regrouped per neighbour corner bc (9 values in
-        // 12); corner blocks 100 floats apart, so the eight corners of a node read
-        // disjoint banks
-        const float4 *Kt = reinterpret_cast<const float4 *>(sK + 576 + 100 * corner_index(dx, dy, dz));
-        for (int base = 0; base < nn; base += kBottomThreads / 8) {
-            const int n = base + (threadIdx.x >> 3);
-            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-            if (n < nn) {
-                const int i = n % L.NX, j = (n / L.NX) % L.NY, k = n / (L.NX * L.NY);
-                const int ex = i - dx, ey = j - dy, ez = k - dz;
-                if (ex >= 0 && ey >= 0 && ez >= 0 && ex < L.nx && ey < L.ny && ez < L.nz) {
-                    const float e = L.E[ex + L.nx * (ey + L.ny * ez)];
-                    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
-#pragma unroll
-                    for (int bc = 0; bc < 8; bc++) {
-                        int bx, by, bz;
-                        corner_bits(bc, bx, by, bz);
-                        const float *u = in + 3 * ((ex + bx) + L.NX * ((ey + by) + L.NY * (ez + bz)));
-                        const float u0 = u[0], u1 = u[1], u2 = u[2];
-                        const float4 k0 = Kt[3 * bc], k1 = Kt[3 * bc + 1], k2 = Kt[3 * bc + 2];
-                        s0 = fmaf(k0.z, u2, fmaf(k0.y, u1, fmaf(k0.x, u0, s0)));
-                        s1 = fmaf(k1.y, u2, fmaf(k1.x, u1, fmaf(k0.w, u0, s1)));
-                        s2 = fmaf(k2.x, u2, fmaf(k1.w, u1, fmaf(k1.z, u0, s2)));
-                    }
-                    a0 = e * s0;
-                    a1 = e * s1;
-                    a2 = e * s2;
-                }
-            }
-#pragma unroll
-            for (int off = 1; off < 8; off <<= 1) {
-                a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-                a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-                a2 += __shfl_xor_sync(0xffffffffu, a2, off);
-            }
-            if (n < nn && corner < 3) {
-                const float a = corner == 0 ? a0 : (corner == 1 ? a1 : a2);
-                out[3 * n + corner] = L.dinv[3 * n + corner] == 0.0f ? 0.0f : a;
-            }
-        }
-        return;
-    }
-    for (int n = threadIdx.x; n < nn; n += kBottomThreads) {
-        const int i = n % L.NX, j = (n / L.NX) % L.NY, k = n / (L.NX * L.NY);
-        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-        for (int dz = 0; dz < 2; dz++)
-            for (int dy = 0; dy < 2; dy++)
-                for (int dx = 0; dx < 2; dx++) {
-                    const int ex = i - dx, ey = j - dy, ez = k - dz;
-                    if (ex < 0 || ey < 0 || ez < 0 || ex >= L.nx || ey >= L.ny || ez >= L.nz) continue;
-                    const float e = L.E[ex + L.nx * (ey + L.ny * ez)];
-                    const float *K = sK + 3 * corner_index(dx, dy, dz) * 24;
-                    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f;
-#pragma unroll
-                    for (int bc = 0; bc < 8; bc++) {
-                        int bx, by, bz;
-                        corner_bits(bc, bx, by, bz);
-                        const float *u = in + 3 * ((ex + bx) + L.NX * ((ey + by) + L.NY * (ez + bz)));
-#pragma unroll
-                        for (int c = 0; c < 3; c++) {
-                            s0 = fmaf(K[3 * bc + c], u[c], s0);
-                            s1 = fmaf(K[24 + 3 * bc + c], u[c], s1);
-                            s2 = fmaf(K[48 + 3 * bc + c], u[c], s2);
-                        }
-                    }
-                    a0 = fmaf(e, s0, a0);
-                    a1 = fmaf(e, s1, a1);
-                    a2 = fmaf(e, s2, a2);
-                }
-        out[3 * n] = L.dinv[3 * n] == 0.0f ? 0.0f : a0;
-        out[3 * n + 1] = L.dinv[3 * n + 1] == 0.0f ? 0.0f : a1;
-        out[3 * n + 2] = L.dinv[3 * n + 2] == 0.0f ? 0.0f : a2;
-    }
-}
-
-// x (+)= Chebyshev-Jacobi smoothing of degree deg for rhs rin (r, d, y scratch)
-__device__ void bottom_smooth(const BottomLevel &L, const float *sK, const float *rin, bool x0_zero, int deg,
-                              float inv_theta, const float *c1, const float *c2) {
-    const int nd = 3 * L.NX * L.NY * L.NZ;
-    for (int q = threadIdx.x; q < nd; q += kBottomThreads) {
-        const float rv = rin[q], dv = L.dinv[q] * rv * inv_theta;
-        L.r[q] = rv;
-        L.d[q] = dv;
-        L.x[q] = x0_zero ? dv : L.x[q] + dv;
-    }
-    __syncthreads();
-    for (int k = 1; k < deg; k++) {
-        bottom_apply(L, sK, L.d, L.y);
-        __syncthreads();
-        for (int q = threadIdx.x; q < nd; q += kBottomThreads) {
-            const float rv = L.r[q] - L.y[q];
-            const float dv = fmaf(c1[k], L.d[q], c2[k] * L.dinv[q] * rv);
-            L.r[q] = rv;
-            L.d[q] = dv;
-            L.x[q] += dv;
-        }
-        __syncthreads();
-    }
-}
-
-// r = b - A x  (0 on Dirichlet dofs)
-__device__ void bottom_residual(const BottomLevel &L, const float *sK) {
-    bottom_apply(L, sK, L.x, L.y);
-    __syncthreads();
-    const int nd = 3 * L.NX * L.NY * L.NZ;
-    for (int q = threadIdx.x; q < nd; q += kBottomThreads) L.r[q] = L.dinv[q] == 0.0f ? 0.0f : L.b[q] - L.y[q];
-    __syncthreads();
-}
-
+// ------------------------------------------------------------- bottom V-cycle
+// The small coarse levels of a design (from its chain head down to its coarsest
+// grid) are solved in one launch, entirely in shared memory, in FP32 on the CUDA
+// cores: the same Chebyshev-Jacobi smoothers, residuals, restriction and
+// prolongation as the level-by-level launches above, without one launch per level
+// operation (mg_bottom_cluster_kernel).
+//
 // Direct coarse solve: the coarsest grid of a bottom chain, when it has at most
 // kCoarseDirectMax dofs, is solved exactly with the inverse of its assembled
 // operator (FP32, formed on the device by mg_coarse_inverse_kernel) instead of a
 // Chebyshev smoother of degree cdeg: one matrix-vector product instead of cdeg - 1
-// operator applications, each a CTA-wide barrier round.  The operator is assembled from
+// operator applications, each a barrier round.  The operator is assembled from
 // the level's moduli and K0 like the level operators (Dirichlet dofs: identity
 // rows and zero columns), so the inverse is symmetric and the V-cycle stays a
 // fixed symmetric preconditioner.
+constexpr int kBottomSmemMax = 200 * 1024;
+// Nodes of the largest level that a batched design's chain starts at; a design of any batch
+// has the same chain.
+constexpr int kBatchMaxHeadNodes = 1024;
+
 struct BottomCheb {
     float inv_theta_s, inv_theta_c;
     float c1s[32], c2s[32], c1c[32], c2c[32];
 };
-
-__global__ void __launch_bounds__(kBottomThreads, 1) mg_bottom_kernel(
-    const MfProblem *__restrict__ probs, const int *__restrict__ heads, const MfState *states,
-    const float *__restrict__ E32, const float *__restrict__ dinv_g, const float *__restrict__ mb,
-    float *__restrict__ mx, const double *__restrict__ K0, BottomCheb cc, int sdeg, int cdeg,
-    const int64_t *__restrict__ coarse_off, const float *__restrict__ coarse_inv,
-    const int *__restrict__ coarse_ok) {
-    pdl_enter();
-    extern __shared__ __align__(16) float sbm[];
-    const int head = heads[blockIdx.x];
-    const MfProblem H = probs[head];
-    if (states[H.root].done) return;
-    float *sK = sbm;  // 576, then the regrouped copy for the eight-lane apply (8 x 100)
-    for (int i = threadIdx.x; i < 576; i += kBottomThreads) sK[i] = (float)K0[i];
-    for (int i = threadIdx.x; i < 800; i += kBottomThreads) {
-        const int a = i / 100, t = i % 100, bc = t / 12, q = t % 12, r = q / 3, c = q % 3;
-        sbm[576 + i] = (t < 96 && q < 9) ? (float)K0[(3 * a + r) * 24 + 3 * bc + c] : 0.0f;
-    }
-    // carve the levels of the chain
-    BottomLevel Lv[kBottomMaxLevels];
-    int pl[kBottomMaxLevels];
-    int m = 0;
-    float *p = sbm + 576 + 800;
-    for (int q = head; q >= 0 && m < kBottomMaxLevels; q = probs[q].coarse) {
-        const MfProblem P = probs[q];
-        BottomLevel &L = Lv[m];
-        L.NX = P.NX; L.NY = P.NY; L.NZ = P.NZ;
-        L.nx = P.nx; L.ny = P.ny; L.nz = P.nz;
-        const int nd = 3 * P.NX * P.NY * P.NZ, ne = P.nx * P.ny * P.nz;
-        L.x = p; p += nd;
-        L.b = p; p += nd;
-        L.r = p; p += nd;
-        L.d = p; p += nd;
-        L.y = p; p += nd;
-        L.dinv = p; p += nd;
-        L.E = p; p += ne;
-        pl[m] = q;
-        m++;
-    }
-    // the coarsest grid's inverse (direct solve), fetched with the level tables
-    const int64_t inv_off = coarse_ok[blockIdx.x] ? coarse_off[blockIdx.x] : -1;
-    float *sInv = p;
-    if (inv_off >= 0) {
-        const BottomLevel &Lc = Lv[m - 1];
-        const int ndc = 3 * Lc.NX * Lc.NY * Lc.NZ;
-        for (int i = threadIdx.x; i < ndc * ndc; i += kBottomThreads) sInv[i] = coarse_inv[inv_off + i];
-    }
-    // load E, D^-1 (and the rhs of the head) from the padded global layout
-    for (int l = 0; l < m; l++) {
-        const MfProblem P = probs[pl[l]];
-        BottomLevel &L = Lv[l];
-        const int ne = P.nx * P.ny * P.nz, nn = P.NX * P.NY * P.NZ;
-        for (int e = threadIdx.x; e < ne; e += kBottomThreads) {
-            const int ex = e % P.nx, ey = (e / P.nx) % P.ny, ez = e / (P.nx * P.ny);
-            L.E[e] = E32[P.elem_off + ((int64_t)ez * P.ny + ey) * P.pitch_e + ex];
-        }
-        for (int q = threadIdx.x; q < 3 * nn; q += kBottomThreads) {
-            const int n = q / 3, c = q - 3 * n;
-            const int i = n % P.NX, j = (n / P.NX) % P.NY, k = n / (P.NX * P.NY);
-            const int64_t g = dof_index(P, i, j, k, c);
-            L.dinv[q] = dinv_g[g];
-            if (l == 0) L.b[q] = L.dinv[q] == 0.0f ? 0.0f : mb[g];
-        }
-    }
-    __syncthreads();
-    // down: smooth, residual, restrict
-    for (int l = 0; l < m - 1; l++) {
-        bottom_smooth(Lv[l], sK, Lv[l].b, true, sdeg, cc.inv_theta_s, cc.c1s, cc.c2s);
-        bottom_residual(Lv[l], sK);
-        const BottomLevel &F = Lv[l], &C = Lv[l + 1];
-        const int ncd = 3 * C.NX * C.NY * C.NZ;
-        for (int q = threadIdx.x; q < ncd; q += kBottomThreads) {
-            const int n = q / 3, c = q - 3 * n;
-            const int I = n % C.NX, J = (n / C.NX) % C.NY, K = n / (C.NX * C.NY);
-            float out = 0.0f;
-            if (C.dinv[q] != 0.0f)
-                for (int dz = -1; dz <= 1; dz++) {
-                    const int kk = 2 * K + dz;
-                    if (kk < 0 || kk >= F.NZ) continue;
-                    for (int dy = -1; dy <= 1; dy++) {
-                        const int jj = 2 * J + dy;
-                        if (jj < 0 || jj >= F.NY) continue;
-                        for (int dx = -1; dx <= 1; dx++) {
-                            const int ii = 2 * I + dx;
-                            if (ii < 0 || ii >= F.NX) continue;
-                            const float w = (dx ? 0.5f : 1.0f) * (dy ? 0.5f : 1.0f) * (dz ? 0.5f : 1.0f);
-                            out = fmaf(w, F.r[3 * (ii + F.NX * (jj + F.NY * kk)) + c], out);
-                        }
-                    }
-                }
-            C.b[q] = out;
-        }
-        __syncthreads();
-    }
-    // coarsest grid of the chain: exact solve with the stored inverse, or smoothing
-    {
-        const BottomLevel &L = Lv[m - 1];
-        if (inv_off >= 0) {
-            // four lanes per row, partial sums met by two shuffles (fixed order)
-            const int nd = 3 * L.NX * L.NY * L.NZ, part = threadIdx.x & 3;
-            for (int q0 = 0; q0 < nd; q0 += kBottomThreads / 4) {
-                const int q = q0 + (threadIdx.x >> 2);
-                float sacc = 0.0f;
-                if (q < nd)
-                    for (int r = part; r < nd; r += 4) sacc = fmaf(sInv[q * nd + r], L.b[r], sacc);
-                sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
-                sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
-                if (q < nd && part == 0) L.x[q] = L.dinv[q] == 0.0f ? 0.0f : sacc;
-            }
-            __syncthreads();
-        } else {
-            bottom_smooth(Lv[m - 1], sK, Lv[m - 1].b, true, cdeg, cc.inv_theta_c, cc.c1c, cc.c2c);
-        }
-    }
-    // up: prolong, residual, post-smooth
-    for (int l = m - 2; l >= 0; l--) {
-        const BottomLevel &F = Lv[l], &C = Lv[l + 1];
-        const int nfd = 3 * F.NX * F.NY * F.NZ;
-        for (int q = threadIdx.x; q < nfd; q += kBottomThreads) {
-            if (F.dinv[q] == 0.0f) continue;
-            const int n = q / 3, c = q - 3 * n;
-            const int ii = n % F.NX, jj = (n / F.NX) % F.NY, kk = n / (F.NX * F.NY);
-            const int Is[2] = {ii >> 1, (ii + 1) >> 1}, Js[2] = {jj >> 1, (jj + 1) >> 1}, Ks[2] = {kk >> 1, (kk + 1) >> 1};
-            const float w = ((ii & 1) ? 0.5f : 1.0f) * ((jj & 1) ? 0.5f : 1.0f) * ((kk & 1) ? 0.5f : 1.0f);
-            float acc = 0.0f;
-            for (int a = 0; a < ((kk & 1) ? 2 : 1); a++)
-                for (int bb = 0; bb < ((jj & 1) ? 2 : 1); bb++)
-                    for (int cc2 = 0; cc2 < ((ii & 1) ? 2 : 1); cc2++)
-                        acc = fmaf(w, C.x[3 * (Is[cc2] + C.NX * (Js[bb] + C.NY * Ks[a])) + c], acc);
-            F.x[q] += acc;
-        }
-        __syncthreads();
-        bottom_residual(Lv[l], sK);
-        // post-smoothing on the residual: x += S(r) (the smoother starts from r in place)
-        bottom_smooth(Lv[l], sK, Lv[l].r, false, sdeg, cc.inv_theta_s, cc.c1s, cc.c2s);
-    }
-    // the head's correction back to the padded global layout
-    {
-        const MfProblem P = probs[head];
-        const int nn = P.NX * P.NY * P.NZ;
-        for (int q = threadIdx.x; q < 3 * nn; q += kBottomThreads) {
-            const int n = q / 3, c = q - 3 * n;
-            const int i = n % P.NX, j = (n / P.NX) % P.NY, k = n / (P.NX * P.NY);
-            mx[dof_index(P, i, j, k, c)] = Lv[0].x[q];
-        }
-    }
-}
 
 // FP32 inverse of a chain's coarsest-grid operator (the direct coarse solve), one
 // CTA per chain, formed whenever the chain's moduli change.  The operator is
@@ -1949,10 +1678,11 @@ __global__ void __launch_bounds__(kCoarseInvThreads, 1) mg_coarse_inverse_kernel
 }
 
 // ------------------------------------------------- bottom V-cycle on a cluster
-// The same bottom V-cycle as mg_bottom_kernel, spread over a thread-block
-// cluster of up to 16 CTAs so that a single design's chain can start at a larger
-// level, for a small design at its own grid: the whole V-cycle and r.z are then
-// one kernel (16x8x8, solve with sensitivities: 2.80 -> 2.24 ms).  CTA r owns the
+// A chain's V-cycle on a thread-block cluster of up to 16 CTAs: all 16 for a single
+// design, whose chain can start at a larger level, for a small design at its own
+// grid (the whole V-cycle and r.z are then one kernel; 16x8x8, solve with
+// sensitivities: 2.80 -> 2.24 ms); in a batch as many as leave every chain its
+// cluster at the same time.  CTA r owns the
 // nodes [r chunk, (r + 1) chunk) of every level of the chain and keeps their x, b,
 // r, d, y in its shared memory, with D^-1 of the nodes and the moduli of the
 // elements around them; a phase reads other CTAs' nodes through distributed shared
@@ -1960,7 +1690,9 @@ __global__ void __launch_bounds__(kCoarseInvThreads, 1) mg_coarse_inverse_kernel
 // separates the phases.  Global memory is touched only at the start (rhs, tables)
 // and at the end (the head's correction).  Every dof is computed by one thread in a
 // fixed order whatever the cluster size, so the correction does not depend on it
-// (r.z of a chain from the own grid does, in its rounding).
+// (r.z of a chain from the own grid does, in its rounding).  Batched chains: 58
+// problems 68 us a launch with one CTA a chain, K0 and the operand both read from
+// shared memory, 41 us with two.
 constexpr int kClusterThreads = 512;
 // Nodes of the largest level that a chain may start at, the design's own grid included: up to here
 // the cluster's phases on 16 SMs beat the level kernels on all of them (us an iteration of single
@@ -2023,7 +1755,8 @@ enum { kClX = 0, kClB, kClR, kClD, kClY };
 __device__ __forceinline__ int cl_slab(const ClusterLevel &L, int v) { return L.s_vec + v * 3 * L.chunk; }
 
 // One phase of the cluster V-cycle on level L: y = A in with eight lanes per node
-// (as bottom_apply), the elementwise update that follows it done by the lanes that
+// (lane dx + 2 dy + 4 dz forms the node's rows of the element node - d, the partial
+// sums meet in a fixed xor butterfly), the elementwise update that follows it done by the lanes that
 // hold each dof's sum, so that the phase needs no second barrier:
 //   step 0, residual:             in = x;   r = b - y
 //   step 1, first smoothing step: in = D^-1 rin theta (formed while staging rin);
@@ -2149,7 +1882,7 @@ __device__ __forceinline__ int cl_fine_addr(const float *sm, const ClusterLevel 
 }
 
 __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
-    const ClusterChain *__restrict__ chain, MfState *states, const float *__restrict__ E32,
+    const ClusterChain *__restrict__ chains, MfState *states, const float *__restrict__ E32,
     const float *__restrict__ dinv, const float *__restrict__ rhs, float *__restrict__ mx, bool from_root,
     const float *__restrict__ k0f, const __grid_constant__ BottomCheb cc, int sdeg, int cdeg,
     const int64_t *__restrict__ coarse_off, const float *__restrict__ coarse_inv, const int *__restrict__ coarse_ok) {
@@ -2163,8 +1896,9 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // (in shared memory: read by level from the constant bank, the tables slowed every phase)
     __shared__ ClusterChain ch;
+    const int chain = blockIdx.x / csize;
     for (int i = threadIdx.x; i < (int)(sizeof(ClusterChain) / 4); i += kClusterThreads)
-        reinterpret_cast<int *>(&ch)[i] = reinterpret_cast<const int *>(chain)[i];
+        reinterpret_cast<int *>(&ch)[i] = reinterpret_cast<const int *>(chains + chain)[i];
     __syncthreads();
     const int m = ch.m;
     int *smi = reinterpret_cast<int *>(sm);
@@ -2231,7 +1965,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) mg_bottom_cluster_kernel(
     }
     // the direct solve's rows of this CTA (one warp per row), loaded now
     const ClusterLevel &Lc = ch.L[m - 1];
-    const int64_t inv_off = coarse_ok[0] ? coarse_off[0] : -1;
+    const int64_t inv_off = coarse_ok[chain] ? coarse_off[chain] : -1;
     const int nnc = Lc.NXY * Lc.NZ, ndc = 3 * nnc;
     const int c0 = rank * Lc.chunk, crows = 3 * max(0, min(nnc, c0 + Lc.chunk) - c0);
     constexpr int kInvPer = (kCoarseDirectMax + 31) / 32;
@@ -3205,8 +2939,6 @@ int configure_kernels() {
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(4)));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(5)));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_fac_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, fac_smem(6)));
-    MG_CUDA_TRY(cudaFuncSetAttribute(mg_bottom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kBottomSmemMax));
     MG_CUDA_TRY(cudaFuncSetAttribute(mg_coarse_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kCoarseInvSmem));
     MG_CUDA_TRY(cudaFuncSetAttribute(mg_bottom_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -3580,105 +3312,85 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.n_pad = dof;
     b.n_elem_pad = el;
     b.n_nodes = nd;
-    // bottom chains: for every design, the first level below the finest with at
-    // most kBottomMaxHeadNodes nodes whose chain (it and all coarser levels) fits
-    // the bottom kernel's shared memory; larger levels run level by level on the
-    // whole GPU (the one-CTA kernel is bound by one SM's shared-memory pipe there).
-    // On a cluster (bottom_cluster: single-design solves), the first level with at
-    // most kClusterMaxHeadNodes nodes, the finest included.
-    // (a device on which no cluster of the bottom kernel can be placed falls back
-    // to the one-CTA chains)
+    // bottom chains: for every design, the first level below the finest with at most
+    // kBatchMaxHeadNodes nodes, larger levels run level by level on the whole GPU; for a
+    // single design (bottom_cluster) the first with at most kClusterMaxHeadNodes, the
+    // finest included.  Chains whose tables no cluster size can hold run level by level.
     int64_t inv_floats = 0;
-    for (int attempt = bottom_cluster && b.n_fine == 1 ? 0 : 1; attempt < 2; attempt++) {
-        const bool use_cluster = attempt == 0;
+    {
+        const bool single = bottom_cluster && b.n_fine == 1;
         b.h_heads.clear();
         b.h_head_root.clear();
         b.bottom_smem = 0;
         b.bottom_cluster = 0;
         b.chains_from_root = false;
         for (MfProblem &T : b.h_probs) T.bottom = 0;
-        for (int r = 0; r < b.n_fine; r++) {
-            // the cluster's chain may start at the design's own grid
-            const bool try_root = use_cluster && b.h_probs[r].coarse >= 0;
-            for (int q = try_root ? r : b.h_probs[r].coarse; q >= 0; q = b.h_probs[q].coarse) {
-                int64_t floats = 576 + 800, depth = 0;
-                for (int t = q; t >= 0; t = b.h_probs[t].coarse, depth++) {
-                    const MfProblem &T = b.h_probs[t];
-                    // x, b, r, d, y, D^-1 per dof and E per element
-                    floats += 18LL * T.NX * T.NY * T.NZ + (int64_t)T.nx * T.ny * T.nz;
-                }
-                const int64_t bytes = floats * 4;
+        for (int r = 0; r < b.n_fine; r++)
+            for (int q = single && b.h_probs[r].coarse >= 0 ? r : b.h_probs[r].coarse; q >= 0; q = b.h_probs[q].coarse) {
+                int64_t depth = 0;
+                for (int t = q; t >= 0; t = b.h_probs[t].coarse) depth++;
                 const MfProblem &Hd = b.h_probs[q];
                 const int64_t head_nodes = (int64_t)Hd.NX * Hd.NY * Hd.NZ;
-                const bool fits = use_cluster ? head_nodes <= kClusterMaxHeadNodes
-                                              : bytes <= kBottomSmemMax && head_nodes <= kBottomMaxHeadNodes;
-                if (depth <= kBottomMaxLevels && fits) {
-                    b.h_heads.push_back(q);
-                    b.h_head_root.push_back(r);
-                    b.bottom_smem = use_cluster ? 0 : std::max(b.bottom_smem, (int)bytes);
-                    for (int t = q; t >= 0; t = b.h_probs[t].coarse) b.h_probs[t].bottom = t != r;
-                    b.chains_from_root = q == r;
-                    break;
-                }
+                if (depth > kBottomMaxLevels || head_nodes > (single ? kClusterMaxHeadNodes : kBatchMaxHeadNodes)) continue;
+                b.h_heads.push_back(q);
+                b.h_head_root.push_back(r);
+                b.chains_from_root = q == r;
+                break;
+            }
+        // the largest clusters (16 CTAs: non-portable size) that the device can place for all
+        // chains at once, one CTA a chain where there are more chains than that.
+        // MASTGPU_BOTTOM_CLUSTER caps the cluster (1, 2, 4, 8 or 16 CTAs): a test knob,
+        // the correction does not depend on the cluster size
+        int cap = kClusterMax;
+        if (const char *env = std::getenv("MASTGPU_BOTTOM_CLUSTER")) cap = std::max(1, std::min(kClusterMax, std::atoi(env)));
+        int first = 1;
+        while (first * 2 <= cap) first *= 2;
+        for (int cs = first; cs >= 1 && !b.bottom_cluster && !b.h_heads.empty(); cs /= 2) {
+            if (cs > 1 && (int64_t)b.h_heads.size() * cs > sms) continue;
+            std::vector<ClusterChain> chains;
+            const int64_t smem = cluster_layout(b, cs, chains);
+            if (smem < 0 || smem > kBottomSmemMax) continue;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(cs * b.h_heads.size()));
+            cfg.blockDim = dim3(kClusterThreads);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)cs;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, mg_bottom_cluster_kernel, &cfg) == cudaSuccess &&
+                n >= (cs > 1 ? (int)b.h_heads.size() : 1)) {
+                b.bottom_cluster = cs;
+                b.bottom_smem = (int)smem;
+                b.h_cl_chains.swap(chains);
+            } else {
+                cudaGetLastError();  // clear the failed query
             }
         }
-        // direct coarse solves: the chains whose coarsest grid is small enough and
-        // whose inverse fits the bottom kernel's shared memory beside the levels
-        {
-            inv_floats = 0;
-            b.h_coarse_off.assign(b.h_heads.size(), -1);
-            for (size_t h = 0; h < b.h_heads.size(); h++) {
-                int64_t floats = 576 + 800;
-                int c = b.h_heads[h];
-                for (int t = c; t >= 0; t = b.h_probs[t].coarse) {
-                    const MfProblem &T = b.h_probs[t];
-                    floats += 18LL * T.NX * T.NY * T.NZ + (int64_t)T.nx * T.ny * T.nz;
-                    c = t;
-                }
-                const MfProblem &C = b.h_probs[c];
-                const int64_t nd = 3LL * C.NX * C.NY * C.NZ;
-                if (nd <= kCoarseDirectMax && (use_cluster || (floats + nd * nd) * 4 <= kBottomSmemMax)) {
-                    b.h_coarse_off[h] = inv_floats;
-                    inv_floats += nd * nd;
-                    if (!use_cluster) b.bottom_smem = std::max(b.bottom_smem, (int)((floats + nd * nd) * 4));
-                }
+        if (!b.bottom_cluster) {
+            b.h_heads.clear();
+            b.h_head_root.clear();
+            b.chains_from_root = false;
+        }
+        // the problems of the chains; direct coarse solves where the coarsest grid is small enough
+        b.h_coarse_off.assign(b.h_heads.size(), -1);
+        for (size_t h = 0; h < b.h_heads.size(); h++) {
+            int c = b.h_heads[h];
+            for (int t = c; t >= 0; t = b.h_probs[t].coarse) {
+                b.h_probs[t].bottom = t != b.h_head_root[h];
+                c = t;
+            }
+            const MfProblem &C = b.h_probs[c];
+            const int64_t nd = 3LL * C.NX * C.NY * C.NZ;
+            if (nd <= kCoarseDirectMax) {
+                b.h_coarse_off[h] = inv_floats;
+                inv_floats += nd * nd;
             }
         }
-        if (!use_cluster || b.h_heads.empty()) break;
-        {
-            // the largest cluster (16 CTAs: non-portable size) the device can place
-            // MASTGPU_BOTTOM_CLUSTER caps the cluster (1, 2, 4, 8 or 16 CTAs): a test knob,
-            // the correction does not depend on the cluster size
-            int cap = kClusterMax;
-            if (const char *env = std::getenv("MASTGPU_BOTTOM_CLUSTER")) cap = std::max(1, std::min(kClusterMax, std::atoi(env)));
-            int first = 1;
-            while (first * 2 <= cap) first *= 2;
-            for (int cs = first; cs >= 1 && !b.bottom_cluster; cs /= 2) {
-                std::vector<ClusterChain> chains;
-                const int64_t smem = cluster_layout(b, cs, chains);
-                if (smem < 0 || smem > kBottomSmemMax) continue;
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3(cs);
-                cfg.blockDim = dim3(kClusterThreads);
-                cfg.dynamicSmemBytes = smem;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeClusterDimension;
-                attr[0].val.clusterDim.x = (unsigned)cs;
-                attr[0].val.clusterDim.y = 1;
-                attr[0].val.clusterDim.z = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, mg_bottom_cluster_kernel, &cfg) == cudaSuccess && n >= 1) {
-                    b.bottom_cluster = cs;
-                    b.bottom_smem = (int)smem;
-                    b.h_cl_chains.swap(chains);
-                }
-                else
-                    cudaGetLastError();  // clear the failed query
-            }
-        }
-        if (b.bottom_cluster) break;
     }
     // node blocks of the transfers, by level: the coarse problems whose fine one is not inside a
     // bottom chain
@@ -3807,8 +3519,9 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         }
         MG_TRY(dev_alloc_n(&b.cl_k0, (size_t)kClusterK0));
         MG_CUDA_TRY(cudaMemcpyAsync(b.cl_k0, k0f.data(), k0f.size() * 4, cudaMemcpyHostToDevice, s));
-        MG_TRY(dev_alloc_n(&b.cl_chain, 1));
-        MG_CUDA_TRY(cudaMemcpyAsync(b.cl_chain, b.h_cl_chains.data(), sizeof(ClusterChain), cudaMemcpyHostToDevice, s));
+        MG_TRY(dev_alloc_n(&b.cl_chains, b.h_cl_chains.size()));
+        MG_CUDA_TRY(cudaMemcpyAsync(b.cl_chains, b.h_cl_chains.data(), b.h_cl_chains.size() * sizeof(ClusterChain),
+                                    cudaMemcpyHostToDevice, s));
         MG_CUDA_TRY(cudaStreamSynchronize(s));  // k0f is a host temporary
     }
     if (!b.h_coarse_off.empty()) {
@@ -3841,7 +3554,7 @@ void mf_batch_free(MfBatch &b) {
                     b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
                     b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_part, b.Bop2, b.fac_tiles, b.fac_maps, b.node_blks,
-                    b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chain, b.sens_offs};
+                    b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chains, b.sens_offs};
     for (void *q : ptrs) dev_free(q);
     if (b.stage_host) cudaFreeHost(b.stage_host);
     if (b.sens_offs_host) cudaFreeHost(b.sens_offs_host);
@@ -4043,8 +3756,8 @@ long long enqueue_smooth(MfBatch &b, bool fac, int prec, int l, const float *rin
 // A problem whose own coarsest grid is level l gets the coarse-grid smoother
 // (degree cdeg) there, whatever the depth of the other problems, so that each
 // problem's preconditioner does not depend on the batch it is solved in.  The
-// small levels of each chain (MfProblem::bottom) are done by one CTA per chain
-// (mg_bottom_kernel) between the down and the up sweep.
+// small levels of each chain (MfProblem::bottom) are done by one launch
+// (mg_bottom_cluster_kernel) between the down and the up sweep.
 long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
     const Cheb cs = cheb_coeffs(b.cheb_lmax, sdeg), cc = cheb_coeffs(b.cheb_lmax, cdeg);
     const int L = b.n_levels;
@@ -4080,15 +3793,10 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
             bc.c1s[k] = cs.c1[k]; bc.c2s[k] = cs.c2[k];
             bc.c1c[k] = cc.c1[k]; bc.c2c[k] = cc.c2[k];
         }
-        if (b.bottom_cluster)
-            launch_cluster_pdl(mg_bottom_cluster_kernel, (unsigned)b.bottom_cluster,
-                               kClusterThreads, b.bottom_smem, b.bottom_cluster, b.stream, b.cl_chain, b.states,
-                               b.E32, b.dinv, b.chains_from_root ? b.r : b.mb, b.mx, b.chains_from_root, b.cl_k0, bc, sdeg,
-                               cdeg, b.coarse_off, b.coarse_inv, b.coarse_ok);
-        else
-            launch_pdl(mg_bottom_kernel, (unsigned)b.h_heads.size(), kBottomThreads, b.bottom_smem, b.stream,
-                b.probs, b.heads, b.states, b.E32, b.dinv, b.mb, b.mx, b.K0, bc, sdeg, cdeg, b.coarse_off,
-                b.coarse_inv, b.coarse_ok);
+        launch_cluster_pdl(mg_bottom_cluster_kernel, (unsigned)(b.h_heads.size() * b.bottom_cluster),
+                           kClusterThreads, b.bottom_smem, b.bottom_cluster, b.stream, b.cl_chains, b.states, b.E32,
+                           b.dinv, b.chains_from_root ? b.r : b.mb, b.mx, b.chains_from_root, b.cl_k0, bc, sdeg, cdeg,
+                           b.coarse_off, b.coarse_inv, b.coarse_ok);
         n += 1;
     }
     for (int l = L - 2; l >= 0; l--) {

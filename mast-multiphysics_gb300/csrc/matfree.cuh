@@ -28,7 +28,7 @@ constexpr int kCX = 7;
 constexpr int kCY = 15;
 constexpr int kCZ = 32;   // most node planes per column
 constexpr int kMaxLevels = 8;                  // multigrid levels per design
-constexpr int kBottomMaxLevels = 6;            // levels of a bottom chain (one-CTA or cluster kernel)
+constexpr int kBottomMaxLevels = 6;            // levels of a bottom chain
 constexpr int kCoarseDirectMax = 144;          // most dofs of a coarsest grid that is solved directly
 
 // Whether a grid gets a coarser level (ceil(n / 2) elements a side): until its dofs fit the
@@ -85,7 +85,7 @@ struct MfProblem {
     int level;            // multigrid level (0 = the design's own grid)
     int root;             // level-0 problem whose solver state drives this one
     int coarse, fine;     // neighbouring levels (-1 if none)
-    int bottom;           // 1: solved inside the one-CTA bottom V-cycle of its chain
+    int bottom;           // 1: solved inside the bottom V-cycle of its chain
 };
 
 struct MfBrick {
@@ -194,10 +194,10 @@ struct MfBatch {
     float *coarse_inv = nullptr;
     int *coarse_ok = nullptr;
     int bottom_smem = 0;        // dynamic shared memory of the bottom kernel
-    int bottom_cluster = 0;     // CTAs per chain of the cluster bottom kernel (0: one-CTA kernel)
+    int bottom_cluster = 0;     // CTAs per chain of the bottom kernel (0: no chains)
     bool chains_from_root = false;  // the cluster chain starts at the design's own grid: the whole V-cycle
-    std::vector<ClusterChain> h_cl_chains;  // its chain's level tables (one: a single design)
-    ClusterChain *cl_chain = nullptr;
+    std::vector<ClusterChain> h_cl_chains;  // the chains' level tables
+    ClusterChain *cl_chains = nullptr;
     float *cl_k0 = nullptr;     // K0 in FP32, regrouped by corners
     // FP64 refinement vectors (padded layout)
     double *u64 = nullptr, *r64 = nullptr, *f64 = nullptr;
@@ -241,9 +241,9 @@ void hex8_box_stiffness(double hx, double hy, double hz, double nu, double K[576
 
 // shapes: the designs' own grids (level 0); max_levels > 1 adds the coarse
 // multigrid levels of every design (mg_coarsens);
-// bottom_cluster: the bottom V-cycle on a thread-block cluster from a larger level
-// on, the design's own grid included (one design only; batches keep the one-CTA
-// form, so a design's preconditioner is the same in every batch)
+// bottom_cluster: the bottom V-cycle from a larger level on, the design's own grid
+// included (one design only; in batches a design's preconditioner is the same in
+// every batch)
 int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, double hy,
                   double hz, double nu, cudaStream_t stream, int max_levels = kMaxLevels,
                   bool bottom_cluster = false);
