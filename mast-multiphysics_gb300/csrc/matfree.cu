@@ -28,6 +28,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
+#include <queue>
+#include <utility>
 
 #include "matfree.cuh"
 
@@ -353,7 +356,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
-// Columns col_lo .. col_hi-1; the input vector is tensor map `in_slot`.
+// This CTA's columns are order[offs[blockIdx.x]] ...; the input vector is tensor map `in_slot`.
 // MODE 1: CG step, gathered u = z + beta p_old (z = in_slot, p_old = map 1 +
 //         parity), p_new (owned) = u, q = A u, per-problem alpha = rz / (p.q).
 // MODE 2: y = rhs - A x.   MODE 3: y = A x.   (Both 0 on Dirichlet dofs.)
@@ -361,7 +364,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 // hand-offs) of *err and ends the block after its copies and MMAs have landed.
 template <int PREC, int MODE>
 __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
-    const MfProblem *__restrict__ probs, const MfCol *__restrict__ cols, int col_lo, int col_hi, int sel,
+    const MfProblem *__restrict__ probs, const MfCol *__restrict__ cols, const int *__restrict__ order,
+    const int *__restrict__ offs, int sel,
     const CUtensorMap *__restrict__ tmaps, int in_slot, int parity, const uint32_t *__restrict__ Bop2,
     const float *__restrict__ dinv, const float *__restrict__ rhs, float *__restrict__ p0,
     float *__restrict__ p1, float *__restrict__ y, MfState *states, double *__restrict__ col_part,
@@ -426,6 +430,9 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
+    // the work lists and the column and problem tables are constant: read the first before the wait
+    const int at0 = offs[blockIdx.x], at_end = offs[blockIdx.x + 1], ci0 = at0 < at_end ? order[at0] : -1;
+    if (tid == 0 && ci0 >= 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(probs + cols[ci0].prob));
     pdl_wait();
 
     if (warp == 0) {
@@ -438,9 +445,9 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
                 return !states[Q.root].done && !Q.bottom && (sel < 0 || sel == (Q.coarse < 0 ? 1 : 0));
             };
             bool ok = true;
-            int ci = col_lo + blockIdx.x;
-            while (ci < col_hi && !usable(ci)) ci += gridDim.x;
-            for (; ci < col_hi && ok;) {
+            for (int at = at0; at < at_end && ok; at++) {
+                const int ci = at == at0 ? ci0 : order[at];
+                if (!usable(ci)) continue;
                 const MfCol cl = cols[ci];
                 const MfProblem &P = probs[cl.prob];
                 const int x0 = cl.cx * kCX, y0 = cl.cy * kCY, z0 = cl.cz * P.col_z;
@@ -467,8 +474,6 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
                                     bar(kCBarRawFull + slot));
                     last_issue[slot] = (int)k;
                 }
-                ci += gridDim.x;
-                while (ci < col_hi && !usable(ci)) ci += gridDim.x;
             }
             if (ok) {
                 // sentinel: no data, the stream ends
@@ -868,7 +873,7 @@ struct FacArgs {
 // A TMA wait that exceeds its bound sets bit 4 of *err and ends the block.
 template <int MODE>
 __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
-    const MfProblem *__restrict__ probs, const MfCol *__restrict__ tiles, int t_lo, int t_hi, int sel,
+    const MfProblem *__restrict__ probs, const MfCol *__restrict__ tiles, const int *__restrict__ offs, int sel,
     const FacK2 K, const CUtensorMap *__restrict__ fmaps, const MfState *__restrict__ states, const FacArgs A,
     int *err) {
     pdl_trigger();
@@ -885,8 +890,9 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
         for (int k = 0; k < kFRing; k++) mbar_init(bar0 + 8 * k, 1);
     // the tile and problem tables are constant: bring the first tile's into the
     // caches while the previous kernel drains, then wait for its results
-    if (t_lo + (int)blockIdx.x < t_hi && tid == 0) {
-        const MfCol T0 = tiles[t_lo + blockIdx.x];
+    const int t_lo = offs[blockIdx.x], t_hi = offs[blockIdx.x + 1];  // this CTA's tiles
+    if (t_lo < t_hi && tid == 0) {
+        const MfCol T0 = tiles[t_lo];
         asm volatile("prefetch.global.L1 [%0];" ::"l"(probs + T0.prob));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(fmaps + (size_t)T0.prob * kFacMaps));
     }
@@ -897,7 +903,7 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
     bool failed = false;
     const bool third = MODE == 2 || MODE == 4 || MODE == 5 || (MODE == 6 && !A.x0_zero);
     const float2 neg1 = make_float2(-1.0f, -1.0f);
-    for (int ti = t_lo + blockIdx.x; ti < t_hi && !failed; ti += gridDim.x) {
+    for (int ti = t_lo; ti < t_hi && !failed; ti++) {
         const MfCol T = tiles[ti];
         const MfProblem P = probs[T.prob];
         if (states[P.root].done || P.bottom || (sel >= 0 && sel != (P.coarse < 0 ? 1 : 0))) continue;
@@ -2840,7 +2846,7 @@ void launch_cluster_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t 
 }
 
 struct ApplyArgs {
-    int col_lo, col_hi, in_slot, parity;  // column range
+    int level, in_slot, parity;
     const float *rhs;
     float *y;
     int sel = -1;  // -1 every problem; 0 problems with a coarser level; 1 those without
@@ -2848,11 +2854,9 @@ struct ApplyArgs {
 
 template <int PREC, int MODE>
 void launch_apply(MfBatch &b, const ApplyArgs &a) {
-    const int nc = a.col_hi - a.col_lo;
-    if (nc <= 0) return;
-    const int grid = std::max(1, std::min(nc, b.col_grid));
-    launch_pdl(mf_col_kernel<PREC, MODE>, grid, kColThreads, kColSmem, b.stream, 
-        b.probs, b.cols, a.col_lo, a.col_hi, a.sel, b.tmaps, a.in_slot, a.parity, b.Bop2, b.dinv,
+    if (!b.lvl_col_ctas[a.level]) return;
+    launch_pdl(mf_col_kernel<PREC, MODE>, b.lvl_col_ctas[a.level], kColThreads, kColSmem, b.stream, 
+        b.probs, b.cols, b.col_order, b.col_offs + b.lvl_col_off[a.level], a.sel, b.tmaps, a.in_slot, a.parity, b.Bop2, b.dinv,
         a.rhs, b.p0, b.p1, a.y, b.states, b.col_part, b.err);
 }
 
@@ -2882,15 +2886,14 @@ int fac_map_of(const MfBatch &b, const float *v) {
 }
 
 template <int MODE>
-void launch_fac(MfBatch &b, int lo, int hi, int sel, const FacArgs &a) {
+void launch_fac(MfBatch &b, int l, int sel, const FacArgs &a) {
     if (a.in_map < 0 || ((MODE == 2 || MODE == 4 || MODE == 5) && a.b_map < 0)) {
         b.enqueue_error = MG_EINVAL;  // reported by the caller of the enqueue
         return;
     }
-    if (hi <= lo) return;
-    const int grid = std::max(1, std::min(hi - lo, b.fac_grid));
-    launch_pdl(mf_fac_kernel<MODE>, grid, kFThreads, fac_smem(MODE), b.stream, b.probs, b.fac_tiles, lo, hi, sel, b.fac2,
-                                                                      b.fac_maps, b.states, a, b.err);
+    if (!b.lvl_fac_ctas[l]) return;
+    launch_pdl(mf_fac_kernel<MODE>, b.lvl_fac_ctas[l], kFThreads, fac_smem(MODE), b.stream, b.probs, b.fac_tiles,
+               b.fac_offs + b.lvl_fac_off[l], sel, b.fac2, b.fac_maps, b.states, a, b.err);
 }
 
 // y = A x (MODE 3) or rhs - A x (MODE 2; z, nullable: D^-1 y, the factored operator only)
@@ -2898,18 +2901,18 @@ template <int MODE>
 void launch_level_op(MfBatch &b, bool fac, int prec, int l, int in_slot, const float *x, const float *rhs,
                      float *y, int sel, float *z = nullptr) {
     if (fac) {
-        launch_fac<MODE>(b, b.lvl_fac_lo[l], b.lvl_fac_hi[l], sel,
+        launch_fac<MODE>(b, l, sel,
                          FacArgs{fac_map_of(b, x), rhs ? fac_map_of(b, rhs) : -1, y, z, nullptr, nullptr, 0.0f, 0.0f,
                                  0.0f, 0});
     } else {
-        ApplyArgs a{b.lvl_col_lo[l], b.lvl_col_hi[l], in_slot, 0, rhs, y, sel};
+        ApplyArgs a{l, in_slot, 0, rhs, y, sel};
         launch_apply_prec<MODE>(b, prec, a);
     }
 }
 
 // CG step on the level-0 bricks (z from map in_slot)
 void launch_cg_apply(MfBatch &b, int prec, int in_slot, int parity) {
-    ApplyArgs a{b.lvl_col_lo[0], b.lvl_col_hi[0], in_slot, parity, nullptr, b.q};
+    ApplyArgs a{0, in_slot, parity, nullptr, b.q};
     launch_apply_prec<1>(b, prec, a);
 }
 
@@ -3149,6 +3152,118 @@ int64_t cluster_layout(const MfBatch &b, int cs, std::vector<ClusterChain> &chai
     return most;
 }
 
+// Work of unequal size dealt to the CTAs of a grid: the largest first, each to the CTA with the
+// least so far (Graham's longest-processing-time rule), equal ones in their order.  order: the
+// pieces CTA by CTA; offs: where each CTA's begin (ctas + 1 entries).  Returns the largest load.
+int deal_work(const std::vector<int> &cost, int ctas, std::vector<int> &order, std::vector<int> &offs) {
+    std::vector<int> by(cost.size());
+    for (size_t i = 0; i < by.size(); i++) by[i] = (int)i;
+    std::stable_sort(by.begin(), by.end(), [&](int a, int c) { return cost[a] > cost[c]; });
+    std::vector<std::vector<int>> own(ctas);
+    typedef std::pair<int, int> Load;  // (load, CTA)
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+    for (int c = 0; c < ctas; c++) heap.push(Load(0, c));
+    int most = 0;
+    for (int i : by) {
+        const Load l = heap.top();
+        heap.pop();
+        own[l.second].push_back(i);
+        most = std::max(most, l.first + cost[i]);
+        heap.push(Load(l.first + cost[i], l.second));
+    }
+    order.clear();
+    offs.assign(1, 0);
+    for (int c = 0; c < ctas; c++) {
+        order.insert(order.end(), own[c].begin(), own[c].end());
+        offs.push_back((int)order.size());
+    }
+    return most;
+}
+
+// Tiles of the factored operator, by level: kFNX x kFNY owned nodes, fac_z node planes.  A tile
+// costs its planes, one element layer more, and about two layers for its start (tables, first
+// loads).  The depth (at most kFMaxZ, the same rule for all problems of the level) is the one
+// whose tiles, dealt out, leave the least to the busiest CTA.  With the deepest tiles dealt round
+// robin, the busiest CTA had 96 layers where the mean is 49 (58 problems of 16x8x8 to 96x48x48) and
+// 69 where it is 34 (two of 192x96x96); MODE 2 on level 0 took 86 and 73 us there, dealt so 66 and 56.
+void plan_fac_tiles(MfBatch &b, int ctas) {
+    b.h_fac_tiles.clear();
+    b.h_fac_offs.clear();
+    b.lvl_fac_off.clear();
+    b.lvl_fac_ctas.clear();
+    for (int l = 0; l < b.n_levels; l++) {
+        auto depth = [](const MfProblem &P, int cap) {
+            const int parts = std::min(32767, (P.NZ + cap - 1) / cap);  // tile numbers are 16 bits
+            return (P.NZ + parts - 1) / parts;
+        };
+        auto tiles_of = [&](int cap, std::vector<MfCol> &tiles, std::vector<int> &cost) {
+            tiles.clear();
+            cost.clear();
+            for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++) {
+                const MfProblem &P = b.h_probs[pi];
+                if (P.bottom) continue;  // solved inside its chain
+                const int tx = (P.NX + kFNX - 1) / kFNX, ty = (P.NY + kFNY - 1) / kFNY, z = depth(P, cap);
+                for (int k = 0; k * z < P.NZ; k++)
+                    for (int j = 0; j < ty; j++)
+                        for (int i = 0; i < tx; i++) {
+                            tiles.push_back(MfCol{pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
+                            cost.push_back(std::min(z, P.NZ - k * z) + 3);
+                        }
+            }
+        };
+        std::vector<MfCol> tiles;
+        std::vector<int> cost, order, offs;
+        int best = 0, best_cap = kFMaxZ;
+        int64_t layers = 0;
+        for (int cap = kFMaxZ; cap >= kFMinZ; cap = cap > 16 ? cap - 8 : cap > 8 ? cap - 2 : cap - 1) {
+            tiles_of(cap, tiles, cost);
+            layers = 0;
+            for (int c : cost) layers += c;
+            if (best && layers >= (int64_t)best * ctas) break;  // shallower tiles only add layers
+            const int most = deal_work(cost, ctas, order, offs);
+            if (!best || most < best) {
+                best = most;
+                best_cap = cap;
+            }
+        }
+        tiles_of(best_cap, tiles, cost);
+        const int used = (int)std::min<int64_t>(ctas, (int64_t)tiles.size());
+        deal_work(cost, used, order, offs);
+        for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++) b.h_probs[pi].fac_z = depth(b.h_probs[pi], best_cap);
+        const int base = (int)b.h_fac_tiles.size();
+        b.lvl_fac_off.push_back((int)b.h_fac_offs.size());
+        b.lvl_fac_ctas.push_back(used);
+        for (int o : offs) b.h_fac_offs.push_back(base + o);
+        for (int i : order) b.h_fac_tiles.push_back(tiles[i]);
+    }
+}
+
+// The columns of the tensor-core operator, by level, dealt out in the same way (58 problems, round
+// robin: 209 layers on the busiest CTA where the mean is 156, 180 us a launch; dealt so 165).  Their numbers, by which the partial
+// sums of p.q are kept, stay those of their problem.
+void plan_cols(MfBatch &b, int ctas) {
+    b.h_col_order.clear();
+    b.h_col_offs.clear();
+    b.lvl_col_off.clear();
+    b.lvl_col_ctas.clear();
+    for (int l = 0; l < b.n_levels; l++) {
+        std::vector<int> cols, cost, order, offs;
+        for (int pi = b.lvl_prob_lo[l]; pi < b.lvl_prob_hi[l]; pi++) {
+            const MfProblem &P = b.h_probs[pi];
+            for (int c = P.col_begin; c < P.col_begin + P.col_count && !P.bottom; c++) {
+                cols.push_back(c);
+                cost.push_back(std::min(P.col_z, P.NZ - b.h_cols[c].cz * P.col_z) + 1);
+            }
+        }
+        const int used = std::min<int>(ctas, (int)cols.size()), base = (int)b.h_col_order.size();
+        deal_work(cost, used, order, offs);
+        b.lvl_col_off.push_back((int)b.h_col_offs.size());
+        b.lvl_col_ctas.push_back(used);
+        for (int o : offs) b.h_col_offs.push_back(base + o);
+        for (int i : order) b.h_col_order.push_back(cols[i]);
+    }
+}
+
 int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, double hy,
                   double hz, double nu, cudaStream_t stream, int max_levels, bool bottom_cluster) {
     MG_TRY(configure_kernels());
@@ -3200,7 +3315,6 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.h_bricks.clear();
     b.h_chunks.clear();
     b.h_cols.clear();
-    b.h_fac_tiles.clear();
     std::vector<int64_t> level_count(b.n_levels + 1, 0);  // problems per multigrid level
     for (const MfProblem &P : b.h_probs) level_count[P.level]++;
     int64_t dofs0 = 0;  // of the designs' own grids, which the vector kernels run over
@@ -3265,21 +3379,6 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
             for (int j = 0; j < cy; j++)
                 for (int i = 0; i < cx; i++)
                     b.h_cols.push_back(MfCol{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
-        // tiles of the factored operator: kFNX x kFNY owned nodes, fac_z node
-        // planes (kFMinZ .. kFMaxZ): as deep as one wave of resident tiles allows
-        {
-            const int tx = (P.NX + kFNX - 1) / kFNX, ty = (P.NY + kFNY - 1) / kFNY;
-            const int64_t fac_slots = 2 * (int64_t)sms;
-            const int64_t per_col = std::max<int64_t>(1, fac_slots / ((int64_t)tx * ty * level_count[P.level]));
-            P.fac_z = (int)std::min<int64_t>(kFMaxZ, std::max<int64_t>(kFMinZ, (P.NZ + per_col - 1) / per_col));
-            const int tz = (P.NZ + P.fac_z - 1) / P.fac_z;
-            P.fac_begin = (int)b.h_fac_tiles.size();
-            P.fac_count = tx * ty * tz;
-            for (int k = 0; k < tz; k++)
-                for (int j = 0; j < ty; j++)
-                    for (int i = 0; i < tx; i++)
-                        b.h_fac_tiles.push_back(MfCol{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
-        }
         P.chunk_begin = nc;
         P.chunk_count = (int)((P.n_pad + chunk - 1) / chunk);
         for (int c = 0; c < P.chunk_count; c++) {
@@ -3296,16 +3395,10 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.n_chunks = nc;
     b.n_cols = (int)b.h_cols.size();
     b.lvl_brick_lo.clear(); b.lvl_brick_hi.clear(); b.lvl_chunk_lo.clear(); b.lvl_chunk_hi.clear();
-    b.lvl_col_lo.clear(); b.lvl_col_hi.clear();
-    b.lvl_fac_lo.clear(); b.lvl_fac_hi.clear();
     for (int l = 0; l < b.n_levels; l++) {
         const MfProblem &A = b.h_probs[b.lvl_prob_lo[l]], &Z = b.h_probs[b.lvl_prob_hi[l] - 1];
         b.lvl_brick_lo.push_back(A.brick_begin);
         b.lvl_brick_hi.push_back(Z.brick_begin + Z.brick_count);
-        b.lvl_col_lo.push_back(A.col_begin);
-        b.lvl_col_hi.push_back(Z.col_begin + Z.col_count);
-        b.lvl_fac_lo.push_back(A.fac_begin);
-        b.lvl_fac_hi.push_back(Z.fac_begin + Z.fac_count);
         b.lvl_chunk_lo.push_back(A.chunk_begin);
         b.lvl_chunk_hi.push_back(Z.chunk_begin + Z.chunk_count);
     }
@@ -3392,6 +3485,8 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
             }
         }
     }
+    plan_fac_tiles(b, 2 * sms);  // two factored-operator CTAs per SM
+    plan_cols(b, kColCtas * sms);
     // node blocks of the transfers, by level: the coarse problems whose fine one is not inside a
     // bottom chain
     {
@@ -3417,14 +3512,15 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.coarse_inv, (size_t)std::max<int64_t>(1, inv_floats)));
     MG_TRY(dev_alloc_n(&b.coarse_ok, std::max<size_t>(1, b.h_coarse_off.size())));
     b.res_grid = std::max(1, std::min(nb, 3 * sms));    // FP64 residual: three CTAs per SM
-    b.col_grid = std::max(1, std::min(b.n_cols, kColCtas * sms));  // column CTAs per SM
-    b.fac_grid = 2 * sms;                                     // two factored-operator CTAs per SM
     b.vec_grid = std::max(1, std::min(nc, 8 * sms));
     MG_TRY(dev_alloc_n(&b.probs, b.h_probs.size()));
     MG_TRY(dev_alloc_n(&b.bricks, b.h_bricks.size()));
     MG_TRY(dev_alloc_n(&b.cols, b.h_cols.size()));
+    MG_TRY(dev_alloc_n(&b.col_order, b.h_col_order.size()));
+    MG_TRY(dev_alloc_n(&b.col_offs, b.h_col_offs.size()));
     MG_TRY(dev_alloc_n(&b.col_part, b.h_cols.size()));
     MG_TRY(dev_alloc_n(&b.fac_tiles, std::max<size_t>(1, b.h_fac_tiles.size())));
+    MG_TRY(dev_alloc_n(&b.fac_offs, b.h_fac_offs.size()));
     MG_TRY(dev_alloc_n(&b.Bop2, 4096));
     MG_TRY(dev_alloc_n(&b.chunks, b.h_chunks.size()));
     MG_TRY(dev_alloc_n(&b.states, (size_t)b.n_probs));
@@ -3497,9 +3593,14 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_CUDA_TRY(cudaMemcpyAsync(b.probs, b.h_probs.data(), b.h_probs.size() * sizeof(MfProblem), cudaMemcpyHostToDevice, s));
     MG_CUDA_TRY(cudaMemcpyAsync(b.bricks, b.h_bricks.data(), b.h_bricks.size() * sizeof(MfBrick), cudaMemcpyHostToDevice, s));
     MG_CUDA_TRY(cudaMemcpyAsync(b.cols, b.h_cols.data(), b.h_cols.size() * sizeof(MfCol), cudaMemcpyHostToDevice, s));
-    if (!b.h_fac_tiles.empty())
-        MG_CUDA_TRY(cudaMemcpyAsync(b.fac_tiles, b.h_fac_tiles.data(), b.h_fac_tiles.size() * sizeof(MfCol),
-                                    cudaMemcpyHostToDevice, s));
+    MG_CUDA_TRY(cudaMemcpyAsync(b.col_order, b.h_col_order.data(), b.h_col_order.size() * sizeof(int),
+                                cudaMemcpyHostToDevice, s));
+    MG_CUDA_TRY(cudaMemcpyAsync(b.col_offs, b.h_col_offs.data(), b.h_col_offs.size() * sizeof(int),
+                                cudaMemcpyHostToDevice, s));
+    MG_CUDA_TRY(cudaMemcpyAsync(b.fac_tiles, b.h_fac_tiles.data(), b.h_fac_tiles.size() * sizeof(MfCol),
+                                cudaMemcpyHostToDevice, s));
+    MG_CUDA_TRY(cudaMemcpyAsync(b.fac_offs, b.h_fac_offs.data(), b.h_fac_offs.size() * sizeof(int),
+                                cudaMemcpyHostToDevice, s));
     {
         std::vector<uint32_t> bop2;
         pack_b_columns(K0, bop2);
@@ -3553,7 +3654,7 @@ void mf_batch_free(MfBatch &b) {
     void *ptrs[] = {b.probs, b.bricks, b.chunks, b.states, b.tmaps, b.E32, b.Edf, b.dE64,
                     b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
-                    b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_part, b.Bop2, b.fac_tiles, b.fac_maps, b.node_blks,
+                    b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_order, b.col_offs, b.col_part, b.Bop2, b.fac_tiles, b.fac_offs, b.fac_maps, b.node_blks,
                     b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chains, b.sens_offs};
     for (void *q : ptrs) dev_free(q);
     if (b.stage_host) cudaFreeHost(b.stage_host);
@@ -3646,10 +3747,10 @@ int mf_apply(MfBatch &b, int precision, const double *x_host, double *y_host, in
     MG_CUDA_TRY(cudaMemcpyAsync(b.mx + P.dof_off, pad.data(), P.n_pad * 4, cudaMemcpyHostToDevice, b.stream));
     MG_CUDA_TRY(cudaMemsetAsync(b.states, 0, b.n_probs * sizeof(MfState), b.stream));
     if (precision == MG_OPERATOR_FACTORED_FP32) {
-        launch_fac<3>(b, P.fac_begin, P.fac_begin + P.fac_count, -1,
+        launch_fac<3>(b, P.level, -1,
                       FacArgs{kFMapMx, -1, b.my, nullptr, nullptr, nullptr, 0.0f, 0.0f, 0.0f, 0});
     } else {
-        ApplyArgs a{P.col_begin, P.col_begin + P.col_count, 4, 0, nullptr, b.my};
+        ApplyArgs a{P.level, 4, 0, nullptr, b.my};
         launch_apply_prec<3>(b, precision, a);
     }
     MG_CUDA_TRY(cudaGetLastError());
@@ -3720,20 +3821,19 @@ long long enqueue_smooth(MfBatch &b, bool fac, int prec, int l, const float *rin
     if (fac && deg >= 2) {
         // fused, from z = D^-1 rin (in b.z): the first two steps in one launch, then one launch
         // per step, the direction alternating md / my (md is never rin)
-        const int lo = b.lvl_fac_lo[l], hi = b.lvl_fac_hi[l];
         if (deg == 2) {
-            launch_fac<6>(b, lo, hi, sel,
+            launch_fac<6>(b, l, sel,
                           FacArgs{kFMapZ, kFMapMx, nullptr, nullptr, nullptr, b.mx, cc.c1[1], cc.c2[1], cc.inv_theta,
                                   x0_zero});
             return 1;
         }
-        launch_fac<5>(b, lo, hi, sel,
+        launch_fac<5>(b, l, sel,
                       FacArgs{kFMapZ, fac_map_of(b, rin), b.md, nullptr, b.mr, b.mx, cc.c1[1], cc.c2[1], cc.inv_theta,
                               x0_zero});
         float *din = b.md, *dout = b.my;
         long long n = 1;
         for (int k = 2; k < deg; k++) {
-            launch_fac<4>(b, lo, hi, sel,
+            launch_fac<4>(b, l, sel,
                           FacArgs{fac_map_of(b, din), kFMapMr, dout, nullptr, b.mr, b.mx, cc.c1[k], cc.c2[k], 0.0f, 0});
             std::swap(din, dout);
             n += 1;

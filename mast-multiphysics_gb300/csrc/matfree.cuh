@@ -79,7 +79,6 @@ struct MfProblem {
     int chunk_begin, chunk_count;
     int col_begin, col_count;
     int col_z;            // node planes per column (kCZ or fewer for small grids)
-    int fac_begin, fac_count;
     int fac_z;            // node planes per tile of the factored CUDA-core operator
     int share_elems;      // >= 0: reuse the element tables of that problem (load cases)
     int level;            // multigrid level (0 = the design's own grid)
@@ -147,7 +146,8 @@ struct MfBatch {
     MfCol *cols = nullptr;
     std::vector<MfCol> h_cols;
     int n_cols = 0;
-    std::vector<int> lvl_col_lo, lvl_col_hi;
+    int *col_order = nullptr, *col_offs = nullptr;  // the columns CTA by CTA and where each CTA's begin, by level
+    std::vector<int> h_col_order, h_col_offs, lvl_col_off, lvl_col_ctas;
     double *col_part = nullptr;   // per-column partial of p.q
     uint32_t *Bop2 = nullptr;     // K0 as the column operator's four (dy, dz) B tiles
     MfNodeBlk *node_blks = nullptr;  // of the level transfers, by coarse level
@@ -155,7 +155,8 @@ struct MfBatch {
     MfCol *fac_tiles = nullptr;   // tiles of the factored CUDA-core operator (cx, cy, cz)
     CUtensorMap *fac_maps = nullptr;  // its tensor maps per problem (node vectors, moduli)
     std::vector<MfCol> h_fac_tiles;
-    std::vector<int> lvl_fac_lo, lvl_fac_hi;
+    int *fac_offs = nullptr;      // where each CTA's tiles begin, by level
+    std::vector<int> h_fac_offs, lvl_fac_off, lvl_fac_ctas;
     FacK<float> fac32{};          // K0 in the per-axis sum/difference basis
     FacK<double> fac64{};
     FacK<dfloat> facdf{};         // fac64 as double-float pairs (the outer residual)
@@ -215,7 +216,7 @@ struct MfBatch {
     std::vector<double> graph_key;    // parameters the graph was captured with
     long long graph_launches = 0;     // kernel nodes in the graph
     int enqueue_error = 0;            // an operator asked for a vector without a tensor map
-    int res_grid = 0, vec_grid = 0, col_grid = 0, fac_grid = 0;
+    int res_grid = 0, vec_grid = 0;
     cudaStream_t stream = nullptr;
 };
 
