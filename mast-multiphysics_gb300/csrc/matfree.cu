@@ -888,13 +888,20 @@ __global__ void __launch_bounds__(kFThreads, 2) mf_fac_kernel(
     const uint32_t bar0 = smem_u32(&bars[0]);
     if (tid == 0)
         for (int k = 0; k < kFRing; k++) mbar_init(bar0 + 8 * k, 1);
-    // the tile and problem tables are constant: bring the first tile's into the
-    // caches while the previous kernel drains, then wait for its results
+    // the work lists, tile and problem tables and the tensor maps are constant: bring the first
+    // tile's into the caches while the previous kernel drains, then wait for its results
     const int t_lo = offs[blockIdx.x], t_hi = offs[blockIdx.x + 1];  // this CTA's tiles
-    if (t_lo < t_hi && tid == 0) {
-        const MfCol T0 = tiles[t_lo];
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(probs + T0.prob));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(fmaps + (size_t)T0.prob * kFacMaps));
+    if (tid == 0) {
+        const int p0 = tiles[t_lo].prob;
+        const char *line = reinterpret_cast<const char *>(probs + p0);
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(line));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(line + 128));
+        const CUtensorMap *m0 = fmaps + (size_t)p0 * kFacMaps;
+        auto prefetch = [&](int k) { asm volatile("prefetch.tensormap [%0];" ::"l"(m0 + k) : "memory"); };
+        prefetch(A.in_map);
+        prefetch(kFMapDinv);
+        prefetch(kFMapE);
+        if (NP == 3 && A.b_map >= 0) prefetch(A.b_map);
     }
     pdl_wait();
     __syncthreads();
