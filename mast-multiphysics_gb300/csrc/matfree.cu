@@ -3373,12 +3373,16 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
                     b.h_bricks.push_back(MfBrick{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
         nb += P.brick_count;
         // columns of the tensor-core operator: as deep as one wave of resident
-        // columns allows (the level's problems share the 3 x SM slots), 4 to kCZ
-        // node planes; a second, partial wave would double the launch's time
+        // columns allows (the level's problems share the CTA slots), up to kCZ
+        // node planes; a second, partial wave would double the launch's time.  A single
+        // small grid's columns are as short as the slots allow, one plane and two element
+        // layers at the least: 16x8x8 54.8 us an iteration with four planes at least, 52.4 with
+        // one; 48x24x24 108.3 and 106.1.  In a batch four at least: a small design's columns,
+        // and with them the order of its p.q, are the same whatever the batch holds
         const int cx = (P.NX + kCX - 1) / kCX, cy = (P.NY + kCY - 1) / kCY;
         const int64_t slots = kColCtas * (int64_t)sms;
         const int64_t col_per = std::max<int64_t>(1, slots / ((int64_t)cx * cy * level_count[P.level]));
-        P.col_z = (int)std::min<int64_t>(kCZ, std::max<int64_t>(4, (P.NZ + col_per - 1) / col_per));
+        P.col_z = (int)std::min<int64_t>(kCZ, std::max<int64_t>(bottom_cluster ? 1 : 4, (P.NZ + col_per - 1) / col_per));
         const int cz = (P.NZ + P.col_z - 1) / P.col_z;
         P.col_begin = (int)b.h_cols.size();
         P.col_count = cx * cy * cz;
