@@ -2335,12 +2335,13 @@ __global__ void __launch_bounds__(kThreads) mf_refine_kernel(
 // after the refinement update: a stopped inner CG sends its problem back to the
 // FP64 residual, or ends it on a breakdown / NaN (one block).  LOOP: the last kernel of a
 // while-loop body; the loop goes on while a problem is unfinished, no wait has timed out
-// and fewer than `limit` bodies have run since the launch (loop[0]; loop[1] counts them all).
+// and fewer than `limit` bodies have run since the launch (loop[0]).  loop[1] counts all
+// bodies, of nested loops those inside (mf_gate_kernel) and loop[2] those around them.
 constexpr int kPhaseThreads = 256;
 template <bool LOOP>
 __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states, int n_fine,
                                                                  cudaGraphConditionalHandle handle, int *loop,
-                                                                 int limit, const int *err) {
+                                                                 int limit, bool nested, const int *err) {
     pdl_enter();
     int active = 0;
     for (int i = threadIdx.x; i < n_fine; i += kPhaseThreads) {
@@ -2363,12 +2364,26 @@ __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states
     if (LOOP) {
         active = __syncthreads_or(active);
         if (threadIdx.x == 0) {
-            const bool more = active && loop[0] + 1 < limit && *err == 0;
-            loop[0] = more ? loop[0] + 1 : 0;
-            loop[1] += 1;
+            const int bodies = loop[0] + 1;
+            const bool more = active && bodies < limit && *err == 0;
+            loop[0] = more ? bodies : 0;
+            loop[nested ? 2 : 1] += 1;
             cudaGraphSetConditional(handle, more ? 1u : 0u);
         }
     }
+}
+
+// The CG loop of a single problem inside its refinement loop goes on while its inner CG does
+// (count: the last kernel of a body; else before the loop).
+__global__ void mf_gate_kernel(const MfState *states, cudaGraphConditionalHandle handle, int *loop, int limit,
+                               bool count, const int *err) {
+    pdl_enter();
+    if (count) {
+        loop[0] += 1;
+        loop[1] += 1;
+    }
+    const bool more = states[0].phase == kPhaseCG && !states[0].done && loop[0] < limit && *err == 0;
+    cudaGraphSetConditional(handle, more ? 1u : 0u);
 }
 
 // FP64 outer residual r = f - K u (double-float arithmetic, factored element
@@ -3552,7 +3567,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.chunk_part, (size_t)2 * nc));
     MG_TRY(dev_alloc_n(&b.err, kErrWords));
     MG_CUDA_TRY(cudaMallocHost(&b.err_host, kErrWords * sizeof(int)));
-    b.loop_bodies = 0;
+    b.loop_bodies = b.loop_outer = 0;
     MG_TRY(dev_alloc_n(&b.diag_list, (size_t)b.n_probs + b.h_heads.size()));
     MG_TRY(dev_alloc_n(&b.sens_offs, (size_t)std::max(1, b.n_fine)));
     MG_CUDA_TRY(cudaMallocHost(&b.sens_offs_host, (size_t)std::max(1, b.n_fine) * sizeof(int64_t)));
@@ -3930,22 +3945,28 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
 //   FP64 residual + stop test (RESID) | inner CG start (INIT) |
 //   [multigrid z = M r, rz, beta] | p, q = A p, alpha | x, r, stop test |
 //   u += d of stopped inner solves | phase transitions.
-// loop_end: this step ends the body of a while loop on that handle (nullable).
 constexpr int kLoopBodies = 64;  // bodies of one loop launch at most: the host looks at the clock between launches
-long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
-                       const cudaGraphConditionalHandle *loop_end = nullptr) {
-    cudaStream_t s = b.stream;
+
+// the residual and the start of the inner CG
+long long enqueue_refine_begin(MfBatch &b, const MfSolveParams &prm) {
     const int n0 = b.lvl_chunk_hi[0], nb0 = b.lvl_brick_hi[0];
     const int vg0 = std::max(1, std::min(n0, b.vec_grid));
-    const bool use_mg = prm.mg && b.n_levels > 1;
     const int maxit = prm.max_iterations > 0 ? prm.max_iterations : 100000;
     const int max_ref = prm.max_refinements > 0 ? prm.max_refinements : 30;
-    launch_pdl(mf_residual64_kernel, std::max(1, std::min(nb0, b.res_grid)), kRThreads, kResidSmem, s, 
+    launch_pdl(mf_residual64_kernel, std::max(1, std::min(nb0, b.res_grid)), kRThreads, kResidSmem, b.stream,
         b.probs, b.bricks, nb0, b.Edf, b.node_fix, b.u64, b.f64, b.facdf, b.r64, b.states,
         b.brick_part, prm.rtol * prm.rtol, max_ref, b.n_fine);
-    launch_pdl(mf_inner_init_kernel, vg0, kThreads, 0, s, 
+    launch_pdl(mf_inner_init_kernel, vg0, kThreads, 0, b.stream,
         b.chunks, n0, b.probs, b.r64, b.x, b.r, b.z, b.p0, b.p1, b.dinv, b.states, b.chunk_part,
         prm.inner_rtol * prm.inner_rtol, maxit, b.n_fine);
+    return 2;
+}
+
+// one iteration of the inner CG
+long long enqueue_cg(MfBatch &b, const MfSolveParams &prm, int parity) {
+    const int n0 = b.lvl_chunk_hi[0];
+    const int vg0 = std::max(1, std::min(n0, b.vec_grid));
+    const bool use_mg = prm.mg && b.n_levels > 1;
     long long n = 2;
     float *pnew = parity ? b.p0 : b.p1;
     if (use_mg) {
@@ -3953,25 +3974,69 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
         const int cdeg = prm.coarse_deg > 0 ? prm.coarse_deg : 8;
         n += enqueue_vcycle(b, prm.mg_operator == 0, mg_precision(prm.precision), sdeg, cdeg);
         if (!b.chains_from_root) {
-            launch_pdl(mf_dot_rz_kernel, vg0, kThreads, 0, s, b.chunks, n0, b.probs, b.r, b.mx, b.states, b.chunk_part);
+            launch_pdl(mf_dot_rz_kernel, vg0, kThreads, 0, b.stream, b.chunks, n0, b.probs, b.r, b.mx, b.states,
+                       b.chunk_part);
             n += 1;
         }
         launch_cg_apply(b, prm.precision, 4, parity);  // p = z + beta p_old, q = A p, alpha
         launch_update(b, pnew, true);                  // x, r, stop test
-        n += 2;
     } else {
         launch_cg_apply(b, prm.precision, 0, parity);
         launch_update(b, pnew, false);                 // also z = D^-1 r, beta
-        n += 2;
     }
-    launch_pdl(mf_refine_kernel, vg0, kThreads, 0, s, b.chunks, b.probs, b.n_fine, b.x, b.u64, b.states);
-    if (loop_end)
-        launch_pdl(mf_phase_kernel<true>, 1, kPhaseThreads, 0, s, b.states, b.n_fine, *loop_end, b.err + 1, kLoopBodies,
-                   b.err);
+    return n;
+}
+
+// the refinement update and the phase transitions; loop_end: the end of a while loop's body on
+// that handle (nullable)
+long long enqueue_refine_end(MfBatch &b, const cudaGraphConditionalHandle *loop_end, bool nested) {
+    const int vg0 = std::max(1, std::min(b.lvl_chunk_hi[0], b.vec_grid));
+    if (nested)  // behind a loop, not behind a kernel: no programmatic launch
+        mf_refine_kernel<<<vg0, kThreads, 0, b.stream>>>(b.chunks, b.probs, b.n_fine, b.x, b.u64, b.states);
     else
-        launch_pdl(mf_phase_kernel<false>, 1, kPhaseThreads, 0, s, b.states, b.n_fine, cudaGraphConditionalHandle{},
-                   nullptr, 0, nullptr);
-    return n + 2;
+        launch_pdl(mf_refine_kernel, vg0, kThreads, 0, b.stream, b.chunks, b.probs, b.n_fine, b.x, b.u64, b.states);
+    if (loop_end)
+        launch_pdl(mf_phase_kernel<true>, 1, kPhaseThreads, 0, b.stream, b.states, b.n_fine, *loop_end, b.err + 1,
+                   kLoopBodies, nested, b.err);
+    else
+        launch_pdl(mf_phase_kernel<false>, 1, kPhaseThreads, 0, b.stream, b.states, b.n_fine,
+                   cudaGraphConditionalHandle{}, nullptr, 0, false, nullptr);
+    return 2;
+}
+
+// a while node in graph g behind deps; its body graph
+cudaError_t add_while(cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, cudaGraphConditionalHandle &handle,
+                      cudaGraphNode_t &node, cudaGraph_t &body) {
+    cudaError_t e = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
+    if (e != cudaSuccess) return e;
+    cudaGraphNodeParams np = {};
+    np.type = cudaGraphNodeTypeConditional;
+    np.conditional.handle = handle;
+    np.conditional.type = cudaGraphCondTypeWhile;
+    np.conditional.size = 1;
+    e = cudaGraphAddNode(&node, g, deps.empty() ? nullptr : deps.data(), nullptr, deps.size(), &np);
+    if (e == cudaSuccess) body = np.conditional.phGraph_out[0];
+    return e;
+}
+
+// what `enqueue` launches, captured into graph g behind deps; last: the nodes it ends on
+template <typename Enqueue>
+cudaError_t capture_into(cudaStream_t s, cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, Enqueue enqueue,
+                         std::vector<cudaGraphNode_t> *last = nullptr) {
+    cudaError_t e = cudaStreamBeginCaptureToGraph(s, g, deps.empty() ? nullptr : deps.data(), nullptr, deps.size(),
+                                                  cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    enqueue();
+    if (last) {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t *nodes = nullptr;
+        size_t n = 0;
+        e = cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &nodes, nullptr, &n);
+        if (e == cudaSuccess && status == cudaStreamCaptureStatusActive) last->assign(nodes, nodes + n);
+    }
+    cudaGraph_t captured = nullptr;
+    const cudaError_t e2 = cudaStreamEndCapture(s, &captured);  // the same graph as g
+    return e != cudaSuccess ? e : e2;
 }
 
 // CUDA graph of `chunk` solver steps (even: the p0/p1 roles alternate per step),
@@ -3979,13 +4044,16 @@ long long enqueue_step(MfBatch &b, const MfSolveParams &prm, int parity,
 // device ends, else they run once per launch.  A solve to completion that returned to the
 // host after every two steps spent 20 us a round trip on it (16x8x8 2.60 -> 2.24 ms looped,
 // 48x24x24 4.64 -> 4.26, 128x64x64 8.21 -> 7.83); the request loop launches single bodies,
-// between which it admits requests.
+// between which it admits requests.  A single problem's CG steps loop inside its refinement
+// loop, so that they do not launch the refinement's four kernels each time to find nothing to do
+// (1.4 to 2.9 us apiece: 90x46x38 6.59 -> 6.51 ms, 64x32x32 BF16X3 6.63 -> 6.59);
+// the problems of a batch are in different phases.
 int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop) {
     const std::vector<double> key = {(double)prm.precision, (double)chunk, (double)prm.mg,
                                      (double)prm.smooth_deg, (double)prm.coarse_deg, prm.rtol,
                                      prm.inner_rtol, (double)prm.max_iterations,
                                      (double)prm.max_refinements, (double)b.vec_grid,
-                                     (double)prm.mg_operator, loop ? 1.0 : 0.0};
+                                     (double)prm.mg_operator, loop ? (b.n_fine == 1 ? 2.0 : 1.0) : 0.0};
     if (b.graph && b.graph_key == key) return MG_OK;
     if (b.graph) {
         cudaGraphExecDestroy(b.graph);
@@ -3993,31 +4061,43 @@ int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop)
     }
     cudaGraph_t g = nullptr;
     MG_CUDA_TRY(cudaGraphCreate(&g, 0));
-    cudaGraph_t body = g;
-    cudaGraphConditionalHandle handle{};
-    cudaError_t e = cudaSuccess;
-    if (loop) {
-        e = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
-        if (e == cudaSuccess) {
-            cudaGraphNodeParams np = {};
-            np.type = cudaGraphNodeTypeConditional;
-            np.conditional.handle = handle;
-            np.conditional.type = cudaGraphCondTypeWhile;
-            np.conditional.size = 1;
-            cudaGraphNode_t node;
-            e = cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &np);
-            if (e == cudaSuccess) body = np.conditional.phGraph_out[0];
-        }
-    }
-    long long n = 0;
+    const bool nested = loop && b.n_fine == 1;
+    cudaGraph_t body = g, inner = nullptr;
+    cudaGraphConditionalHandle handle{}, inner_handle{};
+    cudaGraphNode_t node;
+    cudaError_t e = loop ? add_while(g, {}, handle, node, body) : cudaSuccess;
+    long long n = 0, n_outer = 0;
     b.enqueue_error = 0;
-    if (e == cudaSuccess)
-        e = cudaStreamBeginCaptureToGraph(b.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        for (int it = 0; it < chunk; it++)
-            n += enqueue_step(b, prm, it & 1, loop && it == chunk - 1 ? &handle : nullptr);
-        cudaGraph_t captured = nullptr;
-        e = cudaStreamEndCapture(b.stream, &captured);  // the same graph as body
+    if (e == cudaSuccess && nested) {
+        // the refinement's start and the first decision; the CG loop; the refinement's end.  The
+        // inner loop's handle belongs to the outer body, so its node is made before the capture
+        // of what sets it, and the edge to it afterwards.
+        std::vector<cudaGraphNode_t> last;
+        e = add_while(body, {}, inner_handle, node, inner);
+        if (e == cudaSuccess)
+            e = capture_into(b.stream, body, {}, [&] {
+                n_outer += enqueue_refine_begin(b, prm);
+                launch_pdl(mf_gate_kernel, 1, 1, 0, b.stream, b.states, inner_handle, b.err + 1, kLoopBodies, false, b.err);
+                n_outer += 1;
+            }, &last);
+        for (size_t k = 0; k < last.size() && e == cudaSuccess; k++)
+            e = cudaGraphAddDependencies(body, &last[k], &node, nullptr, 1);
+        if (e == cudaSuccess)
+            e = capture_into(b.stream, inner, {}, [&] {
+                for (int it = 0; it < chunk; it++) n += enqueue_cg(b, prm, it & 1);
+                launch_pdl(mf_gate_kernel, 1, 1, 0, b.stream, b.states, inner_handle, b.err + 1, kLoopBodies, true, b.err);
+                n += 1;
+            });
+        if (e == cudaSuccess)
+            e = capture_into(b.stream, body, {node}, [&] { n_outer += enqueue_refine_end(b, &handle, true); });
+    } else if (e == cudaSuccess) {
+        e = capture_into(b.stream, body, {}, [&] {
+            for (int it = 0; it < chunk; it++) {
+                n += enqueue_refine_begin(b, prm);
+                n += enqueue_cg(b, prm, it & 1);
+                n += enqueue_refine_end(b, loop && it == chunk - 1 ? &handle : nullptr, false);
+            }
+        });
     }
     if (e != cudaSuccess) {
         cudaGraphDestroy(g);
@@ -4038,6 +4118,7 @@ int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop)
     }
     b.graph_key = key;
     b.graph_launches = n;
+    b.graph_outer = n_outer;
     return MG_OK;
 }
 
@@ -4047,7 +4128,7 @@ int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop)
 //   r = f - K u (FP64);  stop when ||r|| <= rtol ||f||;
 //   solve A d = r / ||r|| with FP32 CG to inner_rtol (Jacobi or multigrid
 //   V-cycle preconditioned);  u += ||r|| d.
-// The phases run on the device (enqueue_step); the host only relaunches the
+// The phases run on the device (build_step_graph); the host only relaunches the
 // step graph until every active problem has finished.
 int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm, bool loop) {
     const bool use_mg = prm.mg && b.n_levels > 1;
@@ -4118,8 +4199,10 @@ int mf_batch_step_begin(MfBatch &b) {
 int mf_batch_step_end(MfBatch &b) {
     MG_CUDA_TRY(cudaStreamSynchronize(b.stream));
     // a loop launch reports the bodies it has run
-    count_launches(b.graph_launches * (b.graph_key.back() != 0.0 ? b.err_host[2] - b.loop_bodies : 1));
+    count_launches(b.graph_launches * (b.graph_key.back() != 0.0 ? b.err_host[2] - b.loop_bodies : 1) +
+                   b.graph_outer * (b.err_host[3] - b.loop_outer));
     b.loop_bodies = b.err_host[2];
+    b.loop_outer = b.err_host[3];
     if (*b.err_host) {
         set_error("tensor-core pipeline wait exceeded its bound (error flag %d)", *b.err_host);
         return MG_ETIMEDOUT;

@@ -131,7 +131,7 @@ struct MfState {
     unsigned cnt_apply, cnt_update, cnt_res, pad;
 };
 
-constexpr int kErrWords = 3;
+constexpr int kErrWords = 4;  // error flag; bodies of this launch, of all loops, of all outer loops
 
 struct MfBatch {
     int n_probs = 0;
@@ -165,7 +165,7 @@ struct MfBatch {
     MfState *states = nullptr;
     MfState *states_host = nullptr;  // pinned
     int *err_host = nullptr;         // pinned copy of err
-    int loop_bodies = 0;             // loop bodies run up to the last copy
+    int loop_bodies = 0, loop_outer = 0;  // loop bodies run up to the last copy
     CUtensorMap *tmaps = nullptr;    // kMapsPerProblem per problem
     // element / node tables
     float *E32 = nullptr;
@@ -214,7 +214,8 @@ struct MfBatch {
     double hx = 1, hy = 1, hz = 1, nu = 0.3;
     cudaGraphExec_t graph = nullptr;  // solver steps (see enqueue_step)
     std::vector<double> graph_key;    // parameters the graph was captured with
-    long long graph_launches = 0;     // kernel nodes in the graph
+    long long graph_launches = 0;     // kernel nodes in the graph or its innermost loop body
+    long long graph_outer = 0;        // and in the body of the loop around it
     int enqueue_error = 0;            // an operator asked for a vector without a tensor map
     int res_grid = 0, vec_grid = 0;
     cudaStream_t stream = nullptr;
