@@ -2639,36 +2639,44 @@ __global__ void __launch_bounds__(kRThreads, 3) mf_residual64_kernel(
 }
 
 // Jacobi inverse of the mixed operator: 1 / sum_e E_e K0[3a+c][3a+c];
-// 0 on Dirichlet dofs and padding (marks them for the vector kernels)
-__global__ void mf_diag_kernel(const MfProblem *__restrict__ probs, const int *__restrict__ list,
-                               const float *__restrict__ E32, const uint8_t *__restrict__ node_fix,
-                               const double *__restrict__ K0, float *__restrict__ dinv) {
-    const int pi = list ? list[blockIdx.y] : (int)blockIdx.y;
-    const MfProblem P = probs[pi];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < P.n_pad;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t row = i / P.pitch;
-        const int xin = (int)(i - row * P.pitch);
-        float out = 0.0f;
-        if (xin < 3 * P.NX) {
-            const int gx = xin / 3, c = xin - 3 * gx;
-            const int gy = (int)(row % P.NY), gz = (int)(row / P.NY);
-            const int64_t gn = gx + (int64_t)P.NX * (gy + (int64_t)P.NY * gz);
+// 0 on Dirichlet dofs and padding (marks them for the vector kernels).  Blocks of some 2,048
+// words, whole grid rows (j, k), from a list of all problems; a thread per word.  (A grid of the
+// largest problem's blocks times the problems, 64-bit divisions and K0 converted from FP64 in
+// every thread: 58 designs with their levels 536 us, 131 us so.)
+__host__ __device__ constexpr int diag_rows(int pitch) { return pitch >= 2048 ? 1 : 2048 / pitch; }
+__global__ void __launch_bounds__(256) mf_diag_kernel(const MfProblem *__restrict__ probs,
+                                                      const MfNodeBlk *__restrict__ blks,
+                                                      const float *__restrict__ E32, const uint8_t *__restrict__ node_fix,
+                                                      const double *__restrict__ K0, float *__restrict__ dinv) {
+    __shared__ float sk[24];  // the diagonal of K0
+    if (threadIdx.x < 24) sk[threadIdx.x] = (float)K0[25 * threadIdx.x];
+    const MfNodeBlk B = blks[blockIdx.x];
+    const MfProblem &P = probs[B.prob];
+    const int NX = P.NX, NY = P.NY, nx = P.nx, ny = P.ny, nz = P.nz, pitch = P.pitch;
+    const int row1 = min(B.node + diag_rows(pitch), NY * P.NZ);
+    const float *E = E32 + P.elem_off;
+    const uint8_t *fix = node_fix + P.node_off;
+    float *out = dinv + P.dof_off;
+    __syncthreads();
+    for (int i = threadIdx.x; i < (row1 - B.node) * pitch; i += 256) {
+        const int row = B.node + i / pitch, xin = i % pitch;
+        float v = 0.0f;
+        if (xin < 3 * NX) {
+            const int gx = xin / 3, c = xin - 3 * gx, gy = row % NY, gz = row / NY;
             // FP32 (the Jacobi inverse is stored in FP32; GB300's FP64 pipe issues two
             // DFMA per cycle per SM), the node's elements in a fixed order
             float d = 0.0f;
-            for (int dz = 0; dz < 2; dz++)
-                for (int dy = 0; dy < 2; dy++)
-                    for (int dx = 0; dx < 2; dx++) {
-                        const int ex = gx - dx, ey = gy - dy, ez = gz - dz;
-                        if (ex < 0 || ey < 0 || ez < 0 || ex >= P.nx || ey >= P.ny || ez >= P.nz) continue;
-                        const int k = 3 * corner_index(dx, dy, dz) + c;
-                        d = fmaf(E32[P.elem_off + ((int64_t)ez * P.ny + ey) * P.pitch_e + ex], (float)K0[k * 24 + k], d);
-                    }
-            const bool fixed = (node_fix[P.node_off + gn] >> c) & 1;
-            out = (fixed || d == 0.0f) ? 0.0f : 1.0f / d;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+                const int ex = gx - dx, ey = gy - dy, ez = gz - dz;
+                if (ex < 0 || ey < 0 || ez < 0 || ex >= nx || ey >= ny || ez >= nz) continue;
+                d = fmaf(E[((int64_t)ez * ny + ey) * P.pitch_e + ex], sk[3 * corner_index(dx, dy, dz) + c], d);
+            }
+            const bool fixed = (fix[(int64_t)row * NX + gx] >> c) & 1;
+            v = (fixed || d == 0.0f) ? 0.0f : 1.0f / d;
         }
-        dinv[P.dof_off + i] = out;
+        out[(int64_t)row * pitch + xin] = v;
     }
 }
 
@@ -3017,45 +3025,43 @@ void launch_update(MfBatch &b, float *pnew, bool mg) {
         b.chunks, n0, b.probs, b.x, b.r, b.z, pnew, b.q, b.dinv, b.states, b.chunk_part, mg ? 1 : 0);
 }
 
-int compute_diag(MfBatch &b) {
-    int64_t maxpad = 1;
-    for (const MfProblem &P : b.h_probs) maxpad = std::max(maxpad, P.n_pad);
-    dim3 grid(std::max(1u, std::min(blocks_for(maxpad, 256), 4096u)), b.n_probs);
-    mf_diag_kernel<<<grid, 256, 0, b.stream>>>(b.probs, nullptr, b.E32, b.node_fix, b.K0, b.dinv);
+// Jacobi inverse of blocks [lo, hi) of the list
+int launch_diag(MfBatch &b, int lo, int hi) {
+    if (hi <= lo) return MG_OK;
+    mf_diag_kernel<<<hi - lo, 256, 0, b.stream>>>(b.probs, b.diag_blks + lo, b.E32, b.node_fix, b.K0, b.dinv);
     MG_CUDA_TRY(cudaGetLastError());
     count_launches(1);
+    return MG_OK;
+}
+
+int compute_diag(MfBatch &b) {
+    MG_TRY(launch_diag(b, 0, b.diag_at.back()));
     return MG_OK;  // the operator-only paths need no coarse inverse; activation forms it
 }
 
 // Jacobi inverse of the listed level-0 problems and all their coarse levels, and
 // the inverse of the coarsest grid of their direct chains; nothing waits on the host
 int compute_diag_list(MfBatch &b, const std::vector<int> &level0) {
-    std::vector<int> list, inv;
-    int64_t maxpad = 1;
-    for (int i : level0)
-        for (int q = i; q >= 0; q = b.h_probs[q].coarse) {
-            list.push_back(q);
-            maxpad = std::max(maxpad, b.h_probs[q].n_pad);
-        }
-    if (list.empty()) return MG_OK;
+    std::vector<int> inv;
+    if (level0.empty()) return MG_OK;
     for (size_t h = 0; h < b.h_heads.size(); h++)
         if (b.h_coarse_off[h] >= 0 && std::find(level0.begin(), level0.end(), b.h_head_root[h]) != level0.end())
             inv.push_back((int)h);
-    // the pinned staging buffer: the previous call's copy must have read it
-    if (b.stage_pending) MG_CUDA_TRY(cudaEventSynchronize(b.stage_ev));
-    memcpy(b.stage_host, list.data(), list.size() * sizeof(int));
-    memcpy(b.stage_host + list.size(), inv.data(), inv.size() * sizeof(int));
-    MG_CUDA_TRY(cudaMemcpyAsync(b.diag_list, b.stage_host, (list.size() + inv.size()) * sizeof(int),
-                                cudaMemcpyHostToDevice, b.stream));
-    MG_CUDA_TRY(cudaEventRecord(b.stage_ev, b.stream));
-    b.stage_pending = true;
-    dim3 grid(std::max(1u, std::min(blocks_for(maxpad, 256), 4096u)), (unsigned)list.size());
-    mf_diag_kernel<<<grid, 256, 0, b.stream>>>(b.probs, b.diag_list, b.E32, b.node_fix, b.K0, b.dinv);
-    MG_CUDA_TRY(cudaGetLastError());
-    count_launches(1);
+    // the blocks of a problem and its coarse levels are neighbours in the list
+    if ((int)level0.size() == b.n_fine) {
+        MG_TRY(launch_diag(b, 0, b.diag_at.back()));
+    } else {
+        for (int i : level0) MG_TRY(launch_diag(b, b.diag_at[i], b.diag_at[i + 1]));
+    }
     if (!inv.empty()) {
+        // the pinned staging buffer: the previous call's copy must have read it
+        if (b.stage_pending) MG_CUDA_TRY(cudaEventSynchronize(b.stage_ev));
+        memcpy(b.stage_host, inv.data(), inv.size() * sizeof(int));
+        MG_CUDA_TRY(cudaMemcpyAsync(b.inv_list, b.stage_host, inv.size() * sizeof(int), cudaMemcpyHostToDevice, b.stream));
+        MG_CUDA_TRY(cudaEventRecord(b.stage_ev, b.stream));
+        b.stage_pending = true;
         mg_coarse_inverse_kernel<<<(unsigned)inv.size(), kCoarseInvThreads, kCoarseInvSmem, b.stream>>>(
-            b.probs, b.heads, b.diag_list + list.size(), b.E32, b.dinv, b.K0, b.coarse_off, b.coarse_inv,
+            b.probs, b.heads, b.inv_list, b.E32, b.dinv, b.K0, b.coarse_off, b.coarse_inv,
             b.coarse_ok);
         MG_CUDA_TRY(cudaGetLastError());
         count_launches(1);
@@ -3568,10 +3574,24 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.err, kErrWords));
     MG_CUDA_TRY(cudaMallocHost(&b.err_host, kErrWords * sizeof(int)));
     b.loop_bodies = b.loop_outer = 0;
-    MG_TRY(dev_alloc_n(&b.diag_list, (size_t)b.n_probs + b.h_heads.size()));
+    {
+        std::vector<MfNodeBlk> blks;
+        b.diag_at.assign(1, 0);
+        for (int r = 0; r < b.n_fine; r++) {
+            for (int q = r; q >= 0; q = b.h_probs[q].coarse)
+                for (int row = 0; row < b.h_probs[q].NY * b.h_probs[q].NZ; row += diag_rows(b.h_probs[q].pitch))
+                    blks.push_back(MfNodeBlk{q, row});
+            b.diag_at.push_back((int)blks.size());
+        }
+        MG_TRY(dev_alloc_n(&b.diag_blks, blks.size()));
+        MG_CUDA_TRY(cudaMemcpyAsync(b.diag_blks, blks.data(), blks.size() * sizeof(MfNodeBlk), cudaMemcpyHostToDevice,
+                                    b.stream));
+        MG_CUDA_TRY(cudaStreamSynchronize(b.stream));  // blks is a host temporary
+    }
+    MG_TRY(dev_alloc_n(&b.inv_list, std::max<size_t>(1, b.h_heads.size())));
     MG_TRY(dev_alloc_n(&b.sens_offs, (size_t)std::max(1, b.n_fine)));
     MG_CUDA_TRY(cudaMallocHost(&b.sens_offs_host, (size_t)std::max(1, b.n_fine) * sizeof(int64_t)));
-    MG_CUDA_TRY(cudaMallocHost(&b.stage_host, ((size_t)b.n_probs + b.h_heads.size()) * sizeof(int)));
+    MG_CUDA_TRY(cudaMallocHost(&b.stage_host, std::max<size_t>(1, b.h_heads.size()) * sizeof(int)));
     MG_CUDA_TRY(cudaEventCreateWithFlags(&b.stage_ev, cudaEventDisableTiming));
     MG_TRY(dev_alloc_n(&b.heads, std::max<size_t>(1, b.h_heads.size())));
     MG_TRY(dev_alloc_n(&b.K0, 576));
@@ -3680,7 +3700,7 @@ void mf_batch_free(MfBatch &b) {
     void *ptrs[] = {b.probs, b.bricks, b.chunks, b.states, b.tmaps, b.E32, b.Edf, b.dE64,
                     b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
-                    b.my, b.mr, b.diag_list, b.heads, b.cols, b.col_order, b.col_offs, b.col_part, b.Bop2, b.fac_tiles, b.fac_offs, b.fac_maps, b.node_blks,
+                    b.my, b.mr, b.diag_blks, b.inv_list, b.heads, b.cols, b.col_order, b.col_offs, b.col_part, b.Bop2, b.fac_tiles, b.fac_offs, b.fac_maps, b.node_blks,
                     b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chains, b.sens_offs};
     for (void *q : ptrs) dev_free(q);
     if (b.stage_host) cudaFreeHost(b.stage_host);

@@ -204,8 +204,10 @@ struct MfBatch {
     double *u64 = nullptr, *r64 = nullptr, *f64 = nullptr;
     double *brick_part = nullptr, *chunk_part = nullptr;
     int *err = nullptr;         // error flags of the bounded waits; loop bodies since a launch; in all
-    int *diag_list = nullptr;  // problem list of a partial Jacobi update, then its direct chains
-    int *stage_host = nullptr;  // pinned staging of diag_list
+    MfNodeBlk *diag_blks = nullptr;  // row blocks of the Jacobi inverse, each design's with its levels
+    std::vector<int> diag_at;        // where each design's begin
+    int *inv_list = nullptr;         // chains whose direct coarse solve is formed anew
+    int *stage_host = nullptr;       // pinned staging of inv_list
     int64_t *sens_offs = nullptr, *sens_offs_host = nullptr;  // dC/drho output offsets (device, pinned)
     cudaEvent_t stage_ev = nullptr;  // its last copy
     bool stage_pending = false;
