@@ -3452,11 +3452,16 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         for (MfProblem &T : b.h_probs) T.bottom = 0;
         for (int r = 0; r < b.n_fine; r++)
             for (int q = single && b.h_probs[r].coarse >= 0 ? r : b.h_probs[r].coarse; q >= 0; q = b.h_probs[q].coarse) {
-                int64_t depth = 0;
-                for (int t = q; t >= 0; t = b.h_probs[t].coarse) depth++;
                 const MfProblem &Hd = b.h_probs[q];
                 const int64_t head_nodes = (int64_t)Hd.NX * Hd.NY * Hd.NZ;
+                int64_t depth = 0, words = 6 * head_nodes;  // at most what cluster_layout gives one CTA
+                for (int t = q; t >= 0; t = b.h_probs[t].coarse, depth++) {
+                    const MfProblem &T = b.h_probs[t];
+                    words += 23LL * T.NX * T.NY * T.NZ + (int64_t)T.nx * T.ny * T.nz + kClusterThreads + 32;
+                }
                 if (depth > kBottomMaxLevels || head_nodes > (single ? kClusterMaxHeadNodes : kBatchMaxHeadNodes)) continue;
+                // a batched chain fits one CTA, in whatever batch (a long thin design's levels shrink slowly)
+                if (!single && 4 * words > kBottomSmemMax) continue;
                 b.h_heads.push_back(q);
                 b.h_head_root.push_back(r);
                 b.chains_from_root = q == r;

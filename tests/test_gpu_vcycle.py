@@ -51,6 +51,29 @@ def test_smoother_degrees_match_the_oracle(shape, degree):
         assert np.abs(di - dc_ref).max() / np.abs(dc_ref).max() < 1e-6
 
 
+def test_thin_batched_chains_on_few_ctas(monkeypatch):
+    """Chains of 1,024 nodes with one, two and sixteen CTAs: the same bits.  Beside them a design too
+    slender for FP32 (its solve breaks down), whose 1,024 nodes with all coarser levels do not fit one
+    CTA: its chain starts a level lower and the others keep theirs."""
+    shapes = [(63, 3, 3), (40, 4, 4), (255, 1, 1)]
+    o = M.default_opts(precision=M.MIXED_TF32X3, rtol=1e-8, inner_rtol=1e-2, timeout_s=300.0)
+    out = []
+    for cap in ("1", "2", "16"):
+        monkeypatch.setenv("MASTGPU_BOTTOM_CLUSTER", cap)
+        with M.Batch([dict(nx=s[0], ny=s[1], nz=s[2], rho=reference(s)[0] if s[2] > 1 else np.ones(255), spans=[(0, s[1])])
+                      for s in shapes]) as b:
+            _, reps = b.solve(o, raise_on_error=False)
+            out.append([b.results(d)[:2] for d in (0, 1)])
+        for s, rep, (c, dc) in zip(shapes, reps, out[-1]):
+            _, c_ref, dc_ref = reference(s)
+            assert rep.status == 0 and rep.relres <= 1e-8
+            assert abs(c[0] - c_ref) / c_ref < 1e-6
+            assert np.abs(dc[0] - dc_ref).max() / np.abs(dc_ref).max() < 1e-6
+    for o2 in out[1:]:
+        for (c, dc), (c0, dc0) in zip(o2, out[0]):
+            assert np.array_equal(c, c0) and np.array_equal(dc, dc0)
+
+
 def test_solve_longer_than_one_loop_launch():
     """Jacobi-preconditioned solves of some hundred iterations, two per loop body and 64 bodies a
     launch: the same iterations and the same bits as with 16 per body (one launch or two)."""
