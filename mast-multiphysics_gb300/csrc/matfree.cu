@@ -823,11 +823,13 @@ __global__ void __launch_bounds__(kColThreads, kColCtas) mf_col_kernel(
 // nodes: along x with a warp shuffle (left element + right element), along y
 // inside the thread (rows 2w, 2w+1) or through shared memory (row 2w+1 with the
 // next warp's row 2w+2).  Every node's sum has the same fixed order
-// (deterministic and independent of the tiling).  Issue-bound with 16 warps per
-// SM: 128 registers, no spills (D^-1 and the third plane are read behind the
-// plane's barrier: read before it they spilled, and MODE 6 took 144 us where it
-// takes 85).  MODE 2, 58 problems of 12.9 M dofs: 95 -> 84 us a launch; y = A x at
-// 128x64x64 13.9 -> 12.2 us, at 192x96x96 31.6 -> 27.3 us.
+// (deterministic and independent of the tiling).  Bound by issue (44 % of its slots at
+// 128x64x64) and by the start of a tile (tables and first planes, about 6,000 of 25,000
+// cycles there); 16 warps per SM at 128 registers, no spills (D^-1 and the third plane are
+// read behind the plane's barrier: read before it they spilled, and MODE 6 took 144 us
+// where it takes 85).  MODE 2, 58 problems of 12.9 M dofs: 95 -> 84 us a launch, 66 with the
+// tiles dealt by size (plan_fac_tiles); y = A x at 128x64x64 13.9 -> 12.2 us, at 192x96x96
+// 31.6 -> 27.3 us.
 constexpr int kFEX = 32, kFEY = 16;                // elements per tile plane
 constexpr int kFNX = kFEX - 1, kFNY = kFEY - 1;    // owned nodes per tile plane
 constexpr int kFPX = kFEX + 1, kFPY = kFEY + 1;    // tile node plane (with halo)

@@ -99,7 +99,7 @@ struct MfCol {
 
 constexpr int kNodeBlk = 64;  // nodes per block of the level transfers (256: 48x24x24 prolonged on 17 SMs)
 struct MfNodeBlk {
-    int prob, node;  // nodes [node, node + kNodeBlk) of the problem
+    int prob, node;  // nodes [node, node + kNodeBlk) of the problem (mf_diag_kernel: its rows from node on)
 };
 
 struct MfChunkDesc {
