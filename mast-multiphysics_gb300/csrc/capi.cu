@@ -305,6 +305,9 @@ int create_impl(const mg_mesh_desc *mesh, const mg_material_desc *mat, const mg_
         std::vector<int64_t> fill(p->color_ptr.begin(), p->color_ptr.end() - 1);
         for (int64_t e = 0; e < ne; e++) celems[fill[color[e]]++] = (int32_t)e;
     }
+    // a grid one element thick leaves structured colours without elements: no launch for those
+    p->color_ptr.erase(std::unique(p->color_ptr.begin(), p->color_ptr.end()), p->color_ptr.end());
+    p->n_colors = (int)p->color_ptr.size() - 1;
 
     // ---- sparsity pattern (node-interleaved, shared column list per node) ----
     std::vector<int64_t> aptr;
