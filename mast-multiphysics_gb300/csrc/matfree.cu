@@ -3440,9 +3440,12 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.n_elem_pad = el;
     b.n_nodes = nd;
     // bottom chains: for every design, the first level below the finest with at most
-    // kBatchMaxHeadNodes nodes, larger levels run level by level on the whole GPU; for a
-    // single design (bottom_cluster) the first with at most kClusterMaxHeadNodes, the
-    // finest included.  Chains whose tables no cluster size can hold run level by level.
+    // kBatchMaxHeadNodes nodes whose tables fit one CTA; for a single design (bottom_cluster)
+    // the first with at most kClusterMaxHeadNodes, the finest included, whose tables some
+    // cluster can hold.  The tables hold a halo of NX NY nodes on each side, so a flat
+    // design's wide levels do not fit: 80x64x4 starts at its third level (from the second
+    // 16 CTAs need 209 KB each, from the third 54).  Larger levels run level by level on the
+    // whole GPU; without any chain a solve of 80x64x4 took 74.4 ms, so 38.1 (34x34x3: 25.1, 11.4).
     int64_t inv_floats = 0;
     {
         const bool single = bottom_cluster && b.n_fine == 1;
@@ -3452,6 +3455,43 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         b.bottom_cluster = 0;
         b.chains_from_root = false;
         for (MfProblem &T : b.h_probs) T.bottom = 0;
+        // The chains of b.h_heads on the largest clusters (16 CTAs: non-portable size) that the
+        // device can place for all of them at once, one CTA a chain where there are more chains
+        // than that; false: none that holds the tables.  MASTGPU_BOTTOM_CLUSTER caps the cluster
+        // (1, 2, 4, 8 or 16 CTAs): a test knob, the correction does not depend on the cluster size
+        int cap = kClusterMax;
+        if (const char *env = std::getenv("MASTGPU_BOTTOM_CLUSTER")) cap = std::max(1, std::min(kClusterMax, std::atoi(env)));
+        int first = 1;
+        while (first * 2 <= cap) first *= 2;
+        auto place = [&] {
+            for (int cs = first; cs >= 1; cs /= 2) {
+                if (cs > 1 && (int64_t)b.h_heads.size() * cs > sms) continue;
+                std::vector<ClusterChain> chains;
+                const int64_t smem = cluster_layout(b, cs, chains);
+                if (smem < 0 || smem > kBottomSmemMax) continue;
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3((unsigned)(cs * b.h_heads.size()));
+                cfg.blockDim = dim3(kClusterThreads);
+                cfg.dynamicSmemBytes = smem;
+                cudaLaunchAttribute attr[1];
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = (unsigned)cs;
+                attr[0].val.clusterDim.y = 1;
+                attr[0].val.clusterDim.z = 1;
+                cfg.attrs = attr;
+                cfg.numAttrs = 1;
+                int n = 0;
+                if (cudaOccupancyMaxActiveClusters(&n, mg_bottom_cluster_kernel, &cfg) == cudaSuccess &&
+                    n >= (cs > 1 ? (int)b.h_heads.size() : 1)) {
+                    b.bottom_cluster = cs;
+                    b.bottom_smem = (int)smem;
+                    b.h_cl_chains.swap(chains);
+                    return true;
+                }
+                cudaGetLastError();  // clear the failed query
+            }
+            return false;
+        };
         for (int r = 0; r < b.n_fine; r++)
             for (int q = single && b.h_probs[r].coarse >= 0 ? r : b.h_probs[r].coarse; q >= 0; q = b.h_probs[q].coarse) {
                 const MfProblem &Hd = b.h_probs[q];
@@ -3466,43 +3506,15 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
                 if (!single && 4 * words > kBottomSmemMax) continue;
                 b.h_heads.push_back(q);
                 b.h_head_root.push_back(r);
+                if (single && !place()) {
+                    b.h_heads.clear();
+                    b.h_head_root.clear();
+                    continue;
+                }
                 b.chains_from_root = q == r;
                 break;
             }
-        // the largest clusters (16 CTAs: non-portable size) that the device can place for all
-        // chains at once, one CTA a chain where there are more chains than that.
-        // MASTGPU_BOTTOM_CLUSTER caps the cluster (1, 2, 4, 8 or 16 CTAs): a test knob,
-        // the correction does not depend on the cluster size
-        int cap = kClusterMax;
-        if (const char *env = std::getenv("MASTGPU_BOTTOM_CLUSTER")) cap = std::max(1, std::min(kClusterMax, std::atoi(env)));
-        int first = 1;
-        while (first * 2 <= cap) first *= 2;
-        for (int cs = first; cs >= 1 && !b.bottom_cluster && !b.h_heads.empty(); cs /= 2) {
-            if (cs > 1 && (int64_t)b.h_heads.size() * cs > sms) continue;
-            std::vector<ClusterChain> chains;
-            const int64_t smem = cluster_layout(b, cs, chains);
-            if (smem < 0 || smem > kBottomSmemMax) continue;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(cs * b.h_heads.size()));
-            cfg.blockDim = dim3(kClusterThreads);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = (unsigned)cs;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, mg_bottom_cluster_kernel, &cfg) == cudaSuccess &&
-                n >= (cs > 1 ? (int)b.h_heads.size() : 1)) {
-                b.bottom_cluster = cs;
-                b.bottom_smem = (int)smem;
-                b.h_cl_chains.swap(chains);
-            } else {
-                cudaGetLastError();  // clear the failed query
-            }
-        }
+        if (!single && !b.h_heads.empty()) place();
         if (!b.bottom_cluster) {
             b.h_heads.clear();
             b.h_head_root.clear();
