@@ -136,9 +136,11 @@ typedef struct mg_solve_opts {
     int32_t consistent_jacobian; /* heat: include the dk/dT term */
     int32_t max_refinements; /* mixed: FP64 refinement cap */
     double inner_rtol;       /* mixed: FP32 inner CG tolerance per refinement */
-    double timeout_s;        /* host wall-clock limit for the solve (0 = none) */
+    double timeout_s;        /* wall-clock limit for the solve (0 = none): MG_ETIMEDOUT once it is
+                                past.  Mixed form: looked at after every graph_chunk steps */
     int32_t warm_start;      /* 1: start from the resident solution */
-    int32_t graph_chunk;     /* Krylov iterations per captured CUDA graph (0 = default) */
+    int32_t graph_chunk;     /* Krylov iterations per captured CUDA graph (0 = default: 2 with
+                                multigrid, 16 without) */
     int32_t preconditioner;  /* mixed form: MG_PC_MULTIGRID (default) or MG_PC_JACOBI;
                                 the plain form is Jacobi-preconditioned */
     int32_t smooth_degree;   /* multigrid: Chebyshev degree of the smoothers (0 = 2) */

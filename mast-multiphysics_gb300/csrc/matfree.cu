@@ -2334,18 +2334,37 @@ __global__ void __launch_bounds__(kThreads) mf_refine_kernel(
     });
 }
 
+// Whether a solve's time is up, by the device's own clock: its budget runs from the first look, which is
+// behind the first kernels of its first loop body.  Called by one thread of the loop's deciding kernels,
+// so that a loop of 64 bodies overruns its limit by one body and not by the rest of a launch.  c: *clock,
+// loaded with the kernel's other words (one after another, the loads cost 0.3 us a body: 16x8x8 0.4 %).
+__device__ __forceinline__ bool time_is_up(MfLoopClock *clock, const MfLoopClock &c) {
+    if (c.budget_ns <= 0) return false;
+    int64_t now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    if (c.start_ns == 0) clock->start_ns = now;
+    return now - (c.start_ns ? c.start_ns : now) >= c.budget_ns;
+}
+
 // after the refinement update: a stopped inner CG sends its problem back to the
 // FP64 residual, or ends it on a breakdown / NaN (one block).  LOOP: the last kernel of a
-// while-loop body; the loop goes on while a problem is unfinished, no wait has timed out
-// and fewer than `limit` bodies have run since the launch (loop[0]).  loop[1] counts all
+// while-loop body; the loop goes on while a problem is unfinished, no wait has timed out, the
+// solve has time left and fewer than `limit` bodies have run since the launch (loop[0]).  loop[1] counts all
 // bodies, of nested loops those inside (mf_gate_kernel) and loop[2] those around them.
 constexpr int kPhaseThreads = 256;
 template <bool LOOP>
 __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states, int n_fine,
                                                                  cudaGraphConditionalHandle handle, int *loop,
-                                                                 int limit, bool nested, const int *err) {
+                                                                 int limit, bool nested, const int *err,
+                                                                 MfLoopClock *clock) {
     pdl_enter();
-    int active = 0;
+    int active = 0, bodies = 0, failed = 0;
+    MfLoopClock c{0, 0};
+    if (LOOP && threadIdx.x == 0) {
+        bodies = loop[0] + 1;
+        failed = *err;
+        c = *clock;
+    }
     for (int i = threadIdx.x; i < n_fine; i += kPhaseThreads) {
         MfState *st = states + i;
         if (st->phase == kPhaseCG && st->done) {
@@ -2366,8 +2385,7 @@ __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states
     if (LOOP) {
         active = __syncthreads_or(active);
         if (threadIdx.x == 0) {
-            const int bodies = loop[0] + 1;
-            const bool more = active && bodies < limit && *err == 0;
+            const bool more = active && bodies < limit && failed == 0 && !time_is_up(clock, c);
             loop[0] = more ? bodies : 0;
             loop[nested ? 2 : 1] += 1;
             cudaGraphSetConditional(handle, more ? 1u : 0u);
@@ -2378,13 +2396,17 @@ __global__ void __launch_bounds__(kPhaseThreads) mf_phase_kernel(MfState *states
 // The CG loop of a single problem inside its refinement loop goes on while its inner CG does
 // (count: the last kernel of a body; else before the loop).
 __global__ void mf_gate_kernel(const MfState *states, cudaGraphConditionalHandle handle, int *loop, int limit,
-                               bool count, const int *err) {
+                               bool count, const int *err, MfLoopClock *clock) {
     pdl_enter();
+    const MfLoopClock c = *clock;
+    const int bodies = loop[0] + (count ? 1 : 0), all = loop[1] + 1, failed = *err;
+    const bool active = states[0].phase == kPhaseCG && !states[0].done;
     if (count) {
-        loop[0] += 1;
-        loop[1] += 1;
+        loop[0] = bodies;
+        loop[1] = all;
     }
-    const bool more = states[0].phase == kPhaseCG && !states[0].done && loop[0] < limit && *err == 0;
+    const bool up = time_is_up(clock, c);
+    const bool more = active && bodies < limit && failed == 0 && !up;
     cudaGraphSetConditional(handle, more ? 1u : 0u);
 }
 
@@ -3574,7 +3596,9 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.fac_offs, b.h_fac_offs.size()));
     MG_TRY(dev_alloc_n(&b.Bop2, 4096));
     MG_TRY(dev_alloc_n(&b.chunks, b.h_chunks.size()));
-    MG_TRY(dev_alloc_n(&b.states, (size_t)b.n_probs));
+    static_assert(sizeof(MfLoopClock) <= sizeof(MfState) && alignof(MfLoopClock) <= alignof(MfState), "clock slot");
+    MG_TRY(dev_alloc_n(&b.states, (size_t)b.n_probs + 1));
+    b.clock = reinterpret_cast<MfLoopClock *>(b.states + b.n_probs);
     MG_TRY(dev_alloc_n(&b.tmaps, (size_t)b.n_probs * kMapsPerProblem));
     MG_TRY(dev_alloc_n(&b.fac_maps, (size_t)b.n_probs * kFacMaps));
     MG_CUDA_TRY(cudaMallocHost(reinterpret_cast<void **>(&b.states_host), b.n_probs * sizeof(MfState)));
@@ -3698,7 +3722,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     if (!b.h_heads.empty())
         MG_CUDA_TRY(cudaMemcpyAsync(b.heads, b.h_heads.data(), b.h_heads.size() * sizeof(int),
                                     cudaMemcpyHostToDevice, s));
-    MG_CUDA_TRY(cudaMemsetAsync(b.states, 0, b.n_probs * sizeof(MfState), s));
+    MG_CUDA_TRY(cudaMemsetAsync(b.states, 0, (b.n_probs + 1) * sizeof(MfState), s));
     MG_CUDA_TRY(cudaMemsetAsync(b.err, 0, kErrWords * sizeof(int), s));
     MG_CUDA_TRY(cudaMemsetAsync(b.u64, 0, dof * 8, s));
     MG_CUDA_TRY(cudaMemsetAsync(b.r64, 0, dof * 8, s));
@@ -3984,7 +4008,7 @@ long long enqueue_vcycle(MfBatch &b, bool fac, int prec, int sdeg, int cdeg) {
 //   FP64 residual + stop test (RESID) | inner CG start (INIT) |
 //   [multigrid z = M r, rz, beta] | p, q = A p, alpha | x, r, stop test |
 //   u += d of stopped inner solves | phase transitions.
-constexpr int kLoopBodies = 64;  // bodies of one loop launch at most: the host looks at the clock between launches
+constexpr int kLoopBodies = 64;  // bodies of one loop launch at most
 
 // the residual and the start of the inner CG
 long long enqueue_refine_begin(MfBatch &b, const MfSolveParams &prm) {
@@ -4036,10 +4060,10 @@ long long enqueue_refine_end(MfBatch &b, const cudaGraphConditionalHandle *loop_
         launch_pdl(mf_refine_kernel, vg0, kThreads, 0, b.stream, b.chunks, b.probs, b.n_fine, b.x, b.u64, b.states);
     if (loop_end)
         launch_pdl(mf_phase_kernel<true>, 1, kPhaseThreads, 0, b.stream, b.states, b.n_fine, *loop_end, b.err + 1,
-                   kLoopBodies, nested, b.err);
+                   kLoopBodies, nested, b.err, b.clock);
     else
         launch_pdl(mf_phase_kernel<false>, 1, kPhaseThreads, 0, b.stream, b.states, b.n_fine,
-                   cudaGraphConditionalHandle{}, nullptr, 0, false, nullptr);
+                   cudaGraphConditionalHandle{}, nullptr, 0, false, nullptr, nullptr);
     return 2;
 }
 
@@ -4116,7 +4140,8 @@ int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop)
         if (e == cudaSuccess)
             e = capture_into(b.stream, body, {}, [&] {
                 n_outer += enqueue_refine_begin(b, prm);
-                launch_pdl(mf_gate_kernel, 1, 1, 0, b.stream, b.states, inner_handle, b.err + 1, kLoopBodies, false, b.err);
+                launch_pdl(mf_gate_kernel, 1, 1, 0, b.stream, b.states, inner_handle, b.err + 1, kLoopBodies, false, b.err,
+                           b.clock);
                 n_outer += 1;
             }, &last);
         for (size_t k = 0; k < last.size() && e == cudaSuccess; k++)
@@ -4124,7 +4149,8 @@ int build_step_graph(MfBatch &b, const MfSolveParams &prm, int chunk, bool loop)
         if (e == cudaSuccess)
             e = capture_into(b.stream, inner, {}, [&] {
                 for (int it = 0; it < chunk; it++) n += enqueue_cg(b, prm, it & 1);
-                launch_pdl(mf_gate_kernel, 1, 1, 0, b.stream, b.states, inner_handle, b.err + 1, kLoopBodies, true, b.err);
+                launch_pdl(mf_gate_kernel, 1, 1, 0, b.stream, b.states, inner_handle, b.err + 1, kLoopBodies, true, b.err,
+                           b.clock);
                 n += 1;
             });
         if (e == cudaSuccess)
@@ -4188,15 +4214,18 @@ int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm, bool loop) {
     return build_step_graph(b, p2, chunk, loop);
 }
 
-int mf_batch_reset_states(MfBatch &b) {
-    std::vector<MfState> init(b.n_probs);
+int mf_batch_reset_states(MfBatch &b, double budget_s) {
+    std::vector<MfState> init(b.n_probs + 1);  // and the loop's clock behind the states
     memset(init.data(), 0, init.size() * sizeof(MfState));
     for (int i = 0; i < b.n_probs; i++) {
         init[i].done = 1;
         init[i].ref_done = 1;
         init[i].phase = kPhaseFin;
     }
-    MG_CUDA_TRY(cudaMemcpyAsync(b.states, init.data(), b.n_probs * sizeof(MfState), cudaMemcpyHostToDevice,
+    MfLoopClock clock{0, 0};
+    if (budget_s > 0) clock.budget_ns = (int64_t)std::max(1.0, std::min(budget_s * 1e9, 9e18));
+    memcpy(&init[b.n_probs], &clock, sizeof(clock));
+    MG_CUDA_TRY(cudaMemcpyAsync(b.states, init.data(), init.size() * sizeof(MfState), cudaMemcpyHostToDevice,
                                 b.stream));
     MG_CUDA_TRY(cudaStreamSynchronize(b.stream));  // init is a host temporary
     memcpy(b.states_host, init.data(), b.n_probs * sizeof(MfState));
@@ -4259,7 +4288,8 @@ int mf_batch_finish(MfBatch &b, int i) {
 int mf_batch_solve(MfBatch &b, const MfSolveParams &prm, bool warm_start) {
     const double t0 = wall_time();
     MG_TRY(mf_batch_prepare(b, prm, true));
-    MG_TRY(mf_batch_reset_states(b));
+    // the time left, or none: the loop ends within a body of it
+    MG_TRY(mf_batch_reset_states(b, prm.timeout_s > 0 ? std::max(1e-9, prm.timeout_s - (wall_time() - t0)) : 0.0));
     std::vector<int> act;
     for (int i = 0; i < b.n_fine; i++)
         if (!prm.active || prm.active[i]) act.push_back(i);

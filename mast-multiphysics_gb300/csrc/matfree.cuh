@@ -131,6 +131,12 @@ struct MfState {
     unsigned cnt_apply, cnt_update, cnt_res, pad;
 };
 
+// time limit of a solve that loops on the device (behind the states)
+struct MfLoopClock {
+    int64_t budget_ns;  // 0: no limit
+    int64_t start_ns;   // device clock at the loop's first look; 0 before it
+};
+
 constexpr int kErrWords = 4;  // error flag; bodies of this launch, of all loops, of all outer loops
 
 struct MfBatch {
@@ -163,6 +169,7 @@ struct MfBatch {
     FacK2 fac2{};                 // fac32 as (k, k) pairs for the packed FP32x2 kernels
     MfChunkDesc *chunks = nullptr;
     MfState *states = nullptr;
+    MfLoopClock *clock = nullptr;    // in states' buffer
     MfState *states_host = nullptr;  // pinned
     int *err_host = nullptr;         // pinned copy of err
     int loop_bodies = 0, loop_outer = 0;  // loop bodies run up to the last copy
@@ -259,12 +266,12 @@ int mf_batch_set_moduli(MfBatch &b, int i, const double *E_dev, const double *dE
 int mf_batch_solve(MfBatch &b, const MfSolveParams &prm, bool warm_start);
 // stepping interface (mf_batch_solve and the request loop are built on it):
 // prepare captures the step graph for prm (loop: as a device-side while loop that runs
-// until every problem has finished); reset puts every problem at FIN; activate starts
-// the listed level-0 problems at the FP64 residual (their Jacobi inverses are refreshed;
-// u is zeroed unless warm_start); finish returns a FIN problem's status and zeroes u of a
-// zero-load problem.
+// until every problem has finished or the time is up); reset puts every problem at FIN and
+// sets a loop's time (0: no limit); activate starts the listed level-0 problems at the
+// FP64 residual (their Jacobi inverses are refreshed; u is zeroed unless warm_start);
+// finish returns a FIN problem's status and zeroes u of a zero-load problem.
 int mf_batch_prepare(MfBatch &b, const MfSolveParams &prm, bool loop = false);
-int mf_batch_reset_states(MfBatch &b);
+int mf_batch_reset_states(MfBatch &b, double budget_s = 0.0);
 int mf_batch_activate(MfBatch &b, const std::vector<int> &level0, bool warm_start);
 // one graph launch, in two halves so that several batches can run on the GPU at once:
 // begin launches the graph and the copy of the states, end waits for them (states_host)

@@ -1,0 +1,45 @@
+"""timeout_s: a solve that runs into its limit returns MG_ETIMEDOUT within one graph of solver steps
+(mixed form) or a few iterations (plain form) after it, and the handle solves again afterwards."""
+import time
+
+import numpy as np
+import pytest
+
+import mastgpu as M
+
+pytestmark = pytest.mark.gpu
+
+TRIES = 3  # the least of three: the host may be busy
+
+
+def overrun(solve, limit):
+    times = []
+    for _ in range(TRIES):
+        t0 = time.perf_counter()
+        rc = solve()
+        times.append(time.perf_counter() - t0)
+        assert rc == M.MG_ETIMEDOUT, rc
+    return min(times) - limit
+
+
+@pytest.mark.parametrize("n", [1, 2])  # one design: its CG loops inside its refinement; several: one loop
+def test_mixed_solve_returns_after_its_limit(n):
+    nx, ny, nz = 128, 64, 64
+    rng = np.random.default_rng(41)
+    des = [dict(nx=nx, ny=ny, nz=nz, rho=rng.uniform(0.01, 1.0, nx * ny * nz), spans=[(0, ny)]) for _ in range(n)]
+    # an inner tolerance that FP32 does not reach in the time: one inner solve of thousands of
+    # Jacobi iterations, 16 a graph, about 50 us each
+    o = M.default_opts(precision=M.MIXED_TF32X3, rtol=1e-8, inner_rtol=1e-14, timeout_s=0.002)
+    o.preconditioner = M.PC_JACOBI
+    good = M.default_opts(precision=M.MIXED_TF32X3, rtol=1e-8, inner_rtol=1e-3)
+    with M.Batch(des) as b:
+        b.solve(good)
+        before = b.results(0)
+        b.solve(o, raise_on_error=False)  # captures its graph
+        late = overrun(lambda: b.solve(o, raise_on_error=False)[0], 0.002)
+        b.solve(good)
+        after = b.results(0)
+    # one launch of 64 graphs takes more than 50 ms
+    assert late < 0.02, late
+    assert np.array_equal(before[0], after[0]) and np.array_equal(before[1], after[1])
+
