@@ -137,10 +137,13 @@ typedef struct mg_solve_opts {
     int32_t max_refinements; /* mixed: FP64 refinement cap */
     double inner_rtol;       /* mixed: FP32 inner CG tolerance per refinement */
     double timeout_s;        /* wall-clock limit for the solve (0 = none): MG_ETIMEDOUT once it is
-                                past.  Mixed form: looked at after every graph_chunk steps */
+                                past.  Looked at after every graph_chunk steps (mixed form) or
+                                iterations; a plain solve that one kernel runs looks every 256
+                                iterations while more time than these take is left */
     int32_t warm_start;      /* 1: start from the resident solution */
     int32_t graph_chunk;     /* Krylov iterations per captured CUDA graph (0 = default: 2 with
-                                multigrid, 16 without) */
+                                multigrid, 16 without); a plain solve that one kernel runs has no
+                                graph and uses it for the time limit only */
     int32_t preconditioner;  /* mixed form: MG_PC_MULTIGRID (default) or MG_PC_JACOBI;
                                 the plain form is Jacobi-preconditioned */
     int32_t smooth_degree;   /* multigrid: Chebyshev degree of the smoothers (0 = 2) */

@@ -28,9 +28,14 @@ constexpr int kBS = 256;
 // lanes per node in the SpMV: few lanes keep the FP64 work near one FMA per
 // stored value (GB300's FP64 rate is the binding limit next to HBM)
 constexpr int kSpmvLanes = 4;
-// iterations per launch of the one-kernel form: the host looks at the wall-clock limit
-// between launches (a few ms), a launch and its state copy cost about 20 us
-constexpr int kResidentIters = 256;
+// Iterations per launch of the one-kernel form: the host looks at the wall-clock limit between
+// launches, and a launch with its state copy costs about 20 us.  A launch that could outlast
+// the time left is shorter, down to one graph of the launch-per-phase form.
+constexpr int kResidentIters = 256, kGraphIters = 16;
+
+// microseconds an iteration, before one has been measured (a CG iteration takes 11 at 0.9 M
+// values, 94 at 32 M; BiCGStab has two products)
+double resident_iter_us(int64_t nnz, bool cg) { return (cg ? 1.0 : 2.0) * (20.0 + 4e-6 * (double)nnz); }
 
 template <int NV>
 __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double *partials, int stride) {
@@ -577,9 +582,13 @@ int krylov_solve(mg_problem *p, const CsrMatrix &A, const double *d_b, double *d
     // one cooperative kernel per kResidentIters iterations where the vectors fit the SMs'
     // shared memory (up to about 216,000 HEX8 nodes; faster there at every size measured,
     // krylov_resident.cu)
+    const int fewest = std::min(kResidentIters, o.graph_chunk > 0 ? o.graph_chunk : kGraphIters);
+    double iter_s = 1e-6 * resident_iter_us(A.nnz, krylov == MG_KRYLOV_CG);
     for (;;) {
-        int launched = 0;
-        MG_TRY(krylov_resident_launch(p, A, d_x, krylov == MG_KRYLOV_CG, kResidentIters, &launched));
+        int launched = 0, its = kResidentIters;
+        const double t1 = wall_time();
+        if (o.timeout_s > 0) its = (int)std::max((double)fewest, std::min((double)its, (o.timeout_s - (t1 - t0)) / iter_s));
+        MG_TRY(krylov_resident_launch(p, A, d_x, krylov == MG_KRYLOV_CG, its, &launched));
         if (!launched) break;
         int err = 0;
         MG_CUDA_TRY(cudaMemcpyAsync(&err, w.slot_err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -595,13 +604,15 @@ int krylov_solve(mg_problem *p, const CsrMatrix &A, const double *d_b, double *d
             if (relres) *relres = (h.bb > 0 ? sqrt(h.rr / h.bb) : sqrt(h.rr));
             return h.status;
         }
-        if (o.timeout_s > 0 && wall_time() - t0 > o.timeout_s) {
+        const double t2 = wall_time();
+        if (o.timeout_s > 0 && t2 - t0 > o.timeout_s) {
             set_error("Krylov solve exceeded %.1f s", o.timeout_s);
             return MG_ETIMEDOUT;
         }
+        iter_s = (t2 - t1) / its;
     }
     // CG: p0 = 0 and beta = 0, so the first p update forms p = z
-    const int chunk = o.graph_chunk > 0 ? o.graph_chunk : 16;
+    const int chunk = o.graph_chunk > 0 ? o.graph_chunk : kGraphIters;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     MG_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));

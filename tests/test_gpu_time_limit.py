@@ -43,3 +43,20 @@ def test_mixed_solve_returns_after_its_limit(n):
     assert late < 0.02, late
     assert np.array_equal(before[0], after[0]) and np.array_equal(before[1], after[1])
 
+
+def test_plain_solve_returns_after_its_limit():
+    nx, ny, nz = 80, 40, 40
+    rho = np.random.default_rng(42).uniform(0.2, 1.0, nx * ny * nz)
+    o = M.default_opts(precision=M.PLAIN_FP64, rtol=1e-14, timeout_s=0.002)
+    capped = M.default_opts(precision=M.PLAIN_FP64, rtol=1e-14)
+    capped.max_iterations = 100
+    with M.simp_cantilever(nx, ny, nz) as p:
+        p.set_design(rho)
+        p.solve_resident(capped)
+        before = p.compliance()[0]
+        # about 94 us an iteration: 256 of them take 24 ms
+        late = overrun(lambda: p.solve_resident(o)[0], 0.002)
+        p.solve_resident(capped)
+        after = p.compliance()[0]
+    assert late < 0.01, late
+    assert before == after
