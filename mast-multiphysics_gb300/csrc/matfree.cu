@@ -3367,13 +3367,6 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.h_bricks.clear();
     b.h_chunks.clear();
     b.h_cols.clear();
-    std::vector<int64_t> level_count(b.n_levels + 1, 0);  // problems per multigrid level
-    for (const MfProblem &P : b.h_probs) level_count[P.level]++;
-    int64_t dofs0 = 0;  // of the designs' own grids, which the vector kernels run over
-    for (const MfProblem &P : b.h_probs)
-        if (P.level == 0) dofs0 += (int64_t)((3 * (P.nx + 1) + 3) / 4 * 4) * (P.ny + 1) * (P.nz + 1);
-    int chunk = kMinChunk;
-    while (chunk < kMaxChunk && dofs0 > (int64_t)chunk * kWaveBlocks) chunk *= 2;
     for (size_t pi = 0; pi < b.h_probs.size(); pi++) {
         MfProblem &P = b.h_probs[pi];
         if (P.nx <= 0 || P.ny <= 0 || P.nz <= 0 || P.nx >= kMaxSide || P.ny >= kMaxSide || P.nz >= kMaxSide) {
@@ -3417,17 +3410,21 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
                 for (int i = 0; i < bx; i++)
                     b.h_bricks.push_back(MfBrick{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
         nb += P.brick_count;
-        // columns of the tensor-core operator: as deep as one wave of resident
-        // columns allows (the level's problems share the CTA slots), up to kCZ
-        // node planes; a second, partial wave would double the launch's time.  A single
-        // small grid's columns are as short as the slots allow, one plane and two element
-        // layers at the least: 16x8x8 54.8 us an iteration with four planes at least, 52.4 with
-        // one; 48x24x24 108.3 and 106.1.  In a batch four at least: a small design's columns,
-        // and with them the order of its p.q, are the same whatever the batch holds
+        // Columns of the tensor-core operator: as deep as one wave of resident columns allows, up
+        // to kCZ node planes; a second, partial wave would double the launch's time.  A single
+        // small grid's columns are as short as the slots allow, one plane and two element layers
+        // at the least: 16x8x8 54.8 us an iteration with four planes at least, 52.4 with one;
+        // 48x24x24 108.3 and 106.1.  In a batch a design takes half the slots, eight planes at
+        // least and equal columns where they make one wave, whatever the batch holds: the columns
+        // decide the order of its p.q.  (The slots divided by the level's designs, four planes at
+        // least: 58 problems 44.0 ms a solve where these take 44.4, sixteen 32x16x16 7.7 and 7.5,
+        // one 48x24x24 3.33 and 3.47.  An eighth of the slots: 43.9, 7.5 and 3.57.)
         const int cx = (P.NX + kCX - 1) / kCX, cy = (P.NY + kCY - 1) / kCY;
         const int64_t slots = kColCtas * (int64_t)sms;
-        const int64_t col_per = std::max<int64_t>(1, slots / ((int64_t)cx * cy * level_count[P.level]));
-        P.col_z = (int)std::min<int64_t>(kCZ, std::max<int64_t>(bottom_cluster ? 1 : 4, (P.NZ + col_per - 1) / col_per));
+        const int64_t col_per = std::max<int64_t>(1, (bottom_cluster ? slots : slots / 2) / ((int64_t)cx * cy));
+        P.col_z = (int)std::min<int64_t>(kCZ, std::max<int64_t>(bottom_cluster ? 1 : 8, (P.NZ + col_per - 1) / col_per));
+        const int col_parts = (P.NZ + P.col_z - 1) / P.col_z;
+        if (!bottom_cluster && (int64_t)cx * cy * col_parts <= slots) P.col_z = (P.NZ + col_parts - 1) / col_parts;
         const int cz = (P.NZ + P.col_z - 1) / P.col_z;
         P.col_begin = (int)b.h_cols.size();
         P.col_count = cx * cy * cz;
@@ -3435,6 +3432,8 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
             for (int j = 0; j < cy; j++)
                 for (int i = 0; i < cx; i++)
                     b.h_cols.push_back(MfCol{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
+        int chunk = kMinChunk;
+        while (chunk < kMaxChunk && P.n_pad > (int64_t)chunk * (bottom_cluster ? 8 * sms : 8 * sms / 16)) chunk *= 2;
         P.chunk_begin = nc;
         P.chunk_count = (int)((P.n_pad + chunk - 1) / chunk);
         for (int c = 0; c < P.chunk_count; c++) {

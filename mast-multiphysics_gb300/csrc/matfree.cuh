@@ -15,11 +15,14 @@
 namespace mg {
 
 constexpr int kMaxSide = 8 * 32767;            // elements a side (tile numbers are 16 bits)
-// Dofs per vector-kernel chunk, one to four float4 per thread: the fewest that leave no more
-// chunks than one wave of blocks (8 on each of 152 SMs).  With 4096 throughout, the two
-// vector kernels of a 16x8x8 iteration ran on two blocks each; the rule and the shorter sums
-// took its solve and sensitivities from 3.02 to 2.81 ms, 64x32x32 from 7.52 to 7.03 ms.
-constexpr int kMinChunk = 1024, kMaxChunk = 4096, kWaveBlocks = 8 * 152;
+// Dofs per vector-kernel chunk, one to four float4 per thread: the fewest that leave a single design
+// no more chunks than one wave of blocks (8 per SM), a design of a batch a sixteenth of that, whatever
+// the batch holds: the chunks decide the order of its r.r and r.z.  With 4096 throughout, the two
+// vector kernels of a 16x8x8 iteration ran on two blocks each; the rule and the shorter sums took its
+// solve and sensitivities from 3.02 to 2.81 ms, 64x32x32 from 7.52 to 7.03 ms.  In batches, 4096 / a
+// sixteenth / an eighth / 2048: 58 problems 44.0 / 44.1 / 44.9 / 44.5 ms a solve, sixteen 16x8x8
+// 4.26 / 4.01 / 4.03 / 4.11.
+constexpr int kMinChunk = 1024, kMaxChunk = 4096;
 constexpr int kMapsPerProblem = 6;             // z, p0, p1, E, mg x, mg d (column operator boxes)
 // Column operator: a column owns kCX x kCY nodes in x, y and up to kCZ node
 // planes in z; it streams through its element planes (8 x 16 elements each,
