@@ -2666,22 +2666,31 @@ __global__ void __launch_bounds__(kRThreads, 3) mf_residual64_kernel(
 // 0 on Dirichlet dofs and padding (marks them for the vector kernels).  Blocks of some 2,048
 // words, whole grid rows (j, k), from a list of all problems; a thread per word.  (A grid of the
 // largest problem's blocks times the problems, 64-bit divisions and K0 converted from FP64 in
-// every thread: 58 designs with their levels 536 us, 131 us so.)
+// every thread: 58 designs with their levels 536 us, 131 us so.)  runs > 0: the blocks are those of the
+// runs [first, first + size) of the list: run_end[r] counts the blocks of the runs up to r, run_first
+// follows it (every other of 58 16x8x8 designs started and ended: 1,007 us with a launch a run, 721 so).
 __host__ __device__ constexpr int diag_rows(int pitch) { return pitch >= 2048 ? 1 : 2048 / pitch; }
 __global__ void __launch_bounds__(256) mf_diag_kernel(const MfProblem *__restrict__ probs,
-                                                      const MfNodeBlk *__restrict__ blks,
+                                                      const MfNodeBlk *__restrict__ blks, int runs,
+                                                      const int *__restrict__ run_end,
                                                       const float *__restrict__ E32, const uint8_t *__restrict__ node_fix,
                                                       const double *__restrict__ K0, float *__restrict__ dinv) {
     __shared__ float sk[24];  // the diagonal of K0
+    __shared__ int s_blk;
     if (threadIdx.x < 24) sk[threadIdx.x] = (float)K0[25 * threadIdx.x];
-    const MfNodeBlk B = blks[blockIdx.x];
+    if (runs == 0 && threadIdx.x == 0) s_blk = blockIdx.x;
+    for (int r = threadIdx.x; r < runs; r += 256) {
+        const int lo = r ? run_end[r - 1] : 0, at = (int)blockIdx.x - lo;
+        if (at >= 0 && (int)blockIdx.x < run_end[r]) s_blk = run_end[runs + r] + at;
+    }
+    __syncthreads();
+    const MfNodeBlk B = blks[s_blk];
     const MfProblem &P = probs[B.prob];
     const int NX = P.NX, NY = P.NY, nx = P.nx, ny = P.ny, nz = P.nz, pitch = P.pitch;
     const int row1 = min(B.node + diag_rows(pitch), NY * P.NZ);
     const float *E = E32 + P.elem_off;
     const uint8_t *fix = node_fix + P.node_off;
     float *out = dinv + P.dof_off;
-    __syncthreads();
     for (int i = threadIdx.x; i < (row1 - B.node) * pitch; i += 256) {
         const int row = B.node + i / pitch, xin = i % pitch;
         float v = 0.0f;
@@ -3049,10 +3058,9 @@ void launch_update(MfBatch &b, float *pnew, bool mg) {
         b.chunks, n0, b.probs, b.x, b.r, b.z, pnew, b.q, b.dinv, b.states, b.chunk_part, mg ? 1 : 0);
 }
 
-// Jacobi inverse of blocks [lo, hi) of the list
-int launch_diag(MfBatch &b, int lo, int hi) {
-    if (hi <= lo) return MG_OK;
-    mf_diag_kernel<<<hi - lo, 256, 0, b.stream>>>(b.probs, b.diag_blks + lo, b.E32, b.node_fix, b.K0, b.dinv);
+// Jacobi inverse of n blocks: of the list from `first` on, or of `runs` runs of it
+int launch_diag(MfBatch &b, int first, int n, int runs = 0, const int *run_end = nullptr) {
+    mf_diag_kernel<<<n, 256, 0, b.stream>>>(b.probs, b.diag_blks + first, runs, run_end, b.E32, b.node_fix, b.K0, b.dinv);
     MG_CUDA_TRY(cudaGetLastError());
     count_launches(1);
     return MG_OK;
@@ -3066,26 +3074,45 @@ int compute_diag(MfBatch &b) {
 // Jacobi inverse of the listed level-0 problems and all their coarse levels, and
 // the inverse of the coarsest grid of their direct chains; nothing waits on the host
 int compute_diag_list(MfBatch &b, const std::vector<int> &level0) {
-    std::vector<int> inv;
+    std::vector<int> list;  // the chains, then the runs of blocks (ends, firsts)
     if (level0.empty()) return MG_OK;
     for (size_t h = 0; h < b.h_heads.size(); h++)
         if (b.h_coarse_off[h] >= 0 && std::find(level0.begin(), level0.end(), b.h_head_root[h]) != level0.end())
-            inv.push_back((int)h);
-    // the blocks of a problem and its coarse levels are neighbours in the list
-    if ((int)level0.size() == b.n_fine) {
-        MG_TRY(launch_diag(b, 0, b.diag_at.back()));
-    } else {
-        for (int i : level0) MG_TRY(launch_diag(b, b.diag_at[i], b.diag_at[i + 1]));
+            list.push_back((int)h);
+    const int n_inv = (int)list.size();
+    // the blocks of a problem and its coarse levels are neighbours in the list, as are those of
+    // neighbouring problems
+    std::vector<int> probs(level0), first, end;
+    std::sort(probs.begin(), probs.end());
+    int n = 0;
+    for (size_t k = 0; k < probs.size(); k++) {
+        const int lo = b.diag_at[probs[k]], hi = b.diag_at[probs[k] + 1];
+        if (k && probs[k] == probs[k - 1]) continue;
+        n += hi - lo;
+        if (k && probs[k] == probs[k - 1] + 1) {
+            end.back() = n;
+        } else {
+            first.push_back(lo);
+            end.push_back(n);
+        }
     }
-    if (!inv.empty()) {
+    const int runs = first.size() > 1 ? (int)first.size() : 0;
+    if (runs) {
+        list.insert(list.end(), end.begin(), end.end());
+        list.insert(list.end(), first.begin(), first.end());
+    }
+    if (!list.empty()) {
         // the pinned staging buffer: the previous call's copy must have read it
         if (b.stage_pending) MG_CUDA_TRY(cudaEventSynchronize(b.stage_ev));
-        memcpy(b.stage_host, inv.data(), inv.size() * sizeof(int));
-        MG_CUDA_TRY(cudaMemcpyAsync(b.inv_list, b.stage_host, inv.size() * sizeof(int), cudaMemcpyHostToDevice, b.stream));
+        memcpy(b.stage_host, list.data(), list.size() * sizeof(int));
+        MG_CUDA_TRY(cudaMemcpyAsync(b.start_list, b.stage_host, list.size() * sizeof(int), cudaMemcpyHostToDevice, b.stream));
         MG_CUDA_TRY(cudaEventRecord(b.stage_ev, b.stream));
         b.stage_pending = true;
-        mg_coarse_inverse_kernel<<<(unsigned)inv.size(), kCoarseInvThreads, kCoarseInvSmem, b.stream>>>(
-            b.probs, b.heads, b.inv_list, b.E32, b.dinv, b.K0, b.coarse_off, b.coarse_inv,
+    }
+    MG_TRY(launch_diag(b, runs ? 0 : first[0], n, runs, b.start_list + n_inv));
+    if (n_inv) {
+        mg_coarse_inverse_kernel<<<(unsigned)n_inv, kCoarseInvThreads, kCoarseInvSmem, b.stream>>>(
+            b.probs, b.heads, b.start_list, b.E32, b.dinv, b.K0, b.coarse_off, b.coarse_inv,
             b.coarse_ok);
         MG_CUDA_TRY(cudaGetLastError());
         count_launches(1);
@@ -3630,10 +3657,11 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
                                     b.stream));
         MG_CUDA_TRY(cudaStreamSynchronize(b.stream));  // blks is a host temporary
     }
-    MG_TRY(dev_alloc_n(&b.inv_list, std::max<size_t>(1, b.h_heads.size())));
+    const size_t start_words = b.h_heads.size() + 2 * (size_t)b.n_fine;
+    MG_TRY(dev_alloc_n(&b.start_list, start_words));
     MG_TRY(dev_alloc_n(&b.sens_offs, (size_t)std::max(1, b.n_fine)));
     MG_CUDA_TRY(cudaMallocHost(&b.sens_offs_host, (size_t)std::max(1, b.n_fine) * sizeof(int64_t)));
-    MG_CUDA_TRY(cudaMallocHost(&b.stage_host, std::max<size_t>(1, b.h_heads.size()) * sizeof(int)));
+    MG_CUDA_TRY(cudaMallocHost(&b.stage_host, start_words * sizeof(int)));
     MG_CUDA_TRY(cudaEventCreateWithFlags(&b.stage_ev, cudaEventDisableTiming));
     MG_TRY(dev_alloc_n(&b.heads, std::max<size_t>(1, b.h_heads.size())));
     MG_TRY(dev_alloc_n(&b.K0, 576));
@@ -3742,7 +3770,7 @@ void mf_batch_free(MfBatch &b) {
     void *ptrs[] = {b.probs, b.bricks, b.chunks, b.states, b.tmaps, b.E32, b.Edf, b.dE64,
                     b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
-                    b.my, b.mr, b.diag_blks, b.inv_list, b.heads, b.cols, b.col_order, b.col_offs, b.col_part, b.Bop2, b.fac_tiles, b.fac_offs, b.fac_maps, b.node_blks,
+                    b.my, b.mr, b.diag_blks, b.start_list, b.heads, b.cols, b.col_order, b.col_offs, b.col_part, b.Bop2, b.fac_tiles, b.fac_offs, b.fac_maps, b.node_blks,
                     b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chains, b.sens_offs};
     for (void *q : ptrs) dev_free(q);
     if (b.stage_host) cudaFreeHost(b.stage_host);
@@ -4232,9 +4260,10 @@ int mf_batch_reset_states(MfBatch &b, double budget_s) {
 }
 
 int mf_batch_activate(MfBatch &b, const std::vector<int> &level0, bool warm_start) {
+    for (int i : level0)
+        if (i < 0 || i >= b.n_fine) return MG_EINVAL;
     MG_TRY(compute_diag_list(b, level0));
     for (int i : level0) {
-        if (i < 0 || i >= b.n_fine) return MG_EINVAL;
         const MfProblem &P = b.h_probs[i];
         if (!warm_start) MG_CUDA_TRY(cudaMemsetAsync(b.u64 + P.dof_off, 0, P.n_pad * 8, b.stream));
         // the pinned host mirror entry is the staging buffer; the next

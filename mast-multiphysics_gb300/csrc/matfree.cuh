@@ -216,8 +216,9 @@ struct MfBatch {
     int *err = nullptr;         // error flags of the bounded waits; loop bodies since a launch; in all
     MfNodeBlk *diag_blks = nullptr;  // row blocks of the Jacobi inverse, each design's with its levels
     std::vector<int> diag_at;        // where each design's begin
-    int *inv_list = nullptr;         // chains whose direct coarse solve is formed anew
-    int *stage_host = nullptr;       // pinned staging of inv_list
+    int *start_list = nullptr;       // of the problems that start: chains whose direct coarse solve is
+                                     // formed anew, runs of diag_blks
+    int *stage_host = nullptr;       // pinned staging of start_list
     int64_t *sens_offs = nullptr, *sens_offs_host = nullptr;  // dC/drho output offsets (device, pinned)
     cudaEvent_t stage_ev = nullptr;  // its last copy
     bool stage_pending = false;
