@@ -843,6 +843,7 @@ constexpr int kFModF = kFBoxE * kFEY;              // 576 floats
 constexpr int kFXch = 3 * kFThreads;               // row exchange: 3 floats per thread
 static_assert(kFBoxX * kFPY <= kFPlaneF && kFBoxX >= 3 + 3 * kFPX && kFBoxE >= 3 + kFEX, "boxes");
 static_assert(kFThreads == 32 * (kFEY / 2) && kFEX == 32, "warp = element row pair, lane = x");
+static_assert((kMaxSide + kFNX - 1) / kFNX <= 65536 && (kMaxSide + kFNY - 1) / kFNY <= 65536, "tile numbers");
 // tensor maps per problem for this kernel: node vectors with the 104 x 17 x 1 box
 // and the moduli with the 36 x 16 x 1 box
 enum FacMap { kFMapMx = 0, kFMapMd, kFMapMy, kFMapMb, kFMapR, kFMapDinv, kFMapMr, kFMapZ, kFMapE, kFacMaps };
@@ -2433,6 +2434,7 @@ constexpr int kRLoads = (kRPlane + kRThreads - 1) / kRThreads;
 constexpr int kRMaxZ = 12;
 constexpr int kResidSmem = (2 * kRPlane + 2 * kRPlane + 2 * 12 * kRThreads) * 8;  // planes, raw planes, exchange
 static_assert(kREX * kREY <= kRThreads, "one element and one node per thread");
+static_assert((kMaxSide + kROwnX - 1) / kROwnX <= 32768 && (kMaxSide + kROwnY - 1) / kROwnY <= 32768, "tile numbers");
 
 // block sum of kRThreads threads; valid in thread 0
 __device__ __forceinline__ double resid_sum(double v, double *sh) {
@@ -3285,7 +3287,7 @@ void plan_fac_tiles(MfBatch &b, int ctas) {
                 for (int k = 0; k * z < P.NZ; k++)
                     for (int j = 0; j < ty; j++)
                         for (int i = 0; i < tx; i++) {
-                            tiles.push_back(MfCol{pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
+                            tiles.push_back(MfCol{pi, (uint16_t)i, (uint16_t)j, (uint16_t)k, 0});
                             cost.push_back(std::min(z, P.NZ - k * z) + 3);
                         }
             }
@@ -3458,7 +3460,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         for (int k = 0; k < cz; k++)
             for (int j = 0; j < cy; j++)
                 for (int i = 0; i < cx; i++)
-                    b.h_cols.push_back(MfCol{(int)pi, (int16_t)i, (int16_t)j, (int16_t)k, 0});
+                    b.h_cols.push_back(MfCol{(int)pi, (uint16_t)i, (uint16_t)j, (uint16_t)k, 0});
         int chunk = kMinChunk;
         while (chunk < kMaxChunk && P.n_pad > (int64_t)chunk * (bottom_cluster ? 8 * sms : 8 * sms / 16)) chunk *= 2;
         P.chunk_begin = nc;

@@ -14,7 +14,7 @@
 
 namespace mg {
 
-constexpr int kMaxSide = 8 * 32767;            // elements a side (tile numbers are 16 bits)
+constexpr int kMaxSide = 8 * 32767;            // elements a side, at most
 // Dofs per vector-kernel chunk, one to four float4 per thread: the fewest that leave a single design
 // no more chunks than one wave of blocks (8 per SM), a design of a batch a sixteenth of that, whatever
 // the batch holds: the chunks decide the order of its r.r and r.z.  With 4096 throughout, the two
@@ -97,8 +97,9 @@ struct MfBrick {
 
 struct MfCol {
     int prob;
-    int16_t cx, cy, cz, pad;
+    uint16_t cx, cy, cz, pad;  // unsigned: the longest side has 37,449 columns
 };
+static_assert((kMaxSide + kCX - 1) / kCX <= 65536 && (kMaxSide + kCY - 1) / kCY <= 65536, "column numbers");
 
 constexpr int kNodeBlk = 64;  // nodes per block of the level transfers (256: 48x24x24 prolonged on 17 SMs)
 struct MfNodeBlk {
