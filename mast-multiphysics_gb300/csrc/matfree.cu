@@ -3443,14 +3443,15 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
         // to kCZ node planes; a second, partial wave would double the launch's time.  A single
         // small grid's columns are as short as the slots allow, one plane and two element layers
         // at the least: 16x8x8 54.8 us an iteration with four planes at least, 52.4 with one;
-        // 48x24x24 108.3 and 106.1.  In a batch a design takes half the slots, eight planes at
-        // least and equal columns where they make one wave, whatever the batch holds: the columns
-        // decide the order of its p.q.  (The slots divided by the level's designs, four planes at
-        // least: 58 problems 44.0 ms a solve where these take 44.4, sixteen 32x16x16 7.7 and 7.5,
-        // one 48x24x24 3.33 and 3.47.  An eighth of the slots: 43.9, 7.5 and 3.57.)
+        // 48x24x24 108.3 and 106.1.  In a batch a design takes a quarter of the slots, eight planes
+        // at least and equal columns where they make one wave, whatever the batch holds: the columns
+        // decide the order of its p.q.  ms a solve (the slots divided by the level's designs / half /
+        // a quarter / a sixth of them): 58 problems 44.2 / 44.6 / 44.3 / 44.2, sixteen 32x16x16
+        // 7.75 / 7.56 / 7.56 / 7.55, one 48x24x24 3.36 / 3.51 / 3.50 / 3.57, one 64x32x32 5.62 /
+        // 5.79 / 6.06 / 6.07.
         const int cx = (P.NX + kCX - 1) / kCX, cy = (P.NY + kCY - 1) / kCY;
         const int64_t slots = kColCtas * (int64_t)sms;
-        const int64_t col_per = std::max<int64_t>(1, (bottom_cluster ? slots : slots / 2) / ((int64_t)cx * cy));
+        const int64_t col_per = std::max<int64_t>(1, (bottom_cluster ? slots : slots / 4) / ((int64_t)cx * cy));
         P.col_z = (int)std::min<int64_t>(kCZ, std::max<int64_t>(bottom_cluster ? 1 : 8, (P.NZ + col_per - 1) / col_per));
         const int col_parts = (P.NZ + P.col_z - 1) / P.col_z;
         if (!bottom_cluster && (int64_t)cx * cy * col_parts <= slots) P.col_z = (P.NZ + col_parts - 1) / col_parts;
