@@ -66,7 +66,7 @@ int refresh_moduli(mg_batch *b, int d) {
 }
 
 int64_t batch_bytes(const MfBatch &m) {
-    const int64_t f32_vecs = 13, f64_vecs = 3;
+    const int64_t f32_vecs = 12, f64_vecs = 3;
     return m.n_pad * (4 * f32_vecs + 8 * f64_vecs) + m.n_elem_pad * 20 + m.n_nodes +
            (int64_t)m.n_probs * (sizeof(MfProblem) + sizeof(MfState) + kMapsPerProblem * 128) +
            (int64_t)m.n_bricks * (sizeof(MfBrick) + 16) + (int64_t)m.n_chunks * (sizeof(MfChunkDesc) + 16);

@@ -1713,7 +1713,10 @@ constexpr int kClusterThreads = 512;
 // Nodes of the largest level that a chain may start at, the design's own grid included: up to here
 // the cluster's phases on 16 SMs beat the level kernels on all of them (us an iteration of single
 // designs, chain from the own grid / level by level: 1,377 nodes 57.5 / 72.1, 3,509 78.5 / 80.6,
-// 4,225 76.3 / 80.3, 4,913 77.6 / 83.0; 5,577 85.3 / 84.8).
+// 4,225 76.3 / 80.3, 4,913 77.6 / 83.0; 5,577 85.3 / 84.8).  The line also ends the search below the
+// own grid, where the chain does not take r.z over and the two lie closer (chain from the level of these
+// nodes / from the one below it: 1,377 112.6 / 122.1, 2,420 89.8 / 95.9, 3,312 98.9 / 98.5, 3,432
+// 144.8 / 145.3, 3,549 99.9 / 99.0, 4,225 103.5 / 99.7).
 constexpr int kClusterMaxHeadNodes = 5000;
 constexpr int kClusterMax = 16;
 constexpr int kClusterK0 = 576;  // K0 regrouped by the lanes' corners (floats)
@@ -1730,12 +1733,6 @@ __device__ __forceinline__ unsigned cluster_nctarank() {
 }
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// generic address of p (this CTA's shared memory) in CTA `rank` of the cluster
-__device__ __forceinline__ const float *cl_map(const float *p, int rank) {
-    uint64_t r;
-    asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
-    return reinterpret_cast<const float *>(r);
 }
 // n / d for the level's small divisors by one rounded product (exact for every n
 // of the level: the host checks each reciprocal against integer division)
@@ -2814,8 +2811,6 @@ __global__ void fill_f32_kernel(float *__restrict__ a, const float *__restrict__
 
 inline unsigned blocks_for(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
-// K0 in the UMMA K-major no-swizzle layout (B operand, N = 32 rows, zero padded):
-// [tf32 hi 768 | tf32 lo 768 | bf16 hi 512 | bf16 lo 512] 32-bit words
 // B tiles of the column operator: tile t = dy + 2 dz holds the K0 columns of the
 // corners (0, dy, dz) and (1, dy, dz) (K chunk dx: x, y, z, 0 in TF32; x, y, z
 // and five zeros in BF16) for the 32 N rows n = 3 a + c (libMesh corner a; rows
@@ -2935,9 +2930,6 @@ void launch_apply_prec(MfBatch &b, int prec, const ApplyArgs &a) {
     }
 }
 
-// level operator of the multigrid (MODE 2: y = rhs - A x, MODE 3: y = A x) on
-// level l: the factored CUDA-core operator (fac) or the tensor-core column
-// operator in precision prec (x is the vector of map in_slot there)
 // the factored kernel's tensor map of a batch vector
 int fac_map_of(const MfBatch &b, const float *v) {
     if (v == b.mx) return kFMapMx;
@@ -2961,7 +2953,9 @@ void launch_fac(MfBatch &b, int l, int sel, const FacArgs &a) {
                b.fac_offs + b.lvl_fac_off[l], sel, b.fac2, b.fac_maps, b.states, a, b.err);
 }
 
-// y = A x (MODE 3) or rhs - A x (MODE 2; z, nullable: D^-1 y, the factored operator only)
+// level operator of the multigrid, y = A x (MODE 3) or rhs - A x (MODE 2; z, nullable: D^-1 y,
+// the factored operator only), on level l: the factored CUDA-core operator (fac) or the
+// tensor-core column operator in precision prec (x is the vector of map in_slot there)
 template <int MODE>
 void launch_level_op(MfBatch &b, bool fac, int prec, int l, int in_slot, const float *x, const float *rhs,
                      float *y, int sel, float *z = nullptr) {
@@ -2975,7 +2969,7 @@ void launch_level_op(MfBatch &b, bool fac, int prec, int l, int in_slot, const f
     }
 }
 
-// CG step on the level-0 bricks (z from map in_slot)
+// CG step on the level-0 columns (z from map in_slot)
 void launch_cg_apply(MfBatch &b, int prec, int in_slot, int parity) {
     ApplyArgs a{0, in_slot, parity, nullptr, b.q};
     launch_apply_prec<1>(b, prec, a);
@@ -2986,7 +2980,7 @@ int set_apply_attrs() {
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_col_kernel<PREC, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_col_kernel<PREC, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_col_kernel<PREC, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem));
-    // all of the unified L1/shared storage as shared memory: three CTAs per SM
+    // all of the unified L1/shared storage as shared memory: two CTAs per SM
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_col_kernel<PREC, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_col_kernel<PREC, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     MG_CUDA_TRY(cudaFuncSetAttribute(mf_col_kernel<PREC, 3>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
@@ -3479,10 +3473,9 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     b.n_bricks = nb;
     b.n_chunks = nc;
     b.n_cols = (int)b.h_cols.size();
-    b.lvl_brick_lo.clear(); b.lvl_brick_hi.clear(); b.lvl_chunk_lo.clear(); b.lvl_chunk_hi.clear();
+    b.lvl_brick_hi.clear(); b.lvl_chunk_lo.clear(); b.lvl_chunk_hi.clear();
     for (int l = 0; l < b.n_levels; l++) {
         const MfProblem &A = b.h_probs[b.lvl_prob_lo[l]], &Z = b.h_probs[b.lvl_prob_hi[l] - 1];
-        b.lvl_brick_lo.push_back(A.brick_begin);
         b.lvl_brick_hi.push_back(Z.brick_begin + Z.brick_count);
         b.lvl_chunk_lo.push_back(A.chunk_begin);
         b.lvl_chunk_hi.push_back(Z.chunk_begin + Z.chunk_count);
@@ -3635,7 +3628,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_TRY(dev_alloc_n(&b.Edf, (size_t)el + 4));
     MG_TRY(dev_alloc_n(&b.dE64, (size_t)el + 4));
     MG_TRY(dev_alloc_n(&b.node_fix, (size_t)nd));
-    float **f32s[] = {&b.x, &b.r, &b.z, &b.p0, &b.p1, &b.q, &b.dinv, &b.xdbg,
+    float **f32s[] = {&b.x, &b.r, &b.z, &b.p0, &b.p1, &b.q, &b.dinv,
                       &b.mb, &b.mx, &b.md, &b.my, &b.mr};
     for (float **v : f32s) MG_TRY(dev_alloc_n(v, (size_t)dof));
     MG_TRY(dev_alloc_n(&b.u64, (size_t)dof));
@@ -3761,7 +3754,7 @@ int mf_batch_init(MfBatch &b, const std::vector<MfProblem> &shapes, double hx, d
     MG_CUDA_TRY(cudaMemsetAsync(b.E32, 0, (el + 4) * 4, s));
     MG_CUDA_TRY(cudaMemsetAsync(b.Edf, 0, (el + 4) * sizeof(dfloat), s));
     MG_CUDA_TRY(cudaMemsetAsync(b.dE64, 0, (el + 4) * 8, s));
-    float *zero_vecs[] = {b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.mb, b.mx, b.md, b.my, b.mr};
+    float *zero_vecs[] = {b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.mb, b.mx, b.md, b.my, b.mr};
     for (float *v : zero_vecs) MG_CUDA_TRY(cudaMemsetAsync(v, 0, dof * 4, s));
     MG_CUDA_TRY(cudaStreamSynchronize(s));
     return MG_OK;
@@ -3771,7 +3764,7 @@ void mf_batch_free(MfBatch &b) {
     if (b.stream) cudaStreamSynchronize(b.stream);
     if (b.graph) cudaGraphExecDestroy(b.graph);
     void *ptrs[] = {b.probs, b.bricks, b.chunks, b.states, b.tmaps, b.E32, b.Edf, b.dE64,
-                    b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.xdbg, b.u64, b.r64,
+                    b.node_fix, b.x, b.r, b.z, b.p0, b.p1, b.q, b.dinv, b.u64, b.r64,
                     b.f64, b.brick_part, b.chunk_part, b.err, b.K0, b.mb, b.mx, b.md,
                     b.my, b.mr, b.diag_blks, b.start_list, b.heads, b.cols, b.col_order, b.col_offs, b.col_part, b.Bop2, b.fac_tiles, b.fac_offs, b.fac_maps, b.node_blks,
                     b.coarse_off, b.coarse_inv, b.coarse_ok, b.cl_k0, b.cl_chains, b.sens_offs};

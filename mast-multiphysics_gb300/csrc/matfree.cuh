@@ -185,13 +185,13 @@ struct MfBatch {
     uint8_t *node_fix = nullptr;
     // FP32 inner CG vectors (padded layout)
     float *x = nullptr, *r = nullptr, *z = nullptr, *p0 = nullptr, *p1 = nullptr, *q = nullptr,
-          *dinv = nullptr, *xdbg = nullptr;
+          *dinv = nullptr;
     // multigrid vectors (padded layout, every level): rhs, solution, Chebyshev
     // direction, operator output, residual
     float *mb = nullptr, *mx = nullptr, *md = nullptr, *my = nullptr, *mr = nullptr;
     int n_fine = 0;             // level-0 problems (the designs); problems are ordered by level
     int n_levels = 1;
-    std::vector<int> lvl_prob_lo, lvl_prob_hi, lvl_brick_lo, lvl_brick_hi, lvl_chunk_lo, lvl_chunk_hi;
+    std::vector<int> lvl_prob_lo, lvl_prob_hi, lvl_brick_hi, lvl_chunk_lo, lvl_chunk_hi;
     double cheb_lmax = 0.0;     // Gershgorin bound of D^-1 A (same on every level)
     // bottom V-cycle: the head (first bottom level) of every chain that has one
     std::vector<int> h_heads;

@@ -93,8 +93,8 @@ int64_t chain_bytes(int nx, int ny, int nz, int cases) {
         if (!mg_coarsens(x, y, z)) break;
         x = (x + 1) / 2; y = (y + 1) / 2; z = (z + 1) / 2;
     }
-    // 13 FP32 + 3 FP64 vectors per dof, 3 element tables per design, dc + densities
-    return cases * (dofs * (13 * 4 + 3 * 8) + nodes + 8LL * nx * ny * nz) + elems * 20 +
+    // 12 FP32 + 3 FP64 vectors per dof, 3 element tables per design, dc + densities
+    return cases * (dofs * (12 * 4 + 3 * 8) + nodes + 8LL * nx * ny * nz) + elems * 20 +
            3 * 8LL * nx * ny * nz;
 }
 
